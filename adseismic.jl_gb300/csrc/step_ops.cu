@@ -2,7 +2,7 @@
 // library: AcousticOneStep forward/backward, ScatterAddOps, GatherOps,
 // AddSource and GetReceive.
 //
-// This translation unit is compiled with --fmad=false and keeps the
+// This translation unit is compiled with --fmad=false and the forward keeps the
 // reference's expression order, so the FP64 acoustic forward reproduces
 // AcousticOneStepCpuForward (deps/CustomOps/AcousticOneStepCpu/
 // AcousticOneStepCpu.h:1-48) bit for bit.  Threads map x -> j (the contiguous
@@ -22,13 +22,129 @@ namespace {
 
 constexpr int BJ = 32, BI = 8;
 
+// The scalar factors of one step, each formed on the host by the operations, in
+// the order, that the reference writes them, so they carry its rounding bit for
+// bit.  Forming them in the kernels cost each cell about ten divisions, and an
+// FP64 division is some twenty instructions on a pipe that issues a warp's
+// instruction in 64 cycles: 1001 x 1001 FP64, variant W, one GB300: forward
+// 322 us, gradient 793 us with the factors formed per cell.
 template <typename T>
-__global__ void k_acoustic_fwd_w(const T* __restrict__ w, const T* __restrict__ wold,
-                                 const T* __restrict__ phi, const T* __restrict__ psi,
-                                 const T* __restrict__ sigma, const T* __restrict__ tau,
-                                 const T* __restrict__ c, T dt, T hx, T hy, int NX, int NY,
-                                 T* __restrict__ u, T* __restrict__ phiout,
-                                 T* __restrict__ psiout) {
+struct StepK {
+  T dt, dt2, hx, hy, hx2, hy2;  // hx2 = 2 hx, hy2 = 2 hy
+  T k1, k2;  // 2 dt^2 / hx^2, 2 dt^2 / hy^2
+  T ax, ay;  // dt / hx, dt / hy
+  T cx, cy;  // their squares
+  T fx, fy;  // dt^2 / (2 hx), dt^2 / (2 hy)
+  int plain;  // dt, hx, hy in the range where the undamped short forms hold
+};
+
+template <typename T>
+StepK<T> make_k(double dt_, double hx_, double hy_) {
+  const T dt = T(dt_), hx = T(hx_), hy = T(hy_), two = 2;
+  StepK<T> K;
+  K.dt = dt;
+  K.dt2 = dt * dt;
+  K.hx = hx;
+  K.hy = hy;
+  K.hx2 = two * hx;
+  K.hy2 = two * hy;
+  K.k1 = two * dt * dt / hx / hx;
+  K.k2 = two * dt * dt / hy / hy;
+  K.ax = dt / hx;
+  K.ay = dt / hy;
+  K.cx = K.ax * K.ax;
+  K.cy = K.ay * K.ay;
+  K.fx = K.dt2 / K.hx2;
+  K.fy = K.dt2 / K.hy2;
+  auto ok = [](T x) { return x >= T(1e-15) && x <= T(1e15); };
+  K.plain = ok(dt) && ok(hx) && ok(hy);
+  return K;
+}
+
+// |x| < 2^1023 (2^127): finite, and so is the difference of two of them.  Integer
+// tests: they cost nothing on the FP64 pipe.
+__device__ __forceinline__ bool tame(double x) {
+  return (__double2hiint(x) & 0x7ff00000) < 0x7fe00000;
+}
+__device__ __forceinline__ bool tame(float x) {
+  return (__float_as_int(x) & 0x7f800000) < 0x7f000000;
+}
+// |x| < 2^512 (2^64): its product with a step factor stays finite
+__device__ __forceinline__ bool small(double x) {
+  return (__double2hiint(x) & 0x7ff00000) < 0x5ff00000;
+}
+__device__ __forceinline__ bool small(float x) {
+  return (__float_as_int(x) & 0x7f800000) < 0x5f800000;
+}
+__device__ __forceinline__ bool neg_zero(double x) {
+  return __double2hiint(x) == (int)0x80000000 && __double2loint(x) == 0;
+}
+__device__ __forceinline__ bool neg_zero(float x) {
+  return __float_as_int(x) == (int)0x80000000;
+}
+// x == 0 (either sign) as an integer test
+__device__ __forceinline__ bool is_zero(double x) {
+  return ((__double2hiint(x) << 1) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool is_zero(float x) { return x == 0.f; }
+__device__ __forceinline__ bool zero_bits(double x) {
+  return (__double2hiint(x) | __double2loint(x)) == 0;
+}
+__device__ __forceinline__ bool zero_bits(float x) { return __float_as_int(x) == 0; }
+
+// A cell without damping (sigma = tau = 0): the factors 1 - (sigma + tau) dt/2,
+// 1 + (sigma + tau) dt/2, 1 - dt sigma, 1 - dt tau are exactly 1 and sigma tau
+// dt^2 and dt c (tau - sigma) exactly 0, so their products drop out and the
+// division is by 1; what is left is the same value bit for bit.
+template <typename T>
+__device__ __forceinline__ bool undamped(const StepK<T>& K, T sg, T ta, T c) {
+  return K.plain && is_zero(sg) && is_zero(ta) && small(c);
+}
+
+// phi' = (1 - 0) phi + 0 (difference): phi itself where the difference is
+// finite (0 times it is a zero) and phi is not -0 (which a +0 would turn).
+template <typename T>
+__device__ __forceinline__ bool kept(T phi, T a, T b) {
+  return tame(a) && tame(b) && !neg_zero(phi);
+}
+
+// The field update of one interior cell, in the reference's order (variant W
+// AcousticOneStepCpu.h:18-46; U src/Core.jl:528-549).  Undamped cells take 22
+// FP64 operations of 34 and no division.
+template <typename T, int VARIANT>
+__device__ __forceinline__ T new_u(const StepK<T>& K, int64_t k, int64_t S, T sg, T ta, T ck,
+                                   bool plain, const T* __restrict__ w,
+                                   const T* __restrict__ wold, const T* __restrict__ phi,
+                                   const T* __restrict__ psi) {
+  const T two = 2, one = 1;
+  const T wn = w[k + S], ws = w[k - S], we = w[k + 1], ww = w[k - 1];
+  T a = two;
+  if (!plain) {
+    if (VARIANT == 0) a = two - sg * ta * K.dt * K.dt;
+    else a = two - sg * ta * K.dt2;
+  }
+  T v;
+  if (VARIANT == 0)
+    v = (a - K.k1 * ck - K.k2 * ck) * w[k] + ck * K.ax * K.ax * (wn + ws) +
+        ck * K.ay * K.ay * (we + ww);
+  else
+    v = (a - K.k1 * ck - K.k2 * ck) * w[k] + ck * K.cx * (wn + ws) + ck * K.cy * (we + ww);
+  v = v + K.fx * (phi[k + S] - phi[k - S]) + K.fy * (psi[k + 1] - psi[k - 1]);
+  if (plain) return v - wold[k];
+  v = v - (one - (sg + ta) * K.dt / two) * wold[k];
+  return v / (one + (sg + ta) / two * K.dt);
+}
+
+// One thread per cell.  FP64 issue bounds it (82% of the pipe's active cycles):
+// 22 operations an undamped cell.  75 us at 1001 x 1001 FP64, 322 us with the
+// factors and the division formed in every cell.
+template <typename T>
+__global__ void __launch_bounds__(BJ* BI)
+k_acoustic_fwd_w(const T* __restrict__ w, const T* __restrict__ wold,
+                 const T* __restrict__ phi, const T* __restrict__ psi,
+                 const T* __restrict__ sigma, const T* __restrict__ tau,
+                 const T* __restrict__ c, StepK<T> K, int NX, int NY, T* __restrict__ u,
+                 T* __restrict__ phiout, T* __restrict__ psiout) {
   const int j = blockIdx.x * BJ + threadIdx.x;
   const int i = blockIdx.y * BI + threadIdx.y;
   if (i > NX + 1 || j > NY + 1) return;
@@ -36,169 +152,199 @@ __global__ void k_acoustic_fwd_w(const T* __restrict__ w, const T* __restrict__ 
   const int64_t k = (int64_t)i * S + j;
   if (i == 0 || i == NX + 1 || j == 0 || j == NY + 1) {
     u[k] = 0;
-    phiout[k] = 0;
-    psiout[k] = 0;
-    return;
-  }
-  const T sg = sigma[k], ta = tau[k], ck = c[k];
-  const T two = 2, one = 1, half = 2;
-  T v = (two - sg * ta * dt * dt - two * dt * dt / hx / hx * ck -
-         two * dt * dt / hy / hy * ck) * w[k] +
-        ck * (dt / hx) * (dt / hx) * (w[k + S] + w[k - S]) +
-        ck * (dt / hy) * (dt / hy) * (w[k + 1] + w[k - 1]) +
-        (dt * dt / (T(2.0) * hx)) * (phi[k + S] - phi[k - S]) +
-        (dt * dt / (T(2.0) * hy)) * (psi[k + 1] - psi[k - 1]) -
-        (one - (sg + ta) * dt / half) * wold[k];
-  u[k] = v / (one + (sg + ta) / half * dt);
-  phiout[k] = (one - dt * sg) * phi[k] + dt * ck * (ta - sg) / T(2.0) / hx * (w[k + S] - w[k - S]);
-  psiout[k] = (one - dt * ta) * psi[k] + dt * ck * (sg - ta) / T(2.0) / hy * (w[k + 1] - w[k - 1]);
-}
-
-// Variant U (src/Core.jl:528-549): u over the grid first ...
-template <typename T>
-__global__ void k_acoustic_fwd_u1(const T* __restrict__ w, const T* __restrict__ wold,
-                                  const T* __restrict__ phi, const T* __restrict__ psi,
-                                  const T* __restrict__ sigma, const T* __restrict__ tau,
-                                  const T* __restrict__ c, T dt, T hx, T hy, int NX, int NY,
-                                  T* __restrict__ u) {
-  const int j = blockIdx.x * BJ + threadIdx.x;
-  const int i = blockIdx.y * BI + threadIdx.y;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t S = NY + 2;
-  const int64_t k = (int64_t)i * S + j;
-  if (i == 0 || i == NX + 1 || j == 0 || j == NY + 1) {
-    u[k] = 0;
-    return;
-  }
-  const T sg = sigma[k], ta = tau[k], ck = c[k];
-  const T dt2 = dt * dt, one = 1;
-  const T kx = T(2) * dt2 / (hx * hx), ky = T(2) * dt2 / (hy * hy);
-  const T cx = (dt / hx) * (dt / hx), cy = (dt / hy) * (dt / hy);
-  const T fx = dt2 / (T(2) * hx), fy = dt2 / (T(2) * hy);
-  T v = (T(2) - sg * ta * dt2 - kx * ck - ky * ck) * w[k] + ck * cx * (w[k + S] + w[k - S]) +
-        ck * cy * (w[k + 1] + w[k - 1]) + fx * (phi[k + S] - phi[k - S]) +
-        fy * (psi[k + 1] - psi[k - 1]) - (one - (sg + ta) * dt / T(2)) * wold[k];
-  u[k] = v / (one + (sg + ta) / T(2) * dt);
-}
-
-// ... then phi/psi from the new u.
-template <typename T>
-__global__ void k_acoustic_fwd_u2(const T* __restrict__ u, const T* __restrict__ phi,
-                                  const T* __restrict__ psi, const T* __restrict__ sigma,
-                                  const T* __restrict__ tau, const T* __restrict__ c, T dt,
-                                  T hx, T hy, int NX, int NY, T* __restrict__ phiout,
-                                  T* __restrict__ psiout) {
-  const int j = blockIdx.x * BJ + threadIdx.x;
-  const int i = blockIdx.y * BI + threadIdx.y;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t S = NY + 2;
-  const int64_t k = (int64_t)i * S + j;
-  if (i == 0 || i == NX + 1 || j == 0 || j == NY + 1) {
     phiout[k] = 0;
     psiout[k] = 0;
     return;
   }
   const T sg = sigma[k], ta = tau[k], ck = c[k], one = 1;
-  phiout[k] = (one - dt * sg) * phi[k] + dt * ck * (ta - sg) / (T(2) * hx) * (u[k + S] - u[k - S]);
-  psiout[k] = (one - dt * ta) * psi[k] + dt * ck * (sg - ta) / (T(2) * hy) * (u[k + 1] - u[k - 1]);
+  const bool plain = undamped<T>(K, sg, ta, ck);
+  u[k] = new_u<T, 0>(K, k, S, sg, ta, ck, plain, w, wold, phi, psi);
+  const T pk = phi[k], qk = psi[k];
+  const T wn = w[k + S], ws = w[k - S], we = w[k + 1], ww = w[k - 1];
+  if (plain && kept(pk, wn, ws) && kept(qk, we, ww)) {
+    phiout[k] = pk;
+    psiout[k] = qk;
+  } else {
+    phiout[k] = (one - K.dt * sg) * pk + K.dt * ck * (ta - sg) / T(2.0) / K.hx * (wn - ws);
+    psiout[k] = (one - K.dt * ta) * qk + K.dt * ck * (sg - ta) / T(2.0) / K.hy * (we - ww);
+  }
 }
 
-// Gradient of the new u for variant U: the output gradient plus what phi'/psi'
-// send back through their u differences (interior cells only: u's frame is a
-// constant zero).
+// Variant U: u over a tile and the ring of cells around it, then phi / psi of
+// the tile from the new u: one launch and one read of the fields where two
+// kernels passed u through memory.  Tiles of BI = 8 rows: the ring's second
+// computation is a third of the tile's, but 16- and 32-row tiles leave the last
+// wave emptier (1001 x 1001 FP64: 87.8 us with 8 rows, 88.3 with 16, 98.0 with 32;
+// 1001 x 641: 66.6, 70.6, 79.7).
 template <typename T>
-__device__ __forceinline__ T gu_total(int i, int j, int NX, int NY, int64_t S,
-                                      const T* __restrict__ gu, const T* __restrict__ gp,
-                                      const T* __restrict__ gq, const T* __restrict__ sigma,
-                                      const T* __restrict__ tau, const T* __restrict__ c,
-                                      T dt, T hx, T hy) {
-  if (i < 1 || i > NX || j < 1 || j > NY) return T(0);
+__global__ void __launch_bounds__(BJ* BI)
+k_acoustic_fwd_u(const T* __restrict__ w, const T* __restrict__ wold,
+                 const T* __restrict__ phi, const T* __restrict__ psi,
+                 const T* __restrict__ sigma, const T* __restrict__ tau,
+                 const T* __restrict__ c, StepK<T> K, int NX, int NY, T* __restrict__ u,
+                 T* __restrict__ phiout, T* __restrict__ psiout) {
+  constexpr int W = BJ + 2, H = BI + 2, RING = 2 * W + 2 * BI;
+  __shared__ T su[H][W];
+  const int j0 = blockIdx.x * BJ, i0 = blockIdx.y * BI;
+  const int r = threadIdx.y, q = threadIdx.x, i = i0 + r, j = j0 + q;
+  const int64_t S = NY + 2;
+  const T one = 1;
+  auto cell = [&](int a, int b) -> T {  // u of cell (a, b)
+    if (a < 1 || a > NX || b < 1 || b > NY) return T(0);
+    const int64_t k = (int64_t)a * S + b;
+    const T sg = sigma[k], ta = tau[k], ck = c[k];
+    return new_u<T, 1>(K, k, S, sg, ta, ck, undamped<T>(K, sg, ta, ck), w, wold, phi, psi);
+  };
+  const T v = cell(i, j);
+  su[r + 1][q + 1] = v;
+  const int e = r * BJ + q;
+  if (e < RING) {  // the ring: top and bottom rows, then the two columns
+    const int f = e - 2 * W;
+    const int a = e < W ? -1 : e < 2 * W ? BI : f >> 1;
+    const int b = e < W ? e - 1 : e < 2 * W ? e - W - 1 : (f & 1) ? BJ : -1;
+    su[a + 1][b + 1] = cell(i0 + a, j0 + b);
+  }
+  __syncthreads();
+  if (i > NX + 1 || j > NY + 1) return;
   const int64_t k = (int64_t)i * S + j;
-  T g = gu[k];
-  // y = x - e_i : x is y's i+1 neighbour
-  if (i - 1 >= 1) {
-    const int64_t y = k - S;
-    g += dt * c[y] * (tau[y] - sigma[y]) / (T(2) * hx) * gp[y];
+  u[k] = v;
+  if (i == 0 || i == NX + 1 || j == 0 || j == NY + 1) {
+    phiout[k] = 0;
+    psiout[k] = 0;
+    return;
   }
-  if (i + 1 <= NX) {
-    const int64_t y = k + S;
-    g -= dt * c[y] * (tau[y] - sigma[y]) / (T(2) * hx) * gp[y];
+  const T sg = sigma[k], ta = tau[k], ck = c[k], pk = phi[k], qk = psi[k];
+  const T un = su[r + 2][q + 1], us = su[r][q + 1], ue = su[r + 1][q + 2], uw = su[r + 1][q];
+  if (undamped<T>(K, sg, ta, ck) && kept(pk, un, us) && kept(qk, ue, uw)) {
+    phiout[k] = pk;
+    psiout[k] = qk;
+  } else {
+    phiout[k] = (one - K.dt * sg) * pk + K.dt * ck * (ta - sg) / K.hx2 * (un - us);
+    psiout[k] = (one - K.dt * ta) * qk + K.dt * ck * (sg - ta) / K.hy2 * (ue - uw);
   }
-  if (j - 1 >= 1) {
-    const int64_t y = k - 1;
-    g += dt * c[y] * (sigma[y] - tau[y]) / (T(2) * hy) * gq[y];
-  }
-  if (j + 1 <= NY) {
-    const int64_t y = k + 1;
-    g -= dt * c[y] * (sigma[y] - tau[y]) / (T(2) * hy) * gq[y];
-  }
-  return g;
 }
+
+__device__ __forceinline__ double fm(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
 
 // Gather-form transpose of one step (both variants).  Each output cell sums
 // the contributions the reference's scatter loop (AcousticOneStepCpu.h:76-124)
 // sends it; frame cells receive them too.
+//
+// What a cell y sends is formed once, in shared memory, over a tile and the
+// ring around it: g / den (den = 1 where undamped: no division), c g / den, and
+// in damped cells the phi / psi terms PX = dt c (tau - sigma) / (2 hx) gphi and
+// PY likewise.  Variant U first adds what phi' / psi' send back through their u
+// differences to g, so PX and PY reach one ring further.  An undamped cell takes
+// 17 FP64 operations.  Forming each neighbour's terms again, with its division,
+// took 793 us at 1001 x 1001 FP64 for variant W; this takes 84 us (92 with
+// 16-row tiles, 109 with 32-row ones, whose last wave is nearly empty).
 template <typename T, int VARIANT>
-__global__ void k_acoustic_bwd(T* __restrict__ grad_w, T* __restrict__ grad_wold,
-                               T* __restrict__ grad_phi, T* __restrict__ grad_psi,
-                               T* __restrict__ grad_c, const T* __restrict__ grad_u,
-                               const T* __restrict__ grad_phiout,
-                               const T* __restrict__ grad_psiout, const T* __restrict__ w,
-                               const T* __restrict__ sigma, const T* __restrict__ tau,
-                               const T* __restrict__ c, T dt, T hx, T hy, int NX, int NY,
-                               const T* __restrict__ u) {
-  const int j = blockIdx.x * BJ + threadIdx.x;
-  const int i = blockIdx.y * BI + threadIdx.y;
-  if (i > NX + 1 || j > NY + 1) return;
+__global__ void __launch_bounds__(BJ* BI)
+k_acoustic_bwd(T* __restrict__ grad_w, T* __restrict__ grad_wold, T* __restrict__ grad_phi,
+               T* __restrict__ grad_psi, T* __restrict__ grad_c,
+               const T* __restrict__ grad_u, const T* __restrict__ grad_phiout,
+               const T* __restrict__ grad_psiout, const T* __restrict__ w,
+               const T* __restrict__ sigma, const T* __restrict__ tau,
+               const T* __restrict__ c, StepK<T> K, T kxy, int NX, int NY,
+               const T* __restrict__ u) {
+  constexpr int HP = VARIANT == 0 ? 1 : 2;  // ring of PX, PY
+  constexpr int WP = BJ + 2 * HP, HPR = BI + 2 * HP, W = BJ + 2, H = BI + 2;
+  __shared__ T sx[HPR][WP], sy[HPR][WP], sg_[H][W], sc[H][W];
+  const int j0 = blockIdx.x * BJ, i0 = blockIdx.y * BI;
   const int64_t S = NY + 2;
-  const int64_t k = (int64_t)i * S + j;
   const T one = 1, two = 2;
-  auto interior = [&](int a, int b) { return a >= 1 && a <= NX && b >= 1 && b <= NY; };
-  auto G = [&](int a, int b) -> T {
-    if (VARIANT == 0) return grad_u[(int64_t)a * S + b];
-    return gu_total<T>(a, b, NX, NY, S, grad_u, grad_phiout, grad_psiout, sigma, tau, c,
-                       dt, hx, hy);
-  };
-  auto den = [&](int64_t y) { return one + (sigma[y] + tau[y]) / two * dt; };
-  T gw = 0, gwo = 0, gph = 0, gps = 0, gc = 0;
-  if (interior(i, j)) {
-    const T sg = sigma[k], ta = tau[k], ck = c[k], g = G(i, j), d = den(k);
-    gc = ((-two * dt * dt / hx / hx - two * dt * dt / hy / hy) * w[k] +
-          (dt / hx) * (dt / hx) * (w[k + S] + w[k - S]) +
-          (dt / hy) * (dt / hy) * (w[k + 1] + w[k - 1])) * g / d;
-    gw = (two - sg * ta * dt * dt - two * dt * dt / hx / hx * ck -
-          two * dt * dt / hy / hy * ck) * g / d;
-    gwo = -(one - (sg + ta) * dt / two) * g / d;
-    const T gp = grad_phiout[k], gs = grad_psiout[k];
-    gph = (one - dt * sg) * gp;
-    gps = (one - dt * ta) * gs;
-    if (VARIANT == 0) {
-      gc += dt * (ta - sg) / T(2.0) / hx * (w[k + S] - w[k - S]) * gp;
-      gc += dt * (sg - ta) / T(2.0) / hy * (w[k + 1] - w[k - 1]) * gs;
-    } else {
-      gc += dt * (ta - sg) / (two * hx) * (u[k + S] - u[k - S]) * gp;
-      gc += dt * (sg - ta) / (two * hy) * (u[k + 1] - u[k - 1]) * gs;
+  const int tid = threadIdx.y * BJ + threadIdx.x;
+  auto inside = [&](int i, int j) { return i >= 1 && i <= NX && j >= 1 && j <= NY; };
+  for (int e = tid; e < HPR * WP; e += BJ * BI) {
+    const int r = e / WP, q = e - r * WP;
+    const int i = i0 + r - HP, j = j0 + q - HP;
+    T px = 0, py = 0;
+    if (inside(i, j)) {
+      const int64_t k = (int64_t)i * S + j;
+      const T s = sigma[k], t = tau[k], gp = grad_phiout[k], gq = grad_psiout[k], ck = c[k];
+      // (0 times a gradient that is not finite is kept as the NaN it is)
+      if (!undamped<T>(K, s, t, ck) || !tame(gp) || !tame(gq)) {
+        const T d = K.dt * ck * (t - s);
+        px = d / K.hx2 * gp;
+        py = -d / K.hy2 * gq;
+      }
     }
+    sx[r][q] = px;
+    sy[r][q] = py;
   }
-  // neighbours y whose stencil reaches x
-  const int di[4] = {-1, 1, 0, 0}, dj[4] = {0, 0, -1, 1};
-#pragma unroll
-  for (int n = 0; n < 4; n++) {
-    const int a = i + di[n], b = j + dj[n];
-    if (!interior(a, b)) continue;
-    const int64_t y = (int64_t)a * S + b;
-    const T cy = c[y], g = G(a, b), d = den(y);
-    if (n < 2) {
-      // x is y's i+1 neighbour when n == 0 (y = x - e_i), i-1 neighbour when n == 1
-      const T sgn = n == 0 ? one : -one;
-      gw += cy * (dt / hx) * (dt / hx) * g / d;
-      gph += sgn * (dt * dt / (T(2.0) * hx)) * g / d;
-      if (VARIANT == 0) gw += sgn * dt * cy * (tau[y] - sigma[y]) / T(2.0) / hx * grad_phiout[y];
+  if (VARIANT != 0) __syncthreads();
+  for (int e = tid; e < H * W; e += BJ * BI) {
+    const int r = e / W, q = e - r * W;
+    const int i = i0 + r - 1, j = j0 + q - 1;
+    T g = 0, cg = 0;
+    if (inside(i, j)) {
+      const int64_t k = (int64_t)i * S + j;
+      const T s = sigma[k], t = tau[k], ck = c[k];
+      g = grad_u[k];
+      if (VARIANT != 0) {
+        // PX, PY are zero on the frame and outside the grid
+        const T a = sx[r][q + 1], b = sx[r + 2][q + 1], d = sy[r + 1][q], f = sy[r + 1][q + 2];
+        if (!(zero_bits(a) && zero_bits(b) && zero_bits(d) && zero_bits(f)))
+          g += (a - b) + (d - f);
+      }
+      if (!undamped<T>(K, s, t, ck)) g = g / (one + (s + t) / two * K.dt);
+      cg = ck * g;
+    }
+    sg_[r][q] = g;
+    sc[r][q] = cg;
+  }
+  __syncthreads();
+  const int r = threadIdx.y, q = threadIdx.x, i = i0 + r, j = j0 + q;
+  if (i > NX + 1 || j > NY + 1) return;
+  const int64_t k = (int64_t)i * S + j;
+  // from the neighbours (zero outside the interior)
+  T gw = K.cx * (sc[r][q + 1] + sc[r + 2][q + 1]);
+  gw = fm(K.cy, sc[r + 1][q] + sc[r + 1][q + 2], gw);
+  T gph = K.fx * (sg_[r][q + 1] - sg_[r + 2][q + 1]);
+  T gps = K.fy * (sg_[r + 1][q] - sg_[r + 1][q + 2]);
+  if (VARIANT == 0) {
+    const T a = sx[r][q + 1], b = sx[r + 2][q + 1], d = sy[r + 1][q], f = sy[r + 1][q + 2];
+    if (!(zero_bits(a) && zero_bits(b) && zero_bits(d) && zero_bits(f)))
+      gw += (a - b) + (d - f);
+  }
+  T gwo = 0, gc = 0;
+  if (inside(i, j)) {
+    const T s = sigma[k], t = tau[k], ck = c[k], g = sg_[r + 1][q + 1];
+    const T wn = w[k + S], ws = w[k - S], we = w[k + 1], ww = w[k - 1];
+    const T gp = grad_phiout[k], gq = grad_psiout[k];
+    const bool plain = undamped<T>(K, s, t, ck);
+    T lap = K.cx * (wn + ws);
+    lap = fm(K.cy, we + ww, lap);
+    lap = fm(-kxy, w[k], lap);
+    gc = lap * g;
+    T un, us, ue, uw;  // the field phi' and psi' difference
+    if (VARIANT == 0) {
+      un = wn;
+      us = ws;
+      ue = we;
+      uw = ww;
     } else {
-      const T sgn = n == 2 ? one : -one;
-      gw += cy * (dt / hy) * (dt / hy) * g / d;
-      gps += sgn * (dt * dt / (T(2.0) * hy)) * g / d;
-      if (VARIANT == 0) gw += sgn * dt * cy * (sigma[y] - tau[y]) / T(2.0) / hy * grad_psiout[y];
+      un = u[k + S];
+      us = u[k - S];
+      ue = u[k + 1];
+      uw = u[k - 1];
+    }
+    if (plain) {
+      gw = fm(fm(-kxy, ck, two), g, gw);
+      gwo = -g;
+      gph += gp;
+      gps += gq;
+    } else {
+      gw = fm(fm(-kxy, ck, two - s * t * K.dt2), g, gw);
+      gwo = -(one - (s + t) * K.dt / two) * g;
+      gph = fm(one - K.dt * s, gp, gph);
+      gps = fm(one - K.dt * t, gq, gps);
+    }
+    if (!plain || !(tame(un) && tame(us) && tame(ue) && tame(uw) && tame(gp) && tame(gq))) {
+      const T d = K.dt * (t - s);
+      gc = fm(d / K.hx2 * (un - us), gp, gc);
+      gc = fm(-d / K.hy2 * (ue - uw), gq, gc);
     }
   }
   grad_w[k] = gw;
@@ -218,19 +364,15 @@ int acoustic_fwd(const T* w, const T* wold, const T* phi, const T* psi, const T*
   ADS_REQUIRE(w && wold && phi && psi && sigma && tau && c && u && phiout && psiout,
               "null pointer argument");
   ADS_REQUIRE(variant == 0 || variant == 1, "variant must be 0 (w) or 1 (u)");
-  dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
-  if (variant == 0) {
-    k_acoustic_fwd_w<T><<<grd, blk, 0, st>>>(w, wold, phi, psi, sigma, tau, c, T(dt), T(hx),
-                                              T(hy), (int)NX, (int)NY, u, phiout, psiout);
-    ADS_LAUNCHED(1);
-  } else {
-    k_acoustic_fwd_u1<T><<<grd, blk, 0, st>>>(w, wold, phi, psi, sigma, tau, c, T(dt), T(hx),
-                                               T(hy), (int)NX, (int)NY, u);
-    ADS_LAUNCHED(1);
-    k_acoustic_fwd_u2<T><<<grd, blk, 0, st>>>(u, phi, psi, sigma, tau, c, T(dt), T(hx), T(hy),
-                                               (int)NX, (int)NY, phiout, psiout);
-    ADS_LAUNCHED(1);
-  }
+  const StepK<T> K = make_k<T>(dt, hx, hy);
+  const dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
+  if (variant == 0)
+    k_acoustic_fwd_w<T><<<grd, blk, 0, st>>>(w, wold, phi, psi, sigma, tau, c, K, (int)NX,
+                                             (int)NY, u, phiout, psiout);
+  else
+    k_acoustic_fwd_u<T><<<grd, blk, 0, st>>>(w, wold, phi, psi, sigma, tau, c, K, (int)NX,
+                                             (int)NY, u, phiout, psiout);
+  ADS_LAUNCHED(1);
   return ADS_OK;
 }
 
@@ -246,17 +388,16 @@ int acoustic_bwd(T* grad_w, T* grad_wold, T* grad_phi, T* grad_psi, T* grad_c,
                   grad_phiout && grad_psiout && w && sigma && tau && c,
               "null pointer argument");
   ADS_REQUIRE(variant == 0 || (variant == 1 && u), "variant must be 0, or 1 with u given");
-  dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
-  if (variant == 0)
-    k_acoustic_bwd<T, 0><<<grd, blk, 0, st>>>(grad_w, grad_wold, grad_phi, grad_psi, grad_c,
-                                               grad_u, grad_phiout, grad_psiout, w, sigma,
-                                               tau, c, T(dt), T(hx), T(hy), (int)NX,
-                                               (int)NY, u);
-  else
-    k_acoustic_bwd<T, 1><<<grd, blk, 0, st>>>(grad_w, grad_wold, grad_phi, grad_psi, grad_c,
-                                               grad_u, grad_phiout, grad_psiout, w, sigma,
-                                               tau, c, T(dt), T(hx), T(hy), (int)NX,
-                                               (int)NY, u);
+  const StepK<T> K = make_k<T>(dt, hx, hy);
+  const T kxy = K.k1 + K.k2;
+  const dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
+  auto launch = [&](auto kernel) {
+    kernel<<<grd, blk, 0, st>>>(grad_w, grad_wold, grad_phi, grad_psi, grad_c, grad_u,
+                                grad_phiout, grad_psiout, w, sigma, tau, c, K, kxy, (int)NX,
+                                (int)NY, u);
+  };
+  if (variant == 0) launch(k_acoustic_bwd<T, 0>);
+  else launch(k_acoustic_bwd<T, 1>);
   ADS_LAUNCHED(1);
   return ADS_OK;
 }
