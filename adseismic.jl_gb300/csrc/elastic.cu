@@ -5,10 +5,12 @@
 // The reference composes one step from ~50 gather/scatter custom ops per step
 // (fw1..fw4 + add_source).  Here the single-step operators are two kernels
 // (stresses: fw1+fw2; velocities: fw3+fw4, one thread per cell) and their
-// transpose three; the plans step with one fused row-streaming kernel plus a
-// tiny source/receiver launch, and run each adjoint step as one fused
-// row-streaming kernel (FP32 plans; FP64 plans by default, and any plan on
-// request, as three gather-form row-streaming kernels).  In the plans, per-cell
+// transpose three.  FP64 plans and small FP32 plans step with the same two
+// kernels and a transpose of two; larger FP32 plans with one fused row-streaming
+// kernel a step and one an adjoint step.  On request (adjoint_passes,
+// rows_per_warp) any plan runs the row-streaming kernels, the adjoint fused or as
+// three gather passes.  A tiny source / receiver launch follows each step.  In the
+// plans, per-cell
 // work on the eight memory
 // variables only runs where the 1D CPML profile is active (a != 0 or b != 1);
 // elsewhere the forward memory stays exactly zero and its adjoint never
@@ -51,10 +53,8 @@ struct ElModel {
 
 template <typename T>
 struct ElShot {
-  const T* fin[NF];  // single-step operators: step input state
-  T* f[NF];          // single-step operators: step output state; plans: state
-                     // buffer 0 (buffer 1 follows at f[0] + NF * fs)
-  T* g[NF];          // adjoint state (in place)
+  T* f[NF];          // state buffer 0 (buffer 1 follows at f[0] + NF * fs)
+  T* g[NF];          // adjoint state
   T* tmp[NTMP];
   T* store;          // K slots x NSTORE fields
   T* ckpt;           // nseg x NF fields
@@ -74,279 +74,751 @@ struct ElShot {
   const int* rcv_type;
   int nsrc, nrcv;
   int64_t fs;                   // elements per field
+  double* cacc;                 // cell-kernel plans: NCACC sums, FP64
+  float* cacc32;                // and the FP32 plans' per-segment partials of them
 };
 
+// ---------------------------------------------------------------------------
+// One-thread-per-cell kernels: the single-step operators (both precisions), the
+// FP64 plans, and the FP32 plans whose shots hold too few cells for the
+// row-streaming kernels below.
+//
+// A step is two kernels (stresses: fw1, fw2; velocities: fw3, fw4), its transpose
+// two more.  FP64 kernels are bound by the count of FP64 instructions (a warp's
+// instruction holds the pipe of its SM sub-partition for 64 cycles), so:
+//  * the four-point difference is 27/(24h) (a - b) - 1/(24h) (c - d): 4
+//    operations and no division (a division is some twenty);
+//  * plans fold dt into tables of the averaged moduli and of dt / density
+//    (k_el_tables, once a call), 42 operations a CPML-free cell and step;
+//  * the transpose forms what a cell sends (q, D1..D8 in the comments of the
+//    reference's order: fw4..fw1 transposed) once, in shared memory, over a tile
+//    and the three rows or columns that reach into it, and gathers it there; no
+//    intermediate field goes through memory;
+//  * the plans' parameter gradients are summed where they arise (the products of
+//    strains and stress adjoints at the stress cells, of accelerations and
+//    velocity adjoints at the velocity cells: one multiply-add each) and are
+//    averaged onto the cells of lambda, mu, rho once per call
+//    (k_el_gather_cells), which is the same sum in another order.
+// No row or column is computed twice, and a grid of 47 k cells already gives every
+// SM ten warps, where a strip of rows leaves most of the chip idle: the FP64
+// gradient of 2 shots of 253 x 187, 250 steps, takes 11.6 ms, 113 ms with the
+// row-streaming kernels (FP64 pipe 64% busy in these kernels there); the operator
+// and its transpose on 600 x 300 FP64 take 20 + 22 and 19 + 55 + 43 us (FP64 pipe
+// 74-82% busy).
+// ---------------------------------------------------------------------------
+// offsets within a field: 32 bits in plans (which check it), 64 in the operators
+template <bool PLAN>
+using CellIx = std::conditional_t<PLAN, int, int64_t>;
+
 template <typename T>
-__device__ __forceinline__ T d4(T a0, T am1, T ap1, T am2, T h24) {
-  return (T(27) * a0 - T(27) * am1 - ap1 + am2) / h24;
+struct CellModel {
+  const T *lam, *mu, *rho;                 // operators: averaged per cell
+  const T *lm, *la, *m2, *b3, *b4;         // plans: the tables
+  const T *axi, *axh, *bxi, *bxh, *ayi, *ayh, *byi, *byh;  // 1D, index I-1 / J-1
+  T dt, rdt;                               // dt, 1 / dt
+  T x27, x1, y27, y1;                      // 27 / (24 h), 1 / (24 h)
+  double dtd;                              // dt, unrounded
+  int NX, NY, OFF, P;
+};
+
+__device__ __forceinline__ double el_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float el_fma(float a, float b, float c) { return fmaf(a, b, c); }
+
+// A CPML profile entry that changes nothing (a = 0, b = 1), by its bits: FP64
+// comparisons issue on the FP64 pipe.
+__device__ __forceinline__ bool idle(double a, double b) {
+  return ((__double2hiint(a) << 1) | __double2loint(a)) == 0 &&
+         __double2hiint(b) == 0x3ff00000 && __double2loint(b) == 0;
+}
+__device__ __forceinline__ bool idle(float a, float b) { return a == 0.f && b == 1.f; }
+// finite, and so is the difference of two such values (0 times it is a zero)
+__device__ __forceinline__ bool el_tame(double x) {
+  return (__double2hiint(x) & 0x7ff00000) < 0x7fe00000;
+}
+__device__ __forceinline__ bool el_tame(float x) {
+  return (__float_as_int(x) & 0x7f800000) < 0x7f000000;
 }
 
-#define ELIDX(ii, jj) ((int64_t)(ii) * M.P + (jj) + M.OFF)
+// 27 (a - b) / (24 h) - (c - d) / (24 h)
+template <typename T>
+__device__ __forceinline__ T dif(T a, T b, T c, T d, T k27, T k1) {
+  return el_fma(k27, a - b, -(k1 * (c - d)));
+}
 
-// Stress update (fw1: sxx, syy, m1, m2; fw2: sxy, m3, m4) of the single-step
-// operator: every cell is written (out of place), the memory variables in full.
-template <typename T, bool STORE>
-__global__ void __launch_bounds__(BX* BY)
-k_el_stress(ElModel<T> M, ElShot<T> one, int store_slot) {
-  const ElShot<T>& sh = one;
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  const int NX = M.NX, NY = M.NY;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t x = ELIDX(i, j);
-  const bool b1 = i >= 1 && i <= NX - 1 && j >= 2 && j <= NY;
-  const bool b2 = i >= 2 && i <= NX && j >= 1 && j <= NY - 1;
-  const T* vx = sh.fin[VX];
-  const T* vy = sh.fin[VY];
-  T* st = STORE ? sh.store + (int64_t)store_slot * NSTORE * sh.fs : nullptr;
-  if (b1) {
-    const T lam_ = T(0.5) * (M.lam[ELIDX(i + 1, j)] + M.lam[x]);
-    const T mu_ = T(0.5) * (M.mu[ELIDX(i + 1, j)] + M.mu[x]);
-    const T lm = lam_ + T(2) * mu_;
-    const T dvx = d4<T>(vx[ELIDX(i + 1, j)], vx[x], vx[ELIDX(i + 2, j)], vx[ELIDX(i - 1, j)],
-                        M.hx24);
-    const T dvy = d4<T>(vy[x], vy[ELIDX(i, j - 1)], vy[ELIDX(i, j + 1)], vy[ELIDX(i, j - 2)],
-                        M.hy24);
-    const T m1 = M.bxh[i - 1] * sh.fin[M1 + 0][x] + M.axh[i - 1] * dvx;
-    sh.f[M1 + 0][x] = m1;
-    const T m2 = M.byi[j - 1] * sh.fin[M1 + 1][x] + M.ayi[j - 1] * dvy;
-    sh.f[M1 + 1][x] = m2;
-    const T e1 = dvx + m1, e2 = dvy + m2;
-    sh.f[SXX][x] = sh.fin[SXX][x] + (lm * e1 + lam_ * e2) * M.dt;
-    sh.f[SYY][x] = sh.fin[SYY][x] + (lm * e2 + lam_ * e1) * M.dt;
-    if (STORE) {
-      st[E1 * sh.fs + x] = e1;
-      st[E2 * sh.fs + x] = e2;
+// The strain or acceleration d + m' of one difference d, with its memory
+// variable m' = b m + a d stored at mo.  Plans hold m = 0 where the profile is
+// idle and touch it nowhere there; the operators take any m.
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mem_fwd(T d, T a, T b, const T* mi, T* mo, CellIx<PLAN> x) {
+  if (idle(a, b)) {
+    if (PLAN) return d;
+    if (el_tame(d)) {
+      const T m = mi[x];
+      if (mo) mo[x] = m;
+      return d + m;
     }
-  } else {
-    sh.f[SXX][x] = sh.fin[SXX][x];
-    sh.f[SYY][x] = sh.fin[SYY][x];
-    sh.f[M1 + 0][x] = T(0);
-    sh.f[M1 + 1][x] = T(0);
   }
-  if (b2) {
-    const T mu_ = T(0.5) * (M.mu[x] + M.mu[ELIDX(i, j + 1)]);
-    const T dvydx = d4<T>(vy[x], vy[ELIDX(i - 1, j)], vy[ELIDX(i + 1, j)], vy[ELIDX(i - 2, j)],
-                          M.hx24);
-    const T dvxdy = d4<T>(vx[ELIDX(i, j + 1)], vx[x], vx[ELIDX(i, j + 2)], vx[ELIDX(i, j - 1)],
-                          M.hy24);
-    const T m3 = M.bxi[i - 1] * sh.fin[M1 + 2][x] + M.axi[i - 1] * dvydx;
-    sh.f[M1 + 2][x] = m3;
-    const T m4 = M.byh[j - 1] * sh.fin[M1 + 3][x] + M.ayh[j - 1] * dvxdy;
-    sh.f[M1 + 3][x] = m4;
-    const T e12 = (dvydx + m3) + (dvxdy + m4);
-    sh.f[SXY][x] = sh.fin[SXY][x] + mu_ * e12 * M.dt;
-    if (STORE) st[E12 * sh.fs + x] = e12;
-  } else {
-    sh.f[SXY][x] = sh.fin[SXY][x];
-    sh.f[M1 + 2][x] = T(0);
-    sh.f[M1 + 3][x] = T(0);
-  }
+  const T m = el_fma(b, mi[x], a * d);
+  if (mo) mo[x] = m;
+  return d + m;
 }
 
-// Velocity update (fw3: vx, m5, m6 from the new sxx, sxy; fw4: vy, m7, m8
-// from the new sxy, syy).
+// D = q + a (q + g) of one difference's transpose (g: the memory variable's
+// adjoint, whose new value b (q + g) is stored at go), without the 1/(24h).
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mem_adj(T q, T a, T b, const T* gi, T* go, CellIx<PLAN> x) {
+  if (idle(a, b)) {
+    if (PLAN) return q;
+    if (el_tame(q)) {
+      const T g = gi[x];
+      if (el_tame(g)) {
+        if (go) go[x] = q + g;
+        return q;
+      }
+    }
+  }
+  const T g = q + gi[x];
+  if (go) go[x] = b * g;
+  return el_fma(a, g, q);
+}
+
+// Moduli of the stress cells and dt / density of the velocity cells, times dt.
+template <typename T, bool PLAN>
+__device__ __forceinline__ void mat1(const CellModel<T>& M, CellIx<PLAN> x, T& lm, T& la) {
+  if (PLAN) {
+    lm = M.lm[x];
+    la = M.la[x];
+  } else {
+    const T l = T(0.5) * (M.lam[x + M.P] + M.lam[x]), u = M.mu[x + M.P] + M.mu[x];
+    la = l * M.dt;
+    lm = (l + u) * M.dt;
+  }
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mat2(const CellModel<T>& M, CellIx<PLAN> x) {
+  return PLAN ? M.m2[x] : T(0.5) * M.dt * (M.mu[x] + M.mu[x + 1]);
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mat3(const CellModel<T>& M, CellIx<PLAN> x) {
+  return PLAN ? M.b3[x] : M.dt / M.rho[x];
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mat4(const CellModel<T>& M, CellIx<PLAN> x) {
+  return PLAN ? M.b4[x]
+              : M.dt / (T(0.25) * (M.rho[x] + M.rho[x + M.P] + M.rho[x + M.P + 1] + M.rho[x + 1]));
+}
+
+// Update boxes: fw1 (sxx, syy), fw2 (sxy), fw3 (vx), fw4 (vy).
+template <typename T>
+__device__ __forceinline__ bool box1(const CellModel<T>& M, int i, int j) {
+  return i >= 1 && i <= M.NX - 1 && j >= 2 && j <= M.NY;
+}
+template <typename T>
+__device__ __forceinline__ bool box2(const CellModel<T>& M, int i, int j) {
+  return i >= 2 && i <= M.NX && j >= 1 && j <= M.NY - 1;
+}
+template <typename T>
+__device__ __forceinline__ bool box3(const CellModel<T>& M, int i, int j) {
+  return i >= 2 && i <= M.NX && j >= 2 && j <= M.NY;
+}
+template <typename T>
+__device__ __forceinline__ bool box4(const CellModel<T>& M, int i, int j) {
+  return i >= 1 && i <= M.NX - 1 && j >= 1 && j <= M.NY - 1;
+}
+
+// Strains of the stress cells and accelerations (times density) of the velocity
+// cells at (i, j), x its offset; f: the 13 input fields of fs elements, s the
+// new stresses (sxx, syy, sxy at so[0..2]); the new memory variables go to
+// fo (null: nowhere).
+template <typename T, bool PLAN>
+__device__ __forceinline__ void strain1(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* f,
+                                        int64_t fs, T* fo, T& e1, T& e2) {
+  const T* vx = f + VX * fs;
+  const T* vy = f + VY * fs;
+  const int P = M.P;
+  const T a = dif<T>(vx[x + P], vx[x], vx[x + 2 * P], vx[x - P], M.x27, M.x1);
+  const T b = dif<T>(vy[x], vy[x - 1], vy[x + 1], vy[x - 2], M.y27, M.y1);
+  e1 = mem_fwd<T, PLAN>(a, M.axh[i - 1], M.bxh[i - 1], f + M1 * fs, fo ? fo + M1 * fs : nullptr, x);
+  e2 = mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 1) * fs,
+                        fo ? fo + (M1 + 1) * fs : nullptr, x);
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T strain2(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* f,
+                                     int64_t fs, T* fo) {
+  const T* vx = f + VX * fs;
+  const T* vy = f + VY * fs;
+  const int P = M.P;
+  const T a = dif<T>(vy[x], vy[x - P], vy[x + P], vy[x - 2 * P], M.x27, M.x1);
+  const T b = dif<T>(vx[x + 1], vx[x], vx[x + 2], vx[x - 1], M.y27, M.y1);
+  return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 2) * fs,
+                          fo ? fo + (M1 + 2) * fs : nullptr, x) +
+         mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 3) * fs,
+                          fo ? fo + (M1 + 3) * fs : nullptr, x);
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T accel3(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxx,
+                                    const T* sxy, const T* f, int64_t fs, T* fo) {
+  const int P = M.P;
+  const T a = dif<T>(sxx[x], sxx[x - P], sxx[x + P], sxx[x - 2 * P], M.x27, M.x1);
+  const T b = dif<T>(sxy[x], sxy[x - 1], sxy[x + 1], sxy[x - 2], M.y27, M.y1);
+  return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 4) * fs,
+                          fo ? fo + (M1 + 4) * fs : nullptr, x) +
+         mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 5) * fs,
+                          fo ? fo + (M1 + 5) * fs : nullptr, x);
+}
+template <typename T, bool PLAN>
+__device__ __forceinline__ T accel4(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxy,
+                                    const T* syy, const T* f, int64_t fs, T* fo) {
+  const int P = M.P;
+  const T a = dif<T>(sxy[x + P], sxy[x], sxy[x + 2 * P], sxy[x - P], M.x27, M.x1);
+  const T b = dif<T>(syy[x + 1], syy[x], syy[x + 2], syy[x - 1], M.y27, M.y1);
+  return mem_fwd<T, PLAN>(a, M.axh[i - 1], M.bxh[i - 1], f + (M1 + 6) * fs,
+                          fo ? fo + (M1 + 6) * fs : nullptr, x) +
+         mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 7) * fs,
+                          fo ? fo + (M1 + 7) * fs : nullptr, x);
+}
+
+// Cell of a thread: row blocks along blockIdx.x (their count may pass 65535),
+// column blocks along blockIdx.y.  Plans start at cell (1, 1), whose address is
+// 128-byte aligned; the operators cover the padded grid.
+#define ADS_EL_CELL(FIRST)                                                     \
+  const int tx = threadIdx.x, ty = threadIdx.y;                                \
+  const int i0 = (FIRST) + blockIdx.x * BY, j0 = (FIRST) + blockIdx.y * BX;    \
+  const int i = i0 + ty, j = j0 + tx, P = M.P;                                 \
+  const CellIx<(FIRST) != 0> x = (CellIx<(FIRST) != 0>)i * P + j + M.OFF;      \
+  (void)P, (void)x
+
+// ---- plans: state buffer pin -> the other, only cells a stencil updates
+
 template <typename T, bool STORE>
 __global__ void __launch_bounds__(BX* BY)
-k_el_velocity(ElModel<T> M, ElShot<T> one, int store_slot) {
-  const ElShot<T>& sh = one;
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  const int NX = M.NX, NY = M.NY;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t x = ELIDX(i, j);
-  const bool b3 = i >= 2 && i <= NX && j >= 2 && j <= NY;
-  const bool b4 = i >= 1 && i <= NX - 1 && j >= 1 && j <= NY - 1;
-  const T* sxx = sh.f[SXX];
-  const T* syy = sh.f[SYY];
-  const T* sxy = sh.f[SXY];
-  T* st = STORE ? sh.store + (int64_t)store_slot * NSTORE * sh.fs : nullptr;
-  if (b3) {
-    const T a = d4<T>(sxx[x], sxx[ELIDX(i - 1, j)], sxx[ELIDX(i + 1, j)], sxx[ELIDX(i - 2, j)],
-                      M.hx24);
-    const T b = d4<T>(sxy[x], sxy[ELIDX(i, j - 1)], sxy[ELIDX(i, j + 1)], sxy[ELIDX(i, j - 2)],
-                      M.hy24);
-    const T m5 = M.bxi[i - 1] * sh.fin[M1 + 4][x] + M.axi[i - 1] * a;
-    sh.f[M1 + 4][x] = m5;
-    const T m6 = M.byi[j - 1] * sh.fin[M1 + 5][x] + M.ayi[j - 1] * b;
-    sh.f[M1 + 5][x] = m6;
-    const T e3 = (a + m5) + (b + m6);
-    sh.f[VX][x] = sh.fin[VX][x] + e3 * M.dt / M.rho[x];
-    if (STORE) st[A3 * sh.fs + x] = e3;
-  } else {
-    sh.f[VX][x] = sh.fin[VX][x];
-    sh.f[M1 + 4][x] = T(0);
-    sh.f[M1 + 5][x] = T(0);
+k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+  const ElShot<T>& sh = shots[blockIdx.z];
+  ADS_EL_CELL(1);
+  if (i > M.NX || j > M.NY) return;
+  const int64_t fs = sh.fs;
+  const T* f = sh.f[0] + (int64_t)pin * NF * fs;
+  T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
+  T* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  if (box1(M, i, j)) {
+    T e1, e2, lm, la;
+    strain1<T, true>(M, i, j, x, f, fs, o, e1, e2);
+    mat1<T, true>(M, x, lm, la);
+    o[SXX * fs + x] = el_fma(lm, e1, el_fma(la, e2, f[SXX * fs + x]));
+    o[SYY * fs + x] = el_fma(lm, e2, el_fma(la, e1, f[SYY * fs + x]));
+    if (STORE) {
+      st[E1 * fs + x] = e1;
+      st[E2 * fs + x] = e2;
+    }
   }
-  if (b4) {
-    const T rho_ = T(0.25) * (M.rho[x] + M.rho[ELIDX(i + 1, j)] + M.rho[ELIDX(i + 1, j + 1)] +
-                              M.rho[ELIDX(i, j + 1)]);
-    const T a = d4<T>(sxy[ELIDX(i + 1, j)], sxy[x], sxy[ELIDX(i + 2, j)], sxy[ELIDX(i - 1, j)],
-                      M.hx24);
-    const T b = d4<T>(syy[ELIDX(i, j + 1)], syy[x], syy[ELIDX(i, j + 2)], syy[ELIDX(i, j - 1)],
-                      M.hy24);
-    const T m7 = M.bxh[i - 1] * sh.fin[M1 + 6][x] + M.axh[i - 1] * a;
-    sh.f[M1 + 6][x] = m7;
-    const T m8 = M.byh[j - 1] * sh.fin[M1 + 7][x] + M.ayh[j - 1] * b;
-    sh.f[M1 + 7][x] = m8;
-    const T e4 = (a + m7) + (b + m8);
-    sh.f[VY][x] = sh.fin[VY][x] + e4 * M.dt / rho_;
-    if (STORE) st[A4 * sh.fs + x] = e4;
-  } else {
-    sh.f[VY][x] = sh.fin[VY][x];
-    sh.f[M1 + 6][x] = T(0);
-    sh.f[M1 + 7][x] = T(0);
+  if (box2(M, i, j)) {
+    const T e = strain2<T, true>(M, i, j, x, f, fs, o);
+    o[SXY * fs + x] = el_fma(mat2<T, true>(M, x), e, f[SXY * fs + x]);
+    if (STORE) st[E12 * fs + x] = e;
   }
 }
 
-// Adjoint 1 (velocity cells): transposes of fw3 and fw4.  Writes D5..D8 and
-// R4, updates the memory adjoints m5..m8 and grho (fw3 part) in place.
+template <typename T, bool STORE>
+__global__ void __launch_bounds__(BX* BY)
+k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+  const ElShot<T>& sh = shots[blockIdx.z];
+  ADS_EL_CELL(1);
+  if (i > M.NX || j > M.NY) return;
+  const int64_t fs = sh.fs;
+  const T* f = sh.f[0] + (int64_t)pin * NF * fs;
+  T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
+  T* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  if (box3(M, i, j)) {
+    const T e = accel3<T, true>(M, i, j, x, o + SXX * fs, o + SXY * fs, f, fs, o);
+    o[VX * fs + x] = el_fma(mat3<T, true>(M, x), e, f[VX * fs + x]);
+    if (STORE) st[A3 * fs + x] = e;
+  }
+  if (box4(M, i, j)) {
+    const T e = accel4<T, true>(M, i, j, x, o + SXY * fs, o + SYY * fs, f, fs, o);
+    o[VY * fs + x] = el_fma(mat4<T, true>(M, x), e, f[VY * fs + x]);
+    if (STORE) st[A4 * fs + x] = e;
+  }
+}
+
+// What the velocity cells of a tile and its halo send to the stresses: D5
+// (rows -1..+2 around the tile), D6 (columns -1..+2), D7 (rows -2..+1), D8
+// (columns -2..+1).  One halo value a thread.
+template <typename T>
+struct SendV {
+  T d5[BY + 3][BX], d6[BY][BX + 3], d7[BY + 3][BX], d8[BY][BX + 3];
+};
+// and the stress cells to the velocities: D1 (rows -2..+1), D2 (columns
+// -1..+2), D3 (rows -1..+2), D4 (columns -2..+1)
+template <typename T>
+struct SendS {
+  T d1[BY + 3][BX], d2[BY][BX + 3], d3[BY + 3][BX], d4[BY][BX + 3];
+};
+static_assert(6 * BX + 6 * BY <= BX * BY, "a halo value per thread");
+
+// The thread's halo value: which array (0 none, 1..4), its cell, its place there.
+// Rows above / below: arrays 1 and 3, three rows each; columns: 2 and 4.
+__device__ __forceinline__ int halo_of(int t, int up1, int left2, int up3, int left4, int& di,
+                                       int& dj) {
+  int a, k, up;
+  if (t < 6 * BX) {
+    a = t < 3 * BX ? 1 : 3;
+    if (a == 3) t -= 3 * BX;
+    k = t / BX;
+    up = a == 1 ? up1 : up3;
+    di = k < up ? k - up : BY + k - up;
+    dj = t - k * BX;
+    return a;
+  }
+  t -= 6 * BX;
+  if (t >= 6 * BY) return 0;
+  a = t < 3 * BY ? 2 : 4;
+  if (a == 4) t -= 3 * BY;
+  k = t / BY;
+  up = a == 2 ? left2 : left4;
+  dj = k < up ? k - up : BX + k - up;
+  di = t - k * BY;
+  return a;
+}
+
+// Fills SendV for the tile at (i0, j0): g the 13 adjoint fields, go the new
+// memory adjoints of the tile's own cells (m5..m8).  Returns the thread's own q3, q4.
+template <typename T, bool PLAN>
+__device__ __forceinline__ void send_velocity(const CellModel<T>& M, SendV<T>& S, int i0, int j0,
+                                              const T* g, T* go, int64_t fs, T& q3, T& q4) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  auto put = [&](int a, int di, int dj, T* mo) {
+    const int ii = i0 + di, jj = j0 + dj;
+    const CellIx<PLAN> y = (CellIx<PLAN>)ii * M.P + jj + M.OFF;
+    const bool v3 = a != 3 && a != 4 && box3(M, ii, jj), v4 = a != 1 && a != 2 && box4(M, ii, jj);
+    T q = T(0), p = T(0), r5 = T(0), r6 = T(0), r7 = T(0), r8 = T(0);
+    if (v3) {
+      q = g[VX * fs + y] * mat3<T, PLAN>(M, y);
+      if (a == 0 || a == 1)
+        r5 = mem_adj<T, PLAN>(q, M.axi[ii - 1], M.bxi[ii - 1], g + (M1 + 4) * fs,
+                              mo ? mo + (M1 + 4) * fs : nullptr, y);
+      if (a == 0 || a == 2)
+        r6 = mem_adj<T, PLAN>(q, M.ayi[jj - 1], M.byi[jj - 1], g + (M1 + 5) * fs,
+                              mo ? mo + (M1 + 5) * fs : nullptr, y);
+    }
+    if (v4) {
+      p = g[VY * fs + y] * mat4<T, PLAN>(M, y);
+      if (a == 0 || a == 3)
+        r7 = mem_adj<T, PLAN>(p, M.axh[ii - 1], M.bxh[ii - 1], g + (M1 + 6) * fs,
+                              mo ? mo + (M1 + 6) * fs : nullptr, y);
+      if (a == 0 || a == 4)
+        r8 = mem_adj<T, PLAN>(p, M.ayh[jj - 1], M.byh[jj - 1], g + (M1 + 7) * fs,
+                              mo ? mo + (M1 + 7) * fs : nullptr, y);
+    }
+    if (a == 0 || a == 1) S.d5[di + 1][dj] = r5;
+    if (a == 0 || a == 2) S.d6[di][dj + 1] = r6;
+    if (a == 0 || a == 3) S.d7[di + 2][dj] = r7;
+    if (a == 0 || a == 4) S.d8[di][dj + 2] = r8;
+    if (a == 0) {
+      q3 = q;
+      q4 = p;
+    }
+  };
+  put(0, ty, tx, go);
+  int di, dj;
+  const int a = halo_of(ty * BX + tx, 1, 1, 2, 2, di, dj);
+  if (a == 1) put(1, di, dj, nullptr);
+  else if (a == 2) put(2, di, dj, nullptr);
+  else if (a == 3) put(3, di, dj, nullptr);
+  else if (a == 4) put(4, di, dj, nullptr);
+}
+
+// The stress adjoints gathered from SendV.
+template <typename T>
+__device__ __forceinline__ void gather_stress(const CellModel<T>& M, const SendV<T>& S, T& sxx,
+                                              T& syy, T& sxy) {
+  const int r = threadIdx.y, q = threadIdx.x;
+  sxx += dif<T>(S.d5[r + 1][q], S.d5[r + 2][q], S.d5[r][q], S.d5[r + 3][q], M.x27, M.x1);
+  sxy += dif<T>(S.d6[r][q + 1], S.d6[r][q + 2], S.d6[r][q], S.d6[r][q + 3], M.y27, M.y1);
+  sxy += dif<T>(S.d7[r + 1][q], S.d7[r + 2][q], S.d7[r][q], S.d7[r + 3][q], M.x27, M.x1);
+  syy += dif<T>(S.d8[r][q + 1], S.d8[r][q + 2], S.d8[r][q], S.d8[r][q + 3], M.y27, M.y1);
+}
+
+// Fills SendS from the stress adjoints s (sxx, syy, sxy at fields SXX..SXY of
+// s); g: the old memory adjoints m1..m4, go: the tile's new ones.
+template <typename T, bool PLAN>
+__device__ __forceinline__ void send_stress(const CellModel<T>& M, SendS<T>& S, int i0, int j0,
+                                            const T* s, const T* g, T* go, int64_t fs) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  auto put = [&](int a, int di, int dj, T* mo) {
+    const int ii = i0 + di, jj = j0 + dj;
+    const CellIx<PLAN> y = (CellIx<PLAN>)ii * M.P + jj + M.OFF;
+    T r1 = T(0), r2 = T(0), r3 = T(0), r4 = T(0);
+    if (a != 3 && a != 4 && box1(M, ii, jj)) {
+      const T gx = s[SXX * fs + y], gy = s[SYY * fs + y];
+      T lm, la;
+      mat1<T, PLAN>(M, y, lm, la);
+      if (a == 0 || a == 1)
+        r1 = mem_adj<T, PLAN>(el_fma(lm, gx, la * gy), M.axh[ii - 1], M.bxh[ii - 1], g + M1 * fs,
+                              mo ? mo + M1 * fs : nullptr, y);
+      if (a == 0 || a == 2)
+        r2 = mem_adj<T, PLAN>(el_fma(lm, gy, la * gx), M.ayi[jj - 1], M.byi[jj - 1],
+                              g + (M1 + 1) * fs, mo ? mo + (M1 + 1) * fs : nullptr, y);
+    }
+    if (a != 1 && a != 2 && box2(M, ii, jj)) {
+      const T q = s[SXY * fs + y] * mat2<T, PLAN>(M, y);
+      if (a == 0 || a == 3)
+        r3 = mem_adj<T, PLAN>(q, M.axi[ii - 1], M.bxi[ii - 1], g + (M1 + 2) * fs,
+                              mo ? mo + (M1 + 2) * fs : nullptr, y);
+      if (a == 0 || a == 4)
+        r4 = mem_adj<T, PLAN>(q, M.ayh[jj - 1], M.byh[jj - 1], g + (M1 + 3) * fs,
+                              mo ? mo + (M1 + 3) * fs : nullptr, y);
+    }
+    if (a == 0 || a == 1) S.d1[di + 2][dj] = r1;
+    if (a == 0 || a == 2) S.d2[di][dj + 1] = r2;
+    if (a == 0 || a == 3) S.d3[di + 1][dj] = r3;
+    if (a == 0 || a == 4) S.d4[di][dj + 2] = r4;
+  };
+  put(0, ty, tx, go);
+  int di, dj;
+  const int a = halo_of(ty * BX + tx, 2, 1, 1, 2, di, dj);
+  if (a == 1) put(1, di, dj, nullptr);
+  else if (a == 2) put(2, di, dj, nullptr);
+  else if (a == 3) put(3, di, dj, nullptr);
+  else if (a == 4) put(4, di, dj, nullptr);
+}
+
+template <typename T>
+__device__ __forceinline__ void gather_velocity(const CellModel<T>& M, const SendS<T>& S, T& vx,
+                                                T& vy) {
+  const int r = threadIdx.y, q = threadIdx.x;
+  vx += dif<T>(S.d1[r + 1][q], S.d1[r + 2][q], S.d1[r][q], S.d1[r + 3][q], M.x27, M.x1);
+  vx += dif<T>(S.d4[r][q + 1], S.d4[r][q + 2], S.d4[r][q], S.d4[r][q + 3], M.y27, M.y1);
+  vy += dif<T>(S.d2[r][q + 1], S.d2[r][q + 2], S.d2[r][q], S.d2[r][q + 3], M.y27, M.y1);
+  vy += dif<T>(S.d3[r + 1][q], S.d3[r + 2][q], S.d3[r][q], S.d3[r + 3][q], M.x27, M.x1);
+}
+
+// The sums a cell-kernel plan's gradients are formed from, one field each: FP64
+// accumulators in FP64 plans, the FP32 partials of a segment in FP32 plans.
+enum { CL = 0, CM1, CM2, CR3, CR4, NCACC };
+template <typename T>
+__device__ __forceinline__ void add_cell(const ElShot<T>& sh, int k, int x, T a, T b) {
+  if constexpr (sizeof(T) == 8) {
+    double* p = sh.cacc + (int64_t)k * sh.fs + x;
+    *p = el_fma(a, b, *p);
+  } else {
+    float* p = sh.cacc32 + (int64_t)k * sh.fs + x;
+    *p = el_fma(a, b, *p);
+  }
+}
+
+// Adjoint of a step, velocity cells -> stress adjoints (transposes of fw3, fw4):
+// adjoint buffer pin -> the other.
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
-k_el_adj1(ElModel<T> M, ElShot<T> one, int store_slot) {
-  const ElShot<T>& sh = one;
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  const int NX = M.NX, NY = M.NY;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t x = ELIDX(i, j);
-  const bool b3 = i >= 2 && i <= NX && j >= 2 && j <= NY;
-  const bool b4 = i >= 1 && i <= NX - 1 && j >= 1 && j <= NY - 1;
-  const T* st = sh.store + (int64_t)store_slot * NSTORE * sh.fs;
-  if (b3) {
-    const T gv = sh.g[VX][x], r = M.rho[x];
-    const T q = gv * M.dt / r;
-    T gm5 = q, gm6 = q;
-    gm5 += sh.g[M1 + 4][x];
-    sh.g[M1 + 4][x] = M.bxi[i - 1] * gm5;
-    gm6 += sh.g[M1 + 5][x];
-    sh.g[M1 + 5][x] = M.byi[j - 1] * gm6;
-    sh.tmp[D5][x] = (q + M.axi[i - 1] * gm5) / M.hx24;
-    sh.tmp[D6][x] = (q + M.ayi[j - 1] * gm6) / M.hy24;
-    sh.grho[x] += (double)(-gv * st[A3 * sh.fs + x] * M.dt / (r * r));
-  } else {
-    sh.g[M1 + 4][x] = T(0);
-    sh.g[M1 + 5][x] = T(0);
+k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+  __shared__ SendV<T> S;
+  const ElShot<T>& sh = shots[blockIdx.z];
+  ADS_EL_CELL(1);
+  const int64_t fs = sh.fs;
+  const T* g = sh.g[0] + (int64_t)pin * NF * fs;
+  T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  T q3, q4;
+  send_velocity<T, true>(M, S, i0, j0, g, o, fs, q3, q4);
+  const T* st = sh.store + (int64_t)slot * NSTORE * fs;
+  if (box3(M, i, j)) add_cell<T>(sh, CR3, x, q3, st[A3 * fs + x]);
+  if (box4(M, i, j)) add_cell<T>(sh, CR4, x, q4, st[A4 * fs + x]);
+  __syncthreads();
+  const bool c1 = box1(M, i, j), c2 = box2(M, i, j);
+  T sxx = c1 ? g[SXX * fs + x] : T(0), syy = c1 ? g[SYY * fs + x] : T(0),
+    sxy = c2 ? g[SXY * fs + x] : T(0);
+  gather_stress<T>(M, S, sxx, syy, sxy);
+  if (c1) {
+    o[SXX * fs + x] = sxx;
+    o[SYY * fs + x] = syy;
   }
-  if (b4) {
-    const T gv = sh.g[VY][x];
-    const T rho_ = T(0.25) * (M.rho[x] + M.rho[ELIDX(i + 1, j)] + M.rho[ELIDX(i + 1, j + 1)] +
-                              M.rho[ELIDX(i, j + 1)]);
-    const T q = gv * M.dt / rho_;
-    T gm7 = q, gm8 = q;
-    gm7 += sh.g[M1 + 6][x];
-    sh.g[M1 + 6][x] = M.bxh[i - 1] * gm7;
-    gm8 += sh.g[M1 + 7][x];
-    sh.g[M1 + 7][x] = M.byh[j - 1] * gm8;
-    sh.tmp[D7][x] = (q + M.axh[i - 1] * gm7) / M.hx24;
-    sh.tmp[D8][x] = (q + M.ayh[j - 1] * gm8) / M.hy24;
-    sh.tmp[R4][x] = -gv * st[A4 * sh.fs + x] * M.dt / (rho_ * rho_) * T(0.25);
-  } else {
-    sh.g[M1 + 6][x] = T(0);
-    sh.g[M1 + 7][x] = T(0);
-  }
+  if (c2) o[SXY * fs + x] = sxy;
 }
 
-template <typename T>
-__device__ __forceinline__ T tld(const T* a, const ElModel<T>& M, int i, int j) {
-  return (i >= 0 && i <= M.NX + 1 && j >= 0 && j <= M.NY + 1) ? a[ELIDX(i, j)] : T(0);
-}
-
-// Adjoint 2 (stress cells): gather D5..D8 into the stress adjoints, then the
-// transposes of fw1 and fw2 (D1..D4, memory adjoints m1..m4, lambda/mu parts).
+// Adjoint of a step, stress cells -> velocity adjoints (transposes of fw1, fw2).
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
-k_el_adj2(ElModel<T> M, ElShot<T> one, int store_slot) {
-  const ElShot<T>& sh = one;
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  const int NX = M.NX, NY = M.NY;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t x = ELIDX(i, j);
-  const bool b1 = i >= 1 && i <= NX - 1 && j >= 2 && j <= NY;
-  const bool b2 = i >= 2 && i <= NX && j >= 1 && j <= NY - 1;
-  const T* const* D = sh.tmp;
-  const T gsxx = sh.g[SXX][x] + T(27) * D[D5][x] - T(27) * tld(D[D5], M, i + 1, j) -
-                 tld(D[D5], M, i - 1, j) + tld(D[D5], M, i + 2, j);
-  const T gsxy = sh.g[SXY][x] + T(27) * D[D6][x] - T(27) * tld(D[D6], M, i, j + 1) -
-                 tld(D[D6], M, i, j - 1) + tld(D[D6], M, i, j + 2) +
-                 T(27) * tld(D[D7], M, i - 1, j) - T(27) * D[D7][x] -
-                 tld(D[D7], M, i - 2, j) + tld(D[D7], M, i + 1, j);
-  const T gsyy = sh.g[SYY][x] + T(27) * tld(D[D8], M, i, j - 1) - T(27) * D[D8][x] -
-                 tld(D[D8], M, i, j - 2) + tld(D[D8], M, i, j + 1);
-  sh.g[SXX][x] = gsxx;
-  sh.g[SYY][x] = gsyy;
-  sh.g[SXY][x] = gsxy;
-  const T* st = sh.store + (int64_t)store_slot * NSTORE * sh.fs;
-  if (b1) {
-    const T lam_ = T(0.5) * (M.lam[ELIDX(i + 1, j)] + M.lam[x]);
-    const T mu_ = T(0.5) * (M.mu[ELIDX(i + 1, j)] + M.mu[x]);
-    const T lm = lam_ + T(2) * mu_;
-    const T e1 = st[E1 * sh.fs + x], e2 = st[E2 * sh.fs + x];
-    const T gE1 = M.dt * (lm * gsxx + lam_ * gsyy);
-    const T gE2 = M.dt * (lam_ * gsxx + lm * gsyy);
-    const T glm = M.dt * (e1 * gsxx + e2 * gsyy);
-    const T glam = M.dt * (e2 * gsxx + e1 * gsyy) + glm;
-    sh.tmp[GL1][x] = T(0.5) * glam;
-    sh.tmp[GM1][x] = glm;  // 0.5 * (2 glm) to each of mu[i], mu[i+1]
-    T gm1 = gE1, gm2 = gE2;
-    gm1 += sh.g[M1 + 0][x];
-    sh.g[M1 + 0][x] = M.bxh[i - 1] * gm1;
-    gm2 += sh.g[M1 + 1][x];
-    sh.g[M1 + 1][x] = M.byi[j - 1] * gm2;
-    sh.tmp[D1][x] = (gE1 + M.axh[i - 1] * gm1) / M.hx24;
-    sh.tmp[D2][x] = (gE2 + M.ayi[j - 1] * gm2) / M.hy24;
-  } else {
-    sh.g[M1 + 0][x] = T(0);
-    sh.g[M1 + 1][x] = T(0);
+k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+  __shared__ SendS<T> S;
+  const ElShot<T>& sh = shots[blockIdx.z];
+  ADS_EL_CELL(1);
+  const int64_t fs = sh.fs;
+  const T* g = sh.g[0] + (int64_t)pin * NF * fs;
+  T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  send_stress<T, true>(M, S, i0, j0, o, g, o, fs);
+  const T* st = sh.store + (int64_t)slot * NSTORE * fs;
+  if (box1(M, i, j)) {
+    const T sxx = o[SXX * fs + x], syy = o[SYY * fs + x];
+    const T e1 = st[E1 * fs + x], e2 = st[E2 * fs + x];
+    add_cell<T>(sh, CL, x, e1 + e2, sxx + syy);
+    add_cell<T>(sh, CM1, x, T(1), el_fma(e1, sxx, e2 * syy));
   }
-  if (b2) {
-    const T mu_ = T(0.5) * (M.mu[x] + M.mu[ELIDX(i, j + 1)]);
-    const T q = gsxy * mu_ * M.dt;
-    sh.tmp[GM2][x] = gsxy * st[E12 * sh.fs + x] * M.dt * T(0.5);
-    T gm3 = q, gm4 = q;
-    gm3 += sh.g[M1 + 2][x];
-    sh.g[M1 + 2][x] = M.bxi[i - 1] * gm3;
-    gm4 += sh.g[M1 + 3][x];
-    sh.g[M1 + 3][x] = M.byh[j - 1] * gm4;
-    sh.tmp[D3][x] = (q + M.axi[i - 1] * gm3) / M.hx24;
-    sh.tmp[D4][x] = (q + M.ayh[j - 1] * gm4) / M.hy24;
-  } else {
-    sh.g[M1 + 2][x] = T(0);
-    sh.g[M1 + 3][x] = T(0);
+  if (box2(M, i, j)) add_cell<T>(sh, CM2, x, o[SXY * fs + x], st[E12 * fs + x]);
+  __syncthreads();
+  const bool c3 = box3(M, i, j), c4 = box4(M, i, j);
+  T vx = c3 ? g[VX * fs + x] : T(0), vy = c4 ? g[VY * fs + x] : T(0);
+  gather_velocity<T>(M, S, vx, vy);
+  if (c3) o[VX * fs + x] = vx;
+  if (c4) o[VY * fs + x] = vy;
+}
+
+// The plans' tables from lambda, mu, rho, in FP64, rounded once; zero outside
+// the boxes.
+template <typename T>
+__global__ void k_el_tables(CellModel<T> M, T* __restrict__ tab, int64_t fs) {
+  const int64_t n = (int64_t)M.NX * M.NY;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = 1 + (int)(e / M.NY), j = 1 + (int)(e % M.NY), x = i * M.P + j + M.OFF;
+    const double dt = M.dtd;
+    auto at = [&](const T* p, int y) { return (double)p[y]; };
+    if (box1(M, i, j)) {
+      const double l = 0.5 * (at(M.lam, x + M.P) + at(M.lam, x)),
+                   u = at(M.mu, x + M.P) + at(M.mu, x);
+      tab[x] = (T)((l + u) * dt);
+      tab[fs + x] = (T)(l * dt);
+    }
+    if (box2(M, i, j)) tab[2 * fs + x] = (T)(0.5 * (at(M.mu, x) + at(M.mu, x + 1)) * dt);
+    if (box3(M, i, j)) tab[3 * fs + x] = (T)(dt / at(M.rho, x));
+    if (box4(M, i, j))
+      tab[4 * fs + x] = (T)(dt / (0.25 * (at(M.rho, x) + at(M.rho, x + M.P) +
+                                          at(M.rho, x + M.P + 1) + at(M.rho, x + 1))));
   }
 }
 
-// Adjoint 3 (velocity cells + parameters): gather D1..D4 into the velocity
-// adjoints and the lambda / mu / rho partials into the FP64 accumulators.
+// End of a segment (FP32 plans): accumulators += partials, partials = 0.
+__global__ void k_el_flush_cells(const ElShot<float>* __restrict__ shots) {
+  const ElShot<float>& sh = shots[blockIdx.y];
+  const int64_t n = NCACC * sh.fs;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    sh.cacc[e] += (double)sh.cacc32[e];
+    sh.cacc32[e] = 0.0f;
+  }
+}
+
+// The gradients from the shots' sums: lambda and mu take half of the stress
+// cells they are averaged into, rho its own vx cell and a quarter of the four
+// vy cells around it (d (dt / rho) = - dt / rho^2).
+template <typename T>
+__global__ void k_el_gather_cells(CellModel<T> M, const ElShot<T>* __restrict__ shots,
+                                  int nshots, double* __restrict__ gl, double* __restrict__ gm,
+                                  double* __restrict__ gr) {
+  const int64_t n = (int64_t)(M.NX + 2) * (M.NY + 2);
+  const double dt = M.dtd;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(e / (M.NY + 2)), j = (int)(e % (M.NY + 2)), P = M.P;
+    const int x = i * P + j + M.OFF;
+    double a = 0, b = 0, c = 0;
+    if (i >= 1 && i <= M.NX && j >= 1 && j <= M.NY) {
+      auto rho4 = [&](int y) {
+        return 0.25 * ((double)M.rho[y] + (double)M.rho[y + P] + (double)M.rho[y + P + 1] +
+                       (double)M.rho[y + 1]);
+      };
+      for (int s = 0; s < nshots; s++) {
+        const double* q = shots[s].cacc;
+        const int64_t fs = shots[s].fs;
+        a += q[CL * fs + x] + q[CL * fs + x - P];
+        b += q[CM1 * fs + x] + q[CM1 * fs + x - P] +
+             0.5 * (q[CM2 * fs + x] + q[CM2 * fs + x - 1]);
+        c += q[CR3 * fs + x] / (double)M.rho[x];
+        const double* r = q + CR4 * fs;
+        double d = 0;
+        if (box4(M, i, j)) d += r[x] / rho4(x);
+        if (box4(M, i - 1, j)) d += r[x - P] / rho4(x - P);
+        if (box4(M, i, j - 1)) d += r[x - 1] / rho4(x - 1);
+        if (box4(M, i - 1, j - 1)) d += r[x - P - 1] / rho4(x - P - 1);
+        c += 0.25 * d;
+      }
+    }
+    gl[e] = 0.5 * dt * a;
+    gm[e] = dt * b;
+    gr[e] = -c;
+  }
+}
+
+// ---- single-step operators: every cell of the padded grid is written
+
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
-k_el_adj3(ElModel<T> M, ElShot<T> one) {
-  const ElShot<T>& sh = one;
-  const int j = blockIdx.x * BX + threadIdx.x;
-  const int i = blockIdx.y * BY + threadIdx.y;
-  const int NX = M.NX, NY = M.NY;
-  if (i > NX + 1 || j > NY + 1) return;
-  const int64_t x = ELIDX(i, j);
-  const T* const* D = sh.tmp;
-  sh.g[VX][x] += T(27) * tld(D[D1], M, i - 1, j) - T(27) * D[D1][x] -
-                 tld(D[D1], M, i - 2, j) + tld(D[D1], M, i + 1, j) +
-                 T(27) * tld(D[D4], M, i, j - 1) - T(27) * D[D4][x] -
-                 tld(D[D4], M, i, j - 2) + tld(D[D4], M, i, j + 1);
-  sh.g[VY][x] += T(27) * D[D2][x] - T(27) * tld(D[D2], M, i, j + 1) -
-                 tld(D[D2], M, i, j - 1) + tld(D[D2], M, i, j + 2) + T(27) * D[D3][x] -
-                 T(27) * tld(D[D3], M, i + 1, j) - tld(D[D3], M, i - 1, j) +
-                 tld(D[D3], M, i + 2, j);
-  if (i >= 1 && i <= NX && j >= 1 && j <= NY) {
-    sh.glam[x] += (double)(D[GL1][x] + tld(D[GL1], M, i - 1, j));
-    sh.gmu[x] += (double)(D[GM1][x] + tld(D[GM1], M, i - 1, j) + D[GM2][x] +
-                          tld(D[GM2], M, i, j - 1));
-    sh.grho[x] += (double)(D[R4][x] + tld(D[R4], M, i - 1, j) + tld(D[R4], M, i - 1, j - 1) +
-                           tld(D[R4], M, i, j - 1));
+k_el_op_stress(CellModel<T> M, const T* __restrict__ f, T* __restrict__ o, int64_t fs, T* osxx,
+               T* osyy, T* osxy) {
+  // o: the step's output fields (null: the transpose wants the stresses alone)
+  ADS_EL_CELL(0);
+  if (i > M.NX + 1 || j > M.NY + 1) return;
+  T sxx = f[SXX * fs + x], syy = f[SYY * fs + x], sxy = f[SXY * fs + x];
+  if (box1(M, i, j)) {
+    T e1, e2, lm, la;
+    strain1<T, false>(M, i, j, x, f, fs, o, e1, e2);
+    mat1<T, false>(M, x, lm, la);
+    sxx = el_fma(lm, e1, el_fma(la, e2, sxx));
+    syy = el_fma(lm, e2, el_fma(la, e1, syy));
+  } else if (o) {
+    o[M1 * fs + x] = T(0);
+    o[(M1 + 1) * fs + x] = T(0);
+  }
+  if (box2(M, i, j)) {
+    const T e = strain2<T, false>(M, i, j, x, f, fs, o);
+    sxy = el_fma(mat2<T, false>(M, x), e, sxy);
+  } else if (o) {
+    o[(M1 + 2) * fs + x] = T(0);
+    o[(M1 + 3) * fs + x] = T(0);
+  }
+  osxx[x] = sxx;
+  osyy[x] = syy;
+  osxy[x] = sxy;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(BX* BY)
+k_el_op_velocity(CellModel<T> M, const T* __restrict__ f, T* o, int64_t fs) {
+  ADS_EL_CELL(0);
+  if (i > M.NX + 1 || j > M.NY + 1) return;
+  T vx = f[VX * fs + x], vy = f[VY * fs + x];
+  if (box3(M, i, j)) {
+    const T e = accel3<T, false>(M, i, j, x, o + SXX * fs, o + SXY * fs, f, fs, o);
+    vx = el_fma(mat3<T, false>(M, x), e, vx);
+  } else {
+    o[(M1 + 4) * fs + x] = T(0);
+    o[(M1 + 5) * fs + x] = T(0);
+  }
+  if (box4(M, i, j)) {
+    const T e = accel4<T, false>(M, i, j, x, o + SXY * fs, o + SYY * fs, f, fs, o);
+    vy = el_fma(mat4<T, false>(M, x), e, vy);
+  } else {
+    o[(M1 + 6) * fs + x] = T(0);
+    o[(M1 + 7) * fs + x] = T(0);
+  }
+  o[VX * fs + x] = vx;
+  o[VY * fs + x] = vy;
+}
+
+// Transpose, first half.  f: the step's input state; g: the output's gradient;
+// o: the input's gradient, whose fields M1..M1+2 hold the step's new stresses
+// until the second half overwrites them.  Writes sxx, syy, sxy, m5..m8 of o and
+// adds the density gradient.
+template <typename T, typename G>
+__global__ void __launch_bounds__(BX* BY)
+k_el_op_adj_stress(CellModel<T> M, const T* __restrict__ f, const T* __restrict__ g, T* o,
+                   int64_t fs, G* __restrict__ grho) {
+  __shared__ SendV<T> S;
+  __shared__ T r4[BY + 1][BX + 1];  // vy cells' density terms, one row and column before the tile
+  ADS_EL_CELL(0);
+  T q3, q4;
+  send_velocity<T, false>(M, S, i0, j0, g, o, fs, q3, q4);
+  const T *nsxx = o + M1 * fs, *nsyy = o + (M1 + 1) * fs, *nsxy = o + (M1 + 2) * fs;
+  auto r4_of = [&](int ii, int jj) -> T {
+    if (!box4(M, ii, jj)) return T(0);
+    const int64_t y = (int64_t)ii * P + jj + M.OFF;
+    const T b = mat4<T, false>(M, y);
+    const T e = accel4<T, false>(M, ii, jj, y, nsxy, nsyy, f, fs, (T*)nullptr);
+    return T(-0.25) * (g[VY * fs + y] * b * e) * (b * M.rdt);
+  };
+  r4[ty + 1][tx + 1] = r4_of(i, j);
+  const int t = ty * BX + tx;
+  if (t < BX + 1) r4[0][t] = r4_of(i0 - 1, j0 + t - 1);
+  else if (t >= 2 * BX && t < 2 * BX + BY) r4[t - 2 * BX + 1][0] = r4_of(i0 + t - 2 * BX, j0 - 1);
+  T r3 = T(0);
+  if (box3(M, i, j)) {
+    const T e = accel3<T, false>(M, i, j, x, nsxx, nsxy, f, fs, (T*)nullptr);
+    r3 = -(q3 * e) * (mat3<T, false>(M, x) * M.rdt);
+  } else if (i <= M.NX + 1 && j <= M.NY + 1) {
+    o[(M1 + 4) * fs + x] = T(0);
+    o[(M1 + 5) * fs + x] = T(0);
+  }
+  if (!box4(M, i, j) && i <= M.NX + 1 && j <= M.NY + 1) {
+    o[(M1 + 6) * fs + x] = T(0);
+    o[(M1 + 7) * fs + x] = T(0);
+  }
+  __syncthreads();
+  if (i > M.NX + 1 || j > M.NY + 1) return;
+  T sxx = g[SXX * fs + x], syy = g[SYY * fs + x], sxy = g[SXY * fs + x];
+  gather_stress<T>(M, S, sxx, syy, sxy);
+  o[SXX * fs + x] = sxx;
+  o[SYY * fs + x] = syy;
+  o[SXY * fs + x] = sxy;
+  if (i >= 1 && i <= M.NX && j >= 1 && j <= M.NY) {
+    const double d = (double)r3 + (double)(r4[ty + 1][tx + 1] + r4[ty][tx + 1] + r4[ty][tx] +
+                                           r4[ty + 1][tx]);
+    grho[x] += (G)d;
   }
 }
 
-#undef ELIDX
+// Transpose, second half: writes vx, vy, m1..m4 of o (its stresses come from the
+// first half) and adds the lambda and mu gradients.
+template <typename T, typename G>
+__global__ void __launch_bounds__(BX* BY)
+k_el_op_adj_velocity(CellModel<T> M, const T* __restrict__ f, const T* __restrict__ g, T* o,
+                     int64_t fs, G* __restrict__ glam, G* __restrict__ gmu) {
+  __shared__ SendS<T> S;
+  __shared__ T pl[BY + 1][BX], pm[BY + 1][BX], p2[BY][BX + 1];
+  ADS_EL_CELL(0);
+  send_stress<T, false>(M, S, i0, j0, o, g, o, fs);
+  // lambda and mu terms of the stress cells (one row before the tile) and of the
+  // sxy cells (one column before it)
+  auto terms1 = [&](int ii, int jj, T& a, T& b) {
+    a = b = T(0);
+    if (!box1(M, ii, jj)) return;
+    const int64_t y = (int64_t)ii * P + jj + M.OFF;
+    T e1, e2;
+    strain1<T, false>(M, ii, jj, y, f, fs, (T*)nullptr, e1, e2);
+    const T sxx = o[SXX * fs + y], syy = o[SYY * fs + y];
+    a = T(0.5) * M.dt * ((e1 + e2) * (sxx + syy));
+    b = M.dt * el_fma(e1, sxx, e2 * syy);
+  };
+  auto terms2 = [&](int ii, int jj) -> T {
+    if (!box2(M, ii, jj)) return T(0);
+    const int64_t y = (int64_t)ii * P + jj + M.OFF;
+    return T(0.5) * M.dt * (o[SXY * fs + y] * strain2<T, false>(M, ii, jj, y, f, fs, (T*)nullptr));
+  };
+  terms1(i, j, pl[ty + 1][tx], pm[ty + 1][tx]);
+  p2[ty][tx + 1] = terms2(i, j);
+  const int t = ty * BX + tx;
+  if (t < BX) terms1(i0 - 1, j0 + t, pl[0][t], pm[0][t]);
+  else if (t < BX + BY) p2[t - BX][0] = terms2(i0 + t - BX, j0 - 1);
+  if (i <= M.NX + 1 && j <= M.NY + 1) {
+    if (!box1(M, i, j)) {
+      o[M1 * fs + x] = T(0);
+      o[(M1 + 1) * fs + x] = T(0);
+    }
+    if (!box2(M, i, j)) {
+      o[(M1 + 2) * fs + x] = T(0);
+      o[(M1 + 3) * fs + x] = T(0);
+    }
+  }
+  __syncthreads();
+  if (i > M.NX + 1 || j > M.NY + 1) return;
+  T vx = g[VX * fs + x], vy = g[VY * fs + x];
+  gather_velocity<T>(M, S, vx, vy);
+  o[VX * fs + x] = vx;
+  o[VY * fs + x] = vy;
+  if (i >= 1 && i <= M.NX && j >= 1 && j <= M.NY) {
+    glam[x] += (G)(double)(pl[ty + 1][tx] + pl[ty][tx]);
+    gmu[x] += (G)(double)(pm[ty + 1][tx] + pm[ty][tx] + p2[ty][tx + 1] + p2[ty][tx]);
+  }
+}
+#undef ADS_EL_CELL
+
+template <typename T>
+CellModel<T> make_cells(int NX, int NY, int64_t P, int off, double dt, double dx, double dy,
+                        const T* lam, const T* mu, const T* rho) {
+  CellModel<T> M{};
+  M.lam = lam;
+  M.mu = mu;
+  M.rho = rho;
+  M.dt = (T)dt;
+  M.rdt = (T)(1.0 / dt);
+  M.dtd = dt;
+  M.x27 = (T)(27.0 / (24 * dx));
+  M.x1 = (T)(1.0 / (24 * dx));
+  M.y27 = (T)(27.0 / (24 * dy));
+  M.y1 = (T)(1.0 / (24 * dy));
+  M.NX = NX;
+  M.NY = NY;
+  M.OFF = off;
+  M.P = (int)P;
+  return M;
+}
 
 // ---------------------------------------------------------------------------
 // Row-streaming kernels for the plans (the fused forward step and the three
@@ -2242,6 +2714,15 @@ struct ElPlanBase {
 
 namespace {
 
+// FP32 plans step with the one-thread-per-cell kernels up to this many cells over
+// all shots: below it a step's time is the latency of one warp's chain, which a
+// strip of rows makes 8 rows long and more; above it the row kernels' single read
+// of each field wins.  us per forward step / forward and adjoint step, cell against
+// row kernels: 80 k cells 10.7 / 24.2 against 20.9 / 54.3, 360 k 16.8 / 40.7 against
+// 21.1 / 56.4, 720 k 24.2 / 61.6 against 24.0 / 64.9, 1.44 M 46.1 / 119 against
+// 40.5 / 104.
+constexpr int64_t kCellMax32 = 600000;
+
 template <typename T>
 struct ElPlan final : ElPlanBase {
   ads_elastic_config cfg{};
@@ -2277,6 +2758,14 @@ struct ElPlan final : ElPlanBase {
   int ncola = 0, rows_a = 0, nwta = 0, jsha = 0, isha = 0;
   int nwka[4] = {}, owka[4] = {};
   int* d_wla = nullptr;
+  // one-thread-per-cell kernels: forward steps (cellf) and the reverse sweep's
+  // adjoint steps (cella), their tables and per-shot sums
+  bool cellf = false, cella = false;
+  CellModel<T> C{};
+  T* d_tab = nullptr;
+  dim3 grid_cells() const {
+    return dim3((unsigned)div_up(NX, BY), (unsigned)div_up(NY, BX), (unsigned)nshots);
+  }
   // host copies: the packed CPML rows and the item lists of the current tiling
   std::vector<T> hprof;
   std::vector<int> wl_host, wlf_host, wla_host;
@@ -2286,8 +2775,9 @@ struct ElPlan final : ElPlanBase {
   int upload_lists(cudaStream_t st);
   int autotune(cudaStream_t st, int rw_min, int rf_min);
   static int par(int n) { return n & 1; }
-  int apar(int n) const { return fused ? n & 1 : 0; }  // adjoint buffer of slot n
+  int apar(int n) const { return fused || cella ? n & 1 : 0; }  // adjoint buffer of slot n
   int adj_launches() const {
+    if (cella) return 2;
     if (fused) return (nwka[0] > 0) + (nwka[1] > 0) + (nwka[2] > 0) + (nwka[3] > 0);
     return group_launches(kSplitAdj1, nw_in, nw_pm) +
            2 * group_launches(kSplitAdj23, nw_in, nw_pm);
@@ -2300,6 +2790,7 @@ struct ElPlan final : ElPlanBase {
     return (split ? 2 : 1) * ((n_in > 0) + (n_pm > 0));
   }
   int fwd_launches() const {
+    if (cellf) return 2;
     return (nwk[0] > 0) + (nwk[1] > 0) + (nwk[2] > 0) + (nwk[3] > 0);
   }
   // fn(stream, kind) for each kind with items (nk[kind] > 0), concurrently
@@ -2354,6 +2845,7 @@ struct ElPlan final : ElPlanBase {
 
   int create(const ads_elastic_config& c, const ads_elastic_shot* shots, int64_t ns,
              cudaStream_t st);
+  int step_kernels(cudaStream_t st, int n, bool store, int slot);
   int step(cudaStream_t st, int n, bool store, int slot, bool record);
   int adjoint_step(cudaStream_t st, int slot, int n);
   int issue_forward(cudaStream_t st, int64_t* count);
@@ -2389,9 +2881,14 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   // would not leave room for a plan on the device anyway)
   ADS_REQUIRE((int64_t)(c.NX + 2) * grid_pitch(c.NY) < (int64_t(1) << 31),
               "(NX + 2) x pitch must stay below 2^31 elements");
-  // automatic (0): the fused adjoint for FP32 plans, the three passes for FP64
-  // plans (their fused kernel runs out of registers: measured 1.5x slower)
+  // automatic (0): the cell kernels for FP64 plans and small FP32 plans, the fused
+  // adjoint for larger FP32 plans; with rows_per_warp set, the fused adjoint for
+  // FP32 and the three passes for FP64 plans (whose fused kernel runs out of
+  // registers: measured 1.5x slower)
   fused = c.adjoint_passes == 1 || (c.adjoint_passes == 0 && sizeof(T) == 4);
+  cellf = cella = c.adjoint_passes == 0 && c.rows_per_warp == 0 &&
+                  (sizeof(T) == 8 || (int64_t)c.NX * c.NY * ns <= kCellMax32);
+  if (cella) fused = false;
   if (fused)
     if (int e = el_fadj_prepare<T>()) return e;
   nshots = (int)ns;
@@ -2491,7 +2988,7 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   }
   // ---- layout
   struct Off {
-    size_t state, g, tmp, store, ckpt, acc, acc32, srcv, scell, stype, sdual, rcell, rtype, sptr,
+    size_t state, g, tmp, store, ckpt, acc, acc32, cacc, cacc32, srcv, scell, stype, sdual, rcell, rtype, sptr,
         rptr, gptr, sgptr;
   };
   std::vector<Off> o(ns);
@@ -2509,15 +3006,18 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   zero_fwd_len = used - fwd0;
   const size_t adj0 = used;
   for (int s = 0; s < ns; s++) {
-    o[s].g = take((fused ? 2 : 1) * NF * F);  // the fused adjoint alternates two buffers
-    o[s].acc = take(3 * sizeof(double) * fs);
-    o[s].acc32 = sizeof(T) == 4 ? take(3 * sizeof(float) * fs) : 0;
+    // the fused adjoint and the cell kernels alternate two buffers
+    o[s].g = take((fused || cella ? 2 : 1) * NF * F);
+    o[s].acc = take(cella ? 0 : 3 * sizeof(double) * fs);
+    o[s].acc32 = sizeof(T) == 4 && !cella ? take(3 * sizeof(float) * fs) : 0;
+    o[s].cacc = take(cella ? NCACC * sizeof(double) * fs : 0);
+    o[s].cacc32 = take(cella && sizeof(T) == 4 ? NCACC * sizeof(float) * fs : 0);
   }
   zero_adj_off = adj0;
   zero_adj_len = used - adj0;
   for (int s = 0; s < ns; s++) {
     const ads_elastic_shot& h = shots[s];
-    o[s].tmp = fused ? 0 : take(NTMP * F);  // D1..D8, R4, GL1, GM1, GM2 of the three passes
+    o[s].tmp = fused || cella ? 0 : take(NTMP * F);  // D1..D8, R4, GL1, GM1, GM2 of the three passes
     o[s].ckpt = take((size_t)nseg * NF * F);
     o[s].srcv = take(sizeof(T) * std::max<int64_t>(NSTEP * h.nsrc, 1));
     o[s].scell = take(sizeof(int64_t) * std::max<int64_t>(h.nsrc, 1));
@@ -2531,6 +3031,7 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
     o[s].sgptr = take(sizeof(T*) * std::max<int64_t>(h.nsrc, 1));
   }
   const size_t model_o = take(3 * F);
+  const size_t tab_o = take(cellf || cella ? 5 * F : 0);
   const size_t prof_o = take(sizeof(T) * (4 * NX + 4 * NY));
   const size_t resid_o = take(sizeof(T) * std::max<int64_t>(trace_total, 1));
   const size_t part_o = take(sizeof(double) * kBlocks);
@@ -2603,6 +3104,21 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
                            cudaMemcpyHostToDevice, st));
   M = make_model<T>(NX, NY, P, JOFF, c.dt, c.dx, c.dy, d_lam, d_mu, d_rho,
                     (const T*)(pool + prof_o));
+  C = make_cells<T>(NX, NY, P, JOFF, c.dt, c.dx, c.dy, d_lam, d_mu, d_rho);
+  C.axi = M.axi;
+  C.axh = M.axh;
+  C.bxi = M.bxi;
+  C.bxh = M.bxh;
+  C.ayi = M.ayi;
+  C.ayh = M.ayh;
+  C.byi = M.byi;
+  C.byh = M.byh;
+  d_tab = (T*)(pool + tab_o);
+  C.lm = d_tab;
+  C.la = d_tab + fs;
+  C.m2 = d_tab + 2 * fs;
+  C.b3 = d_tab + 3 * fs;
+  C.b4 = d_tab + 4 * fs;
   // shots
   std::vector<ElShot<T>> hs(ns);
   srcv_dev.assign(ns, nullptr);
@@ -2613,10 +3129,12 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
     ElShot<T>& d = hs[s];
     for (int f = 0; f < NF; f++) {
       d.f[f] = (T*)(pool + o[s].state) + f * fs;
-      d.fin[f] = d.f[f];
       d.g[f] = (T*)(pool + o[s].g) + f * fs;
     }
-    for (int k = 0; k < NTMP; k++) d.tmp[k] = fused ? nullptr : (T*)(pool + o[s].tmp) + k * fs;
+    for (int k = 0; k < NTMP; k++)
+      d.tmp[k] = fused || cella ? nullptr : (T*)(pool + o[s].tmp) + k * fs;
+    d.cacc = cella ? (double*)(pool + o[s].cacc) : nullptr;
+    d.cacc32 = cella && sizeof(T) == 4 ? (float*)(pool + o[s].cacc32) : nullptr;
     d.store = (T*)(pool + o[s].store);
     d.ckpt = (T*)(pool + o[s].ckpt);
     d.glam = (double*)(pool + o[s].acc);
@@ -2728,8 +3246,9 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
     issue_reverse(nullptr, &n);
     nR = n;
   }
-  launches_fwd = 3 + nF;
-  launches_grad = 3 + nF + 2 + nR + 1;
+  const int np = 3 + (cellf || cella ? 1 : 0);  // casts, tables
+  launches_fwd = np + nF;
+  launches_grad = np + nF + 2 + nR + 1;
   if (c.use_graph) {
     ADS_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     for (int which = 0; which < 2; which++) {
@@ -2890,6 +3409,8 @@ int ElPlan<T>::autotune(cudaStream_t st, int rw_min, int rf_min) {
   int rc = ADS_OK;
   int best_f = rows_f, best_w = rows_w;
   float best = 1e30f;
+  const bool cells = cellf;
+  cellf = false;  // the row kernels first
   for (int rf : {12, 16, 20, 24, 32}) {
     if (rf < rf_min || rf > NX) continue;
     build_lists(best_w, rf, rows_a);
@@ -2900,6 +3421,12 @@ int ElPlan<T>::autotune(cudaStream_t st, int rw_min, int rf_min) {
       best_f = rf;
     }
   }
+  if (cells && rc == ADS_OK) {  // then the cell kernels, where this plan has them
+    float ms = 0.f;
+    cellf = true;
+    rc = timed(false, ms);
+    cellf = ms < best;
+  }
   best = 1e30f;
   int best_a = rows_a;
   // the fused adjoint: tile heights as the fused step's; the three passes:
@@ -2907,7 +3434,7 @@ int ElPlan<T>::autotune(cudaStream_t st, int rw_min, int rf_min) {
   const std::vector<int> cand =
       fused ? std::vector<int>{12, 16, 20, 24, 32} : std::vector<int>{6, 8, 12, 16, 24, 32};
   for (int rw : cand) {
-    if (rc != ADS_OK) break;
+    if (rc != ADS_OK || cella) break;
     if ((!fused && rw < rw_min) || rw > NX) continue;  // (the lists hold >= 12-row tiles)
     if (fused) {
       build_lists(best_w, best_f, rw);
@@ -2988,6 +3515,14 @@ int ElPlan<T>::kinds(cudaStream_t st, const int* nk, F&& fn) {
 // other), or the three passes in place.
 template <typename T>
 int ElPlan<T>::adjoint_step(cudaStream_t st, int slot, int n) {
+  if (cella) {
+    const dim3 b(BX, BY);
+    k_el_cell_adj_stress<T><<<grid_cells(), b, 0, st>>>(C, d_shots, apar(n), slot);
+    ADS_LAUNCHED(1);
+    k_el_cell_adj_velocity<T><<<grid_cells(), b, 0, st>>>(C, d_shots, apar(n), slot);
+    ADS_LAUNCHED(1);
+    return ADS_OK;
+  }
   if (fused)
     return kinds(st, nwka, [&](cudaStream_t s, int k) {
       el_fadj<T>(k, grid_rows(nwka[k]), s, M, d_shots, d_wla + owka[k], ncola, rows_a, nwka[k],
@@ -3013,13 +3548,26 @@ int ElPlan<T>::adjoint_step(cudaStream_t st, int slot, int n) {
 // One forward step n (slot n-1 in buffer par(n-1) -> slot n in buffer
 // par(n)) for every shot.
 template <typename T>
+int ElPlan<T>::step_kernels(cudaStream_t st, int n, bool store, int slot) {
+  const int sl = store ? slot : 0, pin = par(n - 1);
+  if (!cellf)
+    return kinds(st, nwk, [&](cudaStream_t s, int k) {
+      el_step<T>(store, k, grid_rows(nwk[k]), s, M, d_shots, d_wlf + owk[k], ncolf, rows_f,
+                 nwk[k], sl, pin, jsh, ish);
+    });
+  const dim3 g = grid_cells(), b(BX, BY);
+  if (store) k_el_cell_stress<T, true><<<g, b, 0, st>>>(C, d_shots, pin, sl);
+  else k_el_cell_stress<T, false><<<g, b, 0, st>>>(C, d_shots, pin, sl);
+  ADS_LAUNCHED(1);
+  if (store) k_el_cell_velocity<T, true><<<g, b, 0, st>>>(C, d_shots, pin, sl);
+  else k_el_cell_velocity<T, false><<<g, b, 0, st>>>(C, d_shots, pin, sl);
+  ADS_LAUNCHED(1);
+  return ADS_OK;
+}
+
+template <typename T>
 int ElPlan<T>::step(cudaStream_t st, int n, bool store, int slot, bool record) {
-  const int sl = store ? slot : 0;
-  if (int e = kinds(st, nwk, [&](cudaStream_t s, int k) {
-        el_step<T>(store, k, grid_rows(nwk[k]), s, M, d_shots, d_wlf + owk[k], ncolf, rows_f,
-                   nwk[k], sl, par(n - 1), jsh, ish);
-      }))
-    return e;
+  if (int e = step_kernels(st, n, store, slot)) return e;
   k_el_src_rcv<T><<<nshots, rcv_threads(), 0, st>>>(d_shots, n, NSTEP + 1, record ? 1 : 0,
                                                     par(n), 1);
   ADS_LAUNCHED(1);
@@ -3091,7 +3639,8 @@ int ElPlan<T>::issue_reverse(cudaStream_t st, int64_t* count) {
       }
     }
     if constexpr (sizeof(T) == 4) {
-      k_el_flush_acc<<<dim3(256, nshots), 256, 0, st>>>(d_shots, fs);
+      if (cella) k_el_flush_cells<<<dim3(256, nshots), 256, 0, st>>>(d_shots);
+      else k_el_flush_acc<<<dim3(256, nshots), 256, 0, st>>>(d_shots, fs);
       ADS_LAUNCHED(1);
     }
   }
@@ -3108,6 +3657,10 @@ int ElPlan<T>::prep(const double* l, const double* m, const double* r, cudaStrea
   ADS_LAUNCHED(1);
   k_el_cast<T><<<g, 256, 0, st>>>(d_rho, r, NX, NY, P, JOFF);
   ADS_LAUNCHED(1);
+  if (cellf || cella) {
+    k_el_tables<T><<<g, 256, 0, st>>>(C, d_tab, fs);
+    ADS_LAUNCHED(1);
+  }
   return ADS_OK;
 }
 
@@ -3147,7 +3700,8 @@ int ElPlan<T>::gradient(const double* l, const double* m, const double* r, const
     return e;
   }
   const unsigned g = (unsigned)std::min<int64_t>(div_up((int64_t)(NX + 2) * (NY + 2), 256), 4096);
-  k_el_gather_grads<T><<<g, 256, 0, st>>>(d_shots, nshots, NX, NY, P, JOFF, gl, gm, gr);
+  if (cella) k_el_gather_cells<T><<<g, 256, 0, st>>>(C, d_shots, nshots, gl, gm, gr);
+  else k_el_gather_grads<T><<<g, 256, 0, st>>>(d_shots, nshots, NX, NY, P, JOFF, gl, gm, gr);
   ADS_LAUNCHED(1);
   if (tr_out)
     ADS_CUDA(cudaMemcpyAsync(tr_out, d_traces, sizeof(T) * trace_total,
@@ -3196,28 +3750,23 @@ int ElPlan<T>::profile(const double* l, const double* m, const double* r, double
   auto wl = [&](bool in) { return in ? d_wl : d_wl + nw_in; };
   auto nw = [&](bool in) { return in ? nw_in : nw_pm; };
   for (int k = 0; k < 2; k++)
-    run(k, [&] {
-      kinds(st, nwk, [&](cudaStream_t s, int kd) {
-        el_step<T>(k == 1, kd, grid_rows(nwk[kd]), s, M, d_shots, d_wlf + owk[kd], ncolf,
-                   rows_f, nwk[kd], 0, 0, jsh, ish);
-      });
-    });
-  if (fused) {  // the fused adjoint in slot 2; slots 3 and 4 stay empty
+    run(k, [&] { step_kernels(st, 1, k == 1, 0); });
+  if (fused || cella) {  // the whole adjoint step in slot 2; slots 3 and 4 stay empty
     run(2, [&] { adjoint_step(st, 0, 1); });
     out[6] = out[8] = 0.0;
     out[7] = out[9] = cells;
   }
-  if (!fused) run(2, [&] {
+  if (!fused && !cella) run(2, [&] {
     group(st, kSplitAdj1, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
       el_adj1<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
     });
   });
-  if (!fused) run(3, [&] {
+  if (!fused && !cella) run(3, [&] {
     group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
       el_adj2<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
     });
   });
-  if (!fused) run(4, [&] {
+  if (!fused && !cella) run(4, [&] {
     group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
       el_adj3<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in));
     });
@@ -3242,17 +3791,22 @@ int ElPlan<T>::profile(const double* l, const double* m, const double* r, double
 // the caller's precision: T = double for the f64 entry points, float for f32.
 // ---------------------------------------------------------------------------
 
-// Profile rows ax, bx, ay, by (2*NX / 2*NY, row 0 integer grid, row 1 half
-// grid) copied into the packed layout the kernels index.
+// The profile rows ax, bx (2*NX) and ay, by (2*NY), row 0 the integer grid and row 1
+// the half grid, as the kernels index them.
 template <typename T>
-int el_copy_profiles(T* prof, const T* ax, const T* bx, const T* ay, const T* by, int64_t NX,
-                     int64_t NY, cudaStream_t st) {
-  ADS_CUDA(cudaMemcpyAsync(prof, ax, sizeof(T) * 2 * NX, cudaMemcpyDeviceToDevice, st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 2 * NX, bx, sizeof(T) * 2 * NX, cudaMemcpyDeviceToDevice, st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 4 * NX, ay, sizeof(T) * 2 * NY, cudaMemcpyDeviceToDevice, st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 4 * NX + 2 * NY, by, sizeof(T) * 2 * NY,
-                           cudaMemcpyDeviceToDevice, st));
-  return ADS_OK;
+void set_profiles(CellModel<T>& M, const T* ax, const T* bx, const T* ay, const T* by) {
+  M.axi = ax;
+  M.axh = ax + M.NX;
+  M.bxi = bx;
+  M.bxh = bx + M.NX;
+  M.ayi = ay;
+  M.ayh = ay + M.NY;
+  M.byi = by;
+  M.byh = by + M.NY;
+}
+
+inline dim3 op_grid(int64_t NX, int64_t NY) {
+  return dim3((unsigned)div_up(NX + 2, BY), (unsigned)div_up(NY + 2, BX));
 }
 
 template <typename T>
@@ -3269,25 +3823,13 @@ int el_step_fwd(const T* state_in, T* state_out, const T* lambda, const T* mu, c
               "invalid source arrays");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t N = (NX + 2) * (NY + 2);
-  // profiles, repacked on the device-side scratch
-  T* prof = nullptr;
-  const size_t prof_n = 4 * NX + 4 * NY;
-  ADS_CUDA(cudaMallocAsync((void**)&prof, sizeof(T) * prof_n, st));
-  if (int e = el_copy_profiles<T>(prof, ax, bx, ay, by, NX, NY, st)) {
-    cudaFreeAsync(prof, st);
-    return e;
-  }
-  ElModel<T> M = make_model<T>((int)NX, (int)NY, NY + 2, 0, dt, dx, dy, lambda, mu, rho, prof);
-  ElShot<T> one{};
-  for (int f = 0; f < NF; f++) {
-    one.fin[f] = state_in + f * N;
-    one.f[f] = state_out + f * N;
-  }
-  one.fs = N;
-  dim3 grd((unsigned)div_up(NY + 2, BX), (unsigned)div_up(NX + 2, BY), 1);
-  k_el_stress<T, false><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
+  CellModel<T> M = make_cells<T>((int)NX, (int)NY, NY + 2, 0, dt, dx, dy, lambda, mu, rho);
+  set_profiles<T>(M, ax, bx, ay, by);
+  const dim3 grd = op_grid(NX, NY), blk(BX, BY);
+  k_el_op_stress<T><<<grd, blk, 0, st>>>(M, state_in, state_out, N, state_out + SXX * N,
+                                         state_out + SYY * N, state_out + SXY * N);
   ADS_LAUNCHED(1);
-  k_el_velocity<T, false><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
+  k_el_op_velocity<T><<<grd, blk, 0, st>>>(M, state_in, state_out, N);
   ADS_LAUNCHED(1);
   if (nsrc > 0) {
     Fields5<T> f5{{state_out, state_out + N, state_out + 2 * N, state_out + 3 * N,
@@ -3295,25 +3837,42 @@ int el_step_fwd(const T* state_in, T* state_out, const T* lambda, const T* mu, c
     k_el_step_src<T><<<1, 32, 0, st>>>(f5, srci, srcj, srctype, srcv, nsrc, (int)NX, (int)NY);
     ADS_LAUNCHED(1);
   }
-  ADS_CUDA(cudaFreeAsync(prof, st));
   return ADS_OK;
 }
 
-// out[e] += (G) acc[e]: the f32 transpose accumulates its parameter gradients in
-// FP64 scratch (as the kernels do) and adds them to the caller's FP32 arrays.
-template <typename G>
-__global__ void k_el_add_grad(G* __restrict__ out, const double* __restrict__ acc, int64_t n) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * blockDim.x)
-    out[e] += (G)acc[e];
+// The transpose's three kernels; state_in must not overlap grad_in (whose memory
+// fields carry the step's new stresses between them).
+template <typename T, typename G>
+int el_bwd_kernels(const T* state_in, const T* grad_out, T* grad_in, G* grad_lambda, G* grad_mu,
+                   G* grad_rho, const T* lambda, const T* mu, const T* rho, const T* ax,
+                   const T* bx, const T* ay, const T* by, double dt, double dx, double dy,
+                   int64_t NX, int64_t NY, cudaStream_t st) {
+  const int64_t N = (NX + 2) * (NY + 2);
+  CellModel<T> M = make_cells<T>((int)NX, (int)NY, NY + 2, 0, dt, dx, dy, lambda, mu, rho);
+  set_profiles<T>(M, ax, bx, ay, by);
+  const dim3 grd = op_grid(NX, NY), blk(BX, BY);
+  k_el_op_stress<T><<<grd, blk, 0, st>>>(M, state_in, (T*)nullptr, N, grad_in + M1 * N,
+                                         grad_in + (M1 + 1) * N, grad_in + (M1 + 2) * N);
+  ADS_LAUNCHED(1);
+  k_el_op_adj_stress<T, G><<<grd, blk, 0, st>>>(M, state_in, grad_out, grad_in, N, grad_rho);
+  ADS_LAUNCHED(1);
+  k_el_op_adj_velocity<T, G>
+      <<<grd, blk, 0, st>>>(M, state_in, grad_out, grad_in, N, grad_lambda, grad_mu);
+  ADS_LAUNCHED(1);
+  return ADS_OK;
 }
 
-template <typename T, typename G>
-int el_step_bwd(const T* state_in, const T* grad_out, T* grad_in, G* grad_lambda, G* grad_mu,
-                G* grad_rho, const T* lambda, const T* mu, const T* rho, const T* ax,
+template <typename T>
+bool overlap13(const T* a, const T* b, int64_t N) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b, n = (uintptr_t)(NF * N * sizeof(T));
+  return x < y + n && y < x + n;
+}
+
+template <typename T>
+int el_step_bwd(const T* state_in, const T* grad_out, T* grad_in, T* grad_lambda, T* grad_mu,
+                T* grad_rho, const T* lambda, const T* mu, const T* rho, const T* ax,
                 const T* bx, const T* ay, const T* by, double dt, double dx, double dy,
                 int64_t NX, int64_t NY, ads_stream_t stream) {
-  constexpr bool kDirect = std::is_same<G, double>::value;  // accumulate into the caller's
   if (int e = require_device()) return e;
   ADS_REQUIRE(NX >= 4 && NY >= 4 && NX < (1 << 24) && NY < (1 << 24), "NX, NY out of range");
   ADS_REQUIRE(state_in && grad_out && grad_in && grad_lambda && grad_mu && grad_rho &&
@@ -3322,64 +3881,23 @@ int el_step_bwd(const T* state_in, const T* grad_out, T* grad_in, G* grad_lambda
   ADS_REQUIRE(grad_in != grad_out, "grad_in must not alias grad_out");
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t N = (NX + 2) * (NY + 2);
-  const size_t prof_n = 4 * NX + 4 * NY;
-  // scratch: profiles, forward output state, per-step store, adjoint temps
-  // (and, for FP32 outputs, three FP64 accumulators)
-  const size_t n_scr = prof_n + (size_t)(NF + NSTORE + NTMP) * N;
-  const size_t n_acc = kDirect ? 0 : (size_t)3 * N;
-  char* scratch = nullptr;
-  const size_t b_scr = sizeof(T) * ((n_scr + 1) & ~size_t(1));
-  ADS_CUDA(cudaMallocAsync((void**)&scratch, b_scr + sizeof(double) * n_acc, st));
-  ADS_CUDA(cudaMemsetAsync(scratch, 0, b_scr + sizeof(double) * n_acc, st));
-  T* prof = (T*)scratch;
-  if (int e = el_copy_profiles<T>(prof, ax, bx, ay, by, NX, NY, st)) {
-    cudaFreeAsync(scratch, st);
-    return e;
+  // the state is read to the end: a caller that takes the gradient into its own
+  // array gets a copy of it
+  T* copy = nullptr;
+  if (overlap13<T>(state_in, grad_in, N)) {
+    ADS_CUDA(cudaMallocAsync((void**)&copy, sizeof(T) * NF * N, st));
+    cudaError_t e =
+        cudaMemcpyAsync(copy, state_in, sizeof(T) * NF * N, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) {
+      cudaFreeAsync(copy, st);
+      ADS_CUDA(e);
+    }
   }
-  T* fout = prof + prof_n;
-  T* store = fout + NF * N;
-  T* tmp = store + NSTORE * N;
-  double* acc = (double*)(scratch + b_scr);
-  ElModel<T> M = make_model<T>((int)NX, (int)NY, NY + 2, 0, dt, dx, dy, lambda, mu, rho, prof);
-  ElShot<T> one{};
-  for (int f = 0; f < NF; f++) {
-    one.fin[f] = state_in + f * N;
-    one.f[f] = fout + f * N;
-    one.g[f] = grad_in + f * N;
-  }
-  for (int k = 0; k < NTMP; k++) one.tmp[k] = tmp + k * N;
-  one.store = store;
-  one.fs = N;
-  if constexpr (kDirect) {
-    one.glam = grad_lambda;
-    one.gmu = grad_mu;
-    one.grho = grad_rho;
-  } else {
-    one.glam = acc;
-    one.gmu = acc + N;
-    one.grho = acc + 2 * N;
-  }
-  dim3 grd((unsigned)div_up(NY + 2, BX), (unsigned)div_up(NX + 2, BY), 1);
-  k_el_stress<T, true><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_velocity<T, true><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  ADS_CUDA(cudaMemcpyAsync(grad_in, grad_out, sizeof(T) * NF * N, cudaMemcpyDeviceToDevice, st));
-  k_el_adj1<T><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_adj2<T><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_adj3<T><<<grd, dim3(BX, BY), 0, st>>>(M, one);
-  ADS_LAUNCHED(1);
-  if constexpr (!kDirect) {
-    const unsigned nb = (unsigned)std::min<int64_t>(div_up(N, 256), 4096);
-    k_el_add_grad<G><<<nb, 256, 0, st>>>(grad_lambda, acc, N);
-    k_el_add_grad<G><<<nb, 256, 0, st>>>(grad_mu, acc + N, N);
-    k_el_add_grad<G><<<nb, 256, 0, st>>>(grad_rho, acc + 2 * N, N);
-    ADS_LAUNCHED(3);
-  }
-  ADS_CUDA(cudaFreeAsync(scratch, st));
-  return ADS_OK;
+  int rc = el_bwd_kernels<T, T>(copy ? copy : state_in, grad_out, grad_in, grad_lambda, grad_mu,
+                                grad_rho, lambda, mu, rho, ax, bx, ay, by, dt, dx, dy, NX, NY,
+                                st);
+  if (copy) ADS_CUDA(cudaFreeAsync(copy, st));
+  return rc;
 }
 
 }  // namespace
@@ -3425,7 +3943,7 @@ int ads_elastic_step_bwd_f64(const double* state_in, const double* grad_out, dou
                              const double* ax, const double* bx, const double* ay,
                              const double* by, double dt, double dx, double dy, int64_t NX,
                              int64_t NY, ads_stream_t stream) {
-  return el_step_bwd<double, double>(state_in, grad_out, grad_in, grad_lambda, grad_mu,
+  return el_step_bwd<double>(state_in, grad_out, grad_in, grad_lambda, grad_mu,
                                      grad_rho, lambda, mu, rho, ax, bx, ay, by, dt, dx, dy, NX,
                                      NY, stream);
 }
@@ -3436,7 +3954,7 @@ int ads_elastic_step_bwd_f32(const float* state_in, const float* grad_out, float
                              const float* ax, const float* bx, const float* ay,
                              const float* by, double dt, double dx, double dy, int64_t NX,
                              int64_t NY, ads_stream_t stream) {
-  return el_step_bwd<float, float>(state_in, grad_out, grad_in, grad_lambda, grad_mu, grad_rho,
+  return el_step_bwd<float>(state_in, grad_out, grad_in, grad_lambda, grad_mu, grad_rho,
                                    lambda, mu, rho, ax, bx, ay, by, dt, dx, dy, NX, NY,
                                    stream);
 }
@@ -3452,17 +3970,15 @@ int ads_elastic_step_bwd_f32(const float* state_in, const float* grad_out, float
 // cudaMalloc bypasses its memory accounting (and can fail once the framework
 // has reserved the device), and time-critical loops that must never enter the
 // CUDA allocator, whose calls can synchronise the device and take unbounded
-// time.  For them the scratch this step needs (forward output state, per-step
-// strains, adjoint temporaries and the packed CPML rows) lives in one fixed
-// array in device global memory, compiled into the library.  Every GPU that
-// loads the library holds the array (34 x 65536 doubles, about 17.8 MB) until
-// the process exits.
+// time.  The kernels themselves need no scratch; only a call whose grad_in
+// overlaps state_in takes a copy of the state, into one fixed array in device
+// global memory, compiled into the library.  Every GPU that loads the library
+// holds the array (13 x 65536 doubles, about 6.8 MB) until the process exits.
 // ---------------------------------------------------------------------------
 namespace {
 
 constexpr int64_t kNoAllocMaxCells = 65536;  // (NX+2)*(NY+2) limit
-constexpr size_t kNoAllocDoubles = (size_t)(NF + NSTORE + NTMP + 4) * kNoAllocMaxCells;
-static __device__ __align__(256) double g_el_bwd_scratch[kNoAllocDoubles];
+static __device__ __align__(256) double g_el_bwd_scratch[(size_t)NF * kNoAllocMaxCells];
 
 std::mutex g_noalloc_mu;
 double* g_noalloc_ptr[128] = {};  // device address of g_el_bwd_scratch, per device
@@ -3512,52 +4028,17 @@ int ads_elastic_step_bwd_f64_noalloc(const double* state_in, const double* grad_
                   lambda && mu && rho && ax && bx && ay && by,
               "null pointer argument");
   ADS_REQUIRE(grad_in != grad_out, "grad_in must not alias grad_out");
-  double* scratch = nullptr;
-  if (int e = noalloc_scratch(&scratch)) return e;
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t prof_n = 4 * NX + 4 * NY;
-  const size_t n_scr = prof_n + (size_t)(NF + NSTORE + NTMP) * N;
-  // the array keeps the previous call's contents: clear the part used here
-  ADS_CUDA(cudaMemsetAsync(scratch, 0, sizeof(double) * n_scr, st));
-  double* prof = scratch;
-  ADS_CUDA(cudaMemcpyAsync(prof, ax, sizeof(double) * 2 * NX, cudaMemcpyDeviceToDevice, st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 2 * NX, bx, sizeof(double) * 2 * NX, cudaMemcpyDeviceToDevice,
-                           st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 4 * NX, ay, sizeof(double) * 2 * NY, cudaMemcpyDeviceToDevice,
-                           st));
-  ADS_CUDA(cudaMemcpyAsync(prof + 4 * NX + 2 * NY, by, sizeof(double) * 2 * NY,
-                           cudaMemcpyDeviceToDevice, st));
-  double* fout = scratch + prof_n;
-  double* store = fout + NF * N;
-  double* tmp = store + NSTORE * N;
-  ElModel<double> M =
-      make_model<double>((int)NX, (int)NY, NY + 2, 0, dt, dx, dy, lambda, mu, rho, prof);
-  ElShot<double> one{};
-  for (int f = 0; f < NF; f++) {
-    one.fin[f] = state_in + f * N;
-    one.f[f] = fout + f * N;
-    one.g[f] = grad_in + f * N;
+  if (overlap13<double>(state_in, grad_in, N)) {
+    double* scratch = nullptr;
+    if (int e = noalloc_scratch(&scratch)) return e;
+    ADS_CUDA(cudaMemcpyAsync(scratch, state_in, sizeof(double) * NF * N,
+                             cudaMemcpyDeviceToDevice, st));
+    state_in = scratch;
   }
-  for (int k = 0; k < NTMP; k++) one.tmp[k] = tmp + k * N;
-  one.store = store;
-  one.fs = N;
-  one.glam = grad_lambda;
-  one.gmu = grad_mu;
-  one.grho = grad_rho;
-  dim3 grd((unsigned)div_up(NY + 2, BX), (unsigned)div_up(NX + 2, BY), 1);
-  k_el_stress<double, true><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_velocity<double, true><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  ADS_CUDA(cudaMemcpyAsync(grad_in, grad_out, sizeof(double) * NF * N,
-                           cudaMemcpyDeviceToDevice, st));
-  k_el_adj1<double><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_adj2<double><<<grd, dim3(BX, BY), 0, st>>>(M, one, 0);
-  ADS_LAUNCHED(1);
-  k_el_adj3<double><<<grd, dim3(BX, BY), 0, st>>>(M, one);
-  ADS_LAUNCHED(1);
-  return ADS_OK;
+  return el_bwd_kernels<double, double>(state_in, grad_out, grad_in, grad_lambda, grad_mu,
+                                        grad_rho, lambda, mu, rho, ax, bx, ay, by, dt, dx, dy,
+                                        NX, NY, st);
 }
 
 int ads_elastic_plan_create(ads_elastic_plan** plan, const ads_elastic_config* cfg,

@@ -140,8 +140,9 @@ class ElasticPlan:
     d loss / d srcv (gradient(..., want_source_grad=True)); the plan then
     rejects (AdsError) sources on the padded frame, the cells the stencil of
     their field does not update.  adjoint_passes: 1 runs each adjoint step
-    as one fused pass, 3 as the three gather passes, 0 (default) the fused
-    pass for FP32 plans and the three passes for FP64 plans."""
+    as one fused pass, 3 as the three gather passes; 0 (default) steps FP64
+    plans and small FP32 plans with one-thread-per-cell kernels and larger
+    FP32 plans with the fused passes."""
 
     def __init__(self, param: ElasticPropagatorParams, shots, precision="f64",
                  use_graph=True, ckpt_every=0, stream=None, rows_per_warp=0,

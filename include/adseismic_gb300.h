@@ -203,16 +203,16 @@ int ads_elastic_step_bwd_f32(const float* state_in, const float* grad_out, float
  * from another framework's custom-call hook (that framework owns the device
  * memory, and a cudaMalloc from an extension bypasses its accounting or fails
  * once it has reserved the device) or time-critical loops that must never enter
- * the CUDA allocator.  Its scratch is one fixed array of 34 x 65536 doubles
- * (about 17.8 MB) compiled into the library and resident on every GPU that
- * loads it until the process exits; grids with (NX+2)*(NY+2) > 65536 are
- * rejected with ADS_ERR_INVALID.  The first call on each device looks up the
- * array's device address and caches it (make that first call before any stream
- * capture); the cache assumes the device's primary context lives until the
- * process exits, so do not call it after cudaDeviceReset.  All calls share the
- * one array, which keeps the last call's contents (each call clears what it
- * uses): calls whose executions overlap on the GPU (different streams without
- * ordering, or threads racing on one device) corrupt each other's scratch. */
+ * the CUDA allocator.  Only a call whose grad_in overlaps state_in needs scratch (a
+ * copy of the state): one fixed array of 13 x 65536 doubles (about 6.8 MB) compiled
+ * into the library and resident on every GPU that loads it until the process exits.
+ * Grids with (NX+2)*(NY+2) > 65536 are rejected with ADS_ERR_INVALID, overlap or
+ * not.  The first call that overlaps looks up the array's device address and caches
+ * it (make it before any stream capture); the cache assumes the device's primary
+ * context lives until the process exits, so do not call it after cudaDeviceReset.
+ * Such calls share the one array: if their executions overlap on the GPU (different
+ * streams without ordering, or threads racing on one device) they corrupt each
+ * other's copy. */
 int ads_elastic_step_bwd_f64_noalloc(const double* state_in, const double* grad_out,
                                      double* grad_in, double* grad_lambda, double* grad_mu,
                                      double* grad_rho, const double* lambda, const double* mu,
@@ -434,12 +434,17 @@ typedef struct ads_elastic_config {
                                 3..NX+1 / 2..NY are updated); 0: not */
   int32_t autotune;          /* 1: time candidate row heights of the fused step and of the
                                 adjoint at plan creation and keep the fastest
-                                (ignored when rows_per_warp is set) */
+                                (ignored when rows_per_warp is set); plans with the
+                                cell kernels time those against the fused step too,
+                                and their adjoint has nothing to tune */
   int32_t adjoint_passes;    /* the reverse sweep's adjoint step: 1 = one fused
                                 row-streaming pass (two adjoint state buffers, no
                                 intermediate fields in device memory); 3 = three gather passes
-                                over intermediate fields, in place; 0 = 1 for FP32
-                                plans, 3 for FP64 plans */
+                                over intermediate fields, in place; 0 = automatic:
+                                one-thread-per-cell kernels (forward and adjoint) for
+                                FP64 plans and FP32 plans of up to 600000 cells over
+                                all shots, 1 for larger FP32 plans; with rows_per_warp
+                                set, 1 for FP32 and 3 for FP64 plans */
   int32_t reserved[3];
 } ads_elastic_config;
 
