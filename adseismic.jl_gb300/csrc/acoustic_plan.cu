@@ -111,11 +111,13 @@ struct AcShot {
   const int* rcv_next; // next receiver on the same cell, or -1 (time-blocked forward)
   T *seg, *ckpt;      // segment store (k+1 fields), checkpoints (nseg x 4 fields)
   T *lu, *lp, *lq;    // adjoint rings (2 fields each)
+  T* dl;              // FP32 one-thread-per-cell adjoint: its increment field, else null
   T *c, *sx, *ty;     // c = vp^2 (pitched), PML profiles along i and j
   // damping tables of the PML profiles (KT_N arrays each): along i, nx + 2
   // entries per array, after sx; along j, ny + 2 entries, after ty
   T *sxk, *tyk;
   T* rdt;  // FP64 plans: 1 / (1 + (sigma + tau) dt/2) per cell (pitched), else null
+  T* cc;   // FP64 plans: c cx per cell (pitched), else null
   double* gc;         // FP64 gradient accumulator (pitched)
   float* gc32;        // FP32 per-segment partial of grad_c (FP32 plans)
   const T* srcv;      // (nstep, nsrc), already multiplied by dt^2
@@ -127,12 +129,17 @@ struct AcShot {
 // Damping tables of a PML profile s (sigma along i, tau along j), one array
 // each, computed in FP64 on the host and rounded once:
 //   r = 1 / (1 + s dt/2), ar = (1 - s dt/2) r, e = 1 - s dt,
-//   ex = s dt / (2 hx), ey = s dt / (2 hy).
-enum { KT_R, KT_AR, KT_E, KT_EX, KT_EY, KT_N };
+//   ex = s dt / (2 hx), ey = s dt / (2 hy),
+//   gx = s dt hx / (2 dt^2), gy = s dt hx^2 / (2 hy dt^2) (over cx = dt^2 / hx^2), times
+//   dt^2 / (2 hx), dt^2 / (2 hy) in FP64 plans (the one-thread-per-cell kernels).
+enum { KT_R, KT_AR, KT_E, KT_EX, KT_EY, KT_GX, KT_GY, KT_N };
 
 // The profile s followed by its KT_N tables.
 template <typename T>
 std::vector<T> with_tables(const std::vector<double>& s, double dt, double hx, double hy) {
+  const double cx = (dt / hx) * (dt / hx);
+  const double gx = dt / 2.0 / hx / cx * (sizeof(T) == 8 ? dt * dt / (2.0 * hx) : 1.0);
+  const double gy = dt / 2.0 / hy / cx * (sizeof(T) == 8 ? dt * dt / (2.0 * hy) : 1.0);
   const size_t n = s.size();
   std::vector<T> o((1 + KT_N) * n);
   for (size_t k = 0; k < n; k++) {
@@ -143,6 +150,8 @@ std::vector<T> with_tables(const std::vector<double>& s, double dt, double hx, d
     o[(1 + KT_E) * n + k] = (T)std::fma(-s[k], dt, 1.0);
     o[(1 + KT_EX) * n + k] = (T)(s[k] * (dt / 2.0 / hx));
     o[(1 + KT_EY) * n + k] = (T)(s[k] * (dt / 2.0 / hy));
+    o[(1 + KT_GX) * n + k] = (T)(s[k] * gx);
+    o[(1 + KT_GY) * n + k] = (T)(s[k] * gy);
   }
   return o;
 }
@@ -150,6 +159,7 @@ std::vector<T> with_tables(const std::vector<double>& s, double dt, double hx, d
 template <typename T>
 struct AcConst {
   T dt, hdt, dt2, cx, cy, kxy, fx, fy, ex, ey;
+  T ry, kk;  // cy / cx, kxy / cx
 };
 
 // ---------------------------------------------------------------- kernels
@@ -1682,6 +1692,496 @@ k_ac_adjphi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
 }
 
 // ---------------------------------------------------------------------------
+// One-thread-per-cell step kernels: FP64 plans, and FP32 plans of few cells
+// (AcPlan::cells).  One launch a step over interior and PML tiles together, in
+// both variants.
+//
+// FP64 issue bounds the FP64 steps (a warp's FP64 instruction holds the pipe of
+// its SM sub-partition for 64 cycles), so the operations are what counts:
+//  * with a table of cc = c cx the undamped update is
+//    cc (w_N + w_S + ry (w_E + w_W) - kk w) + (2 w - w_old): 6 operations, and its
+//    transpose with the gradient 11 (a table of 2 - kxy c would save one of each,
+//    but rounds the coefficient of w: twice the error against 64 bits);
+//  * phi and psi are kept times dt^2 / (2h) and their adjoints divided by it, so
+//    u takes their differences as they are;
+//  * 1 / (1 + (sigma + tau) dt/2) comes from a table, and (r x - (2r - 1) w_old) is
+//    r (x - 2 w_old) + w_old;
+//  * grad_c is summed without its factor cx, which the assembly applies.
+// A damped cell takes about 18 operations forward, 28 in the transpose.  8 shots of
+// 400 x 400, variant W: 31.0 us a forward step (FP64 pipe 78% of its active cycles,
+// 11.6 instructions a warp), 55.6 an adjoint step; 8 shots' 500-step gradient 57.6 ->
+// 43.5 ms against the row kernels.
+//
+// Small grids are bound by the latency of a step: one launch, no row loop, no
+// fork and join of two streams; the launches are chained (grid_wait), so a step's
+// tables are loaded while the step before it runs.  What a cell sends to its
+// neighbours (transpose), and variant U's phi and psi, are formed once over a tile and
+// the ring around it in shared memory, so variant U needs no launch of its own for
+// them.  240 x 240 FP64 forward 4.6 -> 3.5 us a step; 187 x 143 FP32 variant U forward
+// and adjoint 19.3 -> 6.9 us.  Tiles of 4 rows: 8-row ones, whose ring is smaller, were
+// 3% slower on 8 x 400 x 400 and 7% on 240 x 240 (fewer, heavier CTAs).
+// ---------------------------------------------------------------------------
+constexpr int CRF = 4, CRA = 4;  // tile rows (warps of a CTA), forward / adjoint
+
+// AcItem::pad of these tiles: columns (bits 0..7), bit 8 where a column of the
+// tile or beside it is damped, bit 16 + r where row r or one beside it is.
+__host__ __device__ constexpr int cell_near(int pad, int r) {
+  return (pad & 0x100) | ((pad >> (16 + r)) & 1);
+}
+
+__device__ __forceinline__ bool nonzero(double x) {  // not on the FP64 pipe
+  return ((__double2hiint(x) << 1) | __double2loint(x)) != 0;
+}
+__device__ __forceinline__ bool nonzero(float x) { return x != 0.f; }
+__device__ __forceinline__ double fm(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float fm(float a, float b, float c) { return fmaf(a, b, c); }
+
+// cx c of a cell, and what phi' / psi' take from a difference of w is cc times
+// these (phi scaled as above in FP64 plans)
+template <typename T>
+__device__ __forceinline__ T cell_cc(const AcShot<T>& sh, const AcConst<T>& K, int o) {
+  if constexpr (sizeof(T) == 8) return sh.cc[o];
+  else return sh.c[o] * K.cx;
+}
+// The profiles at a cell: whether it is damped, what phi' and psi' take from a
+// difference of w over c cx (kx, ky: the difference of the profiles' GX, GY
+// entries, formed only where both are nonzero) and their damping (er, ec).
+template <typename T>
+struct CellProf {
+  T sg = T(0), ta = T(0), kx = T(0), ky = T(0), er = T(1), ec = T(1);
+  bool damped = false, both = false;
+  __device__ __forceinline__ void load(const AcShot<T>& sh, int i, int j) {
+    const int n = sh.nx + 2, m = sh.ny + 2;
+    sg = sh.sx[i];
+    ta = sh.ty[j];
+    const bool a = nonzero(sg), b = nonzero(ta);
+    damped = a || b;
+    both = a && b;
+    if (b) {
+      kx = sh.tyk[KT_GX * m + j];
+      ky = -sh.tyk[KT_GY * m + j];
+      ec = sh.tyk[KT_E * m + j];
+    }
+    if (a) {
+      const T x = sh.sxk[KT_GX * n + i], y = sh.sxk[KT_GY * n + i];
+      kx = b ? kx - x : -x;
+      ky = b ? ky + y : y;
+      er = sh.sxk[KT_E * n + i];
+    }
+  }
+};
+
+// An item's source or receiver e, or one of no row.
+__device__ __forceinline__ CellRef first_ref(const CellRef* __restrict__ l, int e, int end) {
+  return e < end ? l[e] : CellRef{0, 0, -1};
+}
+
+// Forward step t (MODE, CK as k_ac_fwd; FP32 the increment form).
+template <typename T, int MODE, bool VU, bool CK>
+__global__ void __launch_bounds__(32 * CRF, sizeof(T) == 8 && VU ? 6 : 8)
+k_ac_cell_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
+              const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs, AcConst<T> K,
+              int t, int base, int ckpt_slot) {
+  constexpr bool SEG = MODE != 0, NOREC = MODE == 1, INC = sizeof(T) == 4;
+  __shared__ T sp[VU ? CRF + 2 : 1][32], sq[VU ? CRF : 1][34];
+  const AcItem it = items[blockIdx.x];
+  const AcShot<T>& sh = shots[it.shot];
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5;
+  const int i = it.i0 + r, j = it.j0 + lane, nx = sh.nx, ny = sh.ny, P = (int)sh.pitch;
+  const int width = it.pad & 0xff, o = i * P + j + JOFF;
+  const bool on = i <= nx && lane < width;
+  const bool near = cell_near(it.pad, r) != 0;  // (uniform over the warp)
+  const int64_t fs = sh.fs;
+  const T *w, *wo;
+  T* out;
+  if (SEG) {
+    w = sh.seg + (int64_t)(t - 1 - base) * fs;
+    wo = sh.seg + (int64_t)(t - 2 - base) * fs;
+    out = sh.seg + (int64_t)(t - base) * fs;
+  } else {
+    w = sh.u + (int64_t)((t - 1) & 1) * fs;
+    out = sh.u + (int64_t)(t & 1) * fs;
+    wo = out;
+  }
+  if (INC) wo = sh.d;
+  // phi, psi: variant W reads set (t-1) & 1 and writes t & 1; variant U forms those
+  // of t-1 (set (t-1) & 1) from those of t-2 (set t & 1)
+  const int in = VU ? t & 1 : (t - 1) & 1;
+  const T *pin = sh.p + (int64_t)in * fs, *qin = sh.q + (int64_t)in * fs;
+  T *pout = sh.p + (int64_t)(1 - in) * fs, *qout = sh.q + (int64_t)(1 - in) * fs;
+  // what the time loop never writes
+  T cc = T(0), rd = T(1);
+  CellProf<T> D;
+  if (on) {
+    cc = INC ? sh.c[o] : sh.cc[o];
+    if (near) {
+      D.load(sh, i, j);
+      if (!INC) rd = sh.rdt[o];
+    }
+  }
+  // variant U: this thread's cell of the ring (rows above and below: phi; columns
+  // beside: psi), where it is damped
+  int ra = 0, rb = 0, ro = -1;
+  T rck = T(0), re = T(1);  // c cx kx (ky), its damping
+  const bool rphi = threadIdx.x < 64, ring = VU && it.pad >> 8 && threadIdx.x < 64 + 2 * CRF;
+  if (ring) {
+    ra = rphi ? (r == 0 ? -1 : CRF) : (threadIdx.x - 64) >> 1;
+    rb = rphi ? lane : (threadIdx.x & 1) ? width : -1;
+    const int ii = it.i0 + ra, jj = it.j0 + rb;
+    if (ii >= 1 && ii <= nx && jj >= 1 && jj <= ny) {
+      CellProf<T> C;
+      C.load(sh, ii, jj);
+      if (C.damped) {
+        ro = ii * P + jj + JOFF;
+        rck = cell_cc(sh, K, ro) * (rphi ? C.kx : C.ky);
+        re = rphi ? C.er : C.ec;
+      }
+    }
+  }
+  const CellRef rc0 = NOREC ? CellRef{0, 0, -1} : first_ref(rcvs, it.rcv_b + lane, it.rcv_e);
+  grid_wait();
+  grid_release();
+  T w0 = T(0), wN = T(0), wS = T(0), wE = T(0), wW = T(0), o0 = T(0);
+  if (on) {
+    w0 = w[o];
+    wN = w[o + P];
+    wS = w[o - P];
+    wE = w[o + 1];
+    wW = w[o - 1];
+    o0 = wo[o];
+  }
+  const T cx = INC ? cc * K.cx : cc;              // c cx
+  T p0 = T(0), q0 = T(0), dP = T(0), dQ = T(0);  // phi, psi of t-1 and their differences
+  // e f + c k d, e = 1 where the profile is zero
+  auto mix = [](bool nz, T e, T f, T ck, T d) { return fm(ck, d, nz ? e * f : f); };
+  if constexpr (VU) {
+    if (it.pad >> 8) {
+      // difference of u_{t-1}, less its source values, about cell x
+      const bool srcd = t - 1 >= 2 && it.src_e > it.src_b;
+      auto diff = [&](int x, int h, T a, T b) -> T {
+        if (srcd) {
+          a -= src_at(it, sh, srcs, x + h, t - 1);
+          b -= src_at(it, sh, srcs, x - h, t - 1);
+        }
+        return a - b;
+      };
+      if (on && D.damped) {
+        p0 = mix(nonzero(D.sg), D.er, pin[o], cx * D.kx, diff(o, P, wN, wS));
+        q0 = mix(nonzero(D.ta), D.ec, qin[o], cx * D.ky, diff(o, 1, wE, wW));
+      }
+      if (lane < width) {
+        sp[r + 1][lane] = p0;
+        sq[r][lane + 1] = q0;
+      }
+      if (ring) {
+        T v = T(0);
+        if (ro >= 0) {
+          const int h = rphi ? P : 1;
+          v = fm(rck, diff(ro, h, w[ro + h], w[ro - h]), re * (rphi ? pin : qin)[ro]);
+        }
+        if (rphi) sp[ra + 1][rb] = v;
+        else sq[ra][rb + 1] = v;
+      }
+      __syncthreads();
+      if (on && near) {
+        dP = sp[r + 2][lane] - sp[r][lane];
+        dQ = sq[r][lane + 2] - sq[r][lane];
+        if (D.damped) {
+          pout[o] = p0;
+          qout[o] = q0;
+        }
+      }
+    }
+  } else if (on && near) {
+    p0 = pin[o];
+    q0 = qin[o];
+    dP = pin[o + P] - pin[o - P];
+    dQ = qin[o + 1] - qin[o - 1];
+  }
+  T v = T(0), dn = T(0);
+  if (on) {
+    if constexpr (INC) {
+      const T lap = cc * (K.cx * ((wN - w0) + (wS - w0)) + K.cy * ((wE - w0) + (wW - w0)));
+      if (!near) {
+        dn = o0 + lap;
+      } else {
+        const T s = D.sg + D.ta;
+        dn = (T(1) - s * K.hdt) * o0 + lap - D.sg * D.ta * K.dt2 * w0 + K.fx * dP + K.fy * dQ;
+        dn = pml_damp<T>(dn, s, K);
+      }
+    } else {
+      const T lap = fm(-K.kk, w0, fm(K.ry, wE + wW, wN + wS));
+      if (!near) {
+        v = fm(cc, lap, fm(T(2), w0, -o0));
+      } else {
+        // x - 2 w_old, then r (x - 2 w_old) + w_old
+        T n = fm(cc, lap, fm(T(2), w0 - o0, dP + dQ));
+        if (D.both) n = fm(-(D.sg * D.ta * K.dt2), w0, n);
+        v = fm(rd, n, o0);
+      }
+    }
+    for (int e = it.src_b; e < it.src_e; e++) {
+      const CellRef s = srcs[e];
+      if (s.cell == o) (INC ? dn : v) += sh.srcv[(int64_t)(t - 1) * sh.nsrc + s.idx];
+    }
+    if constexpr (INC) v = w0 + dn;
+    T po = p0, qo = q0;
+    if (!VU && D.damped) {
+      po = mix(nonzero(D.sg), D.er, p0, cx * D.kx, wN - wS);
+      qo = mix(nonzero(D.ta), D.ec, q0, cx * D.ky, wE - wW);
+      pout[o] = po;
+      qout[o] = qo;
+    }
+    out[o] = v;
+    if (INC) sh.d[o] = dn;
+    if (CK && !SEG && ckpt_slot > 0 && ckpt_slot < sh.nseg) {
+      T* ck = sh.ckpt + (int64_t)ckpt_slot * 4 * fs;
+      ck[o] = v;
+      ck[fs + o] = INC ? dn : w0;
+      if (D.damped) {
+        ck[2 * fs + o] = po;
+        ck[3 * fs + o] = qo;
+      }
+    }
+  }
+  if constexpr (!NOREC) {  // the warp's row holds the receivers' values
+    CellRef q = rc0;
+    for (int e = it.rcv_b; e < it.rcv_e; e += 32) {
+      if (e > it.rcv_b) q = first_ref(rcvs, e + lane, it.rcv_e);
+      const bool mine = q.row == i;
+      const T x = __shfl_sync(FULL, v, mine ? (int)(q.cell - (o - lane)) : 0);
+      if (mine) sh.traces[(int64_t)t * sh.nrcv + q.idx] = x;
+    }
+  }
+}
+
+// Adjoint step k (what it computes: k_ac_adj).  FP32 plans take the transpose of the
+// forward's increment form: with Q the adjoint of u_k as the source adds to it and p that
+// of u_{k-1} beyond the increment, g = Q / den, p += L(c g) - sigma tau dt^2 g + phi, psi
+// terms (L(z) as differences of z, p in place), Q_{k-1} = (1 - s dt/2) g + p.  Q is the
+// three-level form's lambdaU; its rounding is relative to the increment p instead of
+// building up over the steps, as the forward's is.  Each thread forms what its own cell
+// sends, and the first 64 + 2 CRA threads that of one cell of the ring, from loads
+// issued together; then one barrier (two in variant U's tiles near damped cells,
+// whose phi and psi terms need lambdaU / den of the cells beside).
+template <typename T, bool VU>
+__global__ void __launch_bounds__(32 * CRA, sizeof(T) == 8 ? 6 : 8)
+k_ac_cell_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
+              const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs, AcConst<T> K,
+              int k, int base, double dt2) {
+  constexpr int HG = VU ? 2 : 1;  // ring of lambdaU / den
+  constexpr bool F64 = sizeof(T) == 8;
+  __shared__ T sz[CRA + 2][34];                 // c cx lambdaU / den
+  __shared__ T sg[CRA + 2 * HG][32 + 2 * HG];   // lambdaU / den (tiles near damped cells)
+  __shared__ T sx_[CRA + 2][32], sy_[CRA][34];  // phi / psi terms
+  const AcItem it = items[blockIdx.x];
+  const AcShot<T>& sh = shots[it.shot];
+  const int tid = threadIdx.x, lane = tid & 31, r = tid >> 5;
+  const int i = it.i0 + r, j = it.j0 + lane, nx = sh.nx, ny = sh.ny, P = (int)sh.pitch;
+  const int width = it.pad & 0xff, o = i * P + j + JOFF;
+  const bool on = i <= nx && lane < width;
+  const bool pml = it.pad >> 8, near = cell_near(it.pad, r) != 0;
+  const int64_t fs = sh.fs;
+  const T* w = sh.seg + (int64_t)(k - 1 - base) * fs;  // u_{k-1}
+  T* lun = sh.lu + (int64_t)((k + 1) & 1) * fs;        // in: lambdaU_{k+1}; out: _{k-1}
+  const T* luc = sh.lu + (int64_t)(k & 1) * fs;        // lambdaU_k
+  const T *lpc = sh.lp + (int64_t)(k & 1) * fs, *lqc = sh.lq + (int64_t)(k & 1) * fs;
+  T *lpo = sh.lp + (int64_t)((k - 1) & 1) * fs, *lqo = sh.lq + (int64_t)((k - 1) & 1) * fs;
+  auto inside = [&](int a, int b) { return a >= 1 && a <= nx && b >= 1 && b <= ny; };
+  // this thread's cell of the ring: rows above and below, columns beside
+  const bool rcol = tid >= 64, ring = tid < 64 + 2 * CRA;
+  const int ra = rcol ? (tid - 64) >> 1 : tid < 32 ? -1 : CRA;
+  const int rb = rcol ? ((tid & 1) ? width : -1) : lane;
+  const int ri = it.i0 + ra, rj = it.j0 + rb, ro = ri * P + rj + JOFF;
+  const bool rin = ring && inside(ri, rj);
+  // what the time loop never writes
+  T cc = T(0), rc = T(0), rd = T(1), rrd = T(1);
+  CellProf<T> D, R;
+  if (on) {
+    cc = cell_cc(sh, K, o);
+    if (near) {
+      D.load(sh, i, j);
+      if constexpr (F64) rd = sh.rdt[o];
+      else rd = inv_den<T>(D.sg + D.ta, K);
+    }
+  }
+  if (rin) {
+    rc = cell_cc(sh, K, ro);
+    if (pml) {
+      R.load(sh, ri, rj);
+      if constexpr (F64) rrd = sh.rdt[ro];
+      else rrd = inv_den<T>(R.sg + R.ta, K);
+    }
+  }
+  // the row's residuals of slot k-1 (made before the sweep), the first 32 of the list
+  int rc0 = -1;
+  T res0 = T(0);
+  if (k - 1 >= 2 && it.rcv_b + lane < it.rcv_e) {
+    const CellRef s = rcvs[it.rcv_b + lane];
+    if (s.row == i) {
+      rc0 = (int)s.cell;
+      res0 = sh.resid[(int64_t)(k - 1) * sh.nrcv + s.idx];
+    }
+  }
+  grid_wait();
+  grid_release();
+  T ln = T(0), w0 = T(0), wN = T(0), wS = T(0), wE = T(0), wW = T(0), gi = T(0), rg = T(0);
+  T lp = T(0), lq = T(0), rl = T(0);
+  using G = typename GradOf<T>::type;
+  G gc = G(0);
+  if (on) {
+    gi = luc[o];
+    ln = F64 ? lun[o] : sh.dl[o];
+    w0 = w[o];
+    wN = w[o + P];
+    wS = w[o - P];
+    wE = w[o + 1];
+    wW = w[o - 1];
+    gc = grad_base(sh)[o];
+    if (D.damped) {
+      lp = lpc[o];
+      lq = lqc[o];
+    }
+  }
+  if (rin) {
+    rg = luc[ro];
+    if (R.damped) rl = rcol ? lqc[ro] : lpc[ro];
+  }
+  T np = T(0), nq = T(0), tx = T(0), ty = T(0), q = T(0);  // q: what came back through phi, psi
+  if (pml) {
+    if (near) gi *= rd;
+    rg *= rrd;
+    // lambdaPhi_{k-1} = er lambdaPhi_k + (lambdaU / den above less below), lambdaPsi alike
+    auto nphi = [&](int a, int b, T e, T l) {
+      T d = sg[a + HG - 1][b + HG] - sg[a + HG + 1][b + HG];
+      if (!F64) d *= K.fx;
+      return fm(e, l, d);
+    };
+    auto npsi = [&](int a, int b, T e, T l) {
+      T d = sg[a + HG][b + HG - 1] - sg[a + HG][b + HG + 1];
+      if (!F64) d *= K.fy;
+      return fm(e, l, d);
+    };
+    auto fill = [&] {
+      if (lane < width) sg[r + HG][lane + HG] = gi;
+      if (ring) sg[ra + HG][rb + HG] = rg;
+    };
+    if constexpr (VU) {
+      // the second ring: two more rows and columns, read where the first is damped
+      if (tid < 64 + 2 * CRA) {
+        const int a = rcol ? ra : tid < 32 ? -2 : CRA + 1;
+        const int b = rcol ? ((tid & 1) ? width + 1 : -2) : lane;
+        const int ii = it.i0 + a, jj = it.j0 + b, x = ii * P + jj + JOFF;
+        T g = T(0);
+        if (inside(ii, jj)) {
+          if constexpr (F64) g = luc[x] * sh.rdt[x];
+          else g = luc[x] * inv_den<T>(sh.sx[ii] + sh.ty[jj], K);
+        }
+        sg[a + HG][b + HG] = g;
+      }
+      fill();
+      __syncthreads();
+      if (D.damped) {
+        lp = np = nphi(r, lane, D.er, lp);
+        lq = nq = npsi(r, lane, D.ec, lq);
+      }
+      if (R.damped) rl = rcol ? npsi(ra, rb, R.ec, rl) : nphi(ra, rb, R.er, rl);
+    } else {
+      fill();
+    }
+    tx = D.kx * lp;
+    ty = D.ky * lq;
+    if (lane < width) {
+      sx_[r + 1][lane] = D.damped ? cc * tx : T(0);
+      sy_[r][lane + 1] = D.damped ? cc * ty : T(0);
+    }
+    if (ring) {
+      const T p = R.damped ? rc * ((rcol ? R.ky : R.kx) * rl) : T(0);
+      if (rcol) sy_[ra][rb + 1] = p;
+      else sx_[ra + 1][rb] = p;
+    }
+  }
+  if (lane < width) sz[r + 1][lane + 1] = cc * gi;
+  if (ring) sz[ra + 1][rb + 1] = rc * rg;
+  __syncthreads();
+  if (on) {
+    if (pml && near) {
+      if constexpr (!VU) {
+        auto up = [&](int a, int b) { return sg[a + HG][b + HG]; };
+        if (D.damped) {
+          T d = up(r - 1, lane) - up(r + 1, lane), e = up(r, lane - 1) - up(r, lane + 1);
+          if (!F64) {
+            d *= K.fx;
+            e *= K.fy;
+          }
+          np = fm(D.er, lp, d);
+          nq = fm(D.ec, lq, e);
+        }
+      }
+      q = (sx_[r][lane] - sx_[r + 2][lane]) + (sy_[r][lane] - sy_[r][lane + 2]);
+    }
+    const T z0 = sz[r + 1][lane + 1], zE = sz[r + 1][lane + 2], zW = sz[r + 1][lane],
+            zN = sz[r + 2][lane + 1], zS = sz[r][lane + 1];
+    T nu, lap;
+    if constexpr (F64) {
+      const T z = fm(-K.kk, z0, fm(K.ry, zE + zW, zN + zS));
+      if (!near) {
+        nu = fm(T(2), gi, -ln) + z;
+      } else {
+        nu = fm(T(2), fm(-rd, ln, gi), ln) + (z + q);
+        if (D.both) nu = fm(-(D.sg * D.ta * K.dt2), gi, nu);
+      }
+      lap = fm(-K.kk, w0, fm(K.ry, wE + wW, wN + wS));
+    } else {
+      T p = ln + (((zN - z0) + (zS - z0)) + K.ry * ((zE - z0) + (zW - z0)));
+      if (near) p += q - D.sg * D.ta * K.dt2 * gi;
+      nu = near ? (T(1) - (D.sg + D.ta) * K.hdt) * gi + p : gi + p;
+      sh.dl[o] = p;
+      lap = K.cx * ((wN - w0) + (wS - w0)) + K.cy * ((wE - w0) + (wW - w0));
+    }
+    if (D.damped) {
+      T dx = wN - wS, dy = wE - wW;
+      if (VU && k - 1 >= 2 && it.src_e > it.src_b) {
+        // u_{k-1} without its source value, as the forward formed phi, psi
+        dx = (wN - src_at(it, sh, srcs, o + P, k - 1)) - (wS - src_at(it, sh, srcs, o - P, k - 1));
+        dy = (wE - src_at(it, sh, srcs, o + 1, k - 1)) - (wW - src_at(it, sh, srcs, o - 1, k - 1));
+      }
+      if constexpr (F64) gc = fm(tx, dx, fm(ty, dy, gc));
+      else lap = fm(lap, gi, K.cx * fm(tx, dx, ty * dy));
+      lpo[o] = np;
+      lqo[o] = nq;
+    }
+    lun[o] = nu;
+    if constexpr (F64) grad_base(sh)[o] = fm(lap, gi, gc);
+    else grad_base(sh)[o] = gc + (D.damped ? lap : lap * gi);
+  }
+  if (k - 1 >= 2 && it.rcv_e > it.rcv_b) {
+    __syncwarp();
+    auto add = [&](int64_t cell, T x) {
+      atomicAdd(lun + cell, x);
+      if (!F64) atomicAdd(sh.dl + cell, x);
+    };
+    if (rc0 >= 0) add(rc0, res0);
+    for (int e = it.rcv_b + 32 + lane; e < it.rcv_e; e += 32) {
+      const CellRef s = rcvs[e];
+      if (s.row == i) add(s.cell, sh.resid[(int64_t)(k - 1) * sh.nrcv + s.idx]);
+    }
+  }
+  // source-time gradient (record_src_grad; variant U: less what came back through
+  // phi_{k-1}, psi_{k-1}, which is q)
+  if (k - 1 >= 2 && it.src_e > it.src_b) {
+    __syncwarp();
+    if (on)
+      for (int e = it.src_b; e < it.src_e; e++) {
+        const CellRef s = srcs[e];
+        if (s.cell == o)
+          sh.gsrc[(int64_t)(k - 2) * sh.nsrc + s.idx] =
+              dt2 * ((double)lun[o] - (VU ? (double)q : 0.0));
+      }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Time-blocked forward (FP32 plans): NS <= KB steps per launch.
 //
 // A CTA of TB_THREADS threads owns one column each: output columns
@@ -1890,14 +2390,18 @@ k_ac_flush_gc(const AcShot<T>* __restrict__ shots) {
 // multiplied by zero adjoint values).
 template <typename T>
 __global__ void k_ac_prep(const AcShot<T>* __restrict__ shots, const double* __restrict__ vp,
-                          int64_t MYp2) {
+                          int64_t MYp2, double cx) {
   const AcShot<T>& sh = shots[blockIdx.y];
   const int64_t n = (int64_t)(sh.nx + 2) * (sh.ny + 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e / (sh.ny + 2), j = e % (sh.ny + 2);
     const double v = vp[(sh.x0 + i) * MYp2 + j];
-    sh.c[i * sh.pitch + j + JOFF] = (T)(v * v);
+    const int64_t x = i * sh.pitch + j + JOFF;
+    sh.c[x] = (T)(v * v);
+    if constexpr (sizeof(T) == 8) {
+      sh.cc[x] = v * v * cx;
+    }
   }
 }
 
@@ -1962,7 +2466,9 @@ __global__ void k_ac_adj_init(const AcShot<T>* __restrict__ shots,
   T* lu = sh.lu + (int64_t)(sh.nstep & 1) * sh.fs;
   for (int e = rcv_b[s] + threadIdx.x; e < rcv_e[s]; e += blockDim.x) {
     const CellRef r = rcvs[e];
-    atomicAdd(lu + r.cell, sh.resid[(int64_t)sh.nstep * sh.nrcv + r.idx]);
+    const T x = sh.resid[(int64_t)sh.nstep * sh.nrcv + r.idx];
+    atomicAdd(lu + r.cell, x);
+    if (sh.dl) atomicAdd(sh.dl + r.cell, x);
   }
   // lambdaU_T is final: source-time gradient of the last row, srcv[T-1]
   __syncthreads();
@@ -1972,11 +2478,12 @@ __global__ void k_ac_adj_init(const AcShot<T>* __restrict__ shots,
   }
 }
 
-// grad_vp = sum over shots covering the cell of (gc * 2) * vp.
+// grad_vp = sum over shots covering the cell of (gc * 2) * vp; gcs: a factor the
+// step kernels left out of gc.
 template <typename T>
 __global__ void k_ac_assemble(const AcShot<T>* __restrict__ shots, int nshots,
                               const double* __restrict__ vp, double* __restrict__ grad,
-                              int64_t MXp2, int64_t MYp2) {
+                              int64_t MXp2, int64_t MYp2, double gcs) {
   const int64_t n = MXp2 * MYp2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -1986,7 +2493,7 @@ __global__ void k_ac_assemble(const AcShot<T>* __restrict__ shots, int nshots,
       const AcShot<T>& sh = shots[s];
       const int64_t li = gi - sh.x0;
       if (li < 0 || li > sh.nx + 1 || j > sh.ny + 1) continue;
-      acc += (sh.gc[li * sh.pitch + j + JOFF] * 2) * vp[e];
+      acc += (sh.gc[li * sh.pitch + j + JOFF] * gcs * 2) * vp[e];
     }
     grad[e] = acc;
   }
@@ -2028,6 +2535,14 @@ struct AcPlanBase {
 };
 
 namespace {
+
+// FP32 plans up to this many cells over all shots (variant W / U) step with the
+// one-thread-per-cell kernels; above it the row-walking kernels, which read each row
+// once for two updates, are ahead.  us per forward / adjoint step, cell against row
+// kernels: W 26.7 k cells 1.9 / 2.6 against 3.9 / 4.7, 160 k 2.7 / 4.0 against 4.2 / 4.7,
+// 320 k 3.9 / 6.0 against 4.5 / 5.2; U 26.7 k 4.4 / 3.7 against 8.9 / 10.4, 640 k
+// 8.1 / 11.5 against 10.7 / 12.7, 1.28 M 12.9 / 20.8 against 12.4 / 18.2.
+constexpr int64_t kCellMaxAc32 = 300000, kCellMaxAc32U = 1000000;
 
 template <typename T>
 struct AcPlan final : AcPlanBase {
@@ -2094,6 +2609,11 @@ struct AcPlan final : AcPlanBase {
   // pm_rows > 0: PML items are cut into items of pm_rows-row tiles (more warps
   // for the heavier PML kernels); 0 keeps them at `rows`
   void build_tiles(int rows, int width, int64_t pitch, TileList& L, int pm_rows = 0) const;
+  // one-thread-per-cell kernels (k_ac_cell_fwd / _adj): their tiles of `rows` rows,
+  // all in the list's PML part
+  bool percell = false;
+  void build_cells(int rows, int64_t pitch, TileList& L) const;
+  void order_items(TileList& L, const std::vector<int>& cost) const;
   int ri_pf = 0, ri_pa = 0;  // row tiles of the PML items (0: same as ri_f / ri)
   int upload_tiles(const TileList& L, DevTiles& D, cudaStream_t st);
   int autotune(cudaStream_t st, int64_t pitch, size_t cap_items);
@@ -2255,6 +2775,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   kc.fy = (T)(dt * dt / (2.0 * hy));
   kc.ex = (T)(dt / 2.0 / hx);
   kc.ey = (T)(dt / 2.0 / hy);
+  kc.ry = (T)(((dt / hy) * (dt / hy)) / ((dt / hx) * (dt / hx)));
+  kc.kk = (T)((2 * dt * dt / hx / hx + 2 * dt * dt / hy / hy) / ((dt / hx) * (dt / hx)));
   // ---- shot order: record length descending (active shots form a prefix)
   order.resize(ns);
   std::iota(order.begin(), order.end(), 0);
@@ -2298,6 +2820,9 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   // steps per launch are tuned only on request (autotune 2): the time-blocked
   // kernel keeps the three-level form, whose FP32 rounding error is larger
   tb_auto = sizeof(T) == 4 && c.autotune >= 2 && c.steps_per_block == 0 && !vu;
+  percell = KB == 1 && c.rows_per_thread <= 0 && c.tma <= 0 &&
+            (sizeof(T) == 8 || cells <= (vu ? kCellMaxAc32U : kCellMaxAc32));
+  if (percell) tb_auto = false;
   inc = sizeof(T) == 4 && KB == 1;
   // ---- trace layout (packed in the caller's shot order)
   trace_off.resize(ns);
@@ -2315,7 +2840,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   size_t off_fwd_begin, off_fwd_end, off_adj_begin, off_adj_end;
   DevPool L;
   struct Offs {
-    size_t u, u2, d, p, q, seg, ckpt, lu, lp, lq, c, rdt, sx, ty, gc, gc32, gsrc, srcv, slist;
+    size_t u, u2, d, p, q, seg, ckpt, lu, lp, lq, dl, c, rdt, cc, sx, ty, gc, gc32, gsrc, srcv, slist;
   };
   std::vector<Offs> offs(ns);
   std::vector<int> nseg(ns);
@@ -2341,6 +2866,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     offs[s].lu = L.take(2 * fs);
     offs[s].lp = L.take(2 * fs);
     offs[s].lq = L.take(2 * fs);
+    offs[s].dl = L.take(percell && sizeof(T) == 4 ? fs : 0);
     offs[s].gc = L.take((shots[order[s]].nx + 2) * pitch * sizeof(double));
     offs[s].gc32 = L.take(sizeof(T) == 4 ? (shots[order[s]].nx + 2) * pitch * sizeof(float) : 0);
     offs[s].gsrc = L.take(sizeof(double) * std::max<int64_t>(shots[order[s]].nstep *
@@ -2352,7 +2878,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     const int64_t fs = (h.nx + 2) * pitch * (int64_t)sizeof(T);
     offs[s].ckpt = L.take((size_t)nseg[s] * 4 * fs);
     offs[s].c = L.take(fs);
-    offs[s].rdt = L.take(sizeof(T) == 8 ? fs : 0);  // FP64 corner warps' 1/den
+    offs[s].rdt = L.take(sizeof(T) == 8 ? fs : 0);  // FP64: 1/den, c cx
+    offs[s].cc = L.take(sizeof(T) == 8 ? fs : 0);
     offs[s].sx = L.take((1 + KT_N) * sizeof(T) * (h.nx + 2));  // sigma, its tables
     offs[s].ty = L.take((1 + KT_N) * sizeof(T) * (MY + 2));    // tau, its tables
     offs[s].srcv = L.take(sizeof(T) * std::max<int64_t>(h.nstep * h.nsrc, 1));
@@ -2404,14 +2931,19 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     ri_f = ri;
   }
   TileList tiles_a, tiles_f;
-  build_tiles(ri, Tile<T>::WA, pitch, tiles_a);
-  build_tiles(ri_f, Tile<T>::WF, pitch, tiles_f);
+  if (percell) {
+    build_cells(CRA, pitch, tiles_a);
+    build_cells(CRF, pitch, tiles_f);
+  } else {
+    build_tiles(ri, Tile<T>::WA, pitch, tiles_a);
+    build_tiles(ri_f, Tile<T>::WF, pitch, tiles_f);
+  }
   auto nitems_of = [](const TileList& L) { return L.in.size() + L.pm.size(); };
   // capacity: the autotuner tries rows down to 2 per thread
   size_t cap_items = std::max(nitems_of(tiles_a), nitems_of(tiles_f));
   size_t cap_refs = std::max({tiles_a.srcs.size(), tiles_f.srcs.size(), tiles_a.rcvs.size(),
                               tiles_f.rcvs.size(), (size_t)1});
-  if (c.autotune) {
+  if (c.autotune && !percell) {
     size_t n2 = 0;
     for (int s = 0; s < ns; s++)
       n2 += (size_t)div_up(shots[order[s]].nx, 2) *
@@ -2581,8 +3113,10 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     d.lu = (T*)(pool + offs[s].lu);
     d.lp = (T*)(pool + offs[s].lp);
     d.lq = (T*)(pool + offs[s].lq);
+    d.dl = percell && sizeof(T) == 4 ? (T*)(pool + offs[s].dl) : nullptr;
     d.c = (T*)(pool + offs[s].c);
     d.rdt = sizeof(T) == 8 ? (T*)(pool + offs[s].rdt) : nullptr;
+    d.cc = sizeof(T) == 8 ? (T*)(pool + offs[s].cc) : nullptr;
     d.sx = (T*)(pool + offs[s].sx);
     d.ty = (T*)(pool + offs[s].ty);
     d.sxk = d.sx + (h.nx + 2);
@@ -2658,7 +3192,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   ADS_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
   ADS_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
   // ---- autotuner: time candidate tilings on the plan's own buffers
-  if (c.autotune)
+  // (the one-thread-per-cell kernels have none)
+  if (c.autotune && !percell)
     if (int e = autotune(st, pitch, cap_items)) return e;
   inc = sizeof(T) == 4 && KB == 1;
   // ---- timing ranges: the first full-length segment the reverse sweep meets
@@ -2683,6 +3218,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   rows[1] = ri;
   rows[2] = ri_pf > 0 ? ri_pf : ri_f;
   rows[3] = ri_pa > 0 ? ri_pa : ri;
+  if (percell) rows[0] = rows[1] = rows[2] = rows[3] = 1;
   launches_fwd = 1 + nF;            // prep + loop
   launches_grad = 1 + nF + 2 + nR + 1;  // prep, loop, misfit+reduce, reverse, assemble
   // ---- graphs
@@ -2702,6 +3238,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
       ADS_CUDA(e);
       cudaGraphExec_t ex = nullptr;
       ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
+      ADS_CUDA(cudaGraphUpload(ex, st));  // (else the first launch waits for it)
       if (which == 0) {
         gF = g;
         eF = ex;
@@ -2904,13 +3441,18 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
     L.in_end[s] = (int)L.in.size();
     L.pm_end[s] = (int)L.pm.size();
   }
-  // Heaviest PML items first.  Their cost varies several-fold (corner warps
-  // take the general form, edge warps a cheaper specialised one, warps past the
-  // profile the interior update), and the blocks start roughly in index order,
-  // so this order lets the launch end on light items.  Items move only within
-  // a group of shots of equal record length: a launch always covers whole
-  // groups (the shots with nstep >= t), so the prefix counts at group ends stay
-  // valid.
+  order_items(L, pm_cost);
+}
+
+// Heaviest PML items first.  Their cost varies several-fold (corner warps
+// take the general form, edge warps a cheaper specialised one, warps past the
+// profile the interior update), and the blocks start roughly in index order,
+// so this order lets the launch end on light items.  Items move only within
+// a group of shots of equal record length: a launch always covers whole
+// groups (the shots with nstep >= t), so the prefix counts at group ends stay
+// valid.
+template <typename T>
+void AcPlan<T>::order_items(TileList& L, const std::vector<int>& cost) const {
   std::vector<int> idx;
   for (int sa = 0; sa < nshots;) {
     int sb = sa + 1;
@@ -2919,12 +3461,102 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
     idx.resize(e - b);
     std::iota(idx.begin(), idx.end(), b);
     std::stable_sort(idx.begin(), idx.end(),
-                     [&](int x, int y) { return pm_cost[x] > pm_cost[y]; });
+                     [&](int x, int y) { return cost[x] > cost[y]; });
     std::vector<AcItem> sorted(e - b);
     for (int k = 0; k < e - b; k++) sorted[k] = L.pm[idx[k]];
     std::copy(sorted.begin(), sorted.end(), L.pm.begin() + b);
     sa = sb;
   }
+}
+
+// Tiles of `rows` rows x at most 32 columns over every sorted shot.  The strips
+// start at column 1; where their number leaves one of them narrower, that is
+// an undamped one next to the left profile (or the last), so the right profile's
+// columns fill whole strips.
+template <typename T>
+void AcPlan<T>::build_cells(int rows, int64_t pitch, TileList& L) const {
+  L = TileList{};
+  L.in_end.assign(nshots, 0);
+  L.pm_end.assign(nshots, 0);
+  const int ny = (int)cfg.MY;
+  const int n = (int)div_up(ny, 32), narrow = ny - 32 * (n - 1);
+  auto near_col = [&](int j) {
+    return hty[j - 1] != 0.0 || hty[j] != 0.0 || hty[j + 1] != 0.0;
+  };
+  int left = 0;  // leading damped columns
+  while (left < ny && near_col(left + 1)) left++;
+  const int at = left < ny ? std::min(n - 1, (int)div_up(left, 32)) : n - 1;
+  std::vector<int> j0(n), jw(n), strip_of(ny + 1);
+  std::vector<char> jn(n, 0);
+  for (int k = 0, j = 1; k < n; k++) {
+    j0[k] = j;
+    jw[k] = k == at ? narrow : 32;
+    for (int q = j; q < j + jw[k]; q++) {
+      strip_of[q] = k;
+      jn[k] |= near_col(q);
+    }
+    j += jw[k];
+  }
+  std::vector<int> cost;
+  for (int s = 0; s < nshots; s++) {
+    const int nx = nxs[s], nti = (int)div_up(nx, rows);
+    std::vector<std::vector<int>> bs((size_t)nti * n), br((size_t)nti * n);
+    for (size_t k = 0; k < hsrc[s].size(); k++) {
+      const int3 q = hsrc[s][k];
+      if (!vu) {
+        bs[(size_t)((q.x - 1) / rows) * n + strip_of[q.y]].push_back((int)k);
+        continue;
+      }
+      // variant U reads u less its source value up to two cells beyond a tile
+      for (int ti = std::max(0, (q.x - 2 - rows) / rows - 1); ti < nti; ti++) {
+        const int i0 = 1 + ti * rows;
+        if (i0 - 2 > q.x) break;
+        if (q.x > i0 + rows + 1) continue;
+        for (int tj = 0; tj < n; tj++)
+          if (q.y >= j0[tj] - 2 && q.y <= j0[tj] + jw[tj] + 1)
+            bs[(size_t)ti * n + tj].push_back((int)k);
+      }
+    }
+    for (size_t k = 0; k < hrcv[s].size(); k++) {
+      const int3 q = hrcv[s][k];
+      br[(size_t)((q.x - 1) / rows) * n + strip_of[q.y]].push_back((int)k);
+    }
+    for (int ti = 0; ti < nti; ti++) {
+      const int i0 = 1 + ti * rows;
+      int mask = 0, nr = 0;
+      for (int r = 0; r < rows && i0 + r <= nx; r++, nr++) {
+        const std::vector<double>& x = hsx[s];
+        const int i = i0 + r;
+        if (x[i - 1] != 0.0 || x[i] != 0.0 || x[i + 1] != 0.0) mask |= 1 << r;
+      }
+      for (int tj = 0; tj < n; tj++) {
+        AcItem it{};
+        it.shot = s;
+        it.i0 = i0;
+        it.j0 = j0[tj];
+        it.pad = jw[tj] | (jn[tj] ? 0x100 : 0) | mask << 16;
+        const size_t b = (size_t)ti * n + tj;
+        it.src_b = (int)L.srcs.size();
+        for (int k : bs[b]) {
+          const int3 q = hsrc[s][k];
+          L.srcs.push_back({(int64_t)q.x * pitch + q.y + JOFF, q.z, q.x});
+        }
+        it.src_e = (int)L.srcs.size();
+        it.rcv_b = (int)L.rcvs.size();
+        for (int k : br[b]) {
+          const int3 q = hrcv[s][k];
+          L.rcvs.push_back({(int64_t)q.x * pitch + q.y + JOFF, q.z, q.x});
+        }
+        it.rcv_e = (int)L.rcvs.size();
+        L.pm.push_back(it);
+        int c = 0;
+        for (int r = 0; r < nr; r++) c += cell_near(it.pad, r) ? 3 : 1;
+        cost.push_back(c);
+      }
+    }
+    L.pm_end[s] = (int)L.pm.size();
+  }
+  order_items(L, cost);
 }
 
 template <typename T>
@@ -2942,7 +3574,7 @@ int AcPlan<T>::upload_tiles(const TileList& L, DevTiles& D, cudaStream_t st) {
     ADS_CUDA(cudaMemcpyAsync(D.rcvs, L.rcvs.data(), sizeof(CellRef) * L.rcvs.size(),
                              cudaMemcpyHostToDevice, st));
   D.pm_off = (int)L.in.size();
-  D.vu = vu ? 1 : 0;
+  D.vu = vu && !percell ? 1 : 0;
   D.in_end = L.in_end;
   D.pm_end = L.pm_end;
   return ADS_OK;
@@ -3019,6 +3651,24 @@ int AcPlan<T>::build_maps(cudaStream_t st) {
 // the PML-item kernel (each launched only when it has items).
 template <typename T>
 int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, int ck) {
+  if (percell) {
+    const int n = tf.pm_upto(na);
+    if (n == 0) return ADS_OK;
+    auto go = [&](auto kernel) {
+      return launch_chained(kernel, dim3(n), dim3(32 * CRF), st, tf.items, d_shots, tf.srcs,
+                            tf.rcvs, kc, t, base, ck);
+    };
+    auto by_mode = [&](auto u) {
+      constexpr bool U = decltype(u)::value;
+      if (mode == 1) return go(k_ac_cell_fwd<T, 1, U, false>);
+      if (mode == 2) return go(k_ac_cell_fwd<T, 2, U, false>);
+      if (ck > 0) return go(k_ac_cell_fwd<T, 0, U, true>);
+      return go(k_ac_cell_fwd<T, 0, U, false>);
+    };
+    ADS_CUDA(vu ? by_mode(std::true_type{}) : by_mode(std::false_type{}));
+    ADS_LAUNCHED(1);
+    return ADS_OK;
+  }
   constexpr int TPB = Tile<T>::TPB;
   const int ni = tf.in_upto(na), np = tf.pm_upto(na);
   const AcItem* pm = tf.items + tf.pm_off;
@@ -3110,6 +3760,15 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, in
 
 template <typename T>
 int AcPlan<T>::launch_adj(cudaStream_t st, int na, int k, int base) {
+  if (percell) {
+    const int n = ta.pm_upto(na);
+    if (n == 0) return ADS_OK;
+    ADS_CUDA(launch_chained(vu ? k_ac_cell_adj<T, true> : k_ac_cell_adj<T, false>, dim3(n),
+                            dim3(32 * CRA), st, ta.items, d_shots, ta.srcs, ta.rcvs, kc, k, base,
+                            dt2d));
+    ADS_LAUNCHED(1);
+    return ADS_OK;
+  }
   constexpr int TPB = Tile<T>::TPB;
   const int ni = ta.in_upto(na), np = ta.pm_upto(na);
   const bool fork = ni > 0 && np > 0;
@@ -3490,7 +4149,7 @@ int AcPlan<T>::run_loop(int which, cudaStream_t st) {
 template <typename T>
 int AcPlan<T>::forward(const double* vp, void* traces, cudaStream_t st) {
   ADS_REQUIRE(vp, "null vp");
-  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2);
+  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2, (cfg.dt / cfg.dx) * (cfg.dt / cfg.dx));
   ADS_LAUNCHED(1);
   if (int e = run_loop(0, st)) return e;
   if (traces)
@@ -3503,7 +4162,7 @@ template <typename T>
 int AcPlan<T>::gradient(const double* vp, const void* obs, double* loss, double* grad,
                         void* traces_out, cudaStream_t st, double* grad_srcv) {
   ADS_REQUIRE(vp && obs && loss && grad, "null argument");
-  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2);
+  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2, (cfg.dt / cfg.dx) * (cfg.dt / cfg.dx));
   ADS_LAUNCHED(1);
   if (int e = run_loop(0, st)) return e;
   k_misfit<T><<<kMisfitBlocks, 256, 0, st>>>(d_traces, (const T*)obs, d_resid, trace_total,
@@ -3514,7 +4173,8 @@ int AcPlan<T>::gradient(const double* vp, const void* obs, double* loss, double*
   if (int e = run_loop(1, st)) return e;
   const int64_t n = (cfg.MX + 2) * (cfg.MY + 2);
   k_ac_assemble<T><<<(unsigned)std::min<int64_t>(div_up(n, 256), 16384), 256, 0, st>>>(
-      d_shots, nshots, vp, grad, cfg.MX + 2, cfg.MY + 2);
+      d_shots, nshots, vp, grad, cfg.MX + 2, cfg.MY + 2,
+      percell && sizeof(T) == 8 ? (cfg.dt / cfg.dx) * (cfg.dt / cfg.dx) : 1.0);
   ADS_LAUNCHED(1);
   if (traces_out)
     ADS_CUDA(cudaMemcpyAsync(traces_out, d_traces, sizeof(T) * trace_total,
@@ -3535,7 +4195,7 @@ int AcPlan<T>::gradient(const double* vp, const void* obs, double* loss, double*
 template <typename T>
 int AcPlan<T>::profile(const double* vp, const void* obs, double* out, cudaStream_t st) {
   ADS_REQUIRE(vp && obs && out, "null argument");
-  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2);
+  k_ac_prep<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, vp, cfg.MY + 2, (cfg.dt / cfg.dx) * (cfg.dt / cfg.dx));
   ADS_LAUNCHED(1);
   timing_run = true;
   int rc = issue_forward(st, nullptr);

@@ -65,6 +65,38 @@ void elastic_cpml(int64_t NX, int64_t NY, double dx, double dy, double dt, int64
                   double* ay, double* by, double* ky);
 
 // ---------------------------------------------------------------------------
+// Programmatic dependent launch, for the chains of short kernels that a plan's time
+// loop is: launch_chained lets the kernel's blocks start while the previous kernel
+// of the stream still runs; grid_wait holds a thread until that kernel is complete
+// and its writes are visible, so before it a kernel may read only what the time
+// loop never writes (items, shot records, tables) and must write nothing.
+// grid_release lets the next kernel's blocks start; after grid_wait, so at most
+// one kernel waits ahead.  Every thread calls both.  Inside stream capture the
+// launches become programmatic graph edges.
+// ---------------------------------------------------------------------------
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
+}
+#endif
+
+// ---------------------------------------------------------------------------
 // Internal grid layout used by the plans: each padded row of ny+2 cells is
 // stored with a pitch that is a multiple of 32 elements and an offset of
 // JOFF = 31, so that interior column j = 1 starts on a 32-element boundary

@@ -271,12 +271,17 @@ typedef struct ads_acoustic_config {
                          both with the whole-path adjoint */
   int32_t use_graph;  /* 1: capture the time loops in CUDA graphs (default) */
   int64_t ckpt_every; /* forward checkpoint spacing k in steps; 0 = automatic */
-  int32_t rows_per_thread; /* stencil tile height (autotuner); 0 = automatic */
+  int32_t rows_per_thread; /* stencil tile height (autotuner) of the row-walking step
+                              kernels; 0 = automatic, which also lets FP64 plans and
+                              small FP32 plans (up to 300000 cells over all shots,
+                              1000000 for variant U) step with one-thread-per-cell
+                              kernels, unless steps_per_block > 1 or tma is set */
   int32_t steps_per_block; /* time steps per forward launch (FP32: 1, 2, 4, 8;
                               FP64: 1); 0 = automatic (1) */
   int32_t block_rows;      /* tile height of the time-blocked forward; 0 = automatic */
   int32_t autotune;        /* 1: time candidate tile heights of the forward and adjoint
-                              kernels at plan creation and keep the fastest; 2: also,
+                              kernels at plan creation and keep the fastest (plans
+                              with the one-thread-per-cell kernels have none); 2: also,
                               for FP32 variant-W plans without resident segments and
                               with steps_per_block 0, time 1, 2 and 4 forward steps
                               per launch and keep the fastest (more than 1 selects
@@ -340,8 +345,8 @@ int64_t ads_acoustic_plan_resident_segments(const ads_acoustic_plan* plan);
 int64_t ads_acoustic_plan_steps_per_block(const ads_acoustic_plan* plan);
 /* Rows per warp of the plan's step items, as created or as the autotuner chose
  * them: forward interior (which = 0), adjoint interior (1), forward PML (2),
- * adjoint PML (3); -1 for a null plan or another `which`.  No reference
- * counterpart. */
+ * adjoint PML (3), each 1 for the one-thread-per-cell kernels; -1 for a null plan
+ * or another `which`.  No reference counterpart. */
 int64_t ads_acoustic_plan_rows(const ads_acoustic_plan* plan, int which);
 /* 1 when the plan's interior forward steps run through tensor-map copies (see
  * ads_acoustic_config.tma), 0 when not, -1 for a null plan.  No reference
