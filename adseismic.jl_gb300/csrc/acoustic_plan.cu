@@ -12,9 +12,12 @@
 //    warp rows are 128/256-byte aligned.  A CTA owns a tile of
 //    rows_per_thread x 128 cells of one shot; each thread slides down i keeping
 //    the i-neighbours in registers and gets j-neighbours by warp shuffles.
-//  * One launch advances every active shot by one step; the launch's grid is
-//    the prefix of the tile list whose shots are still active (shots are sorted
-//    by record length), so uneven NSTEP costs no idle CTAs.
+//  * One launch advances every active shot (of a group) by one step; the launch's
+//    grid is the prefix of the (group's) tile list whose shots are still active
+//    (shots are sorted by record length), so uneven NSTEP costs no idle CTAs.
+//  * Three families of step kernels, chosen by type and cells (kCellMaxAc32 and below):
+//    one thread a cell (FP64 and small FP32 plans), rows walked by warps of four columns
+//    a lane (larger FP32 plans) or two (configured rows, tensor maps, variant U's rest).
 //  * Forward checkpoints (u_t, u_{t-1}, phi_t, psi_t) are written by the step
 //    kernel itself every k steps; the reverse sweep restores a checkpoint,
 //    recomputes its segment into a (k+1)-slot store and runs the adjoint steps
@@ -27,6 +30,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <numeric>
@@ -55,7 +59,18 @@ constexpr unsigned FULL = 0xffffffffu;
 #ifndef ADS_MINB_AI32
 #define ADS_MINB_AI32 9   // 56 registers
 #endif
-
+#ifndef ADS_MINB_WF
+#define ADS_MINB_WF 8     // 64 registers
+#endif
+#ifndef ADS_MINB_PF
+#define ADS_MINB_PF 5     // 96 registers
+#endif
+#ifndef ADS_MINB_PA
+#define ADS_MINB_PA 3     // 168 registers
+#endif
+#ifndef ADS_MINB_WA
+#define ADS_MINB_WA 5     // 96 registers
+#endif
 
 // Tiles: a warp owns a strip of 32 x CF (forward) or 32 x CA (adjoint)
 // columns and rows_per_thread rows of one shot; each thread owns CF / CA
@@ -96,6 +111,8 @@ struct CellRef {
 };
 
 struct AcItem {
+  // pad: columns (low 16 bits) and rows (high) of a row-walking item; the
+  // one-thread-per-cell tiles' own form: cell_near
   int shot, i0, j0, pad;
   int src_b, src_e, rcv_b, rcv_e;
 };
@@ -104,15 +121,16 @@ template <typename T>
 struct AcShot {
   int nx, ny, nstep, x0;
   int64_t pitch, fs;  // row pitch and elements per field
-  int nsrc, nrcv, nseg, pad_;
+  int nsrc, nrcv, nseg;
+  int owner;  // 1 where this shot's tables (c, cc, rdt) are its own, 0 where another's
   T *u, *p, *q;       // forward rings (2 fields each)
   T* d;               // FP32 increment form: d_t = u_t - u_{t-1}, updated in place
   T* u2;              // time-blocked forward: U_{t-1} of the two state sets
   const int* rcv_next; // next receiver on the same cell, or -1 (time-blocked forward)
   T *seg, *ckpt;      // segment store (k+1 fields), checkpoints (nseg x 4 fields)
   T *lu, *lp, *lq;    // adjoint rings (2 fields each)
-  T* dl;              // FP32 one-thread-per-cell adjoint: its increment field, else null
-  T *c, *sx, *ty;     // c = vp^2 (pitched), PML profiles along i and j
+  T* dl;              // increment field of an FP32 reverse sweep in increment form, else null
+  T *c, *sx, *ty;     // c = vp^2 (pitched; shots of one window share it), PML profiles
   // damping tables of the PML profiles (KT_N arrays each): along i, nx + 2
   // entries per array, after sx; along j, ny + 2 entries, after ty
   T *sxk, *tyk;
@@ -391,8 +409,10 @@ k_ac_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
   for (int c = 0; c < C; c++) tj[c] = (j + c <= ny + 1) ? ty[j + c] : T(0);
   const bool tfree = warp_tau_free<T, C>(ty, j, ny);
   auto nz = [&](int r) { return !(tfree && sx[r] == T(0)); };  // phi/psi may be non-zero
-  const int i0 = it.i0 + (threadIdx.x >> 5) * ri, i_end = min(i0 + ri, nx + 1);
-  if (i0 > nx) return;  // whole warps only: every later barrier is warp-level
+  const int i0 = it.i0 + (threadIdx.x >> 5) * ri;
+  const int i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
+  const int jend = min(ny, it.j0 + (it.pad & 0xffff) - 1);  // the item's last column
+  if (i0 >= i_end) return;  // whole warps only: every later barrier is warp-level
   auto off = [&](int r) { return (int64_t)r * P + col; };
   const bool ck_on = CK && !SEG && ckpt_slot > 0 && ckpt_slot < sh.nseg;
   if (INT || interior_rows<T>(tfree, sx, i0, i_end, lane)) {
@@ -462,17 +482,20 @@ k_ac_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
           if constexpr (!INT) {
             for (int e = it.src_b; e < it.src_e; e++) {
               const CellRef r = srcs[e];
-              if (r.cell == row + c) v += srcv[(int64_t)(t - 1) * sh.nsrc + r.idx];
+              if (r.cell != row + c) continue;
+              const T a = srcv[(int64_t)(t - 1) * sh.nsrc + r.idx];
+              v += a;
+              if (INC) dv.v[c] += a;  // (the increment holds the source too)
             }
           }
           vo.v[c] = v;
         }
-        stv<T, C>(out, row, vo, j, ny);
-        if constexpr (INC) stv<T, C>(dd, row, dv, j, ny);
+        stv<T, C>(out, row, vo, j, jend);
+        if constexpr (INC) stv<T, C>(dd, row, dv, j, jend);
         if (ck_on) {
           T* ck = sh.ckpt + (int64_t)ckpt_slot * 4 * fs;
-          stv<T, C>(ck, row, vo, j, ny);
-          stv<T, C>(ck + fs, row, INC ? dv : w0, j, ny);
+          stv<T, C>(ck, row, vo, j, jend);
+          stv<T, C>(ck + fs, row, INC ? dv : w0, j, jend);
         }
       }
 #pragma unroll
@@ -639,19 +662,19 @@ k_ac_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
             qo.v[c] = (T(1) - K.dt * tj[c]) * q0.v[c] + K.ey * cv * (sg - tj[c]) * (wN - wS);
           }
         }
-        stv<T, C>(out, row, vo, j, ny);
-        if constexpr (INC) stv<T, C>(dd, row, dv, j, ny);
+        stv<T, C>(out, row, vo, j, jend);
+        if constexpr (INC) stv<T, C>(dd, row, dv, j, jend);
         if (!VU && n0) {
-          stv<T, C>(pout, row, po, j, ny);
-          stv<T, C>(qout, row, qo, j, ny);
+          stv<T, C>(pout, row, po, j, jend);
+          stv<T, C>(qout, row, qo, j, jend);
         }
         if (ck_on) {
           T* ck = sh.ckpt + (int64_t)ckpt_slot * 4 * fs;
-          stv<T, C>(ck, row, vo, j, ny);
-          stv<T, C>(ck + fs, row, INC ? dv : w0, j, ny);
+          stv<T, C>(ck, row, vo, j, jend);
+          stv<T, C>(ck + fs, row, INC ? dv : w0, j, jend);
           if (n0) {
-            stv<T, C>(ck + 2 * fs, row, VU ? p0 : po, j, ny);
-            stv<T, C>(ck + 3 * fs, row, VU ? q0 : qo, j, ny);
+            stv<T, C>(ck + 2 * fs, row, VU ? p0 : po, j, jend);
+            stv<T, C>(ck + 3 * fs, row, VU ? q0 : qo, j, jend);
           }
         }
       }
@@ -1002,7 +1025,7 @@ __device__ __forceinline__ void record_src_grad(const AcItem& it, const AcShot<T
   for (int e = it.src_b + lane; e < it.src_e; e += 32) {
     const CellRef r = srcs[e];
     const int jc = (int)(r.cell - (int64_t)r.row * sh.pitch) - JOFF;
-    if (r.row < i0 || r.row >= i_end || jc < it.j0 || jc >= it.j0 + 32 * C) continue;
+    if (r.row < i0 || r.row >= i_end || jc < it.j0 || jc >= it.j0 + (it.pad & 0xffff)) continue;
     double g = (double)lun[r.cell];
     if constexpr (VU) {
       const int64_t P = sh.pitch, x = r.cell;
@@ -1031,8 +1054,8 @@ __device__ __forceinline__ T src_at(const AcItem& it, const AcShot<T>& sh,
 }
 
 // Residuals of step k-1 go to receiver cells this warp's lanes wrote in the
-// adjoint step: a warp barrier suffices.
-template <typename T, int C>
+// adjoint step: a warp barrier suffices.  INC: to the increment too.
+template <typename T, bool INC = false>
 __device__ __forceinline__ void inject_residuals(const AcItem& it, const AcShot<T>& sh,
                                                  const CellRef* __restrict__ rcvs, T* lun, int k,
                                                  int lane, int i0, int i_end) {
@@ -1040,8 +1063,11 @@ __device__ __forceinline__ void inject_residuals(const AcItem& it, const AcShot<
   __syncwarp();
   for (int e = it.rcv_b + lane; e < it.rcv_e; e += 32) {
     const CellRef r = rcvs[e];
-    if (r.row >= i0 && r.row < i_end)
-      atomicAdd(lun + r.cell, sh.resid[(int64_t)(k - 1) * sh.nrcv + r.idx]);
+    if (r.row >= i0 && r.row < i_end) {
+      const T x = sh.resid[(int64_t)(k - 1) * sh.nrcv + r.idx];
+      atomicAdd(lun + r.cell, x);
+      if (INC) atomicAdd(sh.dl + r.cell, x);
+    }
   }
 }
 
@@ -1239,7 +1265,7 @@ k_ac_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
       hwq[PF - 1] = hwn;
     }
     if constexpr (!INT) {
-      inject_residuals<T, C>(it, sh, rcvs, lun, k, lane, i0, i_end);
+      inject_residuals<T>(it, sh, rcvs, lun, k, lane, i0, i_end);
       record_src_grad<T, C, VU>(it, sh, srcs, lun, lpc, lqc, K, k, lane, i0, i_end, dt2);
     }
   } else {
@@ -1497,7 +1523,7 @@ k_ac_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
   if (SPEC && tfree) pml_rows(std::integral_constant<int, SPEC ? 1 : 0>{});
   else if (SPEC && sfree) pml_rows(std::integral_constant<int, SPEC ? 2 : 0>{});
   else pml_rows(std::integral_constant<int, SPEC ? 3 : 0>{});
-  inject_residuals<T, C>(it, sh, rcvs, lun, k, lane, i0, i_end);
+  inject_residuals<T>(it, sh, rcvs, lun, k, lane, i0, i_end);
   record_src_grad<T, C, VU>(it, sh, srcs, lun, lpc, lqc, K, k, lane, i0, i_end, dt2);
   }
 }
@@ -1551,8 +1577,10 @@ k_ac_phi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots
   for (int c = 0; c < C; c++) tj[c] = (j + c <= ny + 1) ? ty[j + c] : T(0);
   const bool tfree = warp_tau_free<T, C>(ty, j, ny);
   auto nz = [&](int r) { return !(tfree && sx[r] == T(0)); };
-  const int i0 = it.i0 + (threadIdx.x >> 5) * ri, i_end = min(i0 + ri, nx + 1);
-  if (i0 > nx) return;
+  const int i0 = it.i0 + (threadIdx.x >> 5) * ri;
+  const int i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
+  const int jend = min(ny, it.j0 + (it.pad & 0xffff) - 1);  // the item's last column
+  if (i0 >= i_end) return;
   auto off = [&](int r) { return (int64_t)r * P + col; };
   const bool srcd = t - 1 >= 2 && it.src_e > it.src_b;  // u_{t-1} received source values
   const int64_t hoff = lane == 0 ? -1 : C;
@@ -1593,8 +1621,8 @@ k_ac_phi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots
         po.v[c] = (T(1) - K.dt * sg) * p0.v[c] + K.ex * c0.v[c] * (tj[c] - sg) * dx_;
         qo.v[c] = (T(1) - K.dt * tj[c]) * q0.v[c] + K.ey * c0.v[c] * (sg - tj[c]) * dy_;
       }
-      stv<T, C>(pout, row, po, j, ny);
-      stv<T, C>(qout, row, qo, j, ny);
+      stv<T, C>(pout, row, po, j, jend);
+      stv<T, C>(qout, row, qo, j, jend);
     }
     wm = w0;
     w0 = wp;
@@ -1689,6 +1717,598 @@ k_ac_adjphi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
     hgu = hgun;
     n0 = n1;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Interior steps of the larger FP32 plans: four columns a lane (strips of up to 128
+// columns), rows four at a time.
+//
+// The two-column form of k_ac_fwd / k_ac_adj issues 79 instructions a warp and row of
+// 64 cells forward, and with the PML items' 170 beside it a step ran at 66% of the
+// chip's issue rate at 40% of the DRAM rate: instructions bound it, not bytes.  Four
+// columns share one row's loads (16 bytes a lane), shuffles, halo load, addresses and
+// loop; a neighbour difference serves the two cells it lies between; the
+// vertical part and the update use the packed two-value instructions; and the row
+// registers rotate by unrolling four rows instead of by moves.  Strips start on a
+// multiple of four columns and are a multiple of four wide (the host cuts them so), so
+// a lane's cells are all updated or none.  With the kernels for the items beside them
+// and the shots in groups (kGroupBytes), us per forward / adjoint step, before -> now:
+// 32 shots of 1000 x 500 79.7 / 113.6 -> 46.9 / 99.8 (now DRAM and the adjoint's PML
+// items bound it), 20 of 700 x 400 31.5 / 51.3 -> 18.3 / 32.7, one of 700 x 600
+// 4.8 / 5.7 -> 4.4 / 5.2 (launches).
+//
+// Variant W's reverse sweep here (and in the one-thread-per-cell kernels) is the transpose of the forward's increment form: with
+// Q the adjoint of u_k as a source adds to it (the three-level form's lambdaU) and p that
+// of u_{k-1} beyond the increment, g = Q / den, p += L(c g) - sigma tau dt^2 g + phi, psi
+// terms, Q_{k-1} = (1 - s dt/2) g + p, with L written as differences and p updated in
+// place.  The three-level form rounds Q relative to itself, which builds up like
+// eps sqrt(N) / (w dt); here the rounding is relative to p, as the forward's is to d.
+// ---------------------------------------------------------------------------
+struct alignas(16) F4 {
+  float2 a, b;
+};
+__device__ __forceinline__ float2 add2(float2 x, float2 y) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 r, x, y;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mul.rn.f32x2 r, x, y;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
+  return r;
+}
+__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "mov.b64 z, {%6, %7};\n\tfma.rn.f32x2 r, x, y, z;\n\tmov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
+  return r;
+}
+__device__ __forceinline__ float2 sub2(float2 x, float2 y) {  // x - y
+  return fma2(y, make_float2(-1.f, -1.f), x);
+}
+
+// cx ((x_p - x_0) + (x_m - x_0)) + cy ((x_r - x_0) + (x_l - x_0)) of a lane's four cells:
+// rows m, 0, p; l, r the columns beside them.
+__device__ __forceinline__ F4 lap4(const F4& m, const F4& z, const F4& p, float l, float r,
+                                   float cx, float cy) {
+  const float d01 = z.a.y - z.a.x, d12 = z.b.x - z.a.y, d23 = z.b.y - z.b.x;
+  const float2 ha = make_float2(d01 + (l - z.a.x), d12 - d01);
+  const float2 hb = make_float2(d23 - d12, (r - z.b.y) - d23);
+  const float2 x = make_float2(cx, cx), y = make_float2(cy, cy);
+  F4 o;
+  o.a = fma2(y, ha, mul2(x, add2(sub2(p.a, z.a), sub2(m.a, z.a))));
+  o.b = fma2(y, hb, mul2(x, add2(sub2(p.b, z.b), sub2(m.b, z.b))));
+  return o;
+}
+
+// A 16-byte load / store at a 32-bit element offset of a field, predicated.
+__device__ __forceinline__ F4 ld4(const float* p, int o, bool on) {
+  F4 x;
+  x.a.x = x.a.y = x.b.x = x.b.y = 0.f;
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
+      "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "+f"(x.a.x), "+f"(x.a.y), "+f"(x.b.x), "+f"(x.b.y)
+      : "l"(p + o), "r"((unsigned)on));
+  return x;
+}
+__device__ __forceinline__ void st4(float* p, int o, const F4& x) {
+  *reinterpret_cast<float4*>(p + o) = make_float4(x.a.x, x.a.y, x.b.x, x.b.y);
+}
+__device__ __forceinline__ float ld1v(const float* p, int o, bool on) {
+  float a = 0.f;
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
+               : "+f"(a)
+               : "l"(p + o), "r"((unsigned)on));
+  return a;
+}
+
+// Geometry of a wide item's warp.
+struct Wide {
+  int lane, j, i0, i_end, P, col;
+  bool on, edge;  // the lane has cells; it is the first or last lane that has
+  int hoff;       // an edge lane's halo column, relative to its first cell
+  __device__ Wide(const AcItem& it, int pitch, int ri) {
+    lane = threadIdx.x & 31;
+    const int last = ((it.pad & 0xffff) >> 2) - 1;
+    j = it.j0 + 4 * lane;
+    i0 = it.i0 + (threadIdx.x >> 5) * ri;
+    i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
+    P = pitch;
+    col = j + JOFF;
+    on = lane <= last;
+    edge = lane == 0 || lane == last;
+    hoff = lane == 0 ? -1 : 4;
+  }
+  // the columns left and right of the lane's four, h: the edge lanes' halo (lane 0's
+  // left, the last lane's right; a strip has two lanes or more)
+  __device__ __forceinline__ void beside(const F4& z, float h, float& l, float& r) const {
+    l = __shfl_up_sync(FULL, z.b.y, 1);
+    r = __shfl_down_sync(FULL, z.a.x, 1);
+    if (edge) {
+      if (lane == 0) l = h;
+      else r = h;
+    }
+  }
+};
+
+// Forward step t of an interior item (MODE, CK as k_ac_fwd).
+template <int MODE, bool CK>
+__global__ void __launch_bounds__(128, ADS_MINB_WF)
+k_ac_wide_fwd(const AcItem* __restrict__ items, const AcShot<float>* __restrict__ shots,
+              AcConst<float> K, int t, int base, int ckpt_slot, int ri) {
+  constexpr bool SEG = MODE != 0;
+  const AcItem it = items[blockIdx.x];
+  const AcShot<float>& sh = shots[it.shot];
+  const Wide W(it, (int)sh.pitch, ri);
+  if (W.i0 >= W.i_end) return;  // (whole warps)
+  const int64_t fs = sh.fs;
+  const float* w = SEG ? sh.seg + (int64_t)(t - 1 - base) * fs : sh.u + (int64_t)((t - 1) & 1) * fs;
+  float* out = SEG ? sh.seg + (int64_t)(t - base) * fs : sh.u + (int64_t)(t & 1) * fs;
+  float* dd = sh.d;
+  const float* cc = sh.c;
+  float* ck = CK && !SEG && ckpt_slot > 0 && ckpt_slot < sh.nseg
+                  ? sh.ckpt + (int64_t)ckpt_slot * 4 * fs
+                  : nullptr;
+  const int P = W.P;
+  int o = W.i0 * P + W.col;  // row i
+  F4 u[4], d[2], c[2];
+  float h[2];
+  u[0] = ld4(w, o - P, W.on);
+  u[1] = ld4(w, o, W.on);
+  u[2] = ld4(w, o + P, W.on);
+  d[0] = ld4(dd, o, W.on);
+  c[0] = ld4(cc, o, W.on);
+  h[0] = ld1v(w, o + W.hoff, W.edge);
+  for (int i = W.i0; i < W.i_end; i += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (i + k >= W.i_end) break;  // (uniform)
+      const bool more = W.on && i + k + 1 < W.i_end;
+      const int on = o + P;
+      u[(k + 3) & 3] = ld4(w, on + P, more);
+      d[(k + 1) & 1] = ld4(dd, on, more);
+      c[(k + 1) & 1] = ld4(cc, on, more);
+      h[(k + 1) & 1] = ld1v(w, on + W.hoff, W.edge && more);
+      const F4 &m = u[k & 3], &z = u[(k + 1) & 3], &p = u[(k + 2) & 3];
+      float l, r;
+      W.beside(z, h[k & 1], l, r);
+      const F4 L = lap4(m, z, p, l, r, K.cx, K.cy);
+      F4 dn, v;
+      dn.a = fma2(c[k & 1].a, L.a, d[k & 1].a);
+      dn.b = fma2(c[k & 1].b, L.b, d[k & 1].b);
+      v.a = add2(z.a, dn.a);
+      v.b = add2(z.b, dn.b);
+      if (W.on) {
+        st4(out, o, v);
+        st4(dd, o, dn);
+        if (CK && ck) {
+          st4(ck, o, v);
+          st4(ck + fs, o, dn);
+        }
+      }
+      o = on;
+    }
+  }
+}
+
+// Adjoint step k of an interior item.
+__global__ void __launch_bounds__(128, ADS_MINB_WA)
+k_ac_wide_adj(const AcItem* __restrict__ items, const AcShot<float>* __restrict__ shots,
+              AcConst<float> K, int k_, int base, int ri) {
+  const AcItem it = items[blockIdx.x];
+  const AcShot<float>& sh = shots[it.shot];
+  const Wide W(it, (int)sh.pitch, ri);
+  if (W.i0 >= W.i_end) return;
+  const int64_t fs = sh.fs;
+  const float* w = sh.seg + (int64_t)(k_ - 1 - base) * fs;    // u_{k-1}
+  float* qn = sh.lu + (int64_t)((k_ + 1) & 1) * fs;           // Q_{k-1}
+  const float* qc = sh.lu + (int64_t)(k_ & 1) * fs;           // Q_k
+  float *pp = sh.dl, *gc = sh.gc32;
+  const float* cc = sh.c;
+  const int P = W.P;
+  int o = W.i0 * P + W.col;
+  auto mul4 = [](const F4& x, const F4& y) -> F4 { return {mul2(x.a, y.a), mul2(x.b, y.b)}; };
+  // rows i-1, i, i+1 of z = c Q and of u_{k-1}; Q of rows i, i+1
+  F4 z[4], u[4], Q[2], p[2], g[2];
+  float hz[2], hu[2];
+  auto halo = [&](int x, int off, bool on, float& a, float& b) {
+    a = ld1v(qc, x + off, on) * ld1v(cc, x + off, on);
+    b = ld1v(w, x + off, on);
+  };
+  z[0] = mul4(ld4(qc, o - P, W.on), ld4(cc, o - P, W.on));
+  Q[0] = ld4(qc, o, W.on);
+  z[1] = mul4(Q[0], ld4(cc, o, W.on));
+  Q[1] = ld4(qc, o + P, W.on);
+  F4 cn = ld4(cc, o + P, W.on);
+  u[0] = ld4(w, o - P, W.on);
+  u[1] = ld4(w, o, W.on);
+  u[2] = ld4(w, o + P, W.on);
+  p[0] = ld4(pp, o, W.on);
+  g[0] = ld4(gc, o, W.on);
+  halo(o, W.hoff, W.edge, hz[0], hu[0]);
+  for (int i = W.i0; i < W.i_end; i += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (i + k >= W.i_end) break;
+      const bool more = W.on && i + k + 1 < W.i_end;
+      const int on = o + P;
+      const int a = k & 1, b = (k + 1) & 1;
+      // z of row i+1 from the loads of the row before
+      z[(k + 2) & 3] = mul4(Q[b], cn);
+      const F4 q0 = Q[a];
+      Q[a] = ld4(qc, on + P, more);
+      cn = ld4(cc, on + P, more);
+      u[(k + 3) & 3] = ld4(w, on + P, more);
+      p[b] = ld4(pp, on, more);
+      g[b] = ld4(gc, on, more);
+      halo(on, W.hoff, W.edge && more, hz[b], hu[b]);
+      float l, r;
+      W.beside(z[(k + 1) & 3], hz[a], l, r);
+      const F4 L = lap4(z[k & 3], z[(k + 1) & 3], z[(k + 2) & 3], l, r, K.cx, K.cy);
+      F4 pn, v, gn;
+      pn.a = add2(p[a].a, L.a);
+      pn.b = add2(p[a].b, L.b);
+      v.a = add2(q0.a, pn.a);
+      v.b = add2(q0.b, pn.b);
+      W.beside(u[(k + 1) & 3], hu[a], l, r);
+      const F4 U = lap4(u[k & 3], u[(k + 1) & 3], u[(k + 2) & 3], l, r, K.cx, K.cy);
+      gn.a = fma2(U.a, q0.a, g[a].a);
+      gn.b = fma2(U.b, q0.b, g[a].b);
+      if (W.on) {
+        st4(qn, o, v);
+        st4(pp, o, pn);
+        st4(gc, o, gn);
+      }
+      o = on;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Damped (and source / receiver) items beside the wide interior ones: four columns a
+// lane too, 16 lanes a 64-column strip, so a warp walks two row tiles side by side (its
+// halves take consecutive tiles of ri rows).  The general two-column form issued about
+// 320 instructions a warp and row of 64 cells forward and 390 in the adjoint, most of
+// them per lane and not per cell; this form's are for 128 cells.  Damping is a
+// reciprocal of 1 + s dt/2 refined once, and zero terms are left in: every cell of an
+// item takes one path.  96 and 168 registers (5 and 3 CTAs a SM): in 128 the adjoint
+// spills (32 shots of 1000 x 500, 600 steps: 153 ms a gradient against 114).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float2 bc2(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float rcp1(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+// 1 / x, x >= 1: one Newton-Raphson step r + r (1 - x r) on the hardware's approximation
+// (its relative error, at most 2^-23, squares; what is left is the step's own rounding)
+__device__ __forceinline__ float2 rcp2(float2 x) {
+  const float2 r = make_float2(rcp1(x.x), rcp1(x.y));
+  const float2 e = fma2(make_float2(-x.x, -x.y), r, bc2(1.f));
+  return fma2(r, e, r);
+}
+__device__ __forceinline__ F4 add4(const F4& x, const F4& y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ F4 sub4(const F4& x, const F4& y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
+__device__ __forceinline__ F4 mul4(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
+__device__ __forceinline__ F4 fma4(const F4& x, const F4& y, const F4& z) {
+  return {fma2(x.a, y.a, z.a), fma2(x.b, y.b, z.b)};
+}
+// s x + z and x s + t for scalars
+__device__ __forceinline__ F4 axpy4(float s, const F4& x, const F4& z) {
+  return {fma2(bc2(s), x.a, z.a), fma2(bc2(s), x.b, z.b)};
+}
+__device__ __forceinline__ F4 lin4(float s, const F4& x, float t) {
+  return {fma2(bc2(s), x.a, bc2(t)), fma2(bc2(s), x.b, bc2(t))};
+}
+__device__ __forceinline__ F4 scale4(float s, const F4& x) {
+  return {mul2(bc2(s), x.a), mul2(bc2(s), x.b)};
+}
+// right neighbour less left neighbour of a lane's four cells
+__device__ __forceinline__ F4 cross4(const F4& z, float l, float r) {
+  return {make_float2(z.a.y - l, z.b.x - z.a.x), make_float2(z.b.y - z.a.y, r - z.b.x)};
+}
+
+// Geometry of a half warp of such an item.
+struct Half {
+  int hl, j, i0, i_end, P, col, nv, hoff;
+  int w0, w1;  // rows of the whole warp
+  bool on, edge;
+  F4 T;       // tau of the lane's columns
+  bool tau;   // any of them damped
+  __device__ Half(const AcItem& it, const AcShot<float>& sh, int ri) {
+    const int half = threadIdx.x >> 4, width = it.pad & 0xffff, n = it.pad >> 16;
+    hl = threadIdx.x & 15;
+    const int last = (width - 1) >> 2;
+    j = it.j0 + 4 * hl;
+    i0 = it.i0 + half * ri;
+    i_end = min(i0 + ri, it.i0 + n);
+    w0 = it.i0 + (half & ~1) * ri;
+    w1 = min(w0 + 2 * ri, it.i0 + n);
+    P = (int)sh.pitch;
+    col = j + JOFF;
+    nv = min(4, width - 4 * hl);  // cells of this lane (<= 0: none)
+    on = nv > 0;
+    // an edge lane's halo column: lane 0 the left one, the last lane the right one
+    // (a strip of one lane ends at the grid's last column: its right neighbours are
+    // the frame's zeros, which the idle lanes hold)
+    edge = hl == 0 || (hl == last && nv == 4);
+    hoff = hl == 0 ? -1 : 4;
+    auto t = [&](int c) { return on && j + c <= sh.ny + 1 ? sh.ty[j + c] : 0.f; };
+    T = {make_float2(t(0), t(1)), make_float2(t(2), t(3))};
+    tau = T.a.x != 0.f || T.a.y != 0.f || T.b.x != 0.f || T.b.y != 0.f;
+  }
+  // the columns left and right of the lane's four; h: an edge lane's halo
+  __device__ __forceinline__ void beside(const F4& z, float h, float& l, float& r) const {
+    l = __shfl_up_sync(FULL, z.b.y, 1, 16);
+    r = __shfl_down_sync(FULL, z.a.x, 1, 16);
+    if (edge) {
+      if (hl == 0) l = h;
+      else r = h;
+    }
+  }
+  // four cells, or the ones of a lane cut off by the grid's last column
+  __device__ __forceinline__ void store(float* p, int o, const F4& x) const {
+    if (nv >= 4) {
+      st4(p, o, x);
+    } else {
+      if (nv > 0) p[o] = x.a.x;
+      if (nv > 1) p[o + 1] = x.a.y;
+      if (nv > 2) p[o + 2] = x.b.x;
+    }
+  }
+};
+
+// Forward step t, variant W (MODE, CK as k_ac_fwd).
+template <int MODE, bool CK>
+__global__ void __launch_bounds__(128, ADS_MINB_PF)
+k_ac_pml_fwd(const AcItem* __restrict__ items, const AcShot<float>* __restrict__ shots,
+             const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs,
+             AcConst<float> K, int t, int base, int ckpt_slot, int ri) {
+  constexpr bool SEG = MODE != 0, NOREC = MODE == 1;
+  const AcItem it = items[blockIdx.x];
+  const AcShot<float>& sh = shots[it.shot];
+  const Half W(it, sh, ri);
+  if (W.w0 >= W.w1) return;  // (whole warps)
+  const int64_t fs = sh.fs;
+  const float* w = SEG ? sh.seg + (int64_t)(t - 1 - base) * fs : sh.u + (int64_t)((t - 1) & 1) * fs;
+  float* out = SEG ? sh.seg + (int64_t)(t - base) * fs : sh.u + (int64_t)(t & 1) * fs;
+  float* dd = sh.d;
+  const float* cc = sh.c;
+  const float *pin = sh.p + (int64_t)((t - 1) & 1) * fs, *qin = sh.q + (int64_t)((t - 1) & 1) * fs;
+  float *pout = sh.p + (int64_t)(t & 1) * fs, *qout = sh.q + (int64_t)(t & 1) * fs;
+  const float* sx = sh.sx;
+  float* ck = CK && !SEG && ckpt_slot > 0 && ckpt_slot < sh.nseg
+                  ? sh.ckpt + (int64_t)ckpt_slot * 4 * fs
+                  : nullptr;
+  const int P = W.P;
+  int o = W.i0 * P + W.col;
+  const bool any = W.i0 < W.i_end;  // (this half)
+  const bool on = W.on && any, ed = W.edge && any;
+  auto sig = [&](int r) { return sx[min(r, sh.nx + 1)]; };
+  float s_0 = any ? sig(W.i0) : 0.f, s_1 = any ? sig(W.i0 + 1) : 0.f;
+  const float s_m = any ? sig(W.i0 - 1) : 0.f;
+  F4 um = ld4(w, o - P, on), u0 = ld4(w, o, on), up = ld4(w, o + P, on);
+  F4 pm = ld4(pin, o - P, on && (W.tau || s_m != 0.f)), p0 = ld4(pin, o, on && (W.tau || s_0 != 0.f)),
+     pp = ld4(pin, o + P, on && (W.tau || s_1 != 0.f));
+  F4 q0 = ld4(qin, o, on && (W.tau || s_0 != 0.f));
+  F4 d0 = ld4(dd, o, on), c0 = ld4(cc, o, on);
+  // psi of the halo column: damped there or in this row
+  const float th = ed ? sh.ty[W.j + W.hoff] : 0.f;
+  float hu = ld1v(w, o + W.hoff, ed), hq = ld1v(qin, o + W.hoff, ed && (th != 0.f || s_0 != 0.f));
+#pragma unroll 4
+  for (int k = 0; k < ri; k++) {
+    const int i = W.i0 + k;
+    if (W.w0 + k >= W.w1) break;  // (uniform: the warp's first half is the longer one)
+    const bool act = i < W.i_end, more = i + 1 < W.i_end;
+    const int n = o + P;
+    const bool lon = W.on && more, led = W.edge && more;
+    const float s_2 = more ? sig(i + 2) : 0.f;
+    const F4 un = ld4(w, n + P, lon);
+    const F4 pn = ld4(pin, n + P, lon && (W.tau || s_2 != 0.f));
+    const F4 qn = ld4(qin, n, lon && (W.tau || s_1 != 0.f));
+    const F4 dn_ = ld4(dd, n, lon), cn = ld4(cc, n, lon);
+    const float hun = ld1v(w, n + W.hoff, led),
+                hqn = ld1v(qin, n + W.hoff, led && (th != 0.f || s_1 != 0.f));
+    float l, r, ql, qr;
+    W.beside(u0, hu, l, r);
+    W.beside(q0, hq, ql, qr);
+    const F4 s = lin4(1.f, W.T, s_0);
+    const F4 den = lin4(K.hdt, s, 1.f);
+    F4 x = mul4(lin4(-K.hdt, s, 1.f), d0);
+    x = fma4(c0, lap4(um, u0, up, l, r, K.cx, K.cy), x);
+    x = axpy4(K.fx, sub4(pp, pm), x);
+    x = axpy4(K.fy, cross4(q0, ql, qr), x);
+    if (s_0 != 0.f) x = fma4(scale4(-s_0 * K.dt2, W.T), u0, x);
+    F4 dv = {mul2(x.a, rcp2(den.a)), mul2(x.b, rcp2(den.b))};
+    for (int e = it.src_b; e < it.src_e; e++) {
+      const CellRef q = srcs[e];
+      const int c = (int)q.cell - o;
+      if (c < 0 || c >= 4) continue;
+      const float a = sh.srcv[(int64_t)(t - 1) * sh.nsrc + q.idx];
+      if (c == 0) dv.a.x += a;
+      else if (c == 1) dv.a.y += a;
+      else if (c == 2) dv.b.x += a;
+      else dv.b.y += a;
+    }
+    const F4 v = add4(u0, dv);
+    const bool damped = W.tau || s_0 != 0.f;
+    const F4 kx = lin4(K.ex, W.T, -K.ex * s_0), ky = lin4(-K.ey, W.T, K.ey * s_0);
+    const F4 po = fma4(mul4(c0, kx), sub4(up, um), scale4(1.f - K.dt * s_0, p0));
+    const F4 qo = fma4(mul4(c0, ky), cross4(u0, l, r), mul4(lin4(-K.dt, W.T, 1.f), q0));
+    if (act && W.on) {
+      W.store(out, o, v);
+      W.store(dd, o, dv);
+      if (damped) {
+        W.store(pout, o, po);
+        W.store(qout, o, qo);
+      }
+      if (CK && ck) {
+        W.store(ck, o, v);
+        W.store(ck + fs, o, dv);
+        if (damped) {
+          W.store(ck + 2 * fs, o, po);
+          W.store(ck + 3 * fs, o, qo);
+        }
+      }
+    }
+    um = u0;
+    u0 = up;
+    up = un;
+    pm = p0;
+    p0 = pp;
+    pp = pn;
+    q0 = qn;
+    d0 = dn_;
+    c0 = cn;
+    hu = hun;
+    hq = hqn;
+    s_0 = s_1;
+    s_1 = s_2;
+    o = n;
+  }
+  record_traces<float, 4, NOREC>(it, sh, rcvs, out, t, threadIdx.x & 31, W.w0, W.w1);
+}
+
+// Adjoint step k, variant W (the increment form described at the wide kernels).
+__global__ void __launch_bounds__(128, ADS_MINB_PA)
+k_ac_pml_adj(const AcItem* __restrict__ items, const AcShot<float>* __restrict__ shots,
+             const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs,
+             AcConst<float> K, int kk, int base, int ri, double dt2) {
+  const AcItem it = items[blockIdx.x];
+  const AcShot<float>& sh = shots[it.shot];
+  const Half W(it, sh, ri);
+  if (W.w0 >= W.w1) return;
+  const int64_t fs = sh.fs;
+  const float* w = sh.seg + (int64_t)(kk - 1 - base) * fs;  // u_{k-1}
+  float* qn_ = sh.lu + (int64_t)((kk + 1) & 1) * fs;        // Q_{k-1}
+  const float* qc = sh.lu + (int64_t)(kk & 1) * fs;         // Q_k
+  float *dl = sh.dl, *gcp = sh.gc32;
+  const int in = kk & 1;
+  const float *lpc = sh.lp + (int64_t)in * fs, *lqc = sh.lq + (int64_t)in * fs;
+  float *lpo = sh.lp + (int64_t)((kk - 1) & 1) * fs, *lqo = sh.lq + (int64_t)((kk - 1) & 1) * fs;
+  const float *cc = sh.c, *sx = sh.sx;
+  const int P = W.P;
+  int o = W.i0 * P + W.col;
+  const bool any = W.i0 < W.i_end, on = W.on && any, ed = W.edge && any;
+  auto sig = [&](int r) { return sx[min(r, sh.nx + 1)]; };
+  auto rden = [&](float s) -> F4 {
+    const F4 d = lin4(K.hdt, W.T, fmaf(K.hdt, s, 1.f));
+    return {rcp2(d.a), rcp2(d.b)};
+  };
+  // (tau - sigma) ex of a row: what its phi terms carry
+  auto kxr = [&](float s) { return lin4(K.ex, W.T, -K.ex * s); };
+  float s_m = any ? sig(W.i0 - 1) : 0.f, s_0 = any ? sig(W.i0) : 0.f,
+        s_1 = any ? sig(W.i0 + 1) : 0.f;
+  auto pd = [&](float s) { return W.tau || s != 0.f; };
+  // rows i-1, i: g = Q / den, z = c g, E = c kx lambdaPhi; row i+1 raw
+  F4 gm, zm, Em, g0, z0, E0, l0, cx0;
+  {
+    const F4 c = ld4(cc, o - P, on);
+    gm = mul4(ld4(qc, o - P, on), rden(s_m));
+    zm = mul4(c, gm);
+    Em = mul4(mul4(c, kxr(s_m)), ld4(lpc, o - P, on && pd(s_m)));
+    cx0 = ld4(cc, o, on);
+    l0 = ld4(lpc, o, on && pd(s_0));
+    g0 = mul4(ld4(qc, o, on), rden(s_0));
+    z0 = mul4(cx0, g0);
+    E0 = mul4(mul4(cx0, kxr(s_0)), l0);
+  }
+  F4 Qp = ld4(qc, o + P, on), cp = ld4(cc, o + P, on), lp = ld4(lpc, o + P, on && pd(s_1));
+  F4 um = ld4(w, o - P, on), u0 = ld4(w, o, on), up = ld4(w, o + P, on);
+  F4 m0 = ld4(lqc, o, on && pd(s_0)), d0 = ld4(dl, o, on), a0 = ld4(gcp, o, on);
+  const float th = ed ? sh.ty[W.j + W.hoff] : 0.f;
+  float hQ = ld1v(qc, o + W.hoff, ed), hc = ld1v(cc, o + W.hoff, ed), hw = ld1v(w, o + W.hoff, ed),
+        hl = ld1v(lqc, o + W.hoff, ed && (th != 0.f || s_0 != 0.f));
+#pragma unroll 2
+  for (int k = 0; k < ri; k++) {
+    const int i = W.i0 + k;
+    if (W.w0 + k >= W.w1) break;
+    const bool act = i < W.i_end, more = i + 1 < W.i_end;
+    const int n = o + P;
+    const bool lon = W.on && more, led = W.edge && more;
+    const float s_2 = more ? sig(i + 2) : 0.f;
+    const F4 Qn = ld4(qc, n + P, lon), cn = ld4(cc, n + P, lon), ln = ld4(lpc, n + P, lon && pd(s_2));
+    const F4 un = ld4(w, n + P, lon);
+    const F4 mn = ld4(lqc, n, lon && pd(s_1)), dn = ld4(dl, n, lon), an = ld4(gcp, n, lon);
+    const float hQn = ld1v(qc, n + W.hoff, led), hcn = ld1v(cc, n + W.hoff, led),
+                hwn = ld1v(w, n + W.hoff, led),
+                hln = ld1v(lqc, n + W.hoff, led && (th != 0.f || s_1 != 0.f));
+    // row i+1
+    const F4 gp = mul4(Qp, rden(s_1));
+    const F4 zp = mul4(cp, gp);
+    const F4 Ep = mul4(mul4(cp, kxr(s_1)), lp);
+    // row i: F = c ky lambdaPsi of the lane and of the halo column
+    const F4 kx = kxr(s_0), ky = lin4(-K.ey, W.T, K.ey * s_0);
+    const F4 F = mul4(mul4(cx0, ky), m0);
+    const float hden = fmaf(K.hdt, s_0 + th, 1.f);
+    float hr = rcp1(hden);
+    hr = fmaf(hr, fmaf(-hden, hr, 1.f), hr);
+    const float hg = hQ * hr, hz = hc * hg, hF = hc * (K.ey * (s_0 - th)) * hl;
+    float l, r;
+    W.beside(z0, hz, l, r);
+    F4 x = add4(d0, lap4(zm, z0, zp, l, r, K.cx, K.cy));
+    x = add4(x, sub4(Em, Ep));
+    W.beside(F, hF, l, r);
+    x = sub4(x, cross4(F, l, r));
+    if (s_0 != 0.f) x = fma4(scale4(-s_0 * K.dt2, W.T), g0, x);
+    const F4 A = lin4(-K.hdt, W.T, fmaf(-K.hdt, s_0, 1.f));
+    const F4 Q = fma4(A, g0, x);
+    const F4 np = axpy4(K.fx, sub4(gm, gp), scale4(1.f - K.dt * s_0, l0));
+    W.beside(g0, hg, l, r);
+    const F4 nq = axpy4(-K.fy, cross4(g0, l, r), mul4(lin4(-K.dt, W.T, 1.f), m0));
+    W.beside(u0, hw, l, r);
+    const F4 dx = sub4(up, um), dy = cross4(u0, l, r);
+    F4 g = fma4(lap4(um, u0, up, l, r, K.cx, K.cy), g0, a0);
+    g = fma4(mul4(kx, l0), dx, g);
+    g = fma4(mul4(ky, m0), dy, g);
+    if (act && W.on) {
+      W.store(qn_, o, Q);
+      W.store(dl, o, x);
+      if (pd(s_0)) {
+        W.store(lpo, o, np);
+        W.store(lqo, o, nq);
+      }
+      W.store(gcp, o, g);
+    }
+    gm = g0;
+    zm = z0;
+    Em = E0;
+    g0 = gp;
+    z0 = zp;
+    E0 = Ep;
+    l0 = lp;
+    cx0 = cp;
+    Qp = Qn;
+    cp = cn;
+    lp = ln;
+    um = u0;
+    u0 = up;
+    up = un;
+    m0 = mn;
+    d0 = dn;
+    a0 = an;
+    hQ = hQn;
+    hc = hcn;
+    hw = hwn;
+    hl = hln;
+    s_m = s_0;
+    s_0 = s_1;
+    s_1 = s_2;
+    o = n;
+  }
+  (void)s_m;
+  inject_residuals<float, true>(it, sh, rcvs, qn_, kk, threadIdx.x & 31, W.w0, W.w1);
+  record_src_grad<float, 4, false>(it, sh, srcs, qn_, lpc, lqc, K, kk, threadIdx.x & 31, W.w0, W.w1,
+                                dt2);
 }
 
 // ---------------------------------------------------------------------------
@@ -2392,6 +3012,7 @@ template <typename T>
 __global__ void k_ac_prep(const AcShot<T>* __restrict__ shots, const double* __restrict__ vp,
                           int64_t MYp2, double cx) {
   const AcShot<T>& sh = shots[blockIdx.y];
+  if (!sh.owner) return;
   const int64_t n = (int64_t)(sh.nx + 2) * (sh.ny + 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -2410,6 +3031,7 @@ __global__ void k_ac_prep(const AcShot<T>* __restrict__ shots, const double* __r
 template <typename T>
 __global__ void k_ac_rden(const AcShot<T>* __restrict__ shots, double hdt) {
   const AcShot<T>& sh = shots[blockIdx.y];
+  if (!sh.owner) return;
   const int64_t n = (int64_t)(sh.nx + 2) * (sh.ny + 2);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -2544,6 +3166,31 @@ namespace {
 // 8.1 / 11.5 against 10.7 / 12.7, 1.28 M 12.9 / 20.8 against 12.4 / 18.2.
 constexpr int64_t kCellMaxAc32 = 300000, kCellMaxAc32U = 1000000;
 
+// FP32 plans above that: the interior items through the four-column kernels
+// (k_ac_wide_*), variant W's general items through k_ac_pml_*.  Variant U forward only
+// (k_ac_wide_fwd), from this many cells on; us per forward + adjoint step, two-column
+// against four-column forward: 3 shots of 900 x 500 (1.35 M) 30.5 / 31.5, 10 of
+// 500 x 400 (2 M) 45.6 / 37.9, 16 of 700 x 400 88.3 / 71.0, 12 of 1000 x 500 105 / 100.
+// (Its adjoint stays three-level: in increment form its PML kernel carries one field
+// more, 6 shots of 1000 x 500 51.3 -> 53.2.)
+constexpr int64_t kWideMinU = 1600000;
+// Their tiles take half the rows up to this many cells: twice the warps, where a
+// launch has too few to fill the chip.
+constexpr int64_t kShortRows = 2200000;
+// These plans run their shots in groups with about this many bytes of live fields (three
+// a shot and sweep direction), each group through the whole time loop, so that what one
+// step writes is still in L2 at the next; kChains groups at a time, one's launches filling
+// the tail of the other's.  us per forward / adjoint step, variant W, 32 shots of
+// 1000 x 500: two groups 62.7 / 111.5, 28 MB 47.6 / 100.3 (42 MB: 55 / 108, 21 MB with
+// its 12 groups: 52 / 131); 20 of 700 x 400 19.4 / 39.8 -> 18.4 / 33.0.  Variant U, one
+// group against pairs of up to 42 MB (84 MB: the same): 16 of 700 x 400 28.3 / 54.0 ->
+// 23.9 / 47.1, 10 of 500 x 400 16.7 / 26.3 -> 14.6 / 23.4.
+constexpr int64_t kGroupBytes = (int64_t)28 << 20, kGroupBytesU = (int64_t)42 << 20;
+// Variant U's plans of fewer shots stay one group: 2 of 1200 x 700 31.0 us a step, split
+// 32.6, 6 of 1000 x 500 50.7 / 51.6.  So do plans without a graph, whose launches the host
+// issues (about 10 us a group and step).
+constexpr int kChains = 2, kSplitShotsU = 8;
+
 template <typename T>
 struct AcPlan final : AcPlanBase {
   ads_acoustic_config cfg{};
@@ -2603,7 +3250,12 @@ struct AcPlan final : AcPlanBase {
     std::vector<int> in_end, pm_end;
     int in_upto(int n) const { return n <= 0 ? 0 : in_end[n - 1]; }
     int pm_upto(int n) const { return n <= 0 ? 0 : pm_end[n - 1]; }
-    int launches(int n) const { return (in_upto(n) > 0) + (pm_upto(n) > 0) * (1 + vu); }
+    // items of sorted shots [s0, s1)
+    int in_of(int s0, int s1) const { return s1 > s0 ? in_upto(s1) - in_upto(s0) : 0; }
+    int pm_of(int s0, int s1) const { return s1 > s0 ? pm_upto(s1) - pm_upto(s0) : 0; }
+    int launches(int s0, int s1) const {
+      return (in_of(s0, s1) > 0) + (pm_of(s0, s1) > 0) * (1 + vu);
+    }
   };
   DevTiles tf, ta;  // forward / adjoint items
   // pm_rows > 0: PML items are cut into items of pm_rows-row tiles (more warps
@@ -2612,14 +3264,42 @@ struct AcPlan final : AcPlanBase {
   // one-thread-per-cell kernels (k_ac_cell_fwd / _adj): their tiles of `rows` rows,
   // all in the list's PML part
   bool percell = false;
+  // FP32: interior items through the four-column kernels (k_ac_wide_fwd / _adj)
+  bool wide = false;
+  int ri_wf = 8, ri_wa = 8;  // their rows per warp, forward / adjoint
+  // the reverse sweep in increment form (its p in sh.dl)
+  bool incr_adj() const { return sizeof(T) == 4 && (percell || (wide && !vu)); }
+  void build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L) const;
+  int autotune_wide(cudaStream_t st, int64_t pitch);
+  // row tiles of a general item beside the wide ones: the eight half warps of the
+  // four-column kernels (variant W), the four warps of the two-column ones (U)
+  int pml_tiles() const { return vu ? Tile<T>::G : 2 * Tile<T>::G; }
   void build_cells(int rows, int64_t pitch, TileList& L) const;
   void order_items(TileList& L, const std::vector<int>& cost) const;
   int ri_pf = 0, ri_pa = 0;  // row tiles of the PML items (0: same as ri_f / ri)
   int upload_tiles(const TileList& L, DevTiles& D, cudaStream_t st);
   int autotune(cudaStream_t st, int64_t pitch, size_t cap_items);
-  // step launches over the first na sorted shots (interior and PML kernels)
-  int launch_fwd(cudaStream_t st, int mode, int na, int t, int base, int ck);
-  int launch_adj(cudaStream_t st, int na, int k, int base);
+  // Groups of consecutive sorted shots that take the whole time loop together
+  // (group_shots): group g holds shots [gb[g], gb[g + 1]).  kChains groups run beside
+  // each other, each on a stream of its own.
+  std::vector<int> gb, chain_groups[kChains];
+  int chains() const {  // chains with a group
+    int n = 0;
+    for (const auto& l : chain_groups) n += !l.empty();
+    return n;
+  }
+  size_t rounds() const {
+    size_t n = 0;
+    for (const auto& l : chain_groups) n = std::max(n, l.size());
+    return n;
+  }
+  void group_shots(int64_t pitch);
+  // step launches over sorted shots [s0, s1) (interior and PML kernels) on chain c
+  int launch_fwd(cudaStream_t st, int mode, int s0, int s1, int t, int base, int ck, int c = 0);
+  int launch_adj(cudaStream_t st, int s0, int s1, int k, int base, int c = 0);
+  // the chains' streams, forked from st and joined to it
+  int fork_chains(cudaStream_t st, cudaStream_t (&q)[kChains]);
+  int join_chains(cudaStream_t st);
   std::vector<int> rcv_b_host, rcv_e_host;
   AcConst<T> kc{};
   double dt2d = 0;  // dt^2 in FP64 (source-time gradient)
@@ -2636,10 +3316,11 @@ struct AcPlan final : AcPlanBase {
   size_t zero_fwd_off = 0, zero_fwd_len = 0, zero_adj_off = 0, zero_adj_len = 0;
   std::vector<AcShot<T>> hshots;
   cudaStream_t cap = nullptr;
-  // second stream for the PML-item launch of a step, which runs beside the
-  // interior-item launch (disjoint cells); fork / join through events
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // per chain: its stream (chain 0: the caller's) and a second one for the PML-item
+  // launch of a step, which runs beside the interior-item launch (disjoint cells);
+  // fork / join through events
+  cudaStream_t chain[kChains] = {}, side[kChains] = {};
+  cudaEvent_t ev_fork[kChains] = {}, ev_join[kChains] = {}, ev_chain[kChains] = {};
   cudaGraph_t gF = nullptr, gR = nullptr;
   cudaGraphExec_t eF = nullptr, eR = nullptr;
   int64_t nF = 0, nR = 0;  // kernel launches in each loop
@@ -2684,14 +3365,20 @@ struct AcPlan final : AcPlanBase {
     if (gF) cudaGraphDestroy(gF);
     if (gR) cudaGraphDestroy(gR);
     if (cap) cudaStreamDestroy(cap);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
-    if (side) cudaStreamDestroy(side);
+    for (int c = 0; c < kChains; c++) {
+      for (cudaEvent_t e : {ev_fork[c], ev_join[c], ev_chain[c]})
+        if (e) cudaEventDestroy(e);
+      if (side[c]) cudaStreamDestroy(side[c]);
+      if (chain[c]) cudaStreamDestroy(chain[c]);
+    }
     if (pool) cudaFree(pool);
   }
 
   std::vector<int64_t> cells_prefix;  // interior cells of the first n sorted shots
   int64_t cells_upto(int n) const { return n <= 0 ? 0 : cells_prefix[n - 1]; }
+  int64_t cells_of(int s0, int s1) const {
+    return s1 > s0 ? cells_upto(s1) - cells_upto(s0) : 0;
+  }
   int profile(const double* vp, const void* obs, double* out, cudaStream_t st) override;
   int set_source_values(int64_t shot, const double* srcv, cudaStream_t st) override {
     ADS_REQUIRE(shot >= 0 && shot < nshots, "shot %lld out of range [0, %d)", (long long)shot,
@@ -2699,6 +3386,8 @@ struct AcPlan final : AcPlanBase {
     ADS_REQUIRE(srcv || srcv_n[shot] == 0, "null srcv");
     return cast_scaled(srcv_dev[shot], srcv, srcv_n[shot], cfg.dt * cfg.dt, st);
   }
+  // the autotuner times the first group, as the time loops run it
+  int tune_upto(int t) const { return std::min(gb[1], shots_with_nstep_ge(t)); }
   // number of sorted shots with nstep >= t
   int shots_with_nstep_ge(int t) const {
     int n = 0;
@@ -2824,6 +3513,9 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
             (sizeof(T) == 8 || cells <= (vu ? kCellMaxAc32U : kCellMaxAc32));
   if (percell) tb_auto = false;
   inc = sizeof(T) == 4 && KB == 1;
+  wide = sizeof(T) == 4 && KB == 1 && !percell && !tb_auto && c.rows_per_thread <= 0 &&
+         c.tma <= 0 && (!vu || cells >= kWideMinU);
+  group_shots(grid_pitch(MY));
   // ---- trace layout (packed in the caller's shot order)
   trace_off.resize(ns);
   trace_total = 0;
@@ -2866,20 +3558,32 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     offs[s].lu = L.take(2 * fs);
     offs[s].lp = L.take(2 * fs);
     offs[s].lq = L.take(2 * fs);
-    offs[s].dl = L.take(percell && sizeof(T) == 4 ? fs : 0);
+    offs[s].dl = L.take(incr_adj() ? fs : 0);
     offs[s].gc = L.take((shots[order[s]].nx + 2) * pitch * sizeof(double));
     offs[s].gc32 = L.take(sizeof(T) == 4 ? (shots[order[s]].nx + 2) * pitch * sizeof(float) : 0);
     offs[s].gsrc = L.take(sizeof(double) * std::max<int64_t>(shots[order[s]].nstep *
                                                              shots[order[s]].nsrc, 1));
   }
   off_adj_end = L.used;
+  std::map<std::pair<int64_t, int64_t>, int> windows;  // (x0, nx) -> first sorted shot
+  std::vector<int> table_of(ns);
   for (int s = 0; s < ns; s++) {
     const ads_acoustic_shot& h = shots[order[s]];
     const int64_t fs = (h.nx + 2) * pitch * (int64_t)sizeof(T);
     offs[s].ckpt = L.take((size_t)nseg[s] * 4 * fs);
-    offs[s].c = L.take(fs);
-    offs[s].rdt = L.take(sizeof(T) == 8 ? fs : 0);  // FP64: 1/den, c cx
-    offs[s].cc = L.take(sizeof(T) == 8 ? fs : 0);
+    // the tables depend on the window alone: shots of one window read the same ones,
+    // which then stay in L2 (C3's 64 shots: 2.3 MB instead of 147 MB read a step)
+    const auto w = windows.emplace(std::make_pair(h.x0, h.nx), s).first;
+    table_of[s] = w->second;
+    if (table_of[s] == s) {
+      offs[s].c = L.take(fs);
+      offs[s].rdt = L.take(sizeof(T) == 8 ? fs : 0);  // FP64: 1/den, c cx
+      offs[s].cc = L.take(sizeof(T) == 8 ? fs : 0);
+    } else {
+      offs[s].c = offs[table_of[s]].c;
+      offs[s].rdt = offs[table_of[s]].rdt;
+      offs[s].cc = offs[table_of[s]].cc;
+    }
     offs[s].sx = L.take((1 + KT_N) * sizeof(T) * (h.nx + 2));  // sigma, its tables
     offs[s].ty = L.take((1 + KT_N) * sizeof(T) * (MY + 2));    // tau, its tables
     offs[s].srcv = L.take(sizeof(T) * std::max<int64_t>(h.nstep * h.nsrc, 1));
@@ -2927,6 +3631,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     while (ri_f > rmin && cells / ((int64_t)ri_f * Tile<T>::WF) < 152 * 64) ri_f /= 2;
     ri = 16;
     while (ri > rmin && cells / ((int64_t)ri * Tile<T>::WA) < 152 * 32) ri /= 2;
+    if (wide && !vu) ri_f = ri = cells < kShortRows ? 2 : 4;  // (rows of a half warp)
+    if (wide && cells < kShortRows) ri_wf = ri_wa = 4;
   } else {
     ri_f = ri;
   }
@@ -2934,6 +3640,10 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   if (percell) {
     build_cells(CRA, pitch, tiles_a);
     build_cells(CRF, pitch, tiles_f);
+  } else if (wide) {
+    if (vu) build_tiles(ri, Tile<T>::WA, pitch, tiles_a);
+    else build_wide(ri_wa, ri, pitch, tiles_a);
+    build_wide(ri_wf, ri_f, pitch, tiles_f);
   } else {
     build_tiles(ri, Tile<T>::WA, pitch, tiles_a);
     build_tiles(ri_f, Tile<T>::WF, pitch, tiles_f);
@@ -2949,6 +3659,11 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
       n2 += (size_t)div_up(shots[order[s]].nx, 2) *
             (size_t)div_up(MY, std::min(Tile<T>::WF, Tile<T>::WA));
     cap_items = std::max(cap_items, n2);
+    // a source within one cell of an item's edge is in the neighbours' lists too
+    // (variant U): at most four items
+    size_t n_src = 0;
+    for (const auto& v : hsrc) n_src += v.size();
+    cap_refs = std::max(cap_refs, 4 * n_src);
   }
   // time-blocked tiles (build_tb) for the configured steps per launch and, when
   // the autotuner may choose them, for 2 and 4; the device lists get the
@@ -2990,7 +3705,6 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   const size_t tbm_off = L.take(sizeof(int) * std::max<size_t>(cap_tbm, 1));
   const size_t rnx_off = L.take(sizeof(int) * std::max<size_t>(rcv_next_all.size(), 1));
   const size_t shots_off = L.take(sizeof(AcShot<T>) * ns);
-  // (sources / receivers: each is bucketed into exactly one item of a list)
   const size_t items_off = L.take(sizeof(AcItem) * cap_items);
   const size_t srcs_off = L.take(sizeof(CellRef) * cap_refs);
   const size_t rcvs_off = L.take(sizeof(CellRef) * cap_refs);
@@ -3102,6 +3816,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     d.nsrc = (int)h.nsrc;
     d.nrcv = (int)h.nrcv;
     d.nseg = nseg[s];
+    d.owner = table_of[s] == s;
     d.u = (T*)(pool + offs[s].u);
     d.u2 = (T*)(pool + offs[s].u2);
     d.d = sizeof(T) == 4 ? (T*)(pool + offs[s].d) : nullptr;
@@ -3113,7 +3828,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
     d.lu = (T*)(pool + offs[s].lu);
     d.lp = (T*)(pool + offs[s].lp);
     d.lq = (T*)(pool + offs[s].lq);
-    d.dl = percell && sizeof(T) == 4 ? (T*)(pool + offs[s].dl) : nullptr;
+    d.dl = incr_adj() ? (T*)(pool + offs[s].dl) : nullptr;
     d.c = (T*)(pool + offs[s].c);
     d.rdt = sizeof(T) == 8 ? (T*)(pool + offs[s].rdt) : nullptr;
     d.cc = sizeof(T) == 8 ? (T*)(pool + offs[s].cc) : nullptr;
@@ -3188,13 +3903,19 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   ADS_CUDA(cudaStreamSynchronize(st));  // host staging buffers go out of scope
   if (sizeof(T) == 4 && c.tma > 0)
     if (int e = build_maps(st)) return e;
-  ADS_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-  ADS_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-  ADS_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+  for (int k = 0; k < chains(); k++) {
+    if (k > 0) ADS_CUDA(cudaStreamCreateWithFlags(&chain[k], cudaStreamNonBlocking));
+    ADS_CUDA(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&ev_fork[k], &ev_join[k], &ev_chain[k]})
+      ADS_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
   // ---- autotuner: time candidate tilings on the plan's own buffers
   // (the one-thread-per-cell kernels have none)
-  if (c.autotune && !percell)
+  if (c.autotune && wide) {
+    if (int e = autotune_wide(st, pitch)) return e;
+  } else if (c.autotune && !percell) {
     if (int e = autotune(st, pitch, cap_items)) return e;
+  }
   inc = sizeof(T) == 4 && KB == 1;
   // ---- timing ranges: the first full-length segment the reverse sweep meets
   cells_prefix.resize(ns);
@@ -3219,6 +3940,10 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   rows[2] = ri_pf > 0 ? ri_pf : ri_f;
   rows[3] = ri_pa > 0 ? ri_pa : ri;
   if (percell) rows[0] = rows[1] = rows[2] = rows[3] = 1;
+  if (wide) {
+    rows[0] = ri_wf;
+    if (!vu) rows[1] = ri_wa;
+  }
   launches_fwd = 1 + nF;            // prep + loop
   launches_grad = 1 + nF + 2 + nR + 1;  // prep, loop, misfit+reduce, reverse, assemble
   // ---- graphs
@@ -3405,6 +4130,7 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
         it.shot = s;
         it.i0 = 1 + ti * gh;
         it.j0 = 1 + tj * width;
+        it.pad = width | std::min(gh, nx + 1 - it.i0) << 16;
         const size_t b = (size_t)ti * ntj + tj;
         it.src_b = (int)L.srcs.size();
         for (int k : bs[b]) {
@@ -3427,9 +4153,10 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
         } else if (pm_rows > 0 && pm_rows < rows) {
           // sub-items share the item's source / receiver lists: the kernels
           // match those by cell and row
-          for (int i0 = it.i0; i0 < it.i0 + gh && i0 <= nx; i0 += Tile<T>::G * pm_rows) {
+          for (int i0 = it.i0; i0 < it.i0 + (it.pad >> 16); i0 += Tile<T>::G * pm_rows) {
             AcItem sub = it;
             sub.i0 = i0;
+            sub.pad = width | std::min(Tile<T>::G * pm_rows, it.i0 + (it.pad >> 16) - i0) << 16;
             L.pm.push_back(sub);
             pm_cost.push_back(item_cost(sub, pm_rows, col_free[tj]));
           }
@@ -3444,19 +4171,240 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
   order_items(L, pm_cost);
 }
 
+// Items of the wide kernels and the general kernels beside them, cut along the
+// profiles: the undamped rectangle of a shot (columns from the end of the left
+// profile's 64-column strips to the start of the right one's, a multiple of four) in
+// strips of 128 columns and tiles of 4 rows_in rows; the bands of damped rows above
+// and below it and the strips beside it, in 64-column strips and tiles of 4 rows_pm
+// rows, to the general kernels, as are the tiles of the rectangle that hold a source
+// or receiver.  (Tiles of 8 rows_pm rows: the general kernels' eight half warps.)  A
+// strip of four columns or fewer ends at the grid's last column.
+template <typename T>
+void AcPlan<T>::build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L) const {
+  L = TileList{};
+  L.in_end.assign(nshots, 0);
+  L.pm_end.assign(nshots, 0);
+  const int ny = (int)cfg.MY, gi = Tile<T>::G * rows_in, gp = pml_tiles() * rows_pm;
+  // damped indices 1..n of a profile: leading and trailing runs (all of them where
+  // there are others between)
+  auto runs = [](const std::vector<double>& x, int n, int& lead, int& trail) {
+    auto near = [&](int i) { return x[i - 1] != 0.0 || x[i] != 0.0 || x[i + 1] != 0.0; };
+    lead = trail = 0;
+    while (lead < n && near(lead + 1)) lead++;
+    while (trail < n - lead && near(n - trail)) trail++;
+    for (int i = lead + 1; i <= n - trail; i++)
+      if (near(i)) lead = n, trail = 0;
+  };
+  auto cut64 = [](int left) { return left == 68 ? 60 : std::min(64, left); };
+  int nl, nr;
+  runs(hty, ny, nl, nr);
+  const int jl = 64 * (int)div_up(nl, 64) + 1;
+  int jr = nr > 0 ? ny - 64 * (int)div_up(nr, 64) + 1 : ny + 1;  // first column past the rectangle
+  if (nr > 0) jr += ((1 - jr) % 4 + 4) % 4;
+  else jr -= ((jr - 1) % 4 + 4) % 4;
+  const bool center = jr > jl + 4;
+  std::vector<std::pair<int, int>> side, mid;  // general strips (j0, width)
+  if (center) {
+    for (int j = 1; j < jl; j += 64) side.push_back({j, 64});
+    for (int j = jr; j <= ny; j += 64) side.push_back({j, std::min(64, ny + 1 - j)});
+    for (int j = jl; j < jr;) {
+      const int w = cut64(jr - j);
+      mid.push_back({j, w});
+      j += w;
+    }
+  } else {
+    for (int j = 1; j <= ny; j += 64) side.push_back({j, std::min(64, ny + 1 - j)});
+  }
+  std::vector<int> cost;
+  for (int s = 0; s < nshots; s++) {
+    const int nx = nxs[s];
+    std::vector<int3> src = hsrc[s], rcv = hrcv[s];
+    auto by_row = [](const int3& a, const int3& b) { return a.x < b.x; };
+    std::stable_sort(src.begin(), src.end(), by_row);
+    std::stable_sort(rcv.begin(), rcv.end(), by_row);
+    // those of `v` within m cells of the rectangle, to out (null: whether there are any)
+    auto pick = [&](const std::vector<int3>& v, int i0, int n, int j0, int w, int m,
+                    std::vector<CellRef>* out) {
+      int3 lo{};
+      lo.x = i0 - m;
+      bool any = false;
+      for (auto it = std::lower_bound(v.begin(), v.end(), lo, by_row);
+           it != v.end() && it->x < i0 + n + m; ++it) {
+        if (it->y < j0 - m || it->y >= j0 + w + m) continue;
+        any = true;
+        if (!out) return true;
+        out->push_back({(int64_t)it->x * pitch + it->y + JOFF, it->z, it->x});
+      }
+      return any;
+    };
+    int nt, nb;
+    runs(hsx[s], nx, nt, nb);
+    auto add_pm = [&](int i0, int n, int j0, int w) {
+      for (int i = i0; i < i0 + n; i += gp) {
+        AcItem it{};
+        const int m = std::min(gp, i0 + n - i);
+        it.shot = s;
+        it.i0 = i;
+        it.j0 = j0;
+        it.pad = w | m << 16;
+        it.src_b = (int)L.srcs.size();
+        pick(src, i, m, j0, w, vu ? 1 : 0, &L.srcs);
+        it.src_e = (int)L.srcs.size();
+        it.rcv_b = (int)L.rcvs.size();
+        pick(rcv, i, m, j0, w, 0, &L.rcvs);
+        it.rcv_e = (int)L.rcvs.size();
+        const bool rows = i <= nt || i + m - 1 > nx - nb, cols = j0 < jl || j0 + w > jr;
+        L.pm.push_back(it);
+        cost.push_back(m * (rows && cols ? 4 : rows || cols ? 3 : 1));
+      }
+    };
+    for (const auto& q : side) add_pm(1, nx, q.first, q.second);
+    for (const auto& q : mid) {
+      if (nt > 0) add_pm(1, nt, q.first, q.second);
+      if (nb > 0) add_pm(nx - nb + 1, nb, q.first, q.second);
+    }
+    if (center)
+      for (int i = nt + 1; i <= nx - nb; i += gi)
+        for (int j = jl, w = 0; j < jr; j += w) {
+          const int n = std::min(gi, nx - nb + 1 - i);
+          w = jr - j == 132 ? 124 : std::min(128, jr - j);
+          if (pick(src, i, n, j, w, 0, nullptr) || pick(rcv, i, n, j, w, 0, nullptr)) {
+            for (int q = j; q < j + w;) {
+              const int m = cut64(j + w - q);
+              add_pm(i, n, q, m);
+              q += m;
+            }
+            continue;
+          }
+          AcItem it{};
+          it.shot = s;
+          it.i0 = i;
+          it.j0 = j;
+          it.pad = w | n << 16;
+          L.in.push_back(it);
+        }
+    L.in_end[s] = (int)L.in.size();
+    L.pm_end[s] = (int)L.pm.size();
+  }
+  order_items(L, cost);
+}
+
+// Autotuner of a plan with the wide kernels: rows per warp of the interior, then of
+// the general items, forward and adjoint, on the plan's own buffers.
+template <typename T>
+int AcPlan<T>::autotune_wide(cudaStream_t st, int64_t pitch) {
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  ADS_CUDA(cudaEventCreate(&e0));
+  ADS_CUDA(cudaEventCreate(&e1));
+  const int tf_end = std::min(9, nstep[0]);
+  const int ka_end = std::min(std::min(9, K + 1), nstep[0]);
+  int rc = ADS_OK;
+  for (int which = 0; which < 2 && rc == ADS_OK; which++) {
+    const bool fwd = which == 0;
+    // (variant U's adjoint: one height for both kinds of item)
+    const bool one = vu && !fwd;
+    int &rin = fwd ? ri_wf : one ? ri : ri_wa, &rpm = fwd ? ri_f : ri;
+    DevTiles& D = fwd ? tf : ta;
+    auto set = [&](int a, int b) -> int {
+      TileList L;
+      if (one) {
+        ri = a;
+        build_tiles(a, Tile<T>::WA, pitch, L);
+      } else {
+        rin = a;
+        rpm = b;
+        build_wide(a, b, pitch, L);
+      }
+      return upload_tiles(L, D, st);
+    };
+    auto timed = [&](float& ms) -> int {
+      for (int pass = 0; pass < 2; pass++) {  // pass 0 warms up
+        ADS_CUDA(cudaEventRecord(e0, st));
+        if (fwd) {
+          for (int t = 2; t <= tf_end; t++)
+            if (int e = launch_fwd(st, 0, 0, tune_upto(t), t, 0, 0)) return e;
+        } else {
+          for (int k = 2; k <= ka_end; k++)
+            if (int e = launch_adj(st, 0, tune_upto(k), k, 0)) return e;
+        }
+        ADS_CUDA(cudaEventRecord(e1, st));
+        ADS_CUDA(cudaEventSynchronize(e1));
+        ADS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+      }
+      return ADS_OK;
+    };
+    int best_in = rin, best_pm = rpm;
+    float best = 1e30f, ms = 0.f;
+    for (int a : {4, 8, 16, 32}) {
+      if ((rc = set(a, best_pm)) || (rc = timed(ms))) break;
+      if (ms < best) {
+        best = ms;
+        best_in = a;
+      }
+    }
+    for (int b : {4, 8, 16}) {
+      if (rc != ADS_OK || b == best_pm || one) continue;
+      if ((rc = set(best_in, b)) || (rc = timed(ms))) break;
+      if (ms < best) {
+        best = ms;
+        best_pm = b;
+      }
+    }
+    if (rc == ADS_OK) rc = set(best_in, best_pm);
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  if (rc == ADS_OK) ADS_CUDA(cudaStreamSynchronize(st));
+  return rc;
+}
+
+// Groups of about kGroupBytes of live fields each (Q, u or their like: three a shot), an
+// even number of them, handed to the chain with the least work so far.
+template <typename T>
+void AcPlan<T>::group_shots(int64_t pitch) {
+  gb.assign(1, 0);
+  for (auto& l : chain_groups) l.clear();
+  std::vector<int64_t> live(nshots);
+  int64_t total = 0;
+  for (int s = 0; s < nshots; s++) {
+    live[s] = 3 * (int64_t)(nxs[s] + 2) * pitch * (int64_t)sizeof(T);
+    total += live[s];
+  }
+  const int64_t per = vu ? kGroupBytesU : kGroupBytes;
+  const bool split = wide && cfg.use_graph && nshots >= (vu ? kSplitShotsU : 2);
+  const int64_t n = split ? kChains * div_up(total, kChains * per) : 1;
+  int64_t sum = 0, work[kChains] = {}, w = 0;
+  for (int s = 0, g = 0; s < nshots; s++) {
+    w += live[s] * nstep[s];
+    sum += live[s];
+    // the group ends where the next shot's middle lies past its share
+    const bool end = s + 1 == nshots || (sum + live[s + 1] / 2) * n > (g + 1) * total;
+    if (!end) continue;
+    int c = 0;
+    for (int k = 1; k < kChains; k++)
+      if (work[k] < work[c]) c = k;
+    work[c] += w;
+    chain_groups[c].push_back((int)gb.size() - 1);
+    gb.push_back(s + 1);
+    w = 0;
+    while ((g + 1) * total <= sum * n && g + 1 < n) g++;
+  }
+}
+
 // Heaviest PML items first.  Their cost varies several-fold (corner warps
 // take the general form, edge warps a cheaper specialised one, warps past the
 // profile the interior update), and the blocks start roughly in index order,
 // so this order lets the launch end on light items.  Items move only within
-// a group of shots of equal record length: a launch always covers whole
-// groups (the shots with nstep >= t), so the prefix counts at group ends stay
-// valid.
+// a run of shots of equal record length in one group: a launch always covers whole
+// runs (a group's shots with nstep >= t), so the counts at their ends stay valid.
 template <typename T>
 void AcPlan<T>::order_items(TileList& L, const std::vector<int>& cost) const {
   std::vector<int> idx;
   for (int sa = 0; sa < nshots;) {
     int sb = sa + 1;
-    while (sb < nshots && nstep[sb] == nstep[sa]) sb++;
+    while (sb < nshots && nstep[sb] == nstep[sa] &&
+           !std::binary_search(gb.begin(), gb.end(), sb))
+      sb++;
     const int b = sa > 0 ? L.pm_end[sa - 1] : 0, e = L.pm_end[sb - 1];
     idx.resize(e - b);
     std::iota(idx.begin(), idx.end(), b);
@@ -3650,12 +4598,13 @@ int AcPlan<T>::build_maps(cudaStream_t st) {
 // One forward step of the first na sorted shots: the interior-item kernel and
 // the PML-item kernel (each launched only when it has items).
 template <typename T>
-int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, int ck) {
+int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int s0, int s1, int t, int base, int ck,
+                          int c) {
   if (percell) {
-    const int n = tf.pm_upto(na);
+    const int n = tf.pm_of(s0, s1);
     if (n == 0) return ADS_OK;
     auto go = [&](auto kernel) {
-      return launch_chained(kernel, dim3(n), dim3(32 * CRF), st, tf.items, d_shots, tf.srcs,
+      return launch_chained(kernel, dim3(n), dim3(32 * CRF), st, tf.items + tf.pm_upto(s0), d_shots, tf.srcs,
                             tf.rcvs, kc, t, base, ck);
     };
     auto by_mode = [&](auto u) {
@@ -3670,14 +4619,14 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, in
     return ADS_OK;
   }
   constexpr int TPB = Tile<T>::TPB;
-  const int ni = tf.in_upto(na), np = tf.pm_upto(na);
-  const AcItem* pm = tf.items + tf.pm_off;
+  const int ni = tf.in_of(s0, s1), np = tf.pm_of(s0, s1);
+  const AcItem *in = tf.items + tf.in_upto(s0), *pm = tf.items + tf.pm_off + tf.pm_upto(s0);
   const bool fork = ni > 0 && np > 0;
   cudaStream_t sp = st;  // stream of the PML-item launch
   if (fork) {
-    ADS_CUDA(cudaEventRecord(ev_fork, st));
-    ADS_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
-    sp = side;
+    ADS_CUDA(cudaEventRecord(ev_fork[c], st));
+    ADS_CUDA(cudaStreamWaitEvent(side[c], ev_fork[c], 0));
+    sp = side[c];
   }
 #define ADS_FWD_(M, IN, VUF, CKF, INCF, items_, n_, s_, rows_)                              \
   k_ac_fwd<T, M, IN, VUF, CKF, INCF><<<n_, TPB, 0, s_>>>(items_, d_shots, tf.srcs, tf.rcvs, kc, \
@@ -3701,25 +4650,34 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, in
   auto run_in = [&]() -> int {
     if (ni > 0) {
       if constexpr (sizeof(T) == 4) {
-        if (tma_ok && inc) {
+        if (wide) {
+          if (mode == 1)
+            k_ac_wide_fwd<1, false><<<ni, TPB, 0, st>>>(in, d_shots, kc, t, base, ck, ri_wf);
+          else if (mode == 2)
+            k_ac_wide_fwd<2, false><<<ni, TPB, 0, st>>>(in, d_shots, kc, t, base, ck, ri_wf);
+          else if (ck > 0)
+            k_ac_wide_fwd<0, true><<<ni, TPB, 0, st>>>(in, d_shots, kc, t, base, ck, ri_wf);
+          else
+            k_ac_wide_fwd<0, false><<<ni, TPB, 0, st>>>(in, d_shots, kc, t, base, ck, ri_wf);
+        } else if (tma_ok && inc) {
           const int gh = Tile<T>::G * ri_f;
           if (mode == 1)
-            k_ac_fwd_tma<1, false><<<ni, TPB, TMA_SMEM, st>>>(tf.items, d_shots, d_maps, kc, t,
+            k_ac_fwd_tma<1, false><<<ni, TPB, TMA_SMEM, st>>>(in, d_shots, d_maps, kc, t,
                                                               base, ck, gh, d_err);
           else if (mode == 2)
-            k_ac_fwd_tma<2, false><<<ni, TPB, TMA_SMEM, st>>>(tf.items, d_shots, d_maps, kc, t,
+            k_ac_fwd_tma<2, false><<<ni, TPB, TMA_SMEM, st>>>(in, d_shots, d_maps, kc, t,
                                                               base, ck, gh, d_err);
           else if (ck > 0)
-            k_ac_fwd_tma<0, true><<<ni, TPB, TMA_SMEM, st>>>(tf.items, d_shots, d_maps, kc, t,
+            k_ac_fwd_tma<0, true><<<ni, TPB, TMA_SMEM, st>>>(in, d_shots, d_maps, kc, t,
                                                              base, ck, gh, d_err);
           else
-            k_ac_fwd_tma<0, false><<<ni, TPB, TMA_SMEM, st>>>(tf.items, d_shots, d_maps, kc, t,
+            k_ac_fwd_tma<0, false><<<ni, TPB, TMA_SMEM, st>>>(in, d_shots, d_maps, kc, t,
                                                               base, ck, gh, d_err);
         } else {
-          ADS_FWD_MODE(true, false, tf.items, ni, st, ri_f);
+          ADS_FWD_MODE(true, false, in, ni, st, ri_f);
         }
       } else {
-        ADS_FWD_MODE(true, false, tf.items, ni, st, ri_f);
+        ADS_FWD_MODE(true, false, in, ni, st, ri_f);
       }
       ADS_LAUNCHED(1);
     }
@@ -3728,6 +4686,19 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, in
   auto run_pm = [&]() -> int {
     if (np > 0) {
       const int rows = ri_pf > 0 ? ri_pf : ri_f;
+      if constexpr (sizeof(T) == 4) {
+        if (wide && !vu) {
+          auto go = [&](auto kernel) {
+            kernel<<<np, TPB, 0, sp>>>(pm, d_shots, tf.srcs, tf.rcvs, kc, t, base, ck, rows);
+          };
+          if (mode == 1) go(k_ac_pml_fwd<1, false>);
+          else if (mode == 2) go(k_ac_pml_fwd<2, false>);
+          else if (ck > 0) go(k_ac_pml_fwd<0, true>);
+          else go(k_ac_pml_fwd<0, false>);
+          ADS_LAUNCHED(1);
+          return ADS_OK;
+        }
+      }
       if (vu) {
         // phi_{t-1}, psi_{t-1} from u_{t-1}, then the step reads them
         if (mode == 0)
@@ -3752,36 +4723,45 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int na, int t, int base, in
 #undef ADS_FWD
 #undef ADS_FWD_
   if (fork) {
-    ADS_CUDA(cudaEventRecord(ev_join, side));
-    ADS_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
+    ADS_CUDA(cudaEventRecord(ev_join[c], side[c]));
+    ADS_CUDA(cudaStreamWaitEvent(st, ev_join[c], 0));
   }
   return ADS_OK;
 }
 
 template <typename T>
-int AcPlan<T>::launch_adj(cudaStream_t st, int na, int k, int base) {
+int AcPlan<T>::launch_adj(cudaStream_t st, int s0, int s1, int k, int base, int c) {
   if (percell) {
-    const int n = ta.pm_upto(na);
+    const int n = ta.pm_of(s0, s1);
     if (n == 0) return ADS_OK;
     ADS_CUDA(launch_chained(vu ? k_ac_cell_adj<T, true> : k_ac_cell_adj<T, false>, dim3(n),
-                            dim3(32 * CRA), st, ta.items, d_shots, ta.srcs, ta.rcvs, kc, k, base,
+                            dim3(32 * CRA), st, ta.items + ta.pm_upto(s0), d_shots, ta.srcs, ta.rcvs, kc, k, base,
                             dt2d));
     ADS_LAUNCHED(1);
     return ADS_OK;
   }
   constexpr int TPB = Tile<T>::TPB;
-  const int ni = ta.in_upto(na), np = ta.pm_upto(na);
+  const int ni = ta.in_of(s0, s1), np = ta.pm_of(s0, s1);
+  const AcItem *in = ta.items + ta.in_upto(s0), *pm = ta.items + ta.pm_off + ta.pm_upto(s0);
   const bool fork = ni > 0 && np > 0;
   cudaStream_t sp = st;
   if (fork) {
-    ADS_CUDA(cudaEventRecord(ev_fork, st));
-    ADS_CUDA(cudaStreamWaitEvent(side, ev_fork, 0));
-    sp = side;
+    ADS_CUDA(cudaEventRecord(ev_fork[c], st));
+    ADS_CUDA(cudaStreamWaitEvent(side[c], ev_fork[c], 0));
+    sp = side[c];
   }
   auto run_in = [&]() -> int {
     if (ni > 0) {
-      k_ac_adj<T, true><<<ni, TPB, 0, st>>>(ta.items, d_shots, ta.srcs, ta.rcvs, kc, k, base, ri,
-                                            dt2d);
+      if constexpr (sizeof(T) == 4) {
+        if (wide && !vu)
+          k_ac_wide_adj<<<ni, TPB, 0, st>>>(in, d_shots, kc, k, base, ri_wa);
+        else
+          k_ac_adj<T, true><<<ni, TPB, 0, st>>>(in, d_shots, ta.srcs, ta.rcvs, kc, k, base, ri,
+                                                dt2d);
+      } else {
+        k_ac_adj<T, true><<<ni, TPB, 0, st>>>(in, d_shots, ta.srcs, ta.rcvs, kc, k, base, ri,
+                                              dt2d);
+      }
       ADS_LAUNCHED(1);
     }
     return ADS_OK;
@@ -3789,14 +4769,21 @@ int AcPlan<T>::launch_adj(cudaStream_t st, int na, int k, int base) {
   auto run_pm = [&]() -> int {
     if (np > 0) {
       const int rows = ri_pa > 0 ? ri_pa : ri;
+      if constexpr (sizeof(T) == 4) {
+        if (wide && !vu) {
+          k_ac_pml_adj<<<np, TPB, 0, sp>>>(pm, d_shots, ta.srcs, ta.rcvs, kc, k, base, rows, dt2d);
+          ADS_LAUNCHED(1);
+          return ADS_OK;
+        }
+      }
       if (vu) {
         // lambdaPhi_{k-1}, lambdaPsi_{k-1} first, then the step's transpose
-        k_ac_adjphi_u<T><<<np, TPB, 0, sp>>>(ta.items + ta.pm_off, d_shots, kc, k, rows);
+        k_ac_adjphi_u<T><<<np, TPB, 0, sp>>>(pm, d_shots, kc, k, rows);
         ADS_LAUNCHED(1);
-        k_ac_adj<T, false, true><<<np, TPB, 0, sp>>>(ta.items + ta.pm_off, d_shots, ta.srcs,
+        k_ac_adj<T, false, true><<<np, TPB, 0, sp>>>(pm, d_shots, ta.srcs,
                                                      ta.rcvs, kc, k, base, rows, dt2d);
       } else {
-        k_ac_adj<T, false><<<np, TPB, 0, sp>>>(ta.items + ta.pm_off, d_shots, ta.srcs, ta.rcvs,
+        k_ac_adj<T, false><<<np, TPB, 0, sp>>>(pm, d_shots, ta.srcs, ta.rcvs,
                                                kc, k, base, rows, dt2d);
       }
       ADS_LAUNCHED(1);
@@ -3806,8 +4793,8 @@ int AcPlan<T>::launch_adj(cudaStream_t st, int na, int k, int base) {
   if (int e = run_pm()) return e;  // the PML launch first, as in launch_fwd
   if (int e = run_in()) return e;
   if (fork) {
-    ADS_CUDA(cudaEventRecord(ev_join, side));
-    ADS_CUDA(cudaStreamWaitEvent(st, ev_join, 0));
+    ADS_CUDA(cudaEventRecord(ev_join[c], side[c]));
+    ADS_CUDA(cudaStreamWaitEvent(st, ev_join[c], 0));
   }
   return ADS_OK;
 }
@@ -3841,8 +4828,8 @@ int AcPlan<T>::autotune(cudaStream_t st, int64_t pitch, size_t cap) {
     for (int pass = 0; pass < 2 && rc == ADS_OK; pass++) {  // pass 0 warms up
       if (cudaEventRecord(e0, st) != cudaSuccess) rc = ADS_ERR_CUDA;
       for (int t = 2; t <= tf_end && rc == ADS_OK; t++) {
-        rc = launch_fwd(st, false, shots_with_nstep_ge(t), t, 0, 0);
-        nl += tf.launches(shots_with_nstep_ge(t));
+        rc = launch_fwd(st, 0, 0, tune_upto(t), t, 0, 0);
+        nl += tf.launches(0, tune_upto(t));
       }
       cudaEventRecord(e1, st);
       if (rc != ADS_OK || cudaStreamSynchronize(st) != cudaSuccess ||
@@ -3853,8 +4840,8 @@ int AcPlan<T>::autotune(cudaStream_t st, int64_t pitch, size_t cap) {
       cudaEventElapsedTime(&ms_f, e0, e1);
       cudaEventRecord(e0, st);
       for (int k = 2; k <= ka_end && rc == ADS_OK; k++) {
-        rc = launch_adj(st, shots_with_nstep_ge(k), k, 0);
-        nl += ta.launches(shots_with_nstep_ge(k));
+        rc = launch_adj(st, 0, tune_upto(k), k, 0);
+        nl += ta.launches(0, tune_upto(k));
       }
       cudaEventRecord(e1, st);
       if (rc != ADS_OK || cudaStreamSynchronize(st) != cudaSuccess ||
@@ -3890,10 +4877,10 @@ int AcPlan<T>::autotune(cudaStream_t st, int64_t pitch, size_t cap) {
       ADS_CUDA(cudaEventRecord(e0, st));
       if (fwd) {
         for (int t = 2; t <= tf_end; t++)
-          if (int e = launch_fwd(st, false, shots_with_nstep_ge(t), t, 0, 0)) return e;
+          if (int e = launch_fwd(st, 0, 0, tune_upto(t), t, 0, 0)) return e;
       } else {
         for (int k = 2; k <= ka_end; k++)
-          if (int e = launch_adj(st, shots_with_nstep_ge(k), k, 0)) return e;
+          if (int e = launch_adj(st, 0, tune_upto(k), k, 0)) return e;
       }
       ADS_CUDA(cudaEventRecord(e1, st));
       ADS_CUDA(cudaEventSynchronize(e1));
@@ -3944,7 +4931,7 @@ int AcPlan<T>::autotune(cudaStream_t st, int64_t pitch, size_t cap) {
           const int NS = std::min(kb, t_end - t0 + 1);
           const int na = shots_with_nstep_ge(t0);
           if (kb == 1) {
-            if (int e = launch_fwd(st, 0, na, t0, 0, 0)) return e;
+            if (int e = launch_fwd(st, 0, 0, na, t0, 0, 0)) return e;
           } else if (int e = launch_tb(st, false, tb_items_upto(na), t0, NS, 0, blk & 1, 0)) {
             return e;
           }
@@ -4011,10 +4998,32 @@ int AcPlan<T>::launch_tb(cudaStream_t st, bool seg, int nit, int t0, int NS, int
   }
 }
 
-// Forward time loop (zero the state and traces, then the steps 2..NSTEP: one
-// launch per step, or per block of up to KB steps that never crosses a
-// checkpoint time 1 + sK).  count != nullptr: only count launches and the
-// interior cell-steps of the loop.
+template <typename T>
+int AcPlan<T>::fork_chains(cudaStream_t st, cudaStream_t (&q)[kChains]) {
+  const int n = chains();
+  q[0] = st;
+  if (n > 1) ADS_CUDA(cudaEventRecord(ev_chain[0], st));
+  for (int c = 1; c < n; c++) {
+    q[c] = chain[c];
+    ADS_CUDA(cudaStreamWaitEvent(chain[c], ev_chain[0], 0));
+  }
+  return ADS_OK;
+}
+
+template <typename T>
+int AcPlan<T>::join_chains(cudaStream_t st) {
+  const int n = chains();
+  for (int c = 1; c < n; c++) {
+    ADS_CUDA(cudaEventRecord(ev_chain[c], chain[c]));
+    ADS_CUDA(cudaStreamWaitEvent(st, ev_chain[c], 0));
+  }
+  return ADS_OK;
+}
+
+// Forward time loop (zero the state and traces, then the steps 2..NSTEP of the chains'
+// groups: one launch per step, or per block of up to KB steps that never crosses a
+// checkpoint time 1 + sK).  The chains meet at the end alone.  count != nullptr: only count
+// launches and the interior cell-steps of the loop.
 template <typename T>
 int AcPlan<T>::issue_forward(cudaStream_t st, int64_t* count) {
   if (count) {
@@ -4025,40 +5034,60 @@ int AcPlan<T>::issue_forward(cudaStream_t st, int64_t* count) {
     if (timing_run) ADS_CUDA(cudaEventRecord(ev[0], st));
   }
   const int a_res = res_seg < nseg_max ? 2 + res_seg * K : INT_MAX;  // first resident step
-  int t0 = 2, blk = 0;
-  while (t0 <= nstep[0]) {
-    const int bound = 1 + K * (int)div_up(t0 - 1, K);  // next checkpoint time >= t0
-    const int NS = KB > 1 ? std::min({KB, bound - t0 + 1, nstep[0] - t0 + 1}) : 1;
-    const int t1 = t0 + NS - 1;
-    const int na = shots_with_nstep_ge(t0);
-    // checkpoint s >= 1 holds the state before step a_s = 2 + s K, i.e. after
-    // t = 1 + s K; resident segments need none
-    int ck = ((t1 - 1) % K == 0) ? (t1 - 1) / K : 0;
-    if (ck >= res_seg) ck = 0;
-    const bool res = t0 >= a_res;
-    if (count) {
-      const int nl = (KB > 1 ? 1 : tf.launches(na)) + (t0 == a_res ? 1 : 0);
-      *count += nl;
-      tcount[0] += nl;
-      for (int t = t0; t <= t1; t++) tcount[1] += (double)cells_upto(shots_with_nstep_ge(t));
-    } else if (KB > 1) {
-      if (int e = launch_tb(st, false, tb_items_upto(na), t0, NS, 0, blk & 1, ck)) return e;
-    } else {
-      if (t0 == a_res) {  // u_{a-2}, u_{a-1} into the resident slots
-        k_ac_seed<T><<<dim3(kRowBlocks, na), 256, 0, st>>>(d_shots, a_res, res_base);
-        ADS_LAUNCHED(1);
-      }
-      if (int e = launch_fwd(st, res ? 2 : 0, na, t0, res ? res_base : 0, ck)) return e;
+  const int nc = chains();
+  cudaStream_t q[kChains] = {};
+  if (!count)
+    if (int e = fork_chains(st, q)) return e;
+  for (size_t round = 0; round < rounds(); round++) {
+    int g[kChains], last = 0;  // the chains' groups (-1: none left), their longest record
+    for (int c = 0; c < nc; c++) {
+      g[c] = round < chain_groups[c].size() ? chain_groups[c][round] : -1;
+      if (g[c] >= 0) last = std::max(last, nstep[gb[g[c]]]);
     }
-    t0 = t1 + 1;
-    blk++;
+    int t0 = 2, blk = 0;
+    while (t0 <= last) {
+      const int bound = 1 + K * (int)div_up(t0 - 1, K);  // next checkpoint time >= t0
+      const int NS = KB > 1 ? std::min({KB, bound - t0 + 1, last - t0 + 1}) : 1;
+      const int t1 = t0 + NS - 1;
+      // checkpoint s >= 1 holds the state before step a_s = 2 + s K, i.e. after
+      // t = 1 + s K; resident segments need none
+      int ck = ((t1 - 1) % K == 0) ? (t1 - 1) / K : 0;
+      if (ck >= res_seg) ck = 0;
+      const bool res = t0 >= a_res;
+      for (int c = 0; c < nc; c++) {
+        if (g[c] < 0) continue;
+        const int s0 = gb[g[c]], s1 = std::min(gb[g[c] + 1], shots_with_nstep_ge(t0));
+        if (s1 <= s0) continue;
+        if (count) {
+          const int nl = (KB > 1 ? 1 : tf.launches(s0, s1)) + (t0 == a_res ? 1 : 0);
+          *count += nl;
+          tcount[0] += nl;
+          for (int t = t0; t <= t1; t++)
+            tcount[1] += (double)cells_of(s0, std::min(s1, shots_with_nstep_ge(t)));
+        } else if (KB > 1) {  // (one group)
+          if (int e = launch_tb(st, false, tb_items_upto(s1), t0, NS, 0, blk & 1, ck)) return e;
+        } else {
+          if (t0 == a_res) {  // u_{a-2}, u_{a-1} into the resident slots
+            k_ac_seed<T><<<dim3(kRowBlocks, s1 - s0), 256, 0, q[c]>>>(d_shots + s0, a_res,
+                                                                      res_base);
+            ADS_LAUNCHED(1);
+          }
+          if (int e = launch_fwd(q[c], res ? 2 : 0, s0, s1, t0, res ? res_base : 0, ck, c))
+            return e;
+        }
+      }
+      t0 = t1 + 1;
+      blk++;
+    }
   }
+  if (!count)
+    if (int e = join_chains(st)) return e;
   if (!count && timing_run) ADS_CUDA(cudaEventRecord(ev[1], st));
   return ADS_OK;
 }
 
-// Reverse sweep: zero adjoint state, seed lambdaU_T, then per segment from the
-// last: restore, recompute, adjoint steps.
+// Reverse sweep: zero adjoint state, seed lambdaU_T, then for the chains' groups per
+// segment from the last: restore, recompute, adjoint steps.
 template <typename T>
 int AcPlan<T>::issue_reverse(cudaStream_t st, int64_t* count) {
   int64_t n = 0;
@@ -4068,70 +5097,108 @@ int AcPlan<T>::issue_reverse(cudaStream_t st, int64_t* count) {
     ADS_LAUNCHED(1);
   }
   n++;
-  for (int s = nseg_max - 1; s >= 0; s--) {
-    const int a = 2 + s * K;
-    // shots whose record reaches step a
-    const int na = shots_with_nstep_ge(a);
-    if (na == 0) continue;
-    const int b_max = std::min(a + K - 1, nstep[0]);
-    const bool res = s >= res_seg;  // resident: the store already holds the segment
-    const int base = res ? res_base : a - 2;
-    if (!res) {
-      if (!count) {
-        // phi / psi set the recompute's first step reads: variant W's step a
-        // reads set (a-1) & 1; variant U's pre-pass of step a reads set a & 1
-        k_ac_restore<T><<<dim3(kRowBlocks, na), 256, 0, st>>>(
-            d_shots, s, a, KB > 1 ? 0 : (vu ? (a & 1) : -1), inc ? 1 : 0);
-        ADS_LAUNCHED(1);
-      }
-      n++;
+  const int nc = chains();
+  cudaStream_t q[kChains] = {};
+  if (!count)
+    if (int e = fork_chains(st, q)) return e;
+  for (size_t round = 0; round < rounds(); round++) {
+    int g[kChains], last = 0;
+    for (int c = 0; c < nc; c++) {
+      g[c] = round < chain_groups[c].size() ? chain_groups[c][round] : -1;
+      if (g[c] >= 0) last = std::max(last, nstep[gb[g[c]]]);
     }
-    const bool timed = s == seg_timed;
-    if (timed && timing_run) ADS_CUDA(cudaEventRecord(ev[2], st));
-    if (timed && count) tcount[2] = tcount[3] = tcount[4] = tcount[5] = 0;
-    for (int t0 = a, blk = 0; !res && t0 <= b_max - 1; blk++) {
-      // active while t < b_shot = min(a+K-1, nstep), i.e. nstep >= t+1
-      const int NS = KB > 1 ? std::min(KB, b_max - t0) : 1;
-      const int nt = shots_with_nstep_ge(t0 + 1);
-      const int nl = KB > 1 ? 1 : tf.launches(nt);
-      if (timed && count) {
-        tcount[2] += nl;
-        for (int t = t0; t < t0 + NS; t++) tcount[3] += (double)cells_upto(shots_with_nstep_ge(t + 1));
-      }
-      if (!count) {
-        if (KB > 1) {
-          if (int e = launch_tb(st, true, tb_items_upto(nt), t0, NS, a - 2, blk & 1, 0)) return e;
-        } else {
-          if (int e = launch_fwd(st, 1, nt, t0, a - 2, 0)) return e;
+    const bool first = round == 0;  // profile() times the first round's segment
+    for (int s = nseg_max - 1; s >= 0; s--) {
+      const int a = 2 + s * K;
+      if (last < a) continue;  // no shot's record reaches step a
+      const int b_max = std::min(a + K - 1, last);
+      const bool res = s >= res_seg;  // resident: the store already holds the segment
+      const int base = res ? res_base : a - 2;
+      // shots of chain c whose record reaches step t: [from(c), upto(c, t))
+      auto from = [&](int c) { return g[c] >= 0 ? gb[g[c]] : 0; };
+      auto upto = [&](int c, int t) {
+        return g[c] >= 0 ? std::min(gb[g[c] + 1], shots_with_nstep_ge(t)) : 0;
+      };
+      for (int c = 0; c < nc && !res; c++) {
+        const int s0 = from(c), na = upto(c, a) - s0;
+        if (na <= 0) continue;
+        if (!count) {
+          // phi / psi set the recompute's first step reads: variant W's step a
+          // reads set (a-1) & 1; variant U's pre-pass of step a reads set a & 1
+          k_ac_restore<T><<<dim3(kRowBlocks, na), 256, 0, q[c]>>>(
+              d_shots + s0, s, a, KB > 1 ? 0 : (vu ? (a & 1) : -1), inc ? 1 : 0);
+          ADS_LAUNCHED(1);
         }
+        n++;
       }
-      n += nl;
-      t0 += NS;
-    }
-    if (timed && timing_run) {
-      ADS_CUDA(cudaEventRecord(ev[3], st));
-      ADS_CUDA(cudaEventRecord(ev[4], st));
-    }
-    for (int k = b_max; k >= a; k--) {
-      const int nk = shots_with_nstep_ge(k);
-      if (timed && count) {
-        tcount[4] += ta.launches(nk);
-        tcount[5] += (double)cells_upto(nk);
+      const bool timed = first && s == seg_timed;
+      if (timed && timing_run) {
+        if (int e = join_chains(st)) return e;
+        ADS_CUDA(cudaEventRecord(ev[2], st));
+        if (int e = fork_chains(st, q)) return e;
       }
-      if (!count) {
-        if (int e = launch_adj(st, nk, k, base)) return e;
+      if (timed && count) tcount[2] = tcount[3] = tcount[4] = tcount[5] = 0;
+      for (int t0 = a, blk = 0; !res && t0 <= b_max - 1; blk++) {
+        // active while t < b_shot = min(a+K-1, nstep), i.e. nstep >= t+1
+        const int NS = KB > 1 ? std::min(KB, b_max - t0) : 1;
+        for (int c = 0; c < nc; c++) {
+          const int s0 = from(c), s1 = upto(c, t0 + 1);
+          if (s1 <= s0) continue;
+          const int nl = KB > 1 ? 1 : tf.launches(s0, s1);
+          if (timed && count) {
+            tcount[2] += nl;
+            for (int t = t0; t < t0 + NS; t++) tcount[3] += (double)cells_of(s0, upto(c, t + 1));
+          }
+          if (!count) {
+            if (KB > 1) {
+              if (int e = launch_tb(st, true, tb_items_upto(s1), t0, NS, a - 2, blk & 1, 0))
+                return e;
+            } else {
+              if (int e = launch_fwd(q[c], 1, s0, s1, t0, a - 2, 0, c)) return e;
+            }
+          }
+          n += nl;
+        }
+        t0 += NS;
       }
-      n += ta.launches(nk);
-    }
-    if (timed && timing_run) ADS_CUDA(cudaEventRecord(ev[5], st));
-    if (sizeof(T) == 4) {  // fold the segment's FP32 grad_c partial into FP64
-      if (!count) {
-        k_ac_flush_gc<T><<<dim3(kRowBlocks, na), 256, 0, st>>>(d_shots);
-        ADS_LAUNCHED(1);
+      if (timed && timing_run) {
+        if (int e = join_chains(st)) return e;
+        ADS_CUDA(cudaEventRecord(ev[3], st));
+        ADS_CUDA(cudaEventRecord(ev[4], st));
+        if (int e = fork_chains(st, q)) return e;
       }
-      n++;
+      for (int k = b_max; k >= a; k--)
+        for (int c = 0; c < nc; c++) {
+          const int s0 = from(c), s1 = upto(c, k);
+          if (s1 <= s0) continue;
+          if (timed && count) {
+            tcount[4] += ta.launches(s0, s1);
+            tcount[5] += (double)cells_of(s0, s1);
+          }
+          if (!count) {
+            if (int e = launch_adj(q[c], s0, s1, k, base, c)) return e;
+          }
+          n += ta.launches(s0, s1);
+        }
+      if (timed && timing_run) {
+        if (int e = join_chains(st)) return e;
+        ADS_CUDA(cudaEventRecord(ev[5], st));
+        if (int e = fork_chains(st, q)) return e;
+      }
+      for (int c = 0; c < nc && sizeof(T) == 4; c++) {
+        // fold the segment's FP32 grad_c partial into FP64
+        const int s0 = from(c), na = upto(c, a) - s0;
+        if (na <= 0) continue;
+        if (!count) {
+          k_ac_flush_gc<T><<<dim3(kRowBlocks, na), 256, 0, q[c]>>>(d_shots + s0);
+          ADS_LAUNCHED(1);
+        }
+        n++;
+      }
     }
   }
+  if (!count)
+    if (int e = join_chains(st)) return e;
   if (count) *count = n;
   return ADS_OK;
 }
