@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "ads_internal.h"
+#include "f32x4.h"
 
 namespace ads {
 namespace {
@@ -1744,37 +1745,6 @@ k_ac_adjphi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
 // place.  The three-level form rounds Q relative to itself, which builds up like
 // eps sqrt(N) / (w dt); here the rounding is relative to p, as the forward's is to d.
 // ---------------------------------------------------------------------------
-struct alignas(16) F4 {
-  float2 a, b;
-};
-__device__ __forceinline__ float2 add2(float2 x, float2 y) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "add.rn.f32x2 r, x, y;\n\tmov.b64 {%0, %1}, r;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-  return r;
-}
-__device__ __forceinline__ float2 mul2(float2 x, float2 y) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "mul.rn.f32x2 r, x, y;\n\tmov.b64 {%0, %1}, r;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y));
-  return r;
-}
-__device__ __forceinline__ float2 fma2(float2 x, float2 y, float2 z) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, z, r;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
-      "mov.b64 z, {%6, %7};\n\tfma.rn.f32x2 r, x, y, z;\n\tmov.b64 {%0, %1}, r;\n\t}"
-      : "=f"(r.x), "=f"(r.y)
-      : "f"(x.x), "f"(x.y), "f"(y.x), "f"(y.y), "f"(z.x), "f"(z.y));
-  return r;
-}
-__device__ __forceinline__ float2 sub2(float2 x, float2 y) {  // x - y
-  return fma2(y, make_float2(-1.f, -1.f), x);
-}
-
 // cx ((x_p - x_0) + (x_m - x_0)) + cy ((x_r - x_0) + (x_l - x_0)) of a lane's four cells:
 // rows m, 0, p; l, r the columns beside them.
 __device__ __forceinline__ F4 lap4(const F4& m, const F4& z, const F4& p, float l, float r,
@@ -1787,28 +1757,6 @@ __device__ __forceinline__ F4 lap4(const F4& m, const F4& z, const F4& p, float 
   o.a = fma2(y, ha, mul2(x, add2(sub2(p.a, z.a), sub2(m.a, z.a))));
   o.b = fma2(y, hb, mul2(x, add2(sub2(p.b, z.b), sub2(m.b, z.b))));
   return o;
-}
-
-// A 16-byte load / store at a 32-bit element offset of a field, predicated.
-__device__ __forceinline__ F4 ld4(const float* p, int o, bool on) {
-  F4 x;
-  x.a.x = x.a.y = x.b.x = x.b.y = 0.f;
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\t"
-      "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-      : "+f"(x.a.x), "+f"(x.a.y), "+f"(x.b.x), "+f"(x.b.y)
-      : "l"(p + o), "r"((unsigned)on));
-  return x;
-}
-__device__ __forceinline__ void st4(float* p, int o, const F4& x) {
-  *reinterpret_cast<float4*>(p + o) = make_float4(x.a.x, x.a.y, x.b.x, x.b.y);
-}
-__device__ __forceinline__ float ld1v(const float* p, int o, bool on) {
-  float a = 0.f;
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.f32 %0, [%1];\n\t}"
-               : "+f"(a)
-               : "l"(p + o), "r"((unsigned)on));
-  return a;
 }
 
 // Geometry of a wide item's warp.
@@ -1916,7 +1864,6 @@ k_ac_wide_adj(const AcItem* __restrict__ items, const AcShot<float>* __restrict_
   const float* cc = sh.c;
   const int P = W.P;
   int o = W.i0 * P + W.col;
-  auto mul4 = [](const F4& x, const F4& y) -> F4 { return {mul2(x.a, y.a), mul2(x.b, y.b)}; };
   // rows i-1, i, i+1 of z = c Q and of u_{k-1}; Q of rows i, i+1
   F4 z[4], u[4], Q[2], p[2], g[2];
   float hz[2], hu[2];
@@ -1995,12 +1942,6 @@ __device__ __forceinline__ float2 rcp2(float2 x) {
   const float2 r = make_float2(rcp1(x.x), rcp1(x.y));
   const float2 e = fma2(make_float2(-x.x, -x.y), r, bc2(1.f));
   return fma2(r, e, r);
-}
-__device__ __forceinline__ F4 add4(const F4& x, const F4& y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
-__device__ __forceinline__ F4 sub4(const F4& x, const F4& y) { return {sub2(x.a, y.a), sub2(x.b, y.b)}; }
-__device__ __forceinline__ F4 mul4(const F4& x, const F4& y) { return {mul2(x.a, y.a), mul2(x.b, y.b)}; }
-__device__ __forceinline__ F4 fma4(const F4& x, const F4& y, const F4& z) {
-  return {fma2(x.a, y.a, z.a), fma2(x.b, y.b, z.b)};
 }
 // s x + z and x s + t for scalars
 __device__ __forceinline__ F4 axpy4(float s, const F4& x, const F4& z) {

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "ads_internal.h"
+#include "f32x4.h"
 
 namespace ads {
 namespace {
@@ -81,12 +82,12 @@ struct ElShot {
 // ---------------------------------------------------------------------------
 // One-thread-per-cell kernels: the single-step operators (both precisions), the
 // FP64 plans, and the FP32 plans whose shots hold too few cells for the
-// row-streaming kernels below.
+// row-streaming kernels below (kCellMax32).
 //
 // A step is two kernels (stresses: fw1, fw2; velocities: fw3, fw4), its transpose
 // two more.  FP64 kernels are bound by the count of FP64 instructions (a warp's
 // instruction holds the pipe of its SM sub-partition for 64 cycles), so:
-//  * the four-point difference is 27/(24h) (a - b) - 1/(24h) (c - d): 4
+//  * the four-point difference is (27 (a - b) - (c - d)) times 1/(24h): 4
 //    operations and no division (a division is some twenty);
 //  * plans fold dt into tables of the averaged moduli and of dt / density
 //    (k_el_tables, once a call), 42 operations a CPML-free cell and step;
@@ -101,7 +102,7 @@ struct ElShot {
 //    (k_el_gather_cells), which is the same sum in another order.
 // No row or column is computed twice, and a grid of 47 k cells already gives every
 // SM ten warps, where a strip of rows leaves most of the chip idle: the FP64
-// gradient of 2 shots of 253 x 187, 250 steps, takes 11.6 ms, 113 ms with the
+// gradient of 2 shots of 253 x 187, 250 steps, takes 11.2 ms, 113 ms with the
 // row-streaming kernels (FP64 pipe 64% busy in these kernels there); the operator
 // and its transpose on 600 x 300 FP64 take 20 + 22 and 19 + 55 + 43 us (FP64 pipe
 // 74-82% busy).
@@ -116,7 +117,7 @@ struct CellModel {
   const T *lm, *la, *m2, *b3, *b4;         // plans: the tables
   const T *axi, *axh, *bxi, *bxh, *ayi, *ayh, *byi, *byh;  // 1D, index I-1 / J-1
   T dt, rdt;                               // dt, 1 / dt
-  T x27, x1, y27, y1;                      // 27 / (24 h), 1 / (24 h)
+  T x1, y1;                                // 1 / (24 h)
   double dtd;                              // dt, unrounded
   int NX, NY, OFF, P;
 };
@@ -139,10 +140,11 @@ __device__ __forceinline__ bool el_tame(float x) {
   return (__float_as_int(x) & 0x7f800000) < 0x7f000000;
 }
 
-// 27 (a - b) / (24 h) - (c - d) / (24 h)
+// (27 (a - b) - (c - d)) / (24 h).  27/(24h) and 1/(24h)
+// rounded apart cost as much and leave weights that are no longer 27 : 1.
 template <typename T>
-__device__ __forceinline__ T dif(T a, T b, T c, T d, T k27, T k1) {
-  return el_fma(k27, a - b, -(k1 * (c - d)));
+__device__ __forceinline__ T dif(T a, T b, T c, T d, T k1) {
+  return k1 * el_fma(T(27), a - b, d - c);
 }
 
 // The strain or acceleration d + m' of one difference d, with its memory
@@ -236,8 +238,8 @@ __device__ __forceinline__ void strain1(const CellModel<T>& M, int i, int j, Cel
   const T* vx = f + VX * fs;
   const T* vy = f + VY * fs;
   const int P = M.P;
-  const T a = dif<T>(vx[x + P], vx[x], vx[x + 2 * P], vx[x - P], M.x27, M.x1);
-  const T b = dif<T>(vy[x], vy[x - 1], vy[x + 1], vy[x - 2], M.y27, M.y1);
+  const T a = dif<T>(vx[x + P], vx[x], vx[x + 2 * P], vx[x - P], M.x1);
+  const T b = dif<T>(vy[x], vy[x - 1], vy[x + 1], vy[x - 2], M.y1);
   e1 = mem_fwd<T, PLAN>(a, M.axh[i - 1], M.bxh[i - 1], f + M1 * fs, fo ? fo + M1 * fs : nullptr, x);
   e2 = mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 1) * fs,
                         fo ? fo + (M1 + 1) * fs : nullptr, x);
@@ -248,8 +250,8 @@ __device__ __forceinline__ T strain2(const CellModel<T>& M, int i, int j, CellIx
   const T* vx = f + VX * fs;
   const T* vy = f + VY * fs;
   const int P = M.P;
-  const T a = dif<T>(vy[x], vy[x - P], vy[x + P], vy[x - 2 * P], M.x27, M.x1);
-  const T b = dif<T>(vx[x + 1], vx[x], vx[x + 2], vx[x - 1], M.y27, M.y1);
+  const T a = dif<T>(vy[x], vy[x - P], vy[x + P], vy[x - 2 * P], M.x1);
+  const T b = dif<T>(vx[x + 1], vx[x], vx[x + 2], vx[x - 1], M.y1);
   return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 2) * fs,
                           fo ? fo + (M1 + 2) * fs : nullptr, x) +
          mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 3) * fs,
@@ -259,8 +261,8 @@ template <typename T, bool PLAN>
 __device__ __forceinline__ T accel3(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxx,
                                     const T* sxy, const T* f, int64_t fs, T* fo) {
   const int P = M.P;
-  const T a = dif<T>(sxx[x], sxx[x - P], sxx[x + P], sxx[x - 2 * P], M.x27, M.x1);
-  const T b = dif<T>(sxy[x], sxy[x - 1], sxy[x + 1], sxy[x - 2], M.y27, M.y1);
+  const T a = dif<T>(sxx[x], sxx[x - P], sxx[x + P], sxx[x - 2 * P], M.x1);
+  const T b = dif<T>(sxy[x], sxy[x - 1], sxy[x + 1], sxy[x - 2], M.y1);
   return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 4) * fs,
                           fo ? fo + (M1 + 4) * fs : nullptr, x) +
          mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 5) * fs,
@@ -270,8 +272,8 @@ template <typename T, bool PLAN>
 __device__ __forceinline__ T accel4(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxy,
                                     const T* syy, const T* f, int64_t fs, T* fo) {
   const int P = M.P;
-  const T a = dif<T>(sxy[x + P], sxy[x], sxy[x + 2 * P], sxy[x - P], M.x27, M.x1);
-  const T b = dif<T>(syy[x + 1], syy[x], syy[x + 2], syy[x - 1], M.y27, M.y1);
+  const T a = dif<T>(sxy[x + P], sxy[x], sxy[x + 2 * P], sxy[x - P], M.x1);
+  const T b = dif<T>(syy[x + 1], syy[x], syy[x + 2], syy[x - 1], M.y1);
   return mem_fwd<T, PLAN>(a, M.axh[i - 1], M.bxh[i - 1], f + (M1 + 6) * fs,
                           fo ? fo + (M1 + 6) * fs : nullptr, x) +
          mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 7) * fs,
@@ -288,22 +290,191 @@ __device__ __forceinline__ T accel4(const CellModel<T>& M, int i, int j, CellIx<
   const CellIx<(FIRST) != 0> x = (CellIx<(FIRST) != 0>)i * P + j + M.OFF;      \
   (void)P, (void)x
 
+// A plan's block: a tile of BY x BX cells at (i0, j0), a thread a cell (w = 0), or an
+// interior strip of w columns (a multiple of 4, at most 120) from j0 = 1 mod 4 and
+// rows >> 16 rows from i0, (rows & 0xffff) of them a warp (k_el_* wide parts, FP32).
+struct CellItem {
+  int i0, j0, w, rows;
+};
+
+// ---- FP32 interior strips: four columns a lane, rows walked by a warp
+//
+// The one-thread-per-cell form issues about 10 instructions a cell and kernel in FP32:
+// addresses, loads, box and profile tests, one cell's worth each.  Away from the CPML
+// and the boxes' edges none of the tests remain; four columns share a 16-byte load, the
+// arithmetic runs on packed pairs, and a row's four-row stencil is carried in registers.
+// The first and the last active lane only feed their neighbours (so a strip is 120 of a
+// warp's 128 columns), which leaves no edge case.  The strips run beside the cell tiles
+// of the frame, each kernel with its own registers (in one kernel the tiles, too, would
+// get two blocks a SM: 16 shots of 600 x 300 133 us a forward step instead of 72).  A
+// strip form of the CPML cells issues a quarter of the instructions but waits on its
+// loads row by row: gradient step of 700 k cells 70 us instead of 45.
+struct Span {
+  int x, m, P;    // offset of the lane's first cell in the warp's first row; rows; pitch
+  bool on, out;   // the lane loads; it stores
+  __device__ __forceinline__ Span(const CellItem& it, int P_, int off) {
+    const int lane = threadIdx.x, n = it.w >> 2, r = it.rows & 0xffff;
+    const int d = (int)threadIdx.y * r;
+    P = P_;
+    m = min(r, (it.rows >> 16) - d);
+    on = lane <= n + 1;
+    out = lane >= 1 && lane <= n;
+    x = (it.i0 + d) * P + it.j0 + 4 * lane - 4 + off;
+  }
+};
+__device__ __forceinline__ F4 dif4(const F4& a, const F4& b, const F4& c, const F4& d, float k1) {
+  const float2 p = make_float2(27.f, 27.f), q = make_float2(k1, k1);
+  return {mul2(q, fma2(p, sub2(a.a, b.a), sub2(d.a, c.a))),
+          mul2(q, fma2(p, sub2(a.b, b.b), sub2(d.b, c.b)))};
+}
+// the four-point difference one half cell up (rows or columns -1 .. 2) ...
+__device__ __forceinline__ F4 up_i(const F4& m, const F4& z, const F4& p, const F4& pp, float k1) {
+  return dif4(p, z, pp, m, k1);
+}
+__device__ __forceinline__ F4 up_j(const F4& v, float k1) {
+  const float l1 = __shfl_up_sync(~0u, v.b.y, 1), r1 = __shfl_down_sync(~0u, v.a.x, 1),
+              r2 = __shfl_down_sync(~0u, v.a.y, 1);
+  return dif4({{v.a.y, v.b.x}, {v.b.y, r1}}, v, {{v.b.x, v.b.y}, {r1, r2}},
+              {{l1, v.a.x}, {v.a.y, v.b.x}}, k1);
+}
+// ... and one half cell down (-2 .. 1)
+__device__ __forceinline__ F4 down_i(const F4& mm, const F4& m, const F4& z, const F4& p,
+                                     float k1) {
+  return dif4(z, m, p, mm, k1);
+}
+__device__ __forceinline__ F4 down_j(const F4& v, float k1) {
+  const float l1 = __shfl_up_sync(~0u, v.b.y, 1), l2 = __shfl_up_sync(~0u, v.b.x, 1),
+              r1 = __shfl_down_sync(~0u, v.a.x, 1);
+  return dif4(v, {{l1, v.a.x}, {v.a.y, v.b.x}}, {{v.a.y, v.b.x}, {v.b.y, r1}},
+              {{l2, l1}, {v.a.x, v.a.y}}, k1);
+}
+
+template <bool STORE>
+__global__ void __launch_bounds__(BX* BY, 2)
+k_el_strip_stress(CellModel<float> M, const ElShot<float>* __restrict__ shots,
+    const CellItem* __restrict__ items, int pin, int slot) {
+  const CellItem it = items[blockIdx.x];
+  const ElShot<float>& sh = shots[blockIdx.y];
+  const Span S(it, M.P, M.OFF);
+  const int64_t fs = sh.fs;
+  const float* f = sh.f[0] + (int64_t)pin * NF * fs;
+  float* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
+  float* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  const float *vx = f + VX * fs, *vy = f + VY * fs;
+  const int P = S.P;
+  if (S.m <= 0) return;
+  int x = S.x;
+  F4 X[4], Y[4];  // vx of rows i-1 .. i+2, vy of rows i-2 .. i+1
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    X[k] = ld4(vx, x + (k - 1) * P, S.on);
+    Y[k] = ld4(vy, x + (k - 2) * P, S.on);
+  }
+  for (int r = 0; r < S.m; r += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (r + k >= S.m) break;  // (uniform)
+      X[(k + 3) & 3] = ld4(vx, x + 2 * P, S.on);
+      Y[(k + 3) & 3] = ld4(vy, x + P, S.on);
+      const F4 lm = ld4(M.lm, x, S.out), la = ld4(M.la, x, S.out), m2 = ld4(M.m2, x, S.out);
+      const F4 sxx = ld4(f + SXX * fs, x, S.out), syy = ld4(f + SYY * fs, x, S.out),
+               sxy = ld4(f + SXY * fs, x, S.out);
+      const F4 &x0 = X[(k + 1) & 3], &y0 = Y[(k + 2) & 3];
+      const F4 e1 = up_i(X[k & 3], x0, X[(k + 2) & 3], X[(k + 3) & 3], M.x1);
+      const F4 e2 = down_j(y0, M.y1);
+      const F4 e3 = add4(down_i(Y[k & 3], Y[(k + 1) & 3], y0, Y[(k + 3) & 3], M.x1),
+                         up_j(x0, M.y1));
+      if (S.out) {
+        st4(o + SXX * fs, x, fma4(lm, e1, fma4(la, e2, sxx)));
+        st4(o + SYY * fs, x, fma4(lm, e2, fma4(la, e1, syy)));
+        st4(o + SXY * fs, x, fma4(m2, e3, sxy));
+        if (STORE) {
+          st4(st + E1 * fs, x, e1);
+          st4(st + E2 * fs, x, e2);
+          st4(st + E12 * fs, x, e3);
+        }
+      }
+      x += P;
+    }
+  }
+}
+
+template <bool STORE>
+__global__ void __launch_bounds__(BX* BY, 2)
+k_el_strip_velocity(CellModel<float> M, const ElShot<float>* __restrict__ shots,
+    const CellItem* __restrict__ items, int pin, int slot) {
+  const CellItem it = items[blockIdx.x];
+  const ElShot<float>& sh = shots[blockIdx.y];
+  const Span S(it, M.P, M.OFF);
+  const int64_t fs = sh.fs;
+  const float* f = sh.f[0] + (int64_t)pin * NF * fs;
+  float* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
+  float* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  const float *sxx = o + SXX * fs, *syy = o + SYY * fs, *sxy = o + SXY * fs;
+  const int P = S.P;
+  if (S.m <= 0) return;
+  int x = S.x;
+  F4 X[4], Y[4];  // sxy of rows i-1 .. i+2, sxx of rows i-2 .. i+1
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    X[k] = ld4(sxy, x + (k - 1) * P, S.on);
+    Y[k] = ld4(sxx, x + (k - 2) * P, S.on);
+  }
+  for (int r = 0; r < S.m; r += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (r + k >= S.m) break;
+      X[(k + 3) & 3] = ld4(sxy, x + 2 * P, S.on);
+      Y[(k + 3) & 3] = ld4(sxx, x + P, S.on);
+      const F4 z = ld4(syy, x, S.on);
+      const F4 b3 = ld4(M.b3, x, S.out), b4 = ld4(M.b4, x, S.out);
+      const F4 vx = ld4(f + VX * fs, x, S.out), vy = ld4(f + VY * fs, x, S.out);
+      const F4& x0 = X[(k + 1) & 3];
+      const F4 a3 = add4(down_i(Y[k & 3], Y[(k + 1) & 3], Y[(k + 2) & 3], Y[(k + 3) & 3], M.x1),
+                         down_j(x0, M.y1));
+      const F4 a4 = add4(up_i(X[k & 3], x0, X[(k + 2) & 3], X[(k + 3) & 3], M.x1),
+                         up_j(z, M.y1));
+      if (S.out) {
+        st4(o + VX * fs, x, fma4(b3, a3, vx));
+        st4(o + VY * fs, x, fma4(b4, a4, vy));
+        if (STORE) {
+          st4(st + A3 * fs, x, a3);
+          st4(st + A4 * fs, x, a4);
+        }
+      }
+      x += P;
+    }
+  }
+}
+
 // ---- plans: state buffer pin -> the other, only cells a stencil updates
+#define ADS_EL_ITEM()                                                          \
+  const CellItem it = items[blockIdx.x];                                       \
+  const ElShot<T>& sh = shots[blockIdx.y]
+#define ADS_EL_PLAN_CELL()                                                     \
+  const int tx = threadIdx.x, ty = threadIdx.y, i0 = it.i0, j0 = it.j0;        \
+  const int i = i0 + ty, j = j0 + tx, P = M.P, x = i * P + j + M.OFF;          \
+  (void)P, (void)x
 
 template <typename T, bool STORE>
 __global__ void __launch_bounds__(BX* BY)
-k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
-  const ElShot<T>& sh = shots[blockIdx.z];
-  ADS_EL_CELL(1);
+k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
+                 const CellItem* __restrict__ items, int pin, int slot) {
+  ADS_EL_ITEM();
+  ADS_EL_PLAN_CELL();
   if (i > M.NX || j > M.NY) return;
   const int64_t fs = sh.fs;
   const T* f = sh.f[0] + (int64_t)pin * NF * fs;
   T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
   T* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  T lm = T(0), la = T(0), m2 = T(0);
+  if (box1(M, i, j)) mat1<T, true>(M, x, lm, la);
+  if (box2(M, i, j)) m2 = mat2<T, true>(M, x);
+  grid_wait();
+  grid_release();
   if (box1(M, i, j)) {
-    T e1, e2, lm, la;
+    T e1, e2;
     strain1<T, true>(M, i, j, x, f, fs, o, e1, e2);
-    mat1<T, true>(M, x, lm, la);
     o[SXX * fs + x] = el_fma(lm, e1, el_fma(la, e2, f[SXX * fs + x]));
     o[SYY * fs + x] = el_fma(lm, e2, el_fma(la, e1, f[SYY * fs + x]));
     if (STORE) {
@@ -313,29 +484,34 @@ k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, i
   }
   if (box2(M, i, j)) {
     const T e = strain2<T, true>(M, i, j, x, f, fs, o);
-    o[SXY * fs + x] = el_fma(mat2<T, true>(M, x), e, f[SXY * fs + x]);
+    o[SXY * fs + x] = el_fma(m2, e, f[SXY * fs + x]);
     if (STORE) st[E12 * fs + x] = e;
   }
 }
 
 template <typename T, bool STORE>
 __global__ void __launch_bounds__(BX* BY)
-k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
-  const ElShot<T>& sh = shots[blockIdx.z];
-  ADS_EL_CELL(1);
+k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
+                   const CellItem* __restrict__ items, int pin, int slot) {
+  ADS_EL_ITEM();
+  ADS_EL_PLAN_CELL();
   if (i > M.NX || j > M.NY) return;
   const int64_t fs = sh.fs;
   const T* f = sh.f[0] + (int64_t)pin * NF * fs;
   T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
   T* st = STORE ? sh.store + (int64_t)slot * NSTORE * fs : nullptr;
+  const T b3 = box3(M, i, j) ? mat3<T, true>(M, x) : T(0),
+          b4 = box4(M, i, j) ? mat4<T, true>(M, x) : T(0);
+  grid_wait();
+  grid_release();
   if (box3(M, i, j)) {
     const T e = accel3<T, true>(M, i, j, x, o + SXX * fs, o + SXY * fs, f, fs, o);
-    o[VX * fs + x] = el_fma(mat3<T, true>(M, x), e, f[VX * fs + x]);
+    o[VX * fs + x] = el_fma(b3, e, f[VX * fs + x]);
     if (STORE) st[A3 * fs + x] = e;
   }
   if (box4(M, i, j)) {
     const T e = accel4<T, true>(M, i, j, x, o + SXY * fs, o + SYY * fs, f, fs, o);
-    o[VY * fs + x] = el_fma(mat4<T, true>(M, x), e, f[VY * fs + x]);
+    o[VY * fs + x] = el_fma(b4, e, f[VY * fs + x]);
     if (STORE) st[A4 * fs + x] = e;
   }
 }
@@ -432,10 +608,10 @@ template <typename T>
 __device__ __forceinline__ void gather_stress(const CellModel<T>& M, const SendV<T>& S, T& sxx,
                                               T& syy, T& sxy) {
   const int r = threadIdx.y, q = threadIdx.x;
-  sxx += dif<T>(S.d5[r + 1][q], S.d5[r + 2][q], S.d5[r][q], S.d5[r + 3][q], M.x27, M.x1);
-  sxy += dif<T>(S.d6[r][q + 1], S.d6[r][q + 2], S.d6[r][q], S.d6[r][q + 3], M.y27, M.y1);
-  sxy += dif<T>(S.d7[r + 1][q], S.d7[r + 2][q], S.d7[r][q], S.d7[r + 3][q], M.x27, M.x1);
-  syy += dif<T>(S.d8[r][q + 1], S.d8[r][q + 2], S.d8[r][q], S.d8[r][q + 3], M.y27, M.y1);
+  sxx += dif<T>(S.d5[r + 1][q], S.d5[r + 2][q], S.d5[r][q], S.d5[r + 3][q], M.x1);
+  sxy += dif<T>(S.d6[r][q + 1], S.d6[r][q + 2], S.d6[r][q], S.d6[r][q + 3], M.y1);
+  sxy += dif<T>(S.d7[r + 1][q], S.d7[r + 2][q], S.d7[r][q], S.d7[r + 3][q], M.x1);
+  syy += dif<T>(S.d8[r][q + 1], S.d8[r][q + 2], S.d8[r][q], S.d8[r][q + 3], M.y1);
 }
 
 // Fills SendS from the stress adjoints s (sxx, syy, sxy at fields SXX..SXY of
@@ -486,10 +662,10 @@ template <typename T>
 __device__ __forceinline__ void gather_velocity(const CellModel<T>& M, const SendS<T>& S, T& vx,
                                                 T& vy) {
   const int r = threadIdx.y, q = threadIdx.x;
-  vx += dif<T>(S.d1[r + 1][q], S.d1[r + 2][q], S.d1[r][q], S.d1[r + 3][q], M.x27, M.x1);
-  vx += dif<T>(S.d4[r][q + 1], S.d4[r][q + 2], S.d4[r][q], S.d4[r][q + 3], M.y27, M.y1);
-  vy += dif<T>(S.d2[r][q + 1], S.d2[r][q + 2], S.d2[r][q], S.d2[r][q + 3], M.y27, M.y1);
-  vy += dif<T>(S.d3[r + 1][q], S.d3[r + 2][q], S.d3[r][q], S.d3[r + 3][q], M.x27, M.x1);
+  vx += dif<T>(S.d1[r + 1][q], S.d1[r + 2][q], S.d1[r][q], S.d1[r + 3][q], M.x1);
+  vx += dif<T>(S.d4[r][q + 1], S.d4[r][q + 2], S.d4[r][q], S.d4[r][q + 3], M.y1);
+  vy += dif<T>(S.d2[r][q + 1], S.d2[r][q + 2], S.d2[r][q], S.d2[r][q + 3], M.y1);
+  vy += dif<T>(S.d3[r + 1][q], S.d3[r + 2][q], S.d3[r][q], S.d3[r + 3][q], M.x1);
 }
 
 // The sums a cell-kernel plan's gradients are formed from, one field each: FP64
@@ -506,17 +682,132 @@ __device__ __forceinline__ void add_cell(const ElShot<T>& sh, int k, int x, T a,
   }
 }
 
+// The interior strips' adjoint step (as strip_stress): with no memory variable D5 = D6 =
+// b3 gvx and D7 = D8 = b4 gvy, and the gathers are the forward's differences negated.
+__device__ __forceinline__ void acc4(float* p, int64_t fs, int k, int x, const F4& a, const F4& b) {
+  float* q = p + (int64_t)k * fs;
+  st4(q, x, fma4(a, b, ld4(q, x, true)));
+}
+
+__global__ void __launch_bounds__(BX* BY, 2)
+k_el_strip_adj_stress(CellModel<float> M, const ElShot<float>* __restrict__ shots,
+    const CellItem* __restrict__ items, int pin, int slot) {
+  const CellItem it = items[blockIdx.x];
+  const ElShot<float>& sh = shots[blockIdx.y];
+  const Span S(it, M.P, M.OFF);
+  const int64_t fs = sh.fs;
+  const float* g = sh.g[0] + (int64_t)pin * NF * fs;
+  float* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  const float* st = sh.store + (int64_t)slot * NSTORE * fs;
+  const float *gx = g + VX * fs, *gy = g + VY * fs;
+  const int P = S.P;
+  if (S.m <= 0) return;
+  int x = S.x;
+  F4 X[4], Y[4];  // b3 gvx of rows i-1 .. i+2, b4 gvy of rows i-2 .. i+1
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    X[k] = mul4(ld4(gx, x + (k - 1) * P, S.on), ld4(M.b3, x + (k - 1) * P, S.on));
+    Y[k] = mul4(ld4(gy, x + (k - 2) * P, S.on), ld4(M.b4, x + (k - 2) * P, S.on));
+  }
+  for (int r = 0; r < S.m; r += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (r + k >= S.m) break;
+      const F4 nx = ld4(gx, x + 2 * P, S.on), nb3 = ld4(M.b3, x + 2 * P, S.on),
+               ny = ld4(gy, x + P, S.on), nb4 = ld4(M.b4, x + P, S.on);
+      const F4 sxx = ld4(g + SXX * fs, x, S.out), syy = ld4(g + SYY * fs, x, S.out),
+               sxy = ld4(g + SXY * fs, x, S.out);
+      const F4 a3 = ld4(st + A3 * fs, x, S.out), a4 = ld4(st + A4 * fs, x, S.out);
+      X[(k + 3) & 3] = mul4(nx, nb3);
+      Y[(k + 3) & 3] = mul4(ny, nb4);
+      const F4 &x0 = X[(k + 1) & 3], &y0 = Y[(k + 2) & 3];
+      const F4 d5 = up_i(X[k & 3], x0, X[(k + 2) & 3], X[(k + 3) & 3], M.x1);
+      const F4 d6 = up_j(x0, M.y1);
+      const F4 d7 = down_i(Y[k & 3], Y[(k + 1) & 3], y0, Y[(k + 3) & 3], M.x1);
+      const F4 d8 = down_j(y0, M.y1);
+      if (S.out) {
+        st4(o + SXX * fs, x, sub4(sxx, d5));
+        st4(o + SXY * fs, x, sub4(sub4(sxy, d6), d7));
+        st4(o + SYY * fs, x, sub4(syy, d8));
+        acc4(sh.cacc32, fs, CR3, x, x0, a3);
+        acc4(sh.cacc32, fs, CR4, x, y0, a4);
+      }
+      x += P;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(BX* BY, 2)
+k_el_strip_adj_velocity(CellModel<float> M, const ElShot<float>* __restrict__ shots,
+    const CellItem* __restrict__ items, int pin, int slot) {
+  const CellItem it = items[blockIdx.x];
+  const ElShot<float>& sh = shots[blockIdx.y];
+  const Span S(it, M.P, M.OFF);
+  const int64_t fs = sh.fs;
+  const float* g = sh.g[0] + (int64_t)pin * NF * fs;
+  float* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  const float* st = sh.store + (int64_t)slot * NSTORE * fs;
+  const float *sxx = o + SXX * fs, *syy = o + SYY * fs, *sxy = o + SXY * fs;
+  const int P = S.P;
+  if (S.m <= 0) return;
+  int x = S.x;
+  // lm gxx + la gyy of rows i-2 .. i+1; m2 gxy of rows i-1 .. i+2; lm gyy + la gxx, gxx and
+  // gyy of rows i, i+1
+  F4 R[4], Z[4], W[2], gx[2], gy[2];
+  auto row = [&](int y, F4& r1, F4& r2, F4& a, F4& b) {
+    const F4 lm = ld4(M.lm, y, S.on), la = ld4(M.la, y, S.on);
+    a = ld4(sxx, y, S.on);
+    b = ld4(syy, y, S.on);
+    r1 = fma4(lm, a, mul4(la, b));
+    r2 = fma4(lm, b, mul4(la, a));
+  };
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    row(x + (k - 2) * P, R[k], W[0], gx[0], gy[0]);
+    Z[k] = mul4(ld4(sxy, x + (k - 1) * P, S.on), ld4(M.m2, x + (k - 1) * P, S.on));
+  }
+  for (int r = 0; r < S.m; r += 4) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (r + k >= S.m) break;
+      row(x + P, R[(k + 3) & 3], W[(k + 1) & 1], gx[(k + 1) & 1], gy[(k + 1) & 1]);
+      Z[(k + 3) & 3] = mul4(ld4(sxy, x + 2 * P, S.on), ld4(M.m2, x + 2 * P, S.on));
+      const F4 vx = ld4(g + VX * fs, x, S.out), vy = ld4(g + VY * fs, x, S.out);
+      const F4 e1 = ld4(st + E1 * fs, x, S.out), e2 = ld4(st + E2 * fs, x, S.out),
+               e3 = ld4(st + E12 * fs, x, S.out), gz = ld4(sxy, x, S.out);
+      const F4& z0 = Z[(k + 1) & 3];
+      const F4 d1 = down_i(R[k & 3], R[(k + 1) & 3], R[(k + 2) & 3], R[(k + 3) & 3], M.x1);
+      const F4 d2 = up_j(W[k & 1], M.y1);
+      const F4 d3 = up_i(Z[k & 3], z0, Z[(k + 2) & 3], Z[(k + 3) & 3], M.x1);
+      const F4 d4 = down_j(z0, M.y1);
+      if (S.out) {
+        st4(o + VX * fs, x, sub4(sub4(vx, d1), d4));
+        st4(o + VY * fs, x, sub4(sub4(vy, d2), d3));
+        const F4 &a = gx[k & 1], &b = gy[k & 1];
+        acc4(sh.cacc32, fs, CL, x, add4(e1, e2), add4(a, b));
+        float* q = sh.cacc32 + CM1 * fs;
+        st4(q, x, add4(fma4(e1, a, mul4(e2, b)), ld4(q, x, true)));
+        acc4(sh.cacc32, fs, CM2, x, gz, e3);
+      }
+      x += P;
+    }
+  }
+}
+
 // Adjoint of a step, velocity cells -> stress adjoints (transposes of fw3, fw4):
 // adjoint buffer pin -> the other.
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
-k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
+                     const CellItem* __restrict__ items, int pin, int slot) {
   __shared__ SendV<T> S;
-  const ElShot<T>& sh = shots[blockIdx.z];
-  ADS_EL_CELL(1);
+  ADS_EL_ITEM();
+  ADS_EL_PLAN_CELL();
   const int64_t fs = sh.fs;
   const T* g = sh.g[0] + (int64_t)pin * NF * fs;
   T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  grid_wait();
+  grid_release();
   T q3, q4;
   send_velocity<T, true>(M, S, i0, j0, g, o, fs, q3, q4);
   const T* st = sh.store + (int64_t)slot * NSTORE * fs;
@@ -537,13 +828,16 @@ k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pi
 // Adjoint of a step, stress cells -> velocity adjoints (transposes of fw1, fw2).
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
-k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots, int pin, int slot) {
+k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
+                       const CellItem* __restrict__ items, int pin, int slot) {
   __shared__ SendS<T> S;
-  const ElShot<T>& sh = shots[blockIdx.z];
-  ADS_EL_CELL(1);
+  ADS_EL_ITEM();
+  ADS_EL_PLAN_CELL();
   const int64_t fs = sh.fs;
   const T* g = sh.g[0] + (int64_t)pin * NF * fs;
   T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
+  grid_wait();
+  grid_release();
   send_stress<T, true>(M, S, i0, j0, o, g, o, fs);
   const T* st = sh.store + (int64_t)slot * NSTORE * fs;
   if (box1(M, i, j)) {
@@ -809,9 +1103,7 @@ CellModel<T> make_cells(int NX, int NY, int64_t P, int off, double dt, double dx
   M.dt = (T)dt;
   M.rdt = (T)(1.0 / dt);
   M.dtd = dt;
-  M.x27 = (T)(27.0 / (24 * dx));
   M.x1 = (T)(1.0 / (24 * dx));
-  M.y27 = (T)(27.0 / (24 * dy));
   M.y1 = (T)(1.0 / (24 * dy));
   M.NX = NX;
   M.NY = NY;
@@ -2372,25 +2664,37 @@ __global__ void k_el_flush_acc(const ElShot<float>* __restrict__ shots, int64_t 
 // Sources of slot n (added in order by one thread), then receivers of slot n.
 // par: the state buffer holding slot n (0 for in-place plans); a source on a
 // cell no stencil updates is added to both buffers when dual != 0.
+// Launched chained (as the two kernels after it) beside the one-thread-per-cell
+// kernels: a thread's first source or receiver is looked up ahead of the wait.
 template <typename T>
 __global__ void k_el_src_rcv(const ElShot<T>* __restrict__ shots, int n, int nt, int record,
                              int par, int dual) {
   const ElShot<T>& sh = shots[blockIdx.x];
   const int64_t d = (int64_t)NF * sh.fs, mine = par ? d : 0, other = par ? -d : d;
+  const T* row = sh.srcv + (int64_t)(n - 1) * sh.nsrc;
+  T* p0 = nullptr;
+  T v0 = T(0);
+  if (threadIdx.x == 0 && sh.nsrc > 0) {
+    p0 = sh.src_ptr[0];
+    v0 = row[0];
+  }
+  const T* q = record && threadIdx.x < sh.nrcv ? sh.rcv_ptr[threadIdx.x] : nullptr;
+  grid_wait();
+  grid_release();
   if (threadIdx.x == 0) {
-    const T* row = sh.srcv + (int64_t)(n - 1) * sh.nsrc;
     for (int k = 0; k < sh.nsrc; k++) {
-      T* p = sh.src_ptr[k];
+      T* p = k == 0 ? p0 : sh.src_ptr[k];
       if (!p) continue;
-      p[mine] += row[k];
-      if (dual && sh.src_dual[k]) p[mine + other] += row[k];
+      const T v = k == 0 ? v0 : row[k];
+      p[mine] += v;
+      if (dual && sh.src_dual[k]) p[mine + other] += v;
     }
   }
   if (!record) return;
   __syncthreads();
   for (int r = threadIdx.x; r < sh.nrcv; r += blockDim.x) {
-    const T* p = sh.rcv_ptr[r];
-    sh.traces[(int64_t)r * nt + n] = p ? p[mine] : T(0);
+    if (r != threadIdx.x) q = sh.rcv_ptr[r];
+    sh.traces[(int64_t)r * nt + n] = q ? q[mine] : T(0);
   }
 }
 
@@ -2400,8 +2704,9 @@ template <typename T>
 __global__ void k_el_resid(const ElShot<T>* __restrict__ shots, int n, int nt, int par) {
   const ElShot<T>& sh = shots[blockIdx.y];
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= sh.nrcv) return;
-  T* p = sh.rcv_gptr[r];
+  T* p = r < sh.nrcv ? sh.rcv_gptr[r] : nullptr;
+  grid_wait();
+  grid_release();
   if (p) atomicAdd(p + (par ? (int64_t)NF * sh.fs : 0), sh.resid[(int64_t)r * nt + n]);
 }
 
@@ -2412,6 +2717,8 @@ template <typename T>
 __global__ void k_el_src_grad(const ElShot<T>* __restrict__ shots, int n, int par) {
   const ElShot<T>& sh = shots[blockIdx.y];
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  grid_wait();
+  grid_release();
   if (k >= sh.nsrc) return;
   const T* p = sh.src_gptr[k];
   sh.gsrc[(int64_t)(n - 1) * sh.nsrc + k] =
@@ -2714,14 +3021,27 @@ struct ElPlanBase {
 
 namespace {
 
-// FP32 plans step with the one-thread-per-cell kernels up to this many cells over
-// all shots: below it a step's time is the latency of one warp's chain, which a
-// strip of rows makes 8 rows long and more; above it the row kernels' single read
-// of each field wins.  us per forward step / forward and adjoint step, cell against
-// row kernels: 80 k cells 10.7 / 24.2 against 20.9 / 54.3, 360 k 16.8 / 40.7 against
-// 21.1 / 56.4, 720 k 24.2 / 61.6 against 24.0 / 64.9, 1.44 M 46.1 / 119 against
-// 40.5 / 104.
-constexpr int64_t kCellMax32 = 600000;
+// FP32 plans, by their cells over all shots (us a forward step / a step of the gradient):
+//  * up to kStripMin the one-thread-per-cell kernels alone, chained launches: a step's
+//    time is the latency of one warp's chain, which a strip of rows makes 8 rows long and
+//    more.  80 k cells 10.2 / 22.8 (with strips 11.1 / 25.0, row kernels 20.8 / 53.2);
+//  * up to kCellMax32 those beside interior strips of two rows a warp, of four above
+//    kTallStrips.  240 k 12.0 / 27.8 (cells alone 12.4 / 29.4), 700 k 17.6 / 44.5 (row
+//    kernels 22.4 / 61.3; one row a warp 18.7 / 47.1, four 19.5 / 51.0), 1.2 M 34.9 / 88.9
+//    (row kernels 34.8 / 98.8; two rows 36.8 / 91.9), 1.44 M 28.3 / 78.6 (30.0 / 90.1);
+//  * above, the row kernels, whose single pass over each field wins where the fields do
+//    not stay in L2: 1.8 M 43.4 / 121 (with strips 54.9 / 139), 2.88 M 65 / 171 (72 / 175).
+constexpr int64_t kStripMin = 200000, kTallStrips = 1100000, kCellMax32 = 1500000;
+// FP32 plans of several shots above this many cells run them in two halves beside each
+// other: the CPML kinds' long chains, the receivers and residuals of one half fill the
+// chip under the other's kernels.  Strips, 1 M cells: 24.2 / 68.2 -> 22.3 / 59.8; row
+// kernels, 16 shots of 600 x 300: 76.0 / 184 -> 64.8 / 171, 32: 143 / 322 -> 118 / 278,
+// but 4 (720 k) 23.9 / 65.1 -> 25.1 / 67.2.  More groups of fewer shots (42 MB of fields
+// each: 16 shots 124 / 361) leave too few warps, three or four groups beside each other
+// change 1-2%.  Only plans replayed from a graph: without one the host issues every
+// launch.
+constexpr int64_t kSplitCells = 900000;
+constexpr int kElChains = 2;
 
 template <typename T>
 struct ElPlan final : ElPlanBase {
@@ -2763,9 +3083,29 @@ struct ElPlan final : ElPlanBase {
   bool cellf = false, cella = false;
   CellModel<T> C{};
   T* d_tab = nullptr;
-  dim3 grid_cells() const {
-    return dim3((unsigned)div_up(NX, BY), (unsigned)div_up(NY, BX), (unsigned)nshots);
-  }
+  // A sequence of time-loop launches: shots [s0, s0 + n) on stream st, with the side
+  // streams and events of chain c.
+  struct Run {
+    cudaStream_t st;
+    int s0, n, c;
+  };
+  Run whole(cudaStream_t st) const { return {st, 0, nshots, 0}; }
+  // Groups of shots that take the whole time loop together: chain c runs shots
+  // [gb[c], gb[c + 1]).
+  std::vector<int> gb;
+  void group_shots();
+  // fn(run) for every group; forked from and joined to st
+  template <typename F>
+  int each_group(cudaStream_t st, F&& fn);
+  // the blocks of a shot (CellItem), and whether interior strips are among them
+  CellItem* d_cells = nullptr;
+  int n_cells = 0, n_strips = 0;
+  std::vector<CellItem> cell_items() const;
+  dim3 grid_cells(int n) const { return dim3((unsigned)n_cells, (unsigned)n); }
+  dim3 grid_strips(int n) const { return dim3((unsigned)n_strips, (unsigned)n); }
+  // fn(stream, strips) for the cell tiles and, where the plan has some, the interior strips
+  template <typename F>
+  int cells_and_strips(const Run& q, F&& fn);
   // host copies: the packed CPML rows and the item lists of the current tiling
   std::vector<T> hprof;
   std::vector<int> wl_host, wlf_host, wla_host;
@@ -2777,30 +3117,38 @@ struct ElPlan final : ElPlanBase {
   static int par(int n) { return n & 1; }
   int apar(int n) const { return fused || cella ? n & 1 : 0; }  // adjoint buffer of slot n
   int adj_launches() const {
-    if (cella) return 2;
+    if (cella) return n_strips ? 4 : 2;
     if (fused) return (nwka[0] > 0) + (nwka[1] > 0) + (nwka[2] > 0) + (nwka[3] > 0);
     return group_launches(kSplitAdj1, nw_in, nw_pm) +
            2 * group_launches(kSplitAdj23, nw_in, nw_pm);
   }
-  cudaStream_t side[3] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[3] = {};
+  // per chain: its stream (chain 0: the caller's), the side streams of a step's
+  // launches, and their events
+  struct Chain {
+    cudaStream_t main = nullptr, side[3] = {};
+    cudaEvent_t ev[5] = {};  // fork, joins of the side streams, chain done
+    cudaEvent_t fork() const { return ev[0]; }
+    cudaEvent_t join(int k) const { return ev[1 + k]; }
+    cudaEvent_t done() const { return ev[4]; }
+  } chain[kElChains];
+  int chains() const { return (int)gb.size() - 1; }
   // launches of one row-kernel step over the interior and CPML lists, whole
   // (part 0) or as its two halves (parts 1, 2)
   static int group_launches(bool split, int n_in, int n_pm) {
     return (split ? 2 : 1) * ((n_in > 0) + (n_pm > 0));
   }
   int fwd_launches() const {
-    if (cellf) return 2;
+    if (cellf) return n_strips ? 4 : 2;
     return (nwk[0] > 0) + (nwk[1] > 0) + (nwk[2] > 0) + (nwk[3] > 0);
   }
   // fn(stream, kind) for each kind with items (nk[kind] > 0), concurrently
   template <typename F>
-  int kinds(cudaStream_t st, const int* nk, F&& fn);
+  int kinds(const Run& q, const int* nk, F&& fn);
   // fn(stream, interior, part) for each non-empty list (n_in interior items,
   // n_pm CPML items) and part, launched concurrently on the main stream and
   // the side streams (disjoint outputs)
   template <typename F>
-  int group(cudaStream_t st, bool split, int n_in, int n_pm, F&& fn);
+  int group(const Run& q, bool split, int n_in, int n_pm, F&& fn);
   int max_rcv = 0;                      // most receivers of a shot
   int64_t P = 0, fs = 0;
   char* pool = nullptr;
@@ -2823,33 +3171,36 @@ struct ElPlan final : ElPlanBase {
     if (gF) cudaGraphDestroy(gF);
     if (gR) cudaGraphDestroy(gR);
     if (cap) cudaStreamDestroy(cap);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    for (auto e : ev_join)
-      if (e) cudaEventDestroy(e);
-    for (auto q : side)
-      if (q) cudaStreamDestroy(q);
+    for (auto& c : chain) {
+      for (auto e : c.ev)
+        if (e) cudaEventDestroy(e);
+      if (c.main) cudaStreamDestroy(c.main);
+      for (auto q : c.side)
+        if (q) cudaStreamDestroy(q);
+    }
     if (pool) cudaFree(pool);
   }
 
   dim3 grid3() const {
     return dim3((unsigned)div_up(NY + 2, BX), (unsigned)div_up(NX + 2, BY), (unsigned)nshots);
   }
-  dim3 grid_rows(int nw) const { return dim3((unsigned)div_up(nw, EW), (unsigned)nshots); }
+  dim3 grid_rows(int nw, int n) const { return dim3((unsigned)div_up(nw, EW), (unsigned)n); }
   // sources / receivers: one CTA per shot, a thread per receiver (up to 1024)
   unsigned rcv_threads() const {
     return (unsigned)std::min<int64_t>(1024, std::max<int64_t>(32, div_up(max_rcv, 32) * 32));
   }
-  dim3 grid_resid() const {
-    return dim3((unsigned)std::max<int64_t>(1, div_up(max_rcv, 256)), (unsigned)nshots);
+  dim3 grid_resid(int n) const {
+    return dim3((unsigned)std::max<int64_t>(1, div_up(max_rcv, 256)), (unsigned)n);
   }
 
   int create(const ads_elastic_config& c, const ads_elastic_shot* shots, int64_t ns,
              cudaStream_t st);
-  int step_kernels(cudaStream_t st, int n, bool store, int slot);
-  int step(cudaStream_t st, int n, bool store, int slot, bool record);
-  int adjoint_step(cudaStream_t st, int slot, int n);
+  int step_kernels(const Run& q, int n, bool store, int slot);
+  int step(const Run& q, int n, bool store, int slot, bool record);
+  int adjoint_step(const Run& q, int slot, int n);
   int issue_forward(cudaStream_t st, int64_t* count);
   int issue_reverse(cudaStream_t st, int64_t* count);
+  int reverse_group(const Run& q);
   int prep(const double* l, const double* m, const double* r, cudaStream_t st);
   int forward(const double* l, const double* m, const double* r, void* traces,
               cudaStream_t st) override;
@@ -2998,6 +3349,17 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
     used += (b + 255) & ~size_t(255);
     return r;
   };
+  std::vector<double> ax(2 * NX), bx(2 * NX), kx(2 * NX), ay(2 * NY), by(2 * NY), ky(2 * NY);
+  elastic_cpml(NX, NY, c.dx, c.dy, c.dt, c.npml, c.npower, c.k_max, c.alpha_max, c.vp_ref,
+               c.Rcoef, c.use_pml, ax.data(), bx.data(), kx.data(), ay.data(), by.data(),
+               ky.data());
+  hprof = pack_profiles<T>(NX, NY, ax.data(), bx.data(), ay.data(), by.data());
+  const std::vector<T>& prof = hprof;
+  std::vector<CellItem> cells;
+  if (cellf || cella) cells = cell_items();
+  n_cells = (int)cells.size();
+  for (const CellItem& q : cells) n_strips += q.w > 0;
+  n_cells -= n_strips;
   const size_t F = sizeof(T) * fs;
   const size_t fwd0 = used;
   for (int s = 0; s < ns; s++) o[s].state = take(2 * NF * F);  // two step buffers
@@ -3037,6 +3399,7 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   const size_t part_o = take(sizeof(double) * kBlocks);
   const size_t gsrc_o = take(sizeof(double) * (src_grad ? std::max<int64_t>(src_total, 1) : 1));
   const size_t shots_o = take(sizeof(ElShot<T>) * ns);
+  const size_t cells_o = take(sizeof(CellItem) * (cellf || cella ? cells.size() : 1));
   const size_t wl_o = take(sizeof(int) * std::max(nwt_max, 1));
   const size_t wlf_o = take(sizeof(int) * std::max(nwtf_max, 1));
   const size_t wla_o = take(sizeof(int) * std::max(fused ? nwta_max : 1, 1));
@@ -3085,21 +3448,22 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   d_partial = (double*)(pool + part_o);
   d_gsrc = (double*)(pool + gsrc_o);
   d_shots = (ElShot<T>*)(pool + shots_o);
-  // profiles
-  std::vector<double> ax(2 * NX), bx(2 * NX), kx(2 * NX), ay(2 * NY), by(2 * NY), ky(2 * NY);
-  elastic_cpml(NX, NY, c.dx, c.dy, c.dt, c.npml, c.npower, c.k_max, c.alpha_max, c.vp_ref,
-               c.Rcoef, c.use_pml, ax.data(), bx.data(), kx.data(), ay.data(), by.data(),
-               ky.data());
-  hprof = pack_profiles<T>(NX, NY, ax.data(), bx.data(), ay.data(), by.data());
-  const std::vector<T>& prof = hprof;
+  d_cells = (CellItem*)(pool + cells_o);
+  if (!cells.empty())
+    ADS_CUDA(cudaMemcpyAsync(d_cells, cells.data(), sizeof(CellItem) * cells.size(),
+                             cudaMemcpyHostToDevice, st));
   build_lists(rows_w, rows_f, rows_a);
   d_wl = (int*)(pool + wl_o);
   d_wlf = (int*)(pool + wlf_o);
   d_wla = (int*)(pool + wla_o);
   if (int e = upload_lists(st)) return e;
-  for (auto& q : side) ADS_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
-  ADS_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-  for (auto& e : ev_join) ADS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  group_shots();
+  for (int k = 0; k < chains(); k++) {
+    Chain& h = chain[k];
+    if (k > 0) ADS_CUDA(cudaStreamCreateWithFlags(&h.main, cudaStreamNonBlocking));
+    for (auto& q : h.side) ADS_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+    for (auto& e : h.ev) ADS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  }
   ADS_CUDA(cudaMemcpyAsync(pool + prof_o, prof.data(), sizeof(T) * prof.size(),
                            cudaMemcpyHostToDevice, st));
   M = make_model<T>(NX, NY, P, JOFF, c.dt, c.dx, c.dy, d_lam, d_mu, d_rho,
@@ -3265,6 +3629,7 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
       ADS_CUDA(e);
       cudaGraphExec_t ex = nullptr;
       ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
+      ADS_CUDA(cudaGraphUpload(ex, st));  // (else the first launch waits for it)
       (which == 0 ? gF : gR) = g;
       (which == 0 ? eF : eR) = ex;
     }
@@ -3399,7 +3764,7 @@ int ElPlan<T>::autotune(cudaStream_t st, int rw_min, int rf_min) {
     for (int pass = 0; pass < 2; pass++) {  // pass 0 warms up
       ADS_CUDA(cudaEventRecord(e0, st));
       for (int n = 1; n <= 6; n++)
-        if (int e = adj ? adjoint_step(st, 0, n) : step(st, n, false, 0, false)) return e;
+        if (int e = adj ? adjoint_step(whole(st), 0, n) : step(whole(st), n, false, 0, false)) return e;
       ADS_CUDA(cudaEventRecord(e1, st));
       ADS_CUDA(cudaEventSynchronize(e1));
       ADS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -3458,7 +3823,8 @@ int ElPlan<T>::autotune(cudaStream_t st, int rw_min, int rf_min) {
 // One forward step n (slot n-1 -> slot n) for every shot.
 template <typename T>
 template <typename F>
-int ElPlan<T>::group(cudaStream_t st, bool split, int n_in, int n_pm, F&& fn) {
+int ElPlan<T>::group(const Run& q, bool split, int n_in, int n_pm, F&& fn) {
+  Chain& h = chain[q.c];
   // the CPML items first, as in kinds() (FP64 three-pass gradient, 4 shots
   // on the C4 grid: 1017 against 1059 ms with the CPML-free items first)
   bool in_[4];
@@ -3472,23 +3838,24 @@ int ElPlan<T>::group(cudaStream_t st, bool split, int n_in, int n_pm, F&& fn) {
     }
   }
   if (n > 1) {
-    ADS_CUDA(cudaEventRecord(ev_fork, st));
-    for (int k = 1; k < n; k++) ADS_CUDA(cudaStreamWaitEvent(side[k - 1], ev_fork, 0));
+    ADS_CUDA(cudaEventRecord(h.fork(), q.st));
+    for (int k = 1; k < n; k++) ADS_CUDA(cudaStreamWaitEvent(h.side[k - 1], h.fork(), 0));
   }
   for (int k = 0; k < n; k++) {
-    fn(k == 0 ? st : side[k - 1], in_[k], part_[k]);
+    fn(k == 0 ? q.st : h.side[k - 1], in_[k], part_[k]);
     ADS_LAUNCHED(1);
   }
   for (int k = 1; k < n; k++) {
-    ADS_CUDA(cudaEventRecord(ev_join[k - 1], side[k - 1]));
-    ADS_CUDA(cudaStreamWaitEvent(st, ev_join[k - 1], 0));
+    ADS_CUDA(cudaEventRecord(h.join(k - 1), h.side[k - 1]));
+    ADS_CUDA(cudaStreamWaitEvent(q.st, h.join(k - 1), 0));
   }
   return ADS_OK;
 }
 
 template <typename T>
 template <typename F>
-int ElPlan<T>::kinds(cudaStream_t st, const int* nk, F&& fn) {
+int ElPlan<T>::kinds(const Run& q, const int* nk, F&& fn) {
+  Chain& h = chain[q.c];
   // The CPML kinds first: their few items carry the longest chains, and the
   // launches of a fork start roughly in the order they are issued (measured
   // on the C4 gradient: 20.1 shot-gradients/s against 17.4 with kind 0 first)
@@ -3496,17 +3863,103 @@ int ElPlan<T>::kinds(cudaStream_t st, const int* nk, F&& fn) {
   for (int k = 3; k >= 0; k--)
     if (nk[k] > 0) kd[n++] = k;
   if (n > 1) {
-    ADS_CUDA(cudaEventRecord(ev_fork, st));
-    for (int k = 1; k < n; k++) ADS_CUDA(cudaStreamWaitEvent(side[k - 1], ev_fork, 0));
+    ADS_CUDA(cudaEventRecord(h.fork(), q.st));
+    for (int k = 1; k < n; k++) ADS_CUDA(cudaStreamWaitEvent(h.side[k - 1], h.fork(), 0));
   }
   for (int k = 0; k < n; k++) {
-    fn(k == 0 ? st : side[k - 1], kd[k]);
+    fn(k == 0 ? q.st : h.side[k - 1], kd[k]);
     ADS_LAUNCHED(1);
   }
   for (int k = 1; k < n; k++) {
-    ADS_CUDA(cudaEventRecord(ev_join[k - 1], side[k - 1]));
-    ADS_CUDA(cudaStreamWaitEvent(st, ev_join[k - 1], 0));
+    ADS_CUDA(cudaEventRecord(h.join(k - 1), h.side[k - 1]));
+    ADS_CUDA(cudaStreamWaitEvent(q.st, h.join(k - 1), 0));
   }
+  return ADS_OK;
+}
+
+// The blocks of a shot.  FP32 plans: interior strips over the rectangle of cells with no
+// CPML and no box edge within two rows and columns, its first row and column and its row
+// count such that the frame around it is cut into whole tiles.
+template <typename T>
+std::vector<CellItem> ElPlan<T>::cell_items() const {
+  std::vector<CellItem> v;
+  int it = NX + 1, ib = NX + 1, jl = NY + 1, jr = NY + 1;  // rows [it, ib), columns [jl, jr)
+  if (sizeof(T) == 4 && (int64_t)NX * NY * nshots > kStripMin) {
+    const T *axi = hprof.data(), *axh = axi + NX, *bxi = axh + NX, *bxh = bxi + NX,
+            *ayi = bxh + NX, *ayh = ayi + NY, *byi = ayh + NY, *byh = byi + NY;
+    auto run = [](int n, const T* a, const T* b, const T* c, const T* d, int& lo, int& hi) {
+      // the rows (columns) k, 4 <= k <= n - 3, with idle profiles on k - 2 .. k + 2, around
+      // the middle: [lo, hi)
+      auto ok = [&](int k) {
+        if (k < 4 || k > n - 3) return false;
+        for (int q = k - 2; q <= k + 2; q++)
+          if (a[q - 1] != 0 || b[q - 1] != 1 || c[q - 1] != 0 || d[q - 1] != 1) return false;
+        return true;
+      };
+      lo = hi = n / 2;
+      if (!ok(lo)) return;
+      while (ok(lo - 1)) lo--;
+      while (ok(hi)) hi++;
+    };
+    int a, b;
+    run(NX, axi, bxi, axh, bxh, a, b);
+    it = (int)round_up(a - 1, BY) + 1;
+    ib = it + (b - it) / BY * BY;
+    run(NY, ayi, byi, ayh, byh, a, b);
+    jl = (int)round_up(a - 1, BX) + 1;
+    // the right part of the frame whole tiles wide, as near as multiples of four allow
+    for (int n = (int)div_up(NY + 1 - b, BX); jl < b; n++) {
+      jr = jl + (int)round_up(std::max(0, NY + 1 - BX * n - jl), 4);
+      if (jr <= b) break;
+    }
+    if (jl >= b) jr = jl;
+    if (ib - it < BY || jr - jl < 8) it = ib = NX + 1, jl = jr = NY + 1;
+  }
+  const bool any = ib > it;
+  if (!any) it = ib = NX + 1;
+  auto tiles = [&](int r0, int r1, int c0, int c1) {
+    for (int i = r0; i < r1; i += BY)
+      for (int j = c0; j < c1; j += BX) v.push_back({i, j, 0, 0});
+  };
+  tiles(1, it, 1, NY + 1);
+  if (!any) return v;
+  tiles(it, ib, 1, jl);
+  tiles(it, ib, jr, NY + 1);
+  tiles(ib, NX + 1, 1, NY + 1);
+  // strips of equal width, a multiple of four, at most 120
+  const int ns = (int)div_up(jr - jl, 120), w = (int)round_up(div_up(jr - jl, ns), 4);
+  const int rows = (int64_t)NX * NY * nshots > kTallStrips ? 4 : 2;  // a warp
+  for (int i = it; i < ib; i += BY * rows)
+    for (int j = jl; j < jr; j += w)
+      v.push_back({i, j, std::min(w, jr - j), rows | std::min(BY * rows, ib - i) << 16});
+  return v;
+}
+
+// A launch of the time loop: chained beside the one-thread-per-cell kernels, which are
+// too.
+template <typename... P, typename... A>
+cudaError_t launch_in_loop(bool chained, void (*kernel)(P...), dim3 g, dim3 b, cudaStream_t st,
+                           A... a) {
+  if (chained) return launch_chained(kernel, g, b, st, a...);
+  kernel<<<g, b, 0, st>>>(static_cast<P>(a)...);
+  return cudaGetLastError();
+}
+
+template <typename T>
+template <typename F>
+int ElPlan<T>::cells_and_strips(const Run& q, F&& fn) {
+  Chain& h = chain[q.c];
+  if (n_strips) {
+    ADS_CUDA(cudaEventRecord(h.fork(), q.st));
+    ADS_CUDA(cudaStreamWaitEvent(h.side[0], h.fork(), 0));
+  }
+  ADS_CUDA(fn(n_strips ? h.side[0] : q.st, false));
+  ADS_LAUNCHED(1);
+  if (!n_strips) return ADS_OK;
+  ADS_CUDA(fn(q.st, true));
+  ADS_LAUNCHED(1);
+  ADS_CUDA(cudaEventRecord(h.join(0), h.side[0]));
+  ADS_CUDA(cudaStreamWaitEvent(q.st, h.join(0), 0));
   return ADS_OK;
 }
 
@@ -3514,63 +3967,117 @@ int ElPlan<T>::kinds(cudaStream_t st, const int* nk, F&& fn) {
 // the item kinds (adjoint of slot n in buffer apar(n) -> slot n-1 in the
 // other), or the three passes in place.
 template <typename T>
-int ElPlan<T>::adjoint_step(cudaStream_t st, int slot, int n) {
+int ElPlan<T>::adjoint_step(const Run& q, int slot, int n) {
+  const ElShot<T>* sh = d_shots + q.s0;
   if (cella) {
     const dim3 b(BX, BY);
-    k_el_cell_adj_stress<T><<<grid_cells(), b, 0, st>>>(C, d_shots, apar(n), slot);
-    ADS_LAUNCHED(1);
-    k_el_cell_adj_velocity<T><<<grid_cells(), b, 0, st>>>(C, d_shots, apar(n), slot);
-    ADS_LAUNCHED(1);
-    return ADS_OK;
+    if (int e = cells_and_strips(q, [&](cudaStream_t s, bool strip) {
+          if (!strip)
+            return launch_in_loop(!n_strips, k_el_cell_adj_stress<T>, grid_cells(q.n), b, s, C, sh,
+                                  d_cells, apar(n), slot);
+          if constexpr (sizeof(T) == 4)
+            return launch_in_loop(false, k_el_strip_adj_stress, grid_strips(q.n), b, s, C, sh,
+                                  d_cells + n_cells, apar(n), slot);
+          return cudaSuccess;
+        }))
+      return e;
+    return cells_and_strips(q, [&](cudaStream_t s, bool strip) {
+      if (!strip)
+        return launch_in_loop(!n_strips, k_el_cell_adj_velocity<T>, grid_cells(q.n), b, s, C, sh,
+                              d_cells, apar(n), slot);
+      if constexpr (sizeof(T) == 4)
+        return launch_in_loop(false, k_el_strip_adj_velocity, grid_strips(q.n), b, s, C, sh,
+                              d_cells + n_cells, apar(n), slot);
+      return cudaSuccess;
+    });
   }
   if (fused)
-    return kinds(st, nwka, [&](cudaStream_t s, int k) {
-      el_fadj<T>(k, grid_rows(nwka[k]), s, M, d_shots, d_wla + owka[k], ncola, rows_a, nwka[k],
+    return kinds(q, nwka, [&](cudaStream_t s, int k) {
+      el_fadj<T>(k, grid_rows(nwka[k], q.n), s, M, sh, d_wla + owka[k], ncola, rows_a, nwka[k],
                  slot, apar(n), jsha, isha);
     });
   auto wl = [&](bool in) { return in ? d_wl : d_wl + nw_in; };
   auto nw = [&](bool in) { return in ? nw_in : nw_pm; };
-  if (int e = group(st, kSplitAdj1, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-        el_adj1<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in),
+  if (int e = group(q, kSplitAdj1, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+        el_adj1<T>(in, part, grid_rows(nw(in), q.n), s, M, sh, wl(in), ncolw, rows_w, nw(in),
                    slot);
       }))
     return e;
-  if (int e = group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-        el_adj2<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in),
+  if (int e = group(q, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+        el_adj2<T>(in, part, grid_rows(nw(in), q.n), s, M, sh, wl(in), ncolw, rows_w, nw(in),
                    slot);
       }))
     return e;
-  return group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-    el_adj3<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in));
+  return group(q, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+    el_adj3<T>(in, part, grid_rows(nw(in), q.n), s, M, sh, wl(in), ncolw, rows_w, nw(in));
   });
 }
 
 // One forward step n (slot n-1 in buffer par(n-1) -> slot n in buffer
 // par(n)) for every shot.
 template <typename T>
-int ElPlan<T>::step_kernels(cudaStream_t st, int n, bool store, int slot) {
+int ElPlan<T>::step_kernels(const Run& q, int n, bool store, int slot) {
+  const ElShot<T>* sh = d_shots + q.s0;
   const int sl = store ? slot : 0, pin = par(n - 1);
   if (!cellf)
-    return kinds(st, nwk, [&](cudaStream_t s, int k) {
-      el_step<T>(store, k, grid_rows(nwk[k]), s, M, d_shots, d_wlf + owk[k], ncolf, rows_f,
+    return kinds(q, nwk, [&](cudaStream_t s, int k) {
+      el_step<T>(store, k, grid_rows(nwk[k], q.n), s, M, sh, d_wlf + owk[k], ncolf, rows_f,
                  nwk[k], sl, pin, jsh, ish);
     });
-  const dim3 g = grid_cells(), b(BX, BY);
-  if (store) k_el_cell_stress<T, true><<<g, b, 0, st>>>(C, d_shots, pin, sl);
-  else k_el_cell_stress<T, false><<<g, b, 0, st>>>(C, d_shots, pin, sl);
-  ADS_LAUNCHED(1);
-  if (store) k_el_cell_velocity<T, true><<<g, b, 0, st>>>(C, d_shots, pin, sl);
-  else k_el_cell_velocity<T, false><<<g, b, 0, st>>>(C, d_shots, pin, sl);
+  const dim3 b(BX, BY);
+  if (int e = cells_and_strips(q, [&](cudaStream_t s, bool strip) {
+        if (!strip)
+          return launch_in_loop(!n_strips,
+                                store ? k_el_cell_stress<T, true> : k_el_cell_stress<T, false>,
+                                grid_cells(q.n), b, s, C, sh, d_cells, pin, sl);
+        if constexpr (sizeof(T) == 4)
+          return launch_in_loop(false, store ? k_el_strip_stress<true> : k_el_strip_stress<false>,
+                                grid_strips(q.n), b, s, C, sh, d_cells + n_cells, pin, sl);
+        return cudaSuccess;
+      }))
+    return e;
+  return cells_and_strips(q, [&](cudaStream_t s, bool strip) {
+    if (!strip)
+      return launch_in_loop(!n_strips,
+                            store ? k_el_cell_velocity<T, true> : k_el_cell_velocity<T, false>,
+                            grid_cells(q.n), b, s, C, sh, d_cells, pin, sl);
+    if constexpr (sizeof(T) == 4)
+      return launch_in_loop(false, store ? k_el_strip_velocity<true> : k_el_strip_velocity<false>,
+                            grid_strips(q.n), b, s, C, sh, d_cells + n_cells, pin, sl);
+    return cudaSuccess;
+  });
+}
+
+template <typename T>
+int ElPlan<T>::step(const Run& q, int n, bool store, int slot, bool record) {
+  if (int e = step_kernels(q, n, store, slot)) return e;
+  ADS_CUDA(launch_in_loop(cellf && !n_strips, k_el_src_rcv<T>, dim3(q.n), dim3(rcv_threads()), q.st,
+                          d_shots + q.s0, n, NSTEP + 1, record ? 1 : 0, par(n), 1));
   ADS_LAUNCHED(1);
   return ADS_OK;
 }
 
 template <typename T>
-int ElPlan<T>::step(cudaStream_t st, int n, bool store, int slot, bool record) {
-  if (int e = step_kernels(st, n, store, slot)) return e;
-  k_el_src_rcv<T><<<nshots, rcv_threads(), 0, st>>>(d_shots, n, NSTEP + 1, record ? 1 : 0,
-                                                    par(n), 1);
-  ADS_LAUNCHED(1);
+void ElPlan<T>::group_shots() {
+  const bool split = sizeof(T) == 4 && cfg.use_graph && nshots > 1 &&
+                     (int64_t)NX * NY * nshots > kSplitCells;
+  const int n = split ? std::min(nshots, kElChains) : 1;
+  gb.assign(1, 0);
+  for (int g = 1; g <= n; g++) gb.push_back((int)((int64_t)nshots * g / n));
+}
+
+template <typename T>
+template <typename F>
+int ElPlan<T>::each_group(cudaStream_t st, F&& fn) {
+  const int n = chains();
+  if (n > 1) ADS_CUDA(cudaEventRecord(chain[0].done(), st));
+  for (int c = 0; c < n; c++) {
+    cudaStream_t q = c == 0 ? st : chain[c].main;
+    if (c > 0) ADS_CUDA(cudaStreamWaitEvent(q, chain[0].done(), 0));
+    if (int e = fn(Run{q, gb[c], gb[c + 1] - gb[c], c})) return e;
+    if (c > 0) ADS_CUDA(cudaEventRecord(chain[c].done(), q));
+  }
+  for (int c = 1; c < n; c++) ADS_CUDA(cudaStreamWaitEvent(st, chain[c].done(), 0));
   return ADS_OK;
 }
 
@@ -3580,21 +4087,23 @@ int ElPlan<T>::issue_forward(cudaStream_t st, int64_t* count) {
     int64_t c = 0;
     for (int n = 1; n <= NSTEP; n++)
       c += fwd_launches() + 1 + ((n % K == 0 && n / K < res_seg) ? 1 : 0);
-    *count = c;
+    *count = c * ((int64_t)gb.size() - 1);
     return ADS_OK;
   }
   ADS_CUDA(cudaMemsetAsync(pool + zero_fwd_off, 0, zero_fwd_len, st));
-  for (int n = 1; n <= NSTEP; n++) {
-    // steps of resident segments store what their adjoint steps read
-    const bool res = n >= a_res();
-    if (int e = step(st, n, res, res ? K + n - a_res() : 0, true)) return e;
-    // checkpoint s holds slot s*K (state before step sK+1); resident segments need none
-    if (n % K == 0 && n / K < res_seg) {
-      k_el_ckpt<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, n / K, 1, par(n), 0);
-      ADS_LAUNCHED(1);
+  return each_group(st, [&](const Run& q) -> int {
+    for (int n = 1; n <= NSTEP; n++) {
+      // steps of resident segments store what their adjoint steps read
+      const bool res = n >= a_res();
+      if (int e = step(q, n, res, res ? K + n - a_res() : 0, true)) return e;
+      // checkpoint s holds slot s*K (state before step sK+1); resident segments need none
+      if (n % K == 0 && n / K < res_seg) {
+        k_el_ckpt<T><<<dim3(256, q.n), 256, 0, q.st>>>(d_shots + q.s0, n / K, 1, par(n), 0);
+        ADS_LAUNCHED(1);
+      }
     }
-  }
-  return ADS_OK;
+    return ADS_OK;
+  });
 }
 
 template <typename T>
@@ -3608,39 +4117,48 @@ int ElPlan<T>::issue_reverse(cudaStream_t st, int64_t* count) {
            (b - std::max(a, 2) + 1) + (src_grad ? b - a + 1 : 0) +
            (sizeof(T) == 4 ? 1 : 0);
     }
-    *count = c;
+    *count = c * ((int64_t)gb.size() - 1);
     return ADS_OK;
   }
   ADS_CUDA(cudaMemsetAsync(pool + zero_adj_off, 0, zero_adj_len, st));
-  k_el_resid<T><<<grid_resid(), 256, 0, st>>>(d_shots, NSTEP, NSTEP + 1, apar(NSTEP));
+  return each_group(st, [&](const Run& q) { return reverse_group(q); });
+}
+
+template <typename T>
+int ElPlan<T>::reverse_group(const Run& q) {
+  const ElShot<T>* sh = d_shots + q.s0;
+  ADS_CUDA(launch_in_loop(cella && !n_strips, k_el_resid<T>, grid_resid(q.n), dim3(256), q.st, sh, NSTEP,
+                          NSTEP + 1, apar(NSTEP)));
   ADS_LAUNCHED(1);
   for (int s = nseg - 1; s >= 0; s--) {
     const int a = 1 + s * K, b = std::min(a + K - 1, NSTEP);
     const bool res = s >= res_seg;  // resident: the store already holds the segment
     const int slot0 = res ? K + a - a_res() : 0;  // store slot of step a
     if (!res) {
-      k_el_ckpt<T><<<dim3(256, nshots), 256, 0, st>>>(d_shots, s, 0, 0, 1);
+      k_el_ckpt<T><<<dim3(256, q.n), 256, 0, q.st>>>(sh, s, 0, 0, 1);
       ADS_LAUNCHED(1);
       for (int n = a; n <= b; n++)
-        if (int e = step(st, n, true, n - a, false)) return e;
+        if (int e = step(q, n, true, n - a, false)) return e;
     }
     for (int n = b; n >= a; n--) {
       if (src_grad) {  // the adjoint state refers to slot n, its residual included
-        k_el_src_grad<T><<<dim3((unsigned)div_up(std::max(max_src, 1), 128), nshots), 128, 0,
-                            st>>>(d_shots, n, apar(n));
+        ADS_CUDA(launch_in_loop(cella && !n_strips, k_el_src_grad<T>,
+                                dim3((unsigned)div_up(std::max(max_src, 1), 128), q.n), dim3(128),
+                                q.st, sh, n, apar(n)));
         ADS_LAUNCHED(1);
       }
-      if (int e = adjoint_step(st, slot0 + n - a, n)) return e;
+      if (int e = adjoint_step(q, slot0 + n - a, n)) return e;
       // the adjoint state now refers to slot n-1: add its residual (slot 0 is
       // the constant zero state and takes none)
       if (n - 1 >= 1) {
-        k_el_resid<T><<<grid_resid(), 256, 0, st>>>(d_shots, n - 1, NSTEP + 1, apar(n - 1));
+        ADS_CUDA(launch_in_loop(cella && !n_strips, k_el_resid<T>, grid_resid(q.n), dim3(256), q.st, sh, n - 1,
+                                NSTEP + 1, apar(n - 1)));
         ADS_LAUNCHED(1);
       }
     }
     if constexpr (sizeof(T) == 4) {
-      if (cella) k_el_flush_cells<<<dim3(256, nshots), 256, 0, st>>>(d_shots);
-      else k_el_flush_acc<<<dim3(256, nshots), 256, 0, st>>>(d_shots, fs);
+      if (cella) k_el_flush_cells<<<dim3(256, q.n), 256, 0, q.st>>>(sh);
+      else k_el_flush_acc<<<dim3(256, q.n), 256, 0, q.st>>>(sh, fs);
       ADS_LAUNCHED(1);
     }
   }
@@ -3750,31 +4268,31 @@ int ElPlan<T>::profile(const double* l, const double* m, const double* r, double
   auto wl = [&](bool in) { return in ? d_wl : d_wl + nw_in; };
   auto nw = [&](bool in) { return in ? nw_in : nw_pm; };
   for (int k = 0; k < 2; k++)
-    run(k, [&] { step_kernels(st, 1, k == 1, 0); });
+    run(k, [&] { step_kernels(whole(st), 1, k == 1, 0); });
   if (fused || cella) {  // the whole adjoint step in slot 2; slots 3 and 4 stay empty
-    run(2, [&] { adjoint_step(st, 0, 1); });
+    run(2, [&] { adjoint_step(whole(st), 0, 1); });
     out[6] = out[8] = 0.0;
     out[7] = out[9] = cells;
   }
   if (!fused && !cella) run(2, [&] {
-    group(st, kSplitAdj1, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-      el_adj1<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
+    group(whole(st), kSplitAdj1, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+      el_adj1<T>(in, part, grid_rows(nw(in), nshots), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
     });
   });
   if (!fused && !cella) run(3, [&] {
-    group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-      el_adj2<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
+    group(whole(st), kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+      el_adj2<T>(in, part, grid_rows(nw(in), nshots), s, M, d_shots, wl(in), ncolw, rows_w, nw(in), 0);
     });
   });
   if (!fused && !cella) run(4, [&] {
-    group(st, kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
-      el_adj3<T>(in, part, grid_rows(nw(in)), s, M, d_shots, wl(in), ncolw, rows_w, nw(in));
+    group(whole(st), kSplitAdj23, nw_in, nw_pm, [&](cudaStream_t s, bool in, int part) {
+      el_adj3<T>(in, part, grid_rows(nw(in), nshots), s, M, d_shots, wl(in), ncolw, rows_w, nw(in));
     });
   });
   run(5, [&] {
     k_el_src_rcv<T><<<nshots, rcv_threads(), 0, st>>>(d_shots, 1, NSTEP + 1, 1, 0, 0);
   });
-  run(6, [&] { k_el_resid<T><<<grid_resid(), 256, 0, st>>>(d_shots, 1, NSTEP + 1, 0); });
+  run(6, [&] { k_el_resid<T><<<grid_resid(nshots), 256, 0, st>>>(d_shots, 1, NSTEP + 1, 0); });
   note_launches(2 * (kProfileReps + 1));  // the pairs count their own launches
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
