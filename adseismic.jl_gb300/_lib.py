@@ -94,6 +94,8 @@ _SIGS = {
     "ads_get_receive_bwd_f64": [P] * 6 + [I64, P, P, P, I64, I64, I64, P],
     "ads_elastic_step_fwd_f64": [P] * 11 + [D, D, D, I64, I64, P, P, P, P, I64, P],
     "ads_elastic_step_fwd_f32": [P] * 11 + [D, D, D, I64, I64, P, P, P, P, I64, P],
+    "ads_elastic_add_sources_f64": [P, I64, I64, P, P, P, P, I64, P],
+    "ads_elastic_add_sources_f32": [P, I64, I64, P, P, P, P, I64, P],
     "ads_elastic_step_bwd_f64": [P] * 13 + [D, D, D, I64, I64, P],
     "ads_elastic_step_bwd_f32": [P] * 13 + [D, D, D, I64, I64, P],
     "ads_elastic_step_bwd_f64_noalloc": [P] * 13 + [D, D, D, I64, I64, P],

@@ -20,11 +20,15 @@ from ._lib import ADS_F32, ADS_F64, ADS_VARIANT_U, ADS_VARIANT_W, call, lib
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch.cuda.current_stream(torch.cuda.current_device()).cuda_stream
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
+
+
+def _flat(t, dtype):
+    return t if t.dtype == dtype and t.is_contiguous() else t.contiguous().to(dtype)
 
 
 def _require_cuda(*ts):
@@ -102,7 +106,7 @@ def acoustic_one_step(w, wold, phi, psi, sigma, tau, c, dt, hx, hy, NX, NY,
     ts = [w, wold, phi, psi, sigma, tau, c]
     _require_cuda(*ts)
     dt_ = w.dtype
-    ts = [t.contiguous().to(dt_) for t in ts]
+    ts = [_flat(t, dt_) for t in ts]
     u, po, qo = (torch.empty_like(ts[0]) for _ in range(3))
     name = "ads_acoustic_step_fwd_f64" if dt_ == torch.float64 else "ads_acoustic_step_fwd_f32"
     call(name, *[_ptr(t) for t in ts], dt, hx, hy, NX, NY, _ptr(u), _ptr(po), _ptr(qo),
@@ -116,8 +120,8 @@ def acoustic_one_step_grad(gu, gphi, gpsi, w, wold, phi, psi, sigma, tau, c, dt,
     grad_phi, grad_psi, grad_c (grad_sigma/tau/dt/hx/hy are never produced by the
     reference either)."""
     dt_ = w.dtype
-    ins = [t.contiguous().to(dt_) for t in (gu, gphi, gpsi, w, wold, phi, psi, sigma, tau, c)]
-    tail = [t.contiguous().to(dt_) for t in (u, phiout, psiout)]
+    ins = [_flat(t, dt_) for t in (gu, gphi, gpsi, w, wold, phi, psi, sigma, tau, c)]
+    tail = [_flat(t, dt_) for t in (u, phiout, psiout)]
     _require_cuda(*ins, *tail)
     outs = [torch.empty_like(ins[3]) for _ in range(5)]
     name = "ads_acoustic_step_bwd_f64" if dt_ == torch.float64 else "ads_acoustic_step_bwd_f32"

@@ -76,6 +76,12 @@ def compute_PML_Params(param: ElasticPropagatorParams):
     return tuple(x.reshape(2, -1) for x in a)
 
 
+def _on(a, dev, dtype):
+    if isinstance(a, torch.Tensor) and a.device == dev and a.dtype == dtype:
+        return a.contiguous()
+    return torch.as_tensor(a, device=dev).to(dtype).contiguous()
+
+
 def elastic_one_step(param: ElasticPropagatorParams, rho, lam, mu, state, profiles,
                      srci=None, srcj=None, srcv=None, srctype=None):
     """one_step of src/Core.jl:215-228 on CUDA tensors, float64 (the reference's
@@ -88,23 +94,32 @@ def elastic_one_step(param: ElasticPropagatorParams, rho, lam, mu, state, profil
     dt_ = torch.float32 if state.dtype == torch.float32 else torch.float64
     state = state.contiguous().to(dt_)
     out = torch.empty_like(state)
-    ax, bx, kx, ay, by, ky = [torch.as_tensor(p, device=state.device).to(dt_).contiguous()
-                              for p in profiles]
-    if srci is not None and len(srci):
-        dev = state.device
-        si = torch.as_tensor(np.asarray(srci), dtype=torch.int64, device=dev)
-        sj = torch.as_tensor(np.asarray(srcj), dtype=torch.int64, device=dev)
-        stp = torch.as_tensor(np.asarray(srctype), dtype=torch.int64, device=dev)
-        sv = torch.as_tensor(srcv, device=dev).to(dt_).contiguous()
-        nsrc = len(srci)
-    else:
-        si = sj = stp = sv = None
-        nsrc = 0
+    dev = state.device
+    ax, bx, kx, ay, by, ky = [_on(p, dev, dt_) for p in profiles]
+    si = sj = stp = sv = None
+    nsrc = 0 if srci is None else len(srci)
+    # values that are on the host go along as kernel arguments: a copy to the device would
+    # wait for everything on the stream
+    host = nsrc > 0 and not (isinstance(srcv, torch.Tensor) and srcv.is_cuda)
+    if nsrc and not host:
+        si, sj, stp = (torch.as_tensor(np.asarray(a), dtype=torch.int64, device=dev)
+                       for a in (srci, srcj, srctype))
+        sv = srcv.to(dev).to(dt_).contiguous()
     lam, mu, rho = (t.contiguous().to(dt_) for t in (lam, mu, rho))
-    name = "ads_elastic_step_fwd_f64" if dt_ == torch.float64 else "ads_elastic_step_fwd_f32"
-    call(name, _ptr(state), _ptr(out), _ptr(lam), _ptr(mu), _ptr(rho), _ptr(ax), _ptr(bx),
-         _ptr(kx), _ptr(ay), _ptr(by), _ptr(ky), param.DELTAT, param.DELTAX, param.DELTAY, NX,
-         NY, _ptr(si), _ptr(sj), _ptr(stp), _ptr(sv), nsrc, _stream())
+    suffix = "f64" if dt_ == torch.float64 else "f32"
+    call("ads_elastic_step_fwd_" + suffix, _ptr(state), _ptr(out), _ptr(lam), _ptr(mu),
+         _ptr(rho), _ptr(ax), _ptr(bx), _ptr(kx), _ptr(ay), _ptr(by), _ptr(ky), param.DELTAT,
+         param.DELTAX, param.DELTAY, NX, NY, _ptr(si), _ptr(sj), _ptr(stp), _ptr(sv),
+         0 if host else nsrc, _stream())
+    if host:
+        at = [np.ascontiguousarray(a, dtype=np.int64).reshape(-1) for a in (srci, srcj, srctype)]
+        v = srcv.detach() if isinstance(srcv, torch.Tensor) else srcv
+        at.append(np.ascontiguousarray(v, dtype=np.float64 if suffix == "f64" else np.float32)
+                  .reshape(-1))
+        if min(len(a) for a in at) < nsrc:
+            raise ValueError("srcj, srctype and srcv must have an entry per source")
+        call("ads_elastic_add_sources_" + suffix, _ptr(out), NX, NY,
+             *[a.ctypes.data for a in at], nsrc, _stream())
     return out
 
 
@@ -119,8 +134,7 @@ def elastic_one_step_grad(param: ElasticPropagatorParams, rho, lam, mu, state, g
     gin = torch.empty_like(state)
     N = state.shape[-1]
     gl, gm, gr = (torch.zeros(N, dtype=dt_, device=dev) for _ in range(3))
-    ax, bx, kx, ay, by, ky = [torch.as_tensor(p, device=dev).to(dt_).contiguous()
-                              for p in profiles]
+    ax, bx, kx, ay, by, ky = [_on(p, dev, dt_) for p in profiles]
     lam, mu, rho = (t.contiguous().to(dt_) for t in (lam, mu, rho))
     name = "ads_elastic_step_bwd_f64" if dt_ == torch.float64 else "ads_elastic_step_bwd_f32"
     call(name, _ptr(state), _ptr(gout), _ptr(gin), _ptr(gl), _ptr(gm), _ptr(gr), _ptr(lam),

@@ -178,6 +178,15 @@ int ads_elastic_step_fwd_f32(const float* state_in, float* state_out, const floa
                              double dy, int64_t NX, int64_t NY, const int64_t* srci,
                              const int64_t* srcj, const int64_t* srctype, const float* srcv,
                              int64_t nsrc, ads_stream_t stream);
+/* Adds one time row of sources to a state on its own, as ads_elastic_step_fwd_f64 does
+ * after the step: srci, srcj, srctype, srcv are HOST arrays of nsrc entries here; they go
+ * along as kernel arguments, so nothing is copied or waited for. */
+int ads_elastic_add_sources_f64(double* state, int64_t NX, int64_t NY, const int64_t* srci,
+                                const int64_t* srcj, const int64_t* srctype, const double* srcv,
+                                int64_t nsrc, ads_stream_t stream);
+int ads_elastic_add_sources_f32(float* state, int64_t NX, int64_t NY, const int64_t* srci,
+                                const int64_t* srcj, const int64_t* srctype, const float* srcv,
+                                int64_t nsrc, ads_stream_t stream);
 /* Transpose of one elastic step about state_in: grad_in (13*N, overwritten) is
  * the gradient w.r.t. state_in given grad_out w.r.t. the step's output;
  * grad_lambda, grad_mu, grad_rho are ACCUMULATED (+=).  The TF gradient of
