@@ -46,9 +46,10 @@ BYTES = {
 }
 
 
-# DRAM bytes (read + write) of one step of each kernel on the bench geometry
-# at 16 shots, from ncu --set full captures of both launches of a step
-TRAFFIC_16SHOT = {"k_ac_fwd": 148.9e6, "k_ac_adj": 245.3e6}
+# DRAM bytes (read + write) of one storing forward step and one adjoint step on the
+# bench geometry at 16 shots (four groups), from ncu, caches left alone between launches:
+# a group's fields stay in L2 between its steps, so this is below the algorithmic count
+TRAFFIC_16SHOT = {"k_ac_fwd": 61.8e6, "k_ac_adj": 198.8e6}
 
 
 def workload(nstep=3000, nshots=64, seed=1234):
@@ -628,15 +629,18 @@ def main():
     rc_ms, rc_n, rc_cells = timing["recompute"]
     adj_ms, adj_n, adj_cells = timing["adjoint"]
     nseg = math.ceil((nstep - 1) / 100)
-    # a step is two launches of each kernel (interior items, PML items); the
-    # timed ranges hold whole steps, so per-launch means cover both
+    # a step is two launches of each kernel (interior items, PML items) a group of
+    # shots; the timed ranges hold whole steps, so per-launch means cover both.  The
+    # recompute and adjoint ranges are one segment of the groups that run beside each
+    # other: `rounds` such sets make the plan
     cells_per_step = sum(s["nx"] * MY for s in shots)
+    rounds = cells_per_step * min(100, nstep - 1) / adj_cells
     kern = {
         "k_ac_fwd": dict(ms_per_launch=fwd_ms / fwd_n, bytes=BYTES[("fwd", "f32")] * fwd_cells / fwd_n,
-                         launches=fwd_n + rc_n * (nseg - plan.resident_segments),
+                         launches=fwd_n + rc_n * rounds * (nseg - plan.resident_segments),
                          launches_per_step=fwd_n / (fwd_cells / cells_per_step)),
         "k_ac_adj": dict(ms_per_launch=adj_ms / adj_n, bytes=BYTES[("adj", "f32")] * adj_cells / adj_n,
-                         launches=adj_n * nseg,
+                         launches=adj_n * rounds * nseg,
                          launches_per_step=adj_n / (adj_cells / cells_per_step)),
     }
     for k, v in kern.items():
@@ -644,8 +648,8 @@ def main():
         v["total_ms"] = v["ms_per_launch"] * v["launches"]
     dom = max(kern, key=lambda k: kern[k]["total_ms"])
     d = kern[dom]
-    # DRAM read + write bytes of one step (both launches) from ncu --set full
-    # captures of the same workload at 16 shots, scaled by the shots a step
+    # DRAM read + write bytes of one step (all launches) from ncu captures of the
+    # same workload at 16 shots, scaled by the shots a step
     # processes here (traffic grows with the shot count), per launch like achieved
     per_shot_step = {"k_ac_fwd": TRAFFIC_16SHOT["k_ac_fwd"] / 16,
                      "k_ac_adj": TRAFFIC_16SHOT["k_ac_adj"] / 16}
@@ -656,6 +660,8 @@ def main():
                 "peak_source": peak_kind, "traffic": traffic,
                 "bytes_per_launch": d["bytes"], "ms_per_launch": d["ms_per_launch"],
                 "launches_per_step": round(d["launches_per_step"], 2),
+                "note": "algorithmic bytes; a group's fields stay in L2 between steps, "
+                        "`traffic` is what reaches DRAM",
                 "kernels": {k: {"achieved_gbs": round(v["achieved_gbs"], 1),
                                 "ms_per_launch": round(v["ms_per_launch"], 4),
                                 "launches_per_step": round(v["launches_per_step"], 2),
@@ -663,7 +669,7 @@ def main():
                             for k, v in kern.items()}}
     # the whole gradient: algorithmic bytes of its forward, recompute and
     # adjoint cell-updates over its measured time
-    rc_cu = rc_cells * max(nseg - plan.resident_segments, 0)
+    rc_cu = rc_cells * rounds * max(nseg - plan.resident_segments, 0)
     job_b = (BYTES[("fwd", "f32")] * (cell_steps / world + rc_cu) +
              BYTES[("adj", "f32")] * cell_steps / world)
     roofline["gradient"] = {"bytes": job_b, "achieved_gbs": round(job_b / (ms / 1e3) / 1e9, 1),
