@@ -3904,7 +3904,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
       ADS_CUDA(e);
       cudaGraphExec_t ex = nullptr;
       ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
-      ADS_CUDA(cudaGraphUpload(ex, st));  // (else the first launch waits for it)
+      // (else the first launch waits for it; where it fails, the launch will say so)
+      if (cudaGraphUpload(ex, st) != cudaSuccess) cudaGetLastError();
       if (which == 0) {
         gF = g;
         eF = ex;

@@ -3643,7 +3643,8 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
       ADS_CUDA(e);
       cudaGraphExec_t ex = nullptr;
       ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
-      ADS_CUDA(cudaGraphUpload(ex, st));  // (else the first launch waits for it)
+      // (else the first launch waits for it; where it fails, the launch will say so)
+      if (cudaGraphUpload(ex, st) != cudaSuccess) cudaGetLastError();
       (which == 0 ? gF : gR) = g;
       (which == 0 ? eF : eR) = ex;
     }
