@@ -39,6 +39,7 @@
 
 #include "ads_internal.h"
 #include "f32x4.h"
+#include "wide_split.h"
 
 namespace ads {
 namespace {
@@ -4127,23 +4128,10 @@ void AcPlan<T>::build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L)
   L.in_end.assign(nshots, 0);
   L.pm_end.assign(nshots, 0);
   const int ny = (int)cfg.MY, gi = Tile<T>::G * rows_in, gp = pml_tiles() * rows_pm;
-  // damped indices 1..n of a profile: leading and trailing runs (all of them where
-  // there are others between)
-  auto runs = [](const std::vector<double>& x, int n, int& lead, int& trail) {
-    auto near = [&](int i) { return x[i - 1] != 0.0 || x[i] != 0.0 || x[i + 1] != 0.0; };
-    lead = trail = 0;
-    while (lead < n && near(lead + 1)) lead++;
-    while (trail < n - lead && near(n - trail)) trail++;
-    for (int i = lead + 1; i <= n - trail; i++)
-      if (near(i)) lead = n, trail = 0;
-  };
   auto cut64 = [](int left) { return left == 68 ? 60 : std::min(64, left); };
-  int nl, nr;
-  runs(hty, ny, nl, nr);
-  const int jl = 64 * (int)div_up(nl, 64) + 1;
-  int jr = nr > 0 ? ny - 64 * (int)div_up(nr, 64) + 1 : ny + 1;  // first column past the rectangle
-  if (nr > 0) jr += ((1 - jr) % 4 + 4) % 4;
-  else jr -= ((jr - 1) % 4 + 4) % 4;
+  int nl, nr, jl, jr;
+  damped_runs(hty, ny, nl, nr);
+  wide_columns(ny, nl, nr, jl, jr);
   const bool center = jr > jl + 4;
   std::vector<std::pair<int, int>> side, mid;  // general strips (j0, width)
   if (center) {
@@ -4180,7 +4168,7 @@ void AcPlan<T>::build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L)
       return any;
     };
     int nt, nb;
-    runs(hsx[s], nx, nt, nb);
+    damped_runs(hsx[s], nx, nt, nb);
     auto add_pm = [&](int i0, int n, int j0, int w) {
       for (int i = i0; i < i0 + n; i += gp) {
         AcItem it{};
