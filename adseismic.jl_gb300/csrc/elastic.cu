@@ -118,7 +118,7 @@ struct CellModel {
   const T *axi, *axh, *bxi, *bxh, *ayi, *ayh, *byi, *byh;  // 1D, index I-1 / J-1
   T dt, rdt;                               // dt, 1 / dt
   T x1, y1;                                // 1 / (24 h)
-  double dtd;                              // dt, unrounded
+  double dtd;                              // dt, unrounded; plans: times what x1, y1 lack
   int NX, NY, OFF, P;
 };
 
@@ -1113,6 +1113,26 @@ CellModel<T> make_cells(int NX, int NY, int64_t P, int off, double dt, double dx
   M.OFF = off;
   M.P = (int)P;
   return M;
+}
+
+// FP32 plans: 1/(24 dx) and 1/(24 dy) times a common factor, close to 1, that leaves both
+// almost exact in FP32; the tables and gathered gradients carry its reciprocal (dtd),
+// rounded in FP64.  1/(24h) rounded by itself scales every difference by up to 6e-8, a
+// wave speed error that builds up over the record (h = 10: 5e-8, and 1.3 times the row
+// kernels' error in the traces of 500 steps).  For dx = dy the factor is that rounding.
+inline void scale_differences(CellModel<double>&, double, double, double) {}
+inline void scale_differences(CellModel<float>& M, double dt, double dx, double dy) {
+  const double rx = 1.0 / (24 * dx), ratio = dx / dy;
+  float a = (float)rx;
+  double best = 1.0;
+  for (int k = 0; k < 16; k++, a = std::nextafterf(a, 2 * a)) {
+    const double off = std::fabs((double)(float)(a * ratio) / (a * ratio) - 1.0);
+    if (!(off < best)) continue;
+    best = off;
+    M.x1 = a;
+    M.y1 = (float)(a * ratio);
+    M.dtd = dt * (rx / a);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -3616,6 +3636,8 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   ADS_CUDA(cudaStreamSynchronize(st));
   if (c.autotune && c.rows_per_warp <= 0)
     if (int e = autotune(st, rw_min, rf_min)) return e;
+  // (both sweeps, or the strains one stores are not what the other takes them for)
+  if (cellf && cella) scale_differences(C, c.dt, c.dx, c.dy);
   tiling[0] = fused ? rows_a : rows_w;
   tiling[1] = rows_f;
   for (int k = 0; k < 4; k++) adj_items[k] = fused ? nwka[k] : 0;
