@@ -463,7 +463,6 @@ k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                  const CellItem* __restrict__ items, int pin, int slot) {
   ADS_EL_ITEM();
   ADS_EL_PLAN_CELL();
-  if (i > M.NX || j > M.NY) return;
   const int64_t fs = sh.fs;
   const T* f = sh.f[0] + (int64_t)pin * NF * fs;
   T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
@@ -498,7 +497,6 @@ k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                    const CellItem* __restrict__ items, int pin, int slot) {
   ADS_EL_ITEM();
   ADS_EL_PLAN_CELL();
-  if (i > M.NX || j > M.NY) return;
   const int64_t fs = sh.fs;
   const T* f = sh.f[0] + (int64_t)pin * NF * fs;
   T* o = sh.f[0] + (int64_t)(1 - pin) * NF * fs;
