@@ -90,7 +90,7 @@ struct ElShot {
 //  * the four-point difference is (27 (a - b) - (c - d)) times 1/(24h): 4
 //    operations and no division (a division is some twenty);
 //  * plans fold dt into tables of the averaged moduli and of dt / density
-//    (k_el_tables, once a call), 44 operations a CPML-free cell and step;
+//    (k_el_tables, once a call), 41 operations a CPML-free cell and step;
 //  * the transpose forms what a cell sends (q, D1..D8 in the comments of the
 //    reference's order: fw4..fw1 transposed) once, in shared memory, over a tile
 //    and the three rows or columns that reach into it, and gathers it there; no
@@ -140,12 +140,17 @@ __device__ __forceinline__ bool el_tame(float x) {
   return (__float_as_int(x) & 0x7f800000) < 0x7f000000;
 }
 
+// 27 (a - b) - (c - d)
+template <typename T>
+__device__ __forceinline__ T raw(T a, T b, T c, T d) {
+  return el_fma(T(27), a - b, d - c);
+}
 // (27 (a - b) - (c - d)) / (24 h).  27/(24h) and 1/(24h) rounded apart cost as much and
 // leave weights that are no longer 27 : 1 (FP32 gradients of eight grids, 250 steps, rms
 // error of the loss 1.3e-7 against 0.6e-7, of grad_rho 8.2e-7 against 7.4e-7).
 template <typename T>
 __device__ __forceinline__ T dif(T a, T b, T c, T d, T k1) {
-  return k1 * el_fma(T(27), a - b, d - c);
+  return k1 * raw<T>(a, b, c, d);
 }
 
 // The strain or acceleration d + m' of one difference d, with its memory
@@ -245,40 +250,59 @@ __device__ __forceinline__ void strain1(const CellModel<T>& M, int i, int j, Cel
   e2 = mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 1) * fs,
                         fo ? fo + (M1 + 1) * fs : nullptr, x);
 }
+// Sum of two raw differences (27 (a - b) - (c - d)), scaled, with their memory variables
+// (plans: one operation less than the two sums apart).
+template <typename T, bool PLAN>
+__device__ __forceinline__ T mem_fwd2(T a, T k, T pa, T pb, const T* mi, T* mo, T b, T h, T qa,
+                                      T qb, const T* ni, T* no, CellIx<PLAN> x) {
+  const T d = k * a;
+  if constexpr (PLAN && sizeof(T) == 8) {
+    T s = el_fma(h, b, d);
+    if (!idle(pa, pb)) {
+      const T m = el_fma(pb, mi[x], pa * d);
+      mo[x] = m;
+      s += m;
+    }
+    if (!idle(qa, qb)) {
+      const T n = el_fma(qb, ni[x], qa * (h * b));
+      no[x] = n;
+      s += n;
+    }
+    return s;
+  }
+  return mem_fwd<T, PLAN>(d, pa, pb, mi, mo, x) + mem_fwd<T, PLAN>(h * b, qa, qb, ni, no, x);
+}
 template <typename T, bool PLAN>
 __device__ __forceinline__ T strain2(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* f,
                                      int64_t fs, T* fo) {
   const T* vx = f + VX * fs;
   const T* vy = f + VY * fs;
   const int P = M.P;
-  const T a = dif<T>(vy[x], vy[x - P], vy[x + P], vy[x - 2 * P], M.x1);
-  const T b = dif<T>(vx[x + 1], vx[x], vx[x + 2], vx[x - 1], M.y1);
-  return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 2) * fs,
-                          fo ? fo + (M1 + 2) * fs : nullptr, x) +
-         mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 3) * fs,
-                          fo ? fo + (M1 + 3) * fs : nullptr, x);
+  const T a = raw<T>(vy[x], vy[x - P], vy[x + P], vy[x - 2 * P]);
+  const T b = raw<T>(vx[x + 1], vx[x], vx[x + 2], vx[x - 1]);
+  return mem_fwd2<T, PLAN>(a, M.x1, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 2) * fs,
+                           fo ? fo + (M1 + 2) * fs : nullptr, b, M.y1, M.ayh[j - 1], M.byh[j - 1],
+                           f + (M1 + 3) * fs, fo ? fo + (M1 + 3) * fs : nullptr, x);
 }
 template <typename T, bool PLAN>
 __device__ __forceinline__ T accel3(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxx,
                                     const T* sxy, const T* f, int64_t fs, T* fo) {
   const int P = M.P;
-  const T a = dif<T>(sxx[x], sxx[x - P], sxx[x + P], sxx[x - 2 * P], M.x1);
-  const T b = dif<T>(sxy[x], sxy[x - 1], sxy[x + 1], sxy[x - 2], M.y1);
-  return mem_fwd<T, PLAN>(a, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 4) * fs,
-                          fo ? fo + (M1 + 4) * fs : nullptr, x) +
-         mem_fwd<T, PLAN>(b, M.ayi[j - 1], M.byi[j - 1], f + (M1 + 5) * fs,
-                          fo ? fo + (M1 + 5) * fs : nullptr, x);
+  const T a = raw<T>(sxx[x], sxx[x - P], sxx[x + P], sxx[x - 2 * P]);
+  const T b = raw<T>(sxy[x], sxy[x - 1], sxy[x + 1], sxy[x - 2]);
+  return mem_fwd2<T, PLAN>(a, M.x1, M.axi[i - 1], M.bxi[i - 1], f + (M1 + 4) * fs,
+                           fo ? fo + (M1 + 4) * fs : nullptr, b, M.y1, M.ayi[j - 1], M.byi[j - 1],
+                           f + (M1 + 5) * fs, fo ? fo + (M1 + 5) * fs : nullptr, x);
 }
 template <typename T, bool PLAN>
 __device__ __forceinline__ T accel4(const CellModel<T>& M, int i, int j, CellIx<PLAN> x, const T* sxy,
                                     const T* syy, const T* f, int64_t fs, T* fo) {
   const int P = M.P;
-  const T a = dif<T>(sxy[x + P], sxy[x], sxy[x + 2 * P], sxy[x - P], M.x1);
-  const T b = dif<T>(syy[x + 1], syy[x], syy[x + 2], syy[x - 1], M.y1);
-  return mem_fwd<T, PLAN>(a, M.axh[i - 1], M.bxh[i - 1], f + (M1 + 6) * fs,
-                          fo ? fo + (M1 + 6) * fs : nullptr, x) +
-         mem_fwd<T, PLAN>(b, M.ayh[j - 1], M.byh[j - 1], f + (M1 + 7) * fs,
-                          fo ? fo + (M1 + 7) * fs : nullptr, x);
+  const T a = raw<T>(sxy[x + P], sxy[x], sxy[x + 2 * P], sxy[x - P]);
+  const T b = raw<T>(syy[x + 1], syy[x], syy[x + 2], syy[x - 1]);
+  return mem_fwd2<T, PLAN>(a, M.x1, M.axh[i - 1], M.bxh[i - 1], f + (M1 + 6) * fs,
+                           fo ? fo + (M1 + 6) * fs : nullptr, b, M.y1, M.ayh[j - 1], M.byh[j - 1],
+                           f + (M1 + 7) * fs, fo ? fo + (M1 + 7) * fs : nullptr, x);
 }
 
 // Cell of a thread: row blocks along blockIdx.x (their count may pass 65535),
