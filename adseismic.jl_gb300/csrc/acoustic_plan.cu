@@ -2338,8 +2338,9 @@ __device__ __forceinline__ CellRef first_ref(const CellRef* __restrict__ l, int 
   return e < end ? l[e] : CellRef{0, 0, -1};
 }
 
-// Forward step t (MODE, CK as k_ac_fwd; FP32 the increment form).
-template <typename T, int MODE, bool VU, bool CK>
+// Forward step t (MODE, CK as k_ac_fwd; FP32 the increment form).  LATE: the next
+// launch's blocks start at the end of this one (AcPlan::late_release).
+template <typename T, int MODE, bool VU, bool CK, bool LATE = false>
 __global__ void __launch_bounds__(32 * CRF, sizeof(T) == 8 && VU ? 6 : 8)
 k_ac_cell_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
               const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs, AcConst<T> K,
@@ -2402,7 +2403,7 @@ k_ac_cell_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
   }
   const CellRef rc0 = NOREC ? CellRef{0, 0, -1} : first_ref(rcvs, it.rcv_b + lane, it.rcv_e);
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   T w0 = T(0), wN = T(0), wS = T(0), wE = T(0), wW = T(0), o0 = T(0);
   if (on) {
     w0 = w[o];
@@ -2506,6 +2507,7 @@ k_ac_cell_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
       }
     }
   }
+  if (LATE) grid_release();
   if constexpr (!NOREC) {  // the warp's row holds the receivers' values
     CellRef q = rc0;
     for (int e = it.rcv_b; e < it.rcv_e; e += 32) {
@@ -2526,7 +2528,7 @@ k_ac_cell_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
 // sends, and the first 64 + 2 CRA threads that of one cell of the ring, from loads
 // issued together; then one barrier (two in variant U's tiles near damped cells,
 // whose phi and psi terms need lambdaU / den of the cells beside).
-template <typename T, bool VU>
+template <typename T, bool VU, bool LATE = false>
 __global__ void __launch_bounds__(32 * CRA, sizeof(T) == 8 ? 6 : 8)
 k_ac_cell_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
               const CellRef* __restrict__ srcs, const CellRef* __restrict__ rcvs, AcConst<T> K,
@@ -2586,7 +2588,7 @@ k_ac_cell_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
     }
   }
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   T ln = T(0), w0 = T(0), wN = T(0), wS = T(0), wE = T(0), wW = T(0), gi = T(0), rg = T(0);
   T lp = T(0), lq = T(0), rl = T(0);
   using G = typename GradOf<T>::type;
@@ -2717,6 +2719,7 @@ k_ac_cell_adj(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ sh
     if constexpr (F64) grad_base(sh)[o] = fm(lap, gi, gc);
     else grad_base(sh)[o] = gc + (D.damped ? lap : lap * gi);
   }
+  if (LATE) grid_release();
   if (k - 1 >= 2 && it.rcv_e > it.rcv_b) {
     __syncwarp();
     auto add = [&](int64_t cell, T x) {
@@ -3206,6 +3209,19 @@ struct AcPlan final : AcPlanBase {
   // one-thread-per-cell kernels (k_ac_cell_fwd / _adj): their tiles of `rows` rows,
   // all in the list's PML part
   bool percell = false;
+  // FP64: blocks of their kernels that are resident at once, forward / adjoint.  A launch
+  // of n blocks, over about half of them, leaves too few slots for the whole next launch:
+  // its first blocks wait in those, the rest go to whichever SM is done first, and one SM
+  // ends with all its slots full where another has few.  Latency does not mind, FP64
+  // issue does, so there the next launch starts at the end of this one.  us a step,
+  // release after the wait / at the end, variant W forward: 480 blocks 3.64 / 4.47, 675
+  // 5.70 / 4.61, 830 7.03 / 4.87, 1125 8.53 / 5.68, 1925 6.88 / 7.22 (1216 slots); adjoint:
+  // 300 blocks 4.2 / 4.9, 675 9.6 / 6.6, 968 8.5 / 8.2, 1100 8.2 / 8.6 (912 slots).
+  int slots_f = 0, slots_a = 0;
+  static int late_release(int n, int slots) {
+    return sizeof(T) == 8 && n > 0.55 * slots && n <= 1.1 * slots;
+  }
+  int count_slots();
   // FP32: interior items through the four-column kernels (k_ac_wide_fwd / _adj)
   bool wide = false;
   int ri_wf = 8, ri_wa = 8;  // their rows per warp, forward / adjoint
@@ -3583,6 +3599,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   }
   TileList tiles_a, tiles_f;
   if (percell) {
+    if (sizeof(T) == 8)
+      if (int e = count_slots()) return e;
     build_cells(CRA, pitch, tiles_a);
     build_cells(CRF, pitch, tiles_f);
   } else if (wide) {
@@ -4441,6 +4459,23 @@ void AcPlan<T>::build_cells(int rows, int64_t pitch, TileList& L) const {
 }
 
 template <typename T>
+int AcPlan<T>::count_slots() {
+  int dev = 0, sms = 0;
+  ADS_CUDA(cudaGetDevice(&dev));
+  ADS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  auto blocks = [&](auto kernel, int threads, int& out) -> int {
+    ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out, kernel, threads, 0));
+    out *= sms;
+    return ADS_OK;
+  };
+  if (int e = vu ? blocks(k_ac_cell_fwd<T, 0, true, false>, 32 * CRF, slots_f)
+                 : blocks(k_ac_cell_fwd<T, 0, false, false>, 32 * CRF, slots_f))
+    return e;
+  return vu ? blocks(k_ac_cell_adj<T, true>, 32 * CRA, slots_a)
+            : blocks(k_ac_cell_adj<T, false>, 32 * CRA, slots_a);
+}
+
+template <typename T>
 int AcPlan<T>::upload_tiles(const TileList& L, DevTiles& D, cudaStream_t st) {
   if (!L.in.empty())
     ADS_CUDA(cudaMemcpyAsync(D.items, L.in.data(), sizeof(AcItem) * L.in.size(),
@@ -4540,14 +4575,19 @@ int AcPlan<T>::launch_fwd(cudaStream_t st, int mode, int s0, int s1, int t, int 
       return launch_chained(kernel, dim3(n), dim3(32 * CRF), st, tf.items + tf.pm_upto(s0), d_shots, tf.srcs,
                             tf.rcvs, kc, t, base, ck);
     };
-    auto by_mode = [&](auto u) {
-      constexpr bool U = decltype(u)::value;
-      if (mode == 1) return go(k_ac_cell_fwd<T, 1, U, false>);
-      if (mode == 2) return go(k_ac_cell_fwd<T, 2, U, false>);
-      if (ck > 0) return go(k_ac_cell_fwd<T, 0, U, true>);
-      return go(k_ac_cell_fwd<T, 0, U, false>);
+    constexpr bool F64 = sizeof(T) == 8;
+    auto by_mode = [&](auto u, auto l) {
+      constexpr bool U = decltype(u)::value, L = F64 && decltype(l)::value;
+      if (mode == 1) return go(k_ac_cell_fwd<T, 1, U, false, L>);
+      if (mode == 2) return go(k_ac_cell_fwd<T, 2, U, false, L>);
+      if (ck > 0) return go(k_ac_cell_fwd<T, 0, U, true, L>);
+      return go(k_ac_cell_fwd<T, 0, U, false, L>);
     };
-    ADS_CUDA(vu ? by_mode(std::true_type{}) : by_mode(std::false_type{}));
+    const std::true_type yes{};
+    const std::false_type no{};
+    const bool late = late_release(n, slots_f);
+    ADS_CUDA(vu ? late ? by_mode(yes, yes) : by_mode(yes, no)
+                : late ? by_mode(no, yes) : by_mode(no, no));
     ADS_LAUNCHED(1);
     return ADS_OK;
   }
@@ -4667,9 +4707,12 @@ int AcPlan<T>::launch_adj(cudaStream_t st, int s0, int s1, int k, int base, int 
   if (percell) {
     const int n = ta.pm_of(s0, s1);
     if (n == 0) return ADS_OK;
-    ADS_CUDA(launch_chained(vu ? k_ac_cell_adj<T, true> : k_ac_cell_adj<T, false>, dim3(n),
-                            dim3(32 * CRA), st, ta.items + ta.pm_upto(s0), d_shots, ta.srcs, ta.rcvs, kc, k, base,
-                            dt2d));
+    constexpr bool F64 = sizeof(T) == 8;
+    const bool late = late_release(n, slots_a);
+    auto kernel = vu ? late ? k_ac_cell_adj<T, true, F64> : k_ac_cell_adj<T, true>
+                     : late ? k_ac_cell_adj<T, false, F64> : k_ac_cell_adj<T, false>;
+    ADS_CUDA(launch_chained(kernel, dim3(n), dim3(32 * CRA), st, ta.items + ta.pm_upto(s0), d_shots,
+                            ta.srcs, ta.rcvs, kc, k, base, dt2d));
     ADS_LAUNCHED(1);
     return ADS_OK;
   }

@@ -481,7 +481,8 @@ k_el_strip_velocity(CellModel<float> M, const ElShot<float>* __restrict__ shots,
   const int i = i0 + ty, j = j0 + tx, P = M.P, x = i * P + j + M.OFF;          \
   (void)P, (void)x
 
-template <typename T, bool STORE>
+// LATE: the next launch's blocks start at the end of this one (ElPlan::late_release).
+template <typename T, bool STORE, bool LATE = false>
 __global__ void __launch_bounds__(BX* BY)
 k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                  const CellItem* __restrict__ items, int pin, int slot) {
@@ -495,7 +496,7 @@ k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
   if (box1(M, i, j)) mat1<T, true>(M, x, lm, la);
   if (box2(M, i, j)) m2 = mat2<T, true>(M, x);
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   if (box1(M, i, j)) {
     T e1, e2;
     strain1<T, true>(M, i, j, x, f, fs, o, e1, e2);
@@ -513,9 +514,10 @@ k_el_cell_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
     o[SXY * fs + x] = el_fma(m2, e, f[SXY * fs + x]);
     if (STORE) st[E12 * fs + x] = e;
   }
+  if (LATE) grid_release();
 }
 
-template <typename T, bool STORE>
+template <typename T, bool STORE, bool LATE = false>
 __global__ void __launch_bounds__(BX* BY)
 k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                    const CellItem* __restrict__ items, int pin, int slot) {
@@ -528,7 +530,7 @@ k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
   const T b3 = box3(M, i, j) ? mat3<T, true>(M, x) : T(0),
           b4 = box4(M, i, j) ? mat4<T, true>(M, x) : T(0);
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   if (box3(M, i, j)) {
     const T e = accel3<T, true>(M, i, j, x, o + SXX * fs, o + SXY * fs, f, fs, o);
     o[VX * fs + x] = el_fma(b3, e, f[VX * fs + x]);
@@ -539,6 +541,7 @@ k_el_cell_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
     o[VY * fs + x] = el_fma(b4, e, f[VY * fs + x]);
     if (STORE) st[A4 * fs + x] = e;
   }
+  if (LATE) grid_release();
 }
 
 // What the velocity cells of a tile and its halo send to the stresses: D5
@@ -821,7 +824,7 @@ k_el_strip_adj_velocity(CellModel<float> M, const ElShot<float>* __restrict__ sh
 
 // Adjoint of a step, velocity cells -> stress adjoints (transposes of fw3, fw4):
 // adjoint buffer pin -> the other.
-template <typename T>
+template <typename T, bool LATE = false>
 __global__ void __launch_bounds__(BX* BY)
 k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                      const CellItem* __restrict__ items, int pin, int slot) {
@@ -832,7 +835,7 @@ k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
   const T* g = sh.g[0] + (int64_t)pin * NF * fs;
   T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   T q3, q4;
   send_velocity<T, true>(M, S, i0, j0, g, o, fs, q3, q4);
   const T* st = sh.store + (int64_t)slot * NSTORE * fs;
@@ -848,10 +851,11 @@ k_el_cell_adj_stress(CellModel<T> M, const ElShot<T>* __restrict__ shots,
     o[SYY * fs + x] = syy;
   }
   if (c2) o[SXY * fs + x] = sxy;
+  if (LATE) grid_release();
 }
 
 // Adjoint of a step, stress cells -> velocity adjoints (transposes of fw1, fw2).
-template <typename T>
+template <typename T, bool LATE = false>
 __global__ void __launch_bounds__(BX* BY)
 k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
                        const CellItem* __restrict__ items, int pin, int slot) {
@@ -862,7 +866,7 @@ k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
   const T* g = sh.g[0] + (int64_t)pin * NF * fs;
   T* o = sh.g[0] + (int64_t)(1 - pin) * NF * fs;
   grid_wait();
-  grid_release();
+  if (!LATE) grid_release();
   send_stress<T, true>(M, S, i0, j0, o, g, o, fs);
   const T* st = sh.store + (int64_t)slot * NSTORE * fs;
   if (box1(M, i, j)) {
@@ -878,6 +882,7 @@ k_el_cell_adj_velocity(CellModel<T> M, const ElShot<T>* __restrict__ shots,
   gather_velocity<T>(M, S, vx, vy);
   if (c3) o[VX * fs + x] = vx;
   if (c4) o[VY * fs + x] = vy;
+  if (LATE) grid_release();
 }
 
 // The plans' tables from lambda, mu, rho, in FP64, rounded once; zero outside
@@ -3156,6 +3161,14 @@ struct ElPlan final : ElPlanBase {
   template <typename F>
   int each_group(cudaStream_t st, F&& fn);
   // the blocks of a shot (CellItem), and whether interior strips are among them
+  // FP64: as AcPlan::late_release, from a block an SM on (the blocks hold twice the
+  // threads).  us a forward / gradient step, release after the wait / at the end: 192
+  // blocks 17.0 / 36.1 against 15.6 / 35.1, 357 23.1 / 46.8 against 20.6 / 44.3, 750
+  // 36.3 / 77.1 against 30.9 / 66.9, 80 10.9 / 26.0 against 11.0 / 26.3.
+  int slots = 0;
+  bool late_release(int n) const {
+    return sizeof(T) == 8 && n_cells * n > 0.12 * slots && n_cells * n <= 1.1 * slots;
+  }
   CellItem* d_cells = nullptr;
   int n_cells = 0, n_strips = 0;
   std::vector<CellItem> cell_items() const;
@@ -3414,7 +3427,15 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   hprof = pack_profiles<T>(NX, NY, ax.data(), bx.data(), ay.data(), by.data());
   const std::vector<T>& prof = hprof;
   std::vector<CellItem> cells;
-  if (cellf || cella) cells = cell_items();
+  if (cellf || cella) {
+    int dev = 0, sms = 0;
+    ADS_CUDA(cudaGetDevice(&dev));
+    ADS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    ADS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&slots, k_el_cell_adj_stress<T>,
+                                                           BX * BY, 0));
+    slots *= sms;
+    cells = cell_items();
+  }
   n_cells = (int)cells.size();
   for (const CellItem& q : cells) n_strips += q.w > 0;
   n_cells -= n_strips;
@@ -4031,10 +4052,12 @@ template <typename T>
 int ElPlan<T>::adjoint_step(const Run& q, int slot, int n) {
   const ElShot<T>* sh = d_shots + q.s0;
   if (cella) {
+    constexpr bool F64 = sizeof(T) == 8;
+    const bool late = late_release(q.n);
     const dim3 b(BX, BY);
     if (int e = cells_and_strips(q, [&](cudaStream_t s, bool strip) {
           if (!strip)
-            return launch_in_loop(!n_strips, k_el_cell_adj_stress<T>, grid_cells(q.n), b, s, C, sh,
+            return launch_in_loop(!n_strips, late ? k_el_cell_adj_stress<T, F64> : k_el_cell_adj_stress<T>, grid_cells(q.n), b, s, C, sh,
                                   d_cells, apar(n), slot);
           if constexpr (sizeof(T) == 4)
             return launch_in_loop(false, k_el_strip_adj_stress, grid_strips(q.n), b, s, C, sh,
@@ -4044,7 +4067,7 @@ int ElPlan<T>::adjoint_step(const Run& q, int slot, int n) {
       return e;
     return cells_and_strips(q, [&](cudaStream_t s, bool strip) {
       if (!strip)
-        return launch_in_loop(!n_strips, k_el_cell_adj_velocity<T>, grid_cells(q.n), b, s, C, sh,
+        return launch_in_loop(!n_strips, late ? k_el_cell_adj_velocity<T, F64> : k_el_cell_adj_velocity<T>, grid_cells(q.n), b, s, C, sh,
                               d_cells, apar(n), slot);
       if constexpr (sizeof(T) == 4)
         return launch_in_loop(false, k_el_strip_adj_velocity, grid_strips(q.n), b, s, C, sh,
@@ -4085,11 +4108,14 @@ int ElPlan<T>::step_kernels(const Run& q, int n, bool store, int slot) {
       el_step<T>(store, k, grid_rows(nwk[k], q.n), s, M, sh, d_wlf + owk[k], ncolf, rows_f,
                  nwk[k], sl, pin, jsh, ish);
     });
+  constexpr bool F64 = sizeof(T) == 8;
+  const bool late = late_release(q.n);
   const dim3 b(BX, BY);
   if (int e = cells_and_strips(q, [&](cudaStream_t s, bool strip) {
         if (!strip)
           return launch_in_loop(!n_strips,
-                                store ? k_el_cell_stress<T, true> : k_el_cell_stress<T, false>,
+                                late ? store ? k_el_cell_stress<T, true, F64> : k_el_cell_stress<T, false, F64>
+                                     : store ? k_el_cell_stress<T, true> : k_el_cell_stress<T, false>,
                                 grid_cells(q.n), b, s, C, sh, d_cells, pin, sl);
         if constexpr (sizeof(T) == 4)
           return launch_in_loop(false, store ? k_el_strip_stress<true> : k_el_strip_stress<false>,
@@ -4100,7 +4126,8 @@ int ElPlan<T>::step_kernels(const Run& q, int n, bool store, int slot) {
   return cells_and_strips(q, [&](cudaStream_t s, bool strip) {
     if (!strip)
       return launch_in_loop(!n_strips,
-                            store ? k_el_cell_velocity<T, true> : k_el_cell_velocity<T, false>,
+                            late ? store ? k_el_cell_velocity<T, true, F64> : k_el_cell_velocity<T, false, F64>
+                                 : store ? k_el_cell_velocity<T, true> : k_el_cell_velocity<T, false>,
                             grid_cells(q.n), b, s, C, sh, d_cells, pin, sl);
     if constexpr (sizeof(T) == 4)
       return launch_in_loop(false, store ? k_el_strip_velocity<true> : k_el_strip_velocity<false>,
