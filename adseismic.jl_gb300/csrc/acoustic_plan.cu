@@ -1023,11 +1023,13 @@ __device__ __forceinline__ void record_src_grad(const AcItem& it, const AcShot<T
                                                 const T* lp, const T* lq, const AcConst<T>& K,
                                                 int k, int lane, int i0, int i_end, double dt2) {
   if (k - 1 < 2 || it.src_e <= it.src_b) return;
+  // (the four-column kernels' items may be narrower than a warp's columns)
+  const int width = C == 4 ? it.pad & 0xffff : 32 * C;
   __syncwarp();
   for (int e = it.src_b + lane; e < it.src_e; e += 32) {
     const CellRef r = srcs[e];
     const int jc = (int)(r.cell - (int64_t)r.row * sh.pitch) - JOFF;
-    if (r.row < i0 || r.row >= i_end || jc < it.j0 || jc >= it.j0 + (it.pad & 0xffff)) continue;
+    if (r.row < i0 || r.row >= i_end || jc < it.j0 || jc >= it.j0 + width) continue;
     double g = (double)lun[r.cell];
     if constexpr (VU) {
       const int64_t P = sh.pitch, x = r.cell;
@@ -3108,7 +3110,8 @@ namespace {
 // once for two updates, are ahead.  us per forward / adjoint step, cell against row
 // kernels: W 26.7 k cells 1.9 / 2.6 against 3.9 / 4.7, 160 k 2.7 / 4.0 against 4.2 / 4.7,
 // 320 k 3.9 / 6.0 against 4.5 / 5.2; U 26.7 k 4.4 / 3.7 against 8.9 / 10.4, 640 k
-// 8.1 / 11.5 against 10.7 / 12.7, 1.28 M 12.9 / 20.8 against 12.4 / 18.2.
+// 8.1 / 11.5 against 10.7 / 12.7, 1.28 M 12.9 / 20.8 against 12.4 / 18.2 (below its limit
+// U takes them where they are ahead: AcPlan::cells_ahead_u).
 constexpr int64_t kCellMaxAc32 = 300000, kCellMaxAc32U = 1000000;
 
 // FP32 plans above that: the interior items through the four-column kernels
@@ -3222,6 +3225,7 @@ struct AcPlan final : AcPlanBase {
     return sizeof(T) == 8 && n > 0.55 * slots && n <= 1.1 * slots;
   }
   int count_slots();
+  bool cells_ahead_u() const;
   // FP32: interior items through the four-column kernels (k_ac_wide_fwd / _adj)
   bool wide = false;
   int ri_wf = 8, ri_wa = 8;  // their rows per warp, forward / adjoint
@@ -3465,13 +3469,22 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
               "time blocking is implemented for FP32 plans (steps_per_block 0 or 1 for FP64)");
   ADS_REQUIRE(!vu || KB == 1,
               "time blocking is implemented for variant W (steps_per_block 0 or 1 for U)");
+  // host copies of the PML profiles (the kernels' interior / PML split uses them)
+  hsx.assign(ns, {});
+  hty.assign(MY + 2, 0.0);
+  for (int s = 0; s < ns; s++) {
+    const ads_acoustic_shot& h = shots[order[s]];
+    hsx[s].assign(h.nx + 2, 0.0);
+    acoustic_pml_1d(h.nx, MY, c.dx, c.dy, c.npml, c.vp_ref, c.Rcoef, c.use_pml,
+                    hsx[s].data(), hty.data());
+  }
   tb_cells = cells;
   RB = tb_rows_for(KB);
   // steps per launch are tuned only on request (autotune 2): the time-blocked
   // kernel keeps the three-level form, whose FP32 rounding error is larger
   tb_auto = sizeof(T) == 4 && c.autotune >= 2 && c.steps_per_block == 0 && !vu;
   percell = KB == 1 && c.rows_per_thread <= 0 && c.tma <= 0 &&
-            (sizeof(T) == 8 || cells <= (vu ? kCellMaxAc32U : kCellMaxAc32));
+            (sizeof(T) == 8 || (vu ? cells <= kCellMaxAc32U && cells_ahead_u() : cells <= kCellMaxAc32));
   if (percell) tb_auto = false;
   inc = sizeof(T) == 4 && KB == 1;
   wide = sizeof(T) == 4 && KB == 1 && !percell && !tb_auto && c.rows_per_thread <= 0 &&
@@ -3571,15 +3584,6 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
       shot_rcvs.push_back({(int64_t)i * pitch + j + JOFF, (int)r, i});
     }
     rcv_e_host[s] = (int)shot_rcvs.size();
-  }
-  // host copies of the PML profiles (the kernels' interior / PML split uses them)
-  hsx.assign(ns, {});
-  hty.assign(MY + 2, 0.0);
-  for (int s = 0; s < ns; s++) {
-    const ads_acoustic_shot& h = shots[order[s]];
-    hsx[s].assign(h.nx + 2, 0.0);
-    acoustic_pml_1d(h.nx, MY, c.dx, c.dy, c.npml, c.vp_ref, c.Rcoef, c.use_pml,
-                    hsx[s].data(), hty.data());
   }
   // forward and adjoint warp items (rows per thread chosen separately; the
   // autotuner may replace both once the plan's buffers exist): enough warps
@@ -4456,6 +4460,37 @@ void AcPlan<T>::build_cells(int rows, int64_t pitch, TileList& L) const {
     L.pm_end[s] = (int)L.pm.size();
   }
   order_items(L, cost);
+}
+
+// FP32 variant U up to kCellMaxAc32U cells: whether the one-thread-per-cell kernels take
+// less time a step than the row kernels.  Theirs grows with the rows of 32 columns, of
+// which a damped one costs twice a free one; the row kernels' hides the interior under
+// the damped items' three launches, so it grows with the rows of 64 columns of those,
+// from a higher base.  Fitted to 20 gradients of 0.3-1 M cells, 12 and 40 damped cells a
+// side, within 8%: 0.65 us a thousand free rows, 1.33 damped, + 3.4; 1.41 a thousand
+// rows of damped items, + 17.9.  us a step, cells / rows: one shot of 1000 x 700
+// 18.8-20.5 / 22.7, 4 of 500 x 400 23.1-26.7 / 24.3-28.1, 10 of 320 x 300 29.7-36.1 /
+// 28.8-30.6, one of 1100 x 880 24.6-26.8 / 23.3-23.6.
+template <typename T>
+bool AcPlan<T>::cells_ahead_u() const {
+  auto near = [](const std::vector<double>& x, int i) {
+    return x[i - 1] != 0.0 || x[i] != 0.0 || x[i + 1] != 0.0;
+  };
+  const int ny = (int)cfg.MY;
+  int64_t n32 = div_up(ny, 32), n64 = div_up(ny, 64), d32 = 0, d64 = 0, last32 = -1, last64 = -1;
+  for (int j = 1; j <= ny; j++) {
+    if (!near(hty, j)) continue;
+    if ((j - 1) / 32 != last32) d32++, last32 = (j - 1) / 32;
+    if ((j - 1) / 64 != last64) d64++, last64 = (j - 1) / 64;
+  }
+  double cell = 0, row = 22000;
+  for (int s = 0; s < nshots; s++) {
+    int64_t nx = nxs[s], r = 0;
+    for (int i = 1; i <= nx; i++) r += near(hsx[s], i);
+    cell += (nx - r) * (n32 - d32) + 2.0 * (nx * d32 + r * (n32 - d32));
+    row += 2.2 * (nx * d64 + r * (n64 - d64));
+  }
+  return cell <= row;
 }
 
 template <typename T>
