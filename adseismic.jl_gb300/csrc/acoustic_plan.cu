@@ -3256,6 +3256,7 @@ struct AcPlan final : AcPlanBase {
     return n;
   }
   void group_shots(int64_t pitch);
+  int64_t graph_nodes = 0;  // (an upper estimate)
   // step launches over sorted shots [s0, s1) (interior and PML kernels) on chain c
   int launch_fwd(cudaStream_t st, int mode, int s0, int s1, int t, int base, int ck, int c = 0);
   int launch_adj(cudaStream_t st, int s0, int s1, int k, int base, int c = 0);
@@ -3283,7 +3284,6 @@ struct AcPlan final : AcPlanBase {
   // fork / join through events
   cudaStream_t chain[kChains] = {}, side[kChains] = {};
   cudaEvent_t ev_fork[kChains] = {}, ev_join[kChains] = {}, ev_chain[kChains] = {};
-  cudaGraph_t gF = nullptr, gR = nullptr;
   cudaGraphExec_t eF = nullptr, eR = nullptr;
   int64_t nF = 0, nR = 0;  // kernel launches in each loop
   // Timing events (recorded inside the loops / graphs): [0,1] the forward
@@ -3324,8 +3324,6 @@ struct AcPlan final : AcPlanBase {
       if (e) cudaEventDestroy(e);
     if (eF) cudaGraphExecDestroy(eF);
     if (eR) cudaGraphExecDestroy(eR);
-    if (gF) cudaGraphDestroy(gF);
-    if (gR) cudaGraphDestroy(gR);
     if (cap) cudaStreamDestroy(cap);
     for (int c = 0; c < kChains; c++) {
       for (cudaEvent_t e : {ev_fork[c], ev_join[c], ev_chain[c]})
@@ -3687,7 +3685,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   res_seg = nseg_max;
   {
     std::vector<size_t> fsb(ns);
-    size_t base_bytes = L.used;
+    size_t base_bytes = L.used + (c.use_graph ? graph_nodes * kGraphNodeBytes : 0);
     for (int q = 0; q < ns; q++) {
       fsb[q] = (size_t)(shots[order[q]].nx + 2) * pitch * sizeof(T);
       base_bytes += (K + 2) * fsb[q] + 256;
@@ -3928,17 +3926,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
         return rc;
       }
       ADS_CUDA(e);
-      cudaGraphExec_t ex = nullptr;
-      ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
-      // (else the first launch waits for it; where it fails, the launch will say so)
-      if (cudaGraphUpload(ex, st) != cudaSuccess) cudaGetLastError();
-      if (which == 0) {
-        gF = g;
-        eF = ex;
-      } else {
-        gR = g;
-        eR = ex;
-      }
+      if (int rc = finish_graph(g, st, which == 0 ? &eF : &eR)) return rc;
     }
   }
   return ADS_OK;
@@ -4314,11 +4302,10 @@ int AcPlan<T>::autotune_wide(cudaStream_t st, int64_t pitch) {
 }
 
 // Groups of about kGroupBytes of live fields each (Q, u or their like: three a shot), an
-// even number of them, handed to the chain with the least work so far.
+// even number of them, handed to the chain with the least work so far; fewer where the
+// graphs would pass kMaxGraphNodes.
 template <typename T>
 void AcPlan<T>::group_shots(int64_t pitch) {
-  gb.assign(1, 0);
-  for (auto& l : chain_groups) l.clear();
   std::vector<int64_t> live(nshots);
   int64_t total = 0;
   for (int s = 0; s < nshots; s++) {
@@ -4327,23 +4314,42 @@ void AcPlan<T>::group_shots(int64_t pitch) {
   }
   const int64_t per = vu ? kGroupBytesU : kGroupBytes;
   const bool split = wide && cfg.use_graph && nshots >= (vu ? kSplitShotsU : 2);
-  const int64_t n = split ? kChains * div_up(total, kChains * per) : 1;
-  int64_t sum = 0, work[kChains] = {}, w = 0;
-  for (int s = 0, g = 0; s < nshots; s++) {
-    w += live[s] * nstep[s];
-    sum += live[s];
-    // the group ends where the next shot's middle lies past its share
-    const bool end = s + 1 == nshots || (sum + live[s + 1] / 2) * n > (g + 1) * total;
-    if (!end) continue;
-    int c = 0;
-    for (int k = 1; k < kChains; k++)
-      if (work[k] < work[c]) c = k;
-    work[c] += w;
-    chain_groups[c].push_back((int)gb.size() - 1);
-    gb.push_back(s + 1);
-    w = 0;
-    while ((g + 1) * total <= sum * n && g + 1 < n) g++;
+  // n groups; returns the steps of all of them
+  auto cut = [&](int64_t n) {
+    gb.assign(1, 0);
+    for (auto& l : chain_groups) l.clear();
+    int64_t sum = 0, work[kChains] = {}, w = 0, steps = 0;
+    for (int s = 0, g = 0; s < nshots; s++) {
+      w += live[s] * nstep[s];
+      sum += live[s];
+      // the group ends where the next shot's middle lies past its share
+      const bool end = s + 1 == nshots || (sum + live[s + 1] / 2) * n > (g + 1) * total;
+      if (!end) continue;
+      int c = 0;
+      for (int k = 1; k < kChains; k++)
+        if (work[k] < work[c]) c = k;
+      work[c] += w;
+      steps += nstep[gb.back()];
+      chain_groups[c].push_back((int)gb.size() - 1);
+      gb.push_back(s + 1);
+      w = 0;
+      while ((g + 1) * total <= sum * n && g + 1 < n) g++;
+    }
+    return steps;
+  };
+  const int64_t wanted = split ? kChains * div_up(total, kChains * per) : 1;
+  int64_t n = wanted;
+  // a node a kernel: those of a step forward, recomputed and reversed
+  const int64_t per_step = 3 * (percell ? 1 : vu ? 3 : 2);
+  graph_nodes = cut(n) * per_step;
+  while (n > 1 && graph_nodes > kMaxGraphNodes) {
+    const int64_t fit = n * kMaxGraphNodes / graph_nodes / kChains * kChains;
+    n = std::max<int64_t>(std::min(fit, n - kChains), 1);
+    graph_nodes = cut(n) * per_step;
   }
+  // (groups of twice the bytes find little in L2: one a chain is as good.  128 shots of up
+  // to 1200 x 2000: 128 groups 8.2 s a gradient, 64 9.8, 17 10.4, two 10.3)
+  if (n > kChains && 2 * n <= wanted) graph_nodes = cut(kChains) * per_step;
 }
 
 // Heaviest PML items first.  Their cost varies several-fold (corner warps

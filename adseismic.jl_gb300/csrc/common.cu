@@ -46,6 +46,25 @@ int require_device() {
   return ADS_OK;
 }
 
+int finish_graph(cudaGraph_t g, cudaStream_t st, cudaGraphExec_t* out) {
+  *out = nullptr;
+  cudaError_t e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (e == cudaSuccess) {
+    e = cudaGraphUpload(*out, st);
+    // (refused for another reason, its first launch uploads it)
+    if (e != cudaErrorMemoryAllocation) {
+      if (e != cudaSuccess) cudaGetLastError();
+      return ADS_OK;
+    }
+    cudaGraphExecDestroy(*out);
+    *out = nullptr;
+  }
+  cudaGetLastError();
+  return fail(e == cudaErrorMemoryAllocation ? ADS_ERR_NOMEM : ADS_ERR_CUDA,
+              "the plan's graph could not be made: %s", cudaGetErrorString(e));
+}
+
 // src/Core.jl:738-761 (pml_helper) over x = i*hx and y = j*hy; sigma depends
 // on x only and tau on y only (Core.jl:633-638 evaluates it per (i, j)).
 void acoustic_pml_1d(int64_t NX, int64_t NY, double hx, double hy, int64_t npml,

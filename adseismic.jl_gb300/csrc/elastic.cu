@@ -3157,6 +3157,7 @@ struct ElPlan final : ElPlanBase {
   // [gb[c], gb[c + 1]).
   std::vector<int> gb;
   void group_shots();
+  int64_t graph_nodes = 0;  // (an upper estimate)
   // fn(run) for every group; forked from and joined to st
   template <typename F>
   int each_group(cudaStream_t st, F&& fn);
@@ -3233,14 +3234,11 @@ struct ElPlan final : ElPlanBase {
   size_t zero_fwd_off = 0, zero_fwd_len = 0, zero_adj_off = 0, zero_adj_len = 0;
   cudaStream_t cap = nullptr;
   cudaGraphExec_t eF = nullptr, eR = nullptr;
-  cudaGraph_t gF = nullptr, gR = nullptr;
   int64_t nF = 0, nR = 0;
 
   ~ElPlan() override {
     if (eF) cudaGraphExecDestroy(eF);
     if (eR) cudaGraphExecDestroy(eR);
-    if (gF) cudaGraphDestroy(gF);
-    if (gR) cudaGraphDestroy(gR);
     if (cap) cudaStreamDestroy(cap);
     for (auto& c : chain) {
       for (auto e : c.ev)
@@ -3482,13 +3480,15 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   const size_t wl_o = take(sizeof(int) * std::max(nwt_max, 1));
   const size_t wlf_o = take(sizeof(int) * std::max(nwtf_max, 1));
   const size_t wla_o = take(sizeof(int) * std::max(fused ? nwta_max : 1, 1));
+  group_shots();
   // ---- the shots' stores: K slots for a segment's recompute, then one slot
   // per step of the resident segments (the last ones that fit in the allowed
   // share of the free device memory)
   res_seg = nseg;
   {
     const size_t slot = (size_t)NSTORE * F;
-    const size_t base_bytes = used + (size_t)ns * ((size_t)K * slot + 256);
+    const size_t base_bytes = used + (size_t)ns * ((size_t)K * slot + 256) +
+                              (c.use_graph ? graph_nodes * kGraphNodeBytes : 0);
     if (c.resident_segments >= 0) {
       size_t fr = 0, tot = 0, avail = 0;
       if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr > base_bytes) {
@@ -3536,7 +3536,6 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
   d_wlf = (int*)(pool + wlf_o);
   d_wla = (int*)(pool + wla_o);
   if (int e = upload_lists(st)) return e;
-  group_shots();
   for (int k = 0; k < chains(); k++) {
     Chain& h = chain[k];
     if (k > 0) ADS_CUDA(cudaStreamCreateWithFlags(&h.main, cudaStreamNonBlocking));
@@ -3708,12 +3707,7 @@ int ElPlan<T>::create(const ads_elastic_config& c, const ads_elastic_shot* shots
         return rc;
       }
       ADS_CUDA(e);
-      cudaGraphExec_t ex = nullptr;
-      ADS_CUDA(cudaGraphInstantiate(&ex, g, 0));
-      // (else the first launch waits for it; where it fails, the launch will say so)
-      if (cudaGraphUpload(ex, st) != cudaSuccess) cudaGetLastError();
-      (which == 0 ? gF : gR) = g;
-      (which == 0 ? eF : eR) = ex;
+      if (int rc = finish_graph(g, st, which == 0 ? &eF : &eR)) return rc;
     }
   }
   return ADS_OK;
@@ -4147,8 +4141,12 @@ int ElPlan<T>::step(const Run& q, int n, bool store, int slot, bool record) {
 
 template <typename T>
 void ElPlan<T>::group_shots() {
+  // nodes of a group: at most four kernels and a source / receiver launch a step, forward,
+  // recomputed and reversed
+  const int64_t nodes = (int64_t)NSTEP * 15;
   const bool split = sizeof(T) == 4 && cfg.use_graph && nshots > 1 &&
-                     (int64_t)NX * NY * nshots > kSplitCells;
+                     (int64_t)NX * NY * nshots > kSplitCells && kElChains * nodes <= kMaxGraphNodes;
+  graph_nodes = nodes * (split ? kElChains : 1);
   const int n = split ? std::min(nshots, kElChains) : 1;
   gb.assign(1, 0);
   for (int g = 1; g <= n; g++) gb.push_back((int)((int64_t)nshots * g / n));
