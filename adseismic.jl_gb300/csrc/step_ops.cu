@@ -31,7 +31,7 @@ constexpr int BJ = 32, BI = 8;
 template <typename T>
 struct StepK {
   T dt, dt2, hx, hy, hx2, hy2;  // hx2 = 2 hx, hy2 = 2 hy
-  T k1, k2;  // 2 dt^2 / hx^2, 2 dt^2 / hy^2
+  T k1, k2;  // 2 dt^2 / hx^2, 2 dt^2 / hy^2 (each variant in its own order)
   T ax, ay;  // dt / hx, dt / hy
   T cx, cy;  // their squares
   T fx, fy;  // dt^2 / (2 hx), dt^2 / (2 hy)
@@ -39,7 +39,7 @@ struct StepK {
 };
 
 template <typename T>
-StepK<T> make_k(double dt_, double hx_, double hy_) {
+StepK<T> make_k(double dt_, double hx_, double hy_, int variant) {
   const T dt = T(dt_), hx = T(hx_), hy = T(hy_), two = 2;
   StepK<T> K;
   K.dt = dt;
@@ -48,8 +48,8 @@ StepK<T> make_k(double dt_, double hx_, double hy_) {
   K.hy = hy;
   K.hx2 = two * hx;
   K.hy2 = two * hy;
-  K.k1 = two * dt * dt / hx / hx;
-  K.k2 = two * dt * dt / hy / hy;
+  K.k1 = variant == 0 ? two * dt * dt / hx / hx : two * K.dt2 / (hx * hx);
+  K.k2 = variant == 0 ? two * dt * dt / hy / hy : two * K.dt2 / (hy * hy);
   K.ax = dt / hx;
   K.ay = dt / hy;
   K.cx = K.ax * K.ax;
@@ -364,7 +364,7 @@ int acoustic_fwd(const T* w, const T* wold, const T* phi, const T* psi, const T*
   ADS_REQUIRE(w && wold && phi && psi && sigma && tau && c && u && phiout && psiout,
               "null pointer argument");
   ADS_REQUIRE(variant == 0 || variant == 1, "variant must be 0 (w) or 1 (u)");
-  const StepK<T> K = make_k<T>(dt, hx, hy);
+  const StepK<T> K = make_k<T>(dt, hx, hy, variant);
   const dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
   if (variant == 0)
     k_acoustic_fwd_w<T><<<grd, blk, 0, st>>>(w, wold, phi, psi, sigma, tau, c, K, (int)NX,
@@ -388,7 +388,7 @@ int acoustic_bwd(T* grad_w, T* grad_wold, T* grad_phi, T* grad_psi, T* grad_c,
                   grad_phiout && grad_psiout && w && sigma && tau && c,
               "null pointer argument");
   ADS_REQUIRE(variant == 0 || (variant == 1 && u), "variant must be 0, or 1 with u given");
-  const StepK<T> K = make_k<T>(dt, hx, hy);
+  const StepK<T> K = make_k<T>(dt, hx, hy, 0);  // (the transposes of both sum k1, k2 alike)
   const T kxy = K.k1 + K.k2;
   const dim3 blk(BJ, BI), grd((unsigned)div_up(NY + 2, BJ), (unsigned)div_up(NX + 2, BI));
   auto launch = [&](auto kernel) {
