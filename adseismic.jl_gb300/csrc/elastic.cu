@@ -1131,7 +1131,9 @@ CellModel<T> make_cells(int NX, int NY, int64_t P, int off, double dt, double dx
   M.mu = mu;
   M.rho = rho;
   M.dt = (T)dt;
-  M.rdt = (T)(1.0 / dt);
+  // (a step of no length has no density gradient: 0, not 0 times infinity)
+  const double rdt = 1.0 / dt;
+  M.rdt = std::isfinite((T)rdt) ? (T)rdt : T(0);
   M.dtd = dt;
   M.x1 = (T)(1.0 / (24 * dx));
   M.y1 = (T)(1.0 / (24 * dy));
