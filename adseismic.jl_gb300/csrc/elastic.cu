@@ -305,14 +305,13 @@ __device__ __forceinline__ T accel4(const CellModel<T>& M, int i, int j, CellIx<
                            f + (M1 + 7) * fs, fo ? fo + (M1 + 7) * fs : nullptr, x);
 }
 
-// Cell of a thread: row blocks along blockIdx.x (their count may pass 65535),
-// column blocks along blockIdx.y.  Plans start at cell (1, 1), whose address is
-// 128-byte aligned; the operators cover the padded grid.
-#define ADS_EL_CELL(FIRST)                                                     \
-  const int tx = threadIdx.x, ty = threadIdx.y;                                \
-  const int i0 = (FIRST) + blockIdx.x * BY, j0 = (FIRST) + blockIdx.y * BX;    \
+// Cell of an operator's thread, on the padded grid: the blocks are numbered along
+// blockIdx.x, columns first (along gridDim.y either direction would end at 65535 blocks).
+#define ADS_EL_CELL()                                                          \
+  const int tx = threadIdx.x, ty = threadIdx.y, ncol = (M.NY + 1 + BX) / BX;   \
+  const int i0 = blockIdx.x / ncol * BY, j0 = blockIdx.x % ncol * BX;          \
   const int i = i0 + ty, j = j0 + tx, P = M.P;                                 \
-  const CellIx<(FIRST) != 0> x = (CellIx<(FIRST) != 0>)i * P + j + M.OFF;      \
+  const int64_t x = (int64_t)i * P + j + M.OFF;                                \
   (void)P, (void)x
 
 // A plan's block: a tile of BY x BX cells at (i0, j0), a thread a cell (w = 0), or an
@@ -968,7 +967,7 @@ __global__ void __launch_bounds__(BX* BY)
 k_el_op_stress(CellModel<T> M, const T* __restrict__ f, T* __restrict__ o, int64_t fs, T* osxx,
                T* osyy, T* osxy) {
   // o: the step's output fields (null: the transpose wants the stresses alone)
-  ADS_EL_CELL(0);
+  ADS_EL_CELL();
   if (i > M.NX + 1 || j > M.NY + 1) return;
   T sxx = f[SXX * fs + x], syy = f[SYY * fs + x], sxy = f[SXY * fs + x];
   if (box1(M, i, j)) {
@@ -996,7 +995,7 @@ k_el_op_stress(CellModel<T> M, const T* __restrict__ f, T* __restrict__ o, int64
 template <typename T>
 __global__ void __launch_bounds__(BX* BY)
 k_el_op_velocity(CellModel<T> M, const T* __restrict__ f, T* o, int64_t fs) {
-  ADS_EL_CELL(0);
+  ADS_EL_CELL();
   if (i > M.NX + 1 || j > M.NY + 1) return;
   T vx = f[VX * fs + x], vy = f[VY * fs + x];
   if (box3(M, i, j)) {
@@ -1027,7 +1026,7 @@ k_el_op_adj_stress(CellModel<T> M, const T* __restrict__ f, const T* __restrict_
                    int64_t fs, G* __restrict__ grho) {
   __shared__ SendV<T> S;
   __shared__ T r4[BY + 1][BX + 1];  // vy cells' density terms, one row and column before the tile
-  ADS_EL_CELL(0);
+  ADS_EL_CELL();
   T q3, q4;
   send_velocity<T, false>(M, S, i0, j0, g, o, fs, q3, q4);
   const T *nsxx = o + M1 * fs, *nsyy = o + (M1 + 1) * fs, *nsxy = o + (M1 + 2) * fs;
@@ -1076,7 +1075,7 @@ k_el_op_adj_velocity(CellModel<T> M, const T* __restrict__ f, const T* __restric
                      int64_t fs, G* __restrict__ glam, G* __restrict__ gmu) {
   __shared__ SendS<T> S;
   __shared__ T pl[BY + 1][BX], pm[BY + 1][BX], p2[BY][BX + 1];
-  ADS_EL_CELL(0);
+  ADS_EL_CELL();
   send_stress<T, false>(M, S, i0, j0, o, g, o, fs);
   // lambda and mu terms of the stress cells (one row before the tile) and of the
   // sxy cells (one column before it)
@@ -4412,7 +4411,7 @@ void set_profiles(CellModel<T>& M, const T* ax, const T* bx, const T* ay, const 
 }
 
 inline dim3 op_grid(int64_t NX, int64_t NY) {
-  return dim3((unsigned)div_up(NX + 2, BY), (unsigned)div_up(NY + 2, BX));
+  return dim3((unsigned)(div_up(NX + 2, BY) * div_up(NY + 2, BX)));
 }
 
 template <typename T>
