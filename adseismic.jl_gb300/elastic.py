@@ -116,7 +116,11 @@ def elastic_one_step(param: ElasticPropagatorParams, rho, lam, mu, state, profil
          0 if host else nsrc, _stream())
     if host:
         at = [np.ascontiguousarray(a, dtype=np.int64).reshape(-1) for a in (srci, srcj, srctype)]
-        v = srcv.detach() if isinstance(srcv, torch.Tensor) else srcv
+        v = srcv
+        if isinstance(v, (list, tuple)) and any(isinstance(e, torch.Tensor) for e in v):
+            v = torch.stack([torch.as_tensor(e).detach().to("cpu", torch.float64) for e in v])
+        if isinstance(v, torch.Tensor):
+            v = v.detach().to(torch.float64).numpy()
         at.append(np.ascontiguousarray(v, dtype=np.float64 if suffix == "f64" else np.float32)
                   .reshape(-1))
         if min(len(a) for a in at) < nsrc:
