@@ -3241,6 +3241,8 @@ struct AcPlan final : AcPlanBase {
   int ri_pf = 0, ri_pa = 0;  // row tiles of the PML items (0: same as ri_f / ri)
   int upload_tiles(const TileList& L, DevTiles& D, cudaStream_t st);
   int autotune(cudaStream_t st, int64_t pitch, size_t cap_items);
+  int tune_blocks(cudaStream_t st, int64_t pitch, size_t cap_items);
+  void default_rows();
   // Groups of consecutive sorted shots that take the whole time loop together
   // (group_shots): group g holds shots [gb[g], gb[g + 1]).  kChains groups run beside
   // each other, each on a stream of its own.
@@ -3483,10 +3485,9 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   tb_auto = sizeof(T) == 4 && c.autotune >= 2 && c.steps_per_block == 0 && !vu;
   percell = KB == 1 && c.rows_per_thread <= 0 && c.tma <= 0 &&
             (sizeof(T) == 8 || (vu ? cells <= kCellMaxAc32U && cells_ahead_u() : cells <= kCellMaxAc32));
-  if (percell) tb_auto = false;
   inc = sizeof(T) == 4 && KB == 1;
-  wide = sizeof(T) == 4 && KB == 1 && !percell && !tb_auto && c.rows_per_thread <= 0 &&
-         c.tma <= 0 && (!vu || cells >= kWideMinU);
+  wide = sizeof(T) == 4 && KB == 1 && !percell && c.rows_per_thread <= 0 && c.tma <= 0 &&
+         (!vu || cells >= kWideMinU);
   group_shots(grid_pitch(MY));
   // ---- trace layout (packed in the caller's shot order)
   trace_off.resize(ns);
@@ -3587,15 +3588,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   // autotuner may replace both once the plan's buffers exist): enough warps
   // for several resident waves
   if (c.rows_per_thread <= 0) {
-    ri_f = 8;
-    // FP64 items go down to one row per warp: on small grids a warp's serial
-    // chain of FP64 operations, not the item count, sets a step's duration
-    const int rmin = sizeof(T) == 8 ? 1 : 2;
-    while (ri_f > rmin && cells / ((int64_t)ri_f * Tile<T>::WF) < 152 * 64) ri_f /= 2;
-    ri = 16;
-    while (ri > rmin && cells / ((int64_t)ri * Tile<T>::WA) < 152 * 32) ri /= 2;
-    if (wide && !vu) ri_f = ri = cells < kShortRows ? 2 : 4;  // (rows of a half warp)
-    if (wide && cells < kShortRows) ri_wf = ri_wa = 4;
+    default_rows();
   } else {
     ri_f = ri;
   }
@@ -3618,7 +3611,7 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   size_t cap_items = std::max(nitems_of(tiles_a), nitems_of(tiles_f));
   size_t cap_refs = std::max({tiles_a.srcs.size(), tiles_f.srcs.size(), tiles_a.rcvs.size(),
                               tiles_f.rcvs.size(), (size_t)1});
-  if (c.autotune && !percell) {
+  if (c.autotune && (!percell || tb_auto)) {
     size_t n2 = 0;
     for (int s = 0; s < ns; s++)
       n2 += (size_t)div_up(shots[order[s]].nx, 2) *
@@ -3881,6 +3874,8 @@ int AcPlan<T>::create(const ads_acoustic_config& c, const ads_acoustic_shot* sho
   } else if (c.autotune && !percell) {
     if (int e = autotune(st, pitch, cap_items)) return e;
   }
+  if (tb_auto)
+    if (int e = tune_blocks(st, pitch, cap_items)) return e;
   inc = sizeof(T) == 4 && KB == 1;
   // ---- timing ranges: the first full-length segment the reverse sweep meets
   cells_prefix.resize(ns);
@@ -4499,6 +4494,20 @@ bool AcPlan<T>::cells_ahead_u() const {
   return cell <= row;
 }
 
+// Row heights of the row-walking kernels where none are configured.
+template <typename T>
+void AcPlan<T>::default_rows() {
+  ri_f = 8;
+  // FP64 items go down to one row per warp: on small grids a warp's serial
+  // chain of FP64 operations, not the item count, sets a step's duration
+  const int rmin = sizeof(T) == 8 ? 1 : 2;
+  while (ri_f > rmin && tb_cells / ((int64_t)ri_f * Tile<T>::WF) < 152 * 64) ri_f /= 2;
+  ri = 16;
+  while (ri > rmin && tb_cells / ((int64_t)ri * Tile<T>::WA) < 152 * 32) ri /= 2;
+  if (wide && !vu) ri_f = ri = tb_cells < kShortRows ? 2 : 4;  // (rows of a half warp)
+  if (wide && tb_cells < kShortRows) ri_wf = ri_wa = 4;
+}
+
 template <typename T>
 int AcPlan<T>::count_slots() {
   int dev = 0, sms = 0;
@@ -4937,55 +4946,85 @@ int AcPlan<T>::autotune(cudaStream_t st, int64_t pitch, size_t cap) {
     build_tiles(rows, width, pitch, L, pm);
     if (int e = upload_tiles(L, D, st)) return e;
   }
-  // third phase (tb_auto): steps per forward launch, 1 (the tiles chosen
-  // above) against the time-blocked kernel at 2 and 4, over the same steps
-  if (tb_auto && !tb_cand.empty()) {
-    const int t_end = std::min(9, nstep[0]);
-    auto time_tb = [&](int kb, float& ms) -> int {
-      for (int pass = 0; pass < 2; pass++) {
-        ADS_CUDA(cudaEventRecord(e0, st));
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  ADS_CUDA(cudaStreamSynchronize(st));
+  return ADS_OK;
+}
+
+// Steps per forward launch (tb_auto): the plan's own kernels, group by group as its time
+// loops run them, against the time-blocked kernel at 2 and 4 steps, over the same steps.
+// Where that wins, the plan steps forward with it and back with the row kernels' transpose
+// of its three-level form.
+template <typename T>
+int AcPlan<T>::tune_blocks(cudaStream_t st, int64_t pitch, size_t cap) {
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  ADS_CUDA(cudaEventCreate(&e0));
+  ADS_CUDA(cudaEventCreate(&e1));
+  const int t_end = std::min(9, nstep[0]);
+  auto timed = [&](int kb, float& ms) -> int {
+    for (int pass = 0; pass < 2; pass++) {  // pass 0 warms up
+      ADS_CUDA(cudaEventRecord(e0, st));
+      if (kb == 1) {
+        for (size_t g = 0; g + 1 < gb.size(); g++)
+          for (int t = 2; t <= t_end; t++) {
+            const int s1 = std::min(gb[g + 1], shots_with_nstep_ge(t));
+            if (s1 <= gb[g]) break;
+            if (int e = launch_fwd(st, 0, gb[g], s1, t, 0, 0)) return e;
+          }
+      } else {
         for (int t0 = 2, blk = 0; t0 <= t_end; blk++) {
           const int NS = std::min(kb, t_end - t0 + 1);
-          const int na = shots_with_nstep_ge(t0);
-          if (kb == 1) {
-            if (int e = launch_fwd(st, 0, 0, na, t0, 0, 0)) return e;
-          } else if (int e = launch_tb(st, false, tb_items_upto(na), t0, NS, 0, blk & 1, 0)) {
+          if (int e = launch_tb(st, false, tb_items_upto(shots_with_nstep_ge(t0)), t0, NS, 0,
+                                blk & 1, 0))
             return e;
-          }
           t0 += NS;
         }
-        ADS_CUDA(cudaEventRecord(e1, st));
-        ADS_CUDA(cudaEventSynchronize(e1));
-        ADS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
       }
-      return ADS_OK;
-    };
+      ADS_CUDA(cudaEventRecord(e1, st));
+      ADS_CUDA(cudaEventSynchronize(e1));
+      ADS_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+    }
+    return ADS_OK;
+  };
+  auto run = [&]() -> int {
     float best = 0.f;
-    KB = 1;
-    if (int e = time_tb(1, best)) return e;
+    if (int e = timed(1, best)) return e;
     int best_kb = 1;
     for (const auto& cand : tb_cand) {
       if (int e = upload_tb(cand.second, st)) return e;
       KB = cand.first;
       RB = tb_rows_for(KB);
       float ms = 0.f;
-      if (int e = time_tb(KB, ms)) return e;
+      if (int e = timed(KB, ms)) return e;
       if (ms < best) {
         best = ms;
         best_kb = KB;
       }
+    }
+    KB = 1;
+    if (best_kb > 1 && (percell || wide)) {
+      percell = wide = false;
+      group_shots(pitch);
+      default_rows();
+      for (auto& h : hshots) h.dl = nullptr;  // (incr_adj() no more)
+      ADS_CUDA(cudaMemcpyAsync(d_shots, hshots.data(), sizeof(AcShot<T>) * nshots,
+                               cudaMemcpyHostToDevice, st));
+      if (int e = autotune(st, pitch, cap)) return e;
     }
     KB = best_kb;
     RB = tb_rows_for(KB);
     for (const auto& cand : tb_cand)
       if (cand.first == KB)
         if (int e = upload_tb(cand.second, st)) return e;
-    tb_cand.clear();
-  }
+    return ADS_OK;
+  };
+  const int rc = run();
+  tb_cand.clear();
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  ADS_CUDA(cudaStreamSynchronize(st));
-  return ADS_OK;
+  if (rc == ADS_OK) ADS_CUDA(cudaStreamSynchronize(st));
+  return rc;
 }
 
 template <typename T>

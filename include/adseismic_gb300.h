@@ -292,9 +292,10 @@ typedef struct ads_acoustic_config {
                               kernels at plan creation and keep the fastest (plans
                               with the one-thread-per-cell kernels have none); 2: also,
                               for FP32 variant-W plans without resident segments and
-                              with steps_per_block 0, time 1, 2 and 4 forward steps
-                              per launch and keep the fastest (more than 1 selects
-                              the time-blocked three-level form) */
+                              with steps_per_block 0, time 2 and 4 forward steps
+                              per launch against the plan's own kernels and keep the
+                              fastest (more than 1 selects the time-blocked
+                              three-level form and the row-walking adjoint) */
   int32_t resident_segments; /* checkpoint segments (the last ones) whose forward
                                 wavefields stay in device memory for the reverse sweep,
                                 which then neither restores nor recomputes them:
