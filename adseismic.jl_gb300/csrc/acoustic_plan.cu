@@ -112,9 +112,15 @@ struct CellRef {
   int row;       // its row (1-based padded grid)
 };
 
+// Columns (up to 128) and rows (up to 2^24, as many as a plan may be configured to walk) of
+// an item.
+constexpr int item_pad(int width, int rows) { return (int)((unsigned)rows << 8 | width); }
+__host__ __device__ constexpr int item_width(int pad) { return pad & 0xff; }
+__host__ __device__ constexpr int item_rows(int pad) { return (int)((unsigned)pad >> 8); }
+
 struct AcItem {
-  // pad: columns (low 16 bits) and rows (high) of a row-walking item; the
-  // one-thread-per-cell tiles' own form: cell_near
+  // pad: columns and rows of a row-walking item (item_pad); the one-thread-per-cell
+  // tiles' own form: cell_near
   int shot, i0, j0, pad;
   int src_b, src_e, rcv_b, rcv_e;
 };
@@ -412,8 +418,8 @@ k_ac_fwd(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots,
   const bool tfree = warp_tau_free<T, C>(ty, j, ny);
   auto nz = [&](int r) { return !(tfree && sx[r] == T(0)); };  // phi/psi may be non-zero
   const int i0 = it.i0 + (threadIdx.x >> 5) * ri;
-  const int i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
-  const int jend = min(ny, it.j0 + (it.pad & 0xffff) - 1);  // the item's last column
+  const int i_end = min(i0 + ri, it.i0 + item_rows(it.pad));
+  const int jend = min(ny, it.j0 + item_width(it.pad) - 1);  // the item's last column
   if (i0 >= i_end) return;  // whole warps only: every later barrier is warp-level
   auto off = [&](int r) { return (int64_t)r * P + col; };
   const bool ck_on = CK && !SEG && ckpt_slot > 0 && ckpt_slot < sh.nseg;
@@ -1024,7 +1030,7 @@ __device__ __forceinline__ void record_src_grad(const AcItem& it, const AcShot<T
                                                 int k, int lane, int i0, int i_end, double dt2) {
   if (k - 1 < 2 || it.src_e <= it.src_b) return;
   // (the four-column kernels' items may be narrower than a warp's columns)
-  const int width = C == 4 ? it.pad & 0xffff : 32 * C;
+  const int width = C == 4 ? item_width(it.pad) : 32 * C;
   __syncwarp();
   for (int e = it.src_b + lane; e < it.src_e; e += 32) {
     const CellRef r = srcs[e];
@@ -1582,8 +1588,8 @@ k_ac_phi_u(const AcItem* __restrict__ items, const AcShot<T>* __restrict__ shots
   const bool tfree = warp_tau_free<T, C>(ty, j, ny);
   auto nz = [&](int r) { return !(tfree && sx[r] == T(0)); };
   const int i0 = it.i0 + (threadIdx.x >> 5) * ri;
-  const int i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
-  const int jend = min(ny, it.j0 + (it.pad & 0xffff) - 1);  // the item's last column
+  const int i_end = min(i0 + ri, it.i0 + item_rows(it.pad));
+  const int jend = min(ny, it.j0 + item_width(it.pad) - 1);  // the item's last column
   if (i0 >= i_end) return;
   auto off = [&](int r) { return (int64_t)r * P + col; };
   const bool srcd = t - 1 >= 2 && it.src_e > it.src_b;  // u_{t-1} received source values
@@ -1769,10 +1775,10 @@ struct Wide {
   int hoff;       // an edge lane's halo column, relative to its first cell
   __device__ Wide(const AcItem& it, int pitch, int ri) {
     lane = threadIdx.x & 31;
-    const int last = ((it.pad & 0xffff) >> 2) - 1;
+    const int last = (item_width(it.pad) >> 2) - 1;
     j = it.j0 + 4 * lane;
     i0 = it.i0 + (threadIdx.x >> 5) * ri;
-    i_end = min(i0 + ri, it.i0 + (it.pad >> 16));
+    i_end = min(i0 + ri, it.i0 + item_rows(it.pad));
     P = pitch;
     col = j + JOFF;
     on = lane <= last;
@@ -1969,7 +1975,7 @@ struct Half {
   F4 T;       // tau of the lane's columns
   bool tau;   // any of them damped
   __device__ Half(const AcItem& it, const AcShot<float>& sh, int ri) {
-    const int half = threadIdx.x >> 4, width = it.pad & 0xffff, n = it.pad >> 16;
+    const int half = threadIdx.x >> 4, width = item_width(it.pad), n = item_rows(it.pad);
     hl = threadIdx.x & 15;
     const int last = (width - 1) >> 2;
     j = it.j0 + 4 * hl;
@@ -4081,7 +4087,7 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
         it.shot = s;
         it.i0 = 1 + ti * gh;
         it.j0 = 1 + tj * width;
-        it.pad = width | std::min(gh, nx + 1 - it.i0) << 16;
+        it.pad = item_pad(width, std::min(gh, nx + 1 - it.i0));
         const size_t b = (size_t)ti * ntj + tj;
         it.src_b = (int)L.srcs.size();
         for (int k : bs[b]) {
@@ -4104,10 +4110,10 @@ void AcPlan<T>::build_tiles(int rows, int width, int64_t pitch, TileList& L,
         } else if (pm_rows > 0 && pm_rows < rows) {
           // sub-items share the item's source / receiver lists: the kernels
           // match those by cell and row
-          for (int i0 = it.i0; i0 < it.i0 + (it.pad >> 16); i0 += Tile<T>::G * pm_rows) {
+          for (int i0 = it.i0; i0 < it.i0 + item_rows(it.pad); i0 += Tile<T>::G * pm_rows) {
             AcItem sub = it;
             sub.i0 = i0;
-            sub.pad = width | std::min(Tile<T>::G * pm_rows, it.i0 + (it.pad >> 16) - i0) << 16;
+            sub.pad = item_pad(width, std::min(Tile<T>::G * pm_rows, it.i0 + item_rows(it.pad) - i0));
             L.pm.push_back(sub);
             pm_cost.push_back(item_cost(sub, pm_rows, col_free[tj]));
           }
@@ -4184,7 +4190,7 @@ void AcPlan<T>::build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L)
         it.shot = s;
         it.i0 = i;
         it.j0 = j0;
-        it.pad = w | m << 16;
+        it.pad = item_pad(w, m);
         it.src_b = (int)L.srcs.size();
         pick(src, i, m, j0, w, vu ? 1 : 0, &L.srcs);
         it.src_e = (int)L.srcs.size();
@@ -4218,7 +4224,7 @@ void AcPlan<T>::build_wide(int rows_in, int rows_pm, int64_t pitch, TileList& L)
           it.shot = s;
           it.i0 = i;
           it.j0 = j;
-          it.pad = w | n << 16;
+          it.pad = item_pad(w, n);
           L.in.push_back(it);
         }
     L.in_end[s] = (int)L.in.size();
