@@ -4453,6 +4453,12 @@ int el_add_sources(T* state, int64_t NX, int64_t NY, const int64_t* srci, const 
   ADS_REQUIRE(state, "null pointer argument");
   ADS_REQUIRE(nsrc >= 0 && (nsrc == 0 || (srci && srcj && srctype && srcv)),
               "invalid source arrays");
+  if (nsrc > 0) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    ADS_CUDA(cudaStreamIsCapturing((cudaStream_t)stream, &capture));
+    ADS_REQUIRE(capture == cudaStreamCaptureStatusNone,
+                "source values on the host cannot be captured: a graph would replay those of now");
+  }
   ArgSources<T> s{};
   int n = 0;
   for (int64_t k = 0; k < nsrc; k++) {

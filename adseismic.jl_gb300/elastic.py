@@ -101,9 +101,6 @@ def elastic_one_step(param: ElasticPropagatorParams, rho, lam, mu, state, profil
     # values that are on the host go along as kernel arguments: a copy to the device would
     # wait for everything on the stream
     host = nsrc > 0 and not (isinstance(srcv, torch.Tensor) and srcv.is_cuda)
-    if host and torch.cuda.is_current_stream_capturing():
-        raise RuntimeError("elastic_one_step: sources from the host cannot be captured: a graph "
-                           "would replay the values of now")
     if nsrc and not host:
         si, sj, stp = (torch.as_tensor(np.asarray(a), dtype=torch.int64, device=dev)
                        for a in (srci, srcj, srctype))

@@ -180,7 +180,8 @@ int ads_elastic_step_fwd_f32(const float* state_in, float* state_out, const floa
                              int64_t nsrc, ads_stream_t stream);
 /* Adds one time row of sources to a state on its own, as ads_elastic_step_fwd_f64 does
  * after the step: srci, srcj, srctype, srcv are HOST arrays of nsrc entries here; they go
- * along as kernel arguments, so nothing is copied or waited for. */
+ * along as kernel arguments, so nothing is copied or waited for.  A stream that is being
+ * captured is refused (ADS_ERR_INVALID): its graph would replay the values of now. */
 int ads_elastic_add_sources_f64(double* state, int64_t NX, int64_t NY, const int64_t* srci,
                                 const int64_t* srcj, const int64_t* srctype, const double* srcv,
                                 int64_t nsrc, ads_stream_t stream);
