@@ -2263,7 +2263,7 @@ k_ac_pml_adj(const AcItem* __restrict__ items, const AcShot<float>* __restrict__
 
 // ---------------------------------------------------------------------------
 // One-thread-per-cell step kernels: FP64 plans, and FP32 plans of few cells
-// (AcPlan::cells).  One launch a step over interior and PML tiles together, in
+// (AcPlan::percell).  One launch a step over interior and PML tiles together, in
 // both variants.
 //
 // FP64 issue bounds the FP64 steps (a warp's FP64 instruction holds the pipe of
@@ -2278,9 +2278,9 @@ k_ac_pml_adj(const AcItem* __restrict__ items, const AcShot<float>* __restrict__
 //    r (x - 2 w_old) + w_old;
 //  * grad_c is summed without its factor cx, which the assembly applies.
 // A damped cell takes about 18 operations forward, 28 in the transpose.  8 shots of
-// 400 x 400, variant W: 31.0 us a forward step (FP64 pipe 78% of its active cycles,
-// 11.6 instructions a warp), 55.6 an adjoint step; 8 shots' 500-step gradient 57.6 ->
-// 43.5 ms against the row kernels.
+// 400 x 400, variant W: 30.9 us a forward step (11.0 FP64 operations a cell, the pipe 73%
+// of its active cycles), 55.3 an adjoint step (19.3, 78%); 8 shots' 500-step gradient
+// 57.6 -> 42.9 ms against the row kernels.
 //
 // Small grids are bound by the latency of a step: one launch, no row loop, no
 // fork and join of two streams; the launches are chained (grid_wait), so a step's

@@ -102,10 +102,10 @@ struct ElShot {
 //    (k_el_gather_cells), which is the same sum in another order.
 // No row or column is computed twice, and a grid of 47 k cells already gives every
 // SM ten warps, where a strip of rows leaves most of the chip idle: the FP64
-// gradient of 2 shots of 253 x 187, 250 steps, takes 11.2 ms, 113 ms with the
-// row-streaming kernels (FP64 pipe 64% busy in these kernels there); the operator
-// and its transpose on 600 x 300 FP64 take 20 + 22 and 19 + 55 + 43 us (FP64 pipe
-// 74-82% busy).
+// gradient of 2 shots of 253 x 187, 250 steps, takes 10.7 ms, 113 ms with the
+// row-streaming kernels (FP64 pipe 57-65% busy in these kernels there); the operator
+// and its transpose on 600 x 300 FP64 take 20 + 22 and 20 + 54 + 42 us (FP64 pipe
+// 73-82% busy).
 // ---------------------------------------------------------------------------
 // offsets within a field: 32 bits in plans (which check it), 64 in the operators
 template <bool PLAN>

@@ -136,8 +136,9 @@ __device__ __forceinline__ T new_u(const StepK<T>& K, int64_t k, int64_t S, T sg
 }
 
 // One thread per cell.  FP64 issue bounds it (82% of the pipe's active cycles):
-// 22 operations an undamped cell.  75 us at 1001 x 1001 FP64, 322 us with the
-// factors and the division formed in every cell.
+// 22 operations an undamped cell, 28 a cell at 1001 x 1001 with a PML of 12, whose cells
+// divide five times.  75 us there in FP64, 322 us with the factors and the division
+// formed in every cell.
 template <typename T>
 __global__ void __launch_bounds__(BJ* BI)
 k_acoustic_fwd_w(const T* __restrict__ w, const T* __restrict__ wold,

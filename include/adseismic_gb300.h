@@ -283,9 +283,11 @@ typedef struct ads_acoustic_config {
   int64_t ckpt_every; /* forward checkpoint spacing k in steps; 0 = automatic */
   int32_t rows_per_thread; /* stencil tile height (autotuner) of the row-walking step
                               kernels; 0 = automatic, which also lets FP64 plans and
-                              small FP32 plans (up to 300000 cells over all shots,
-                              1000000 for variant U) step with one-thread-per-cell
-                              kernels, unless steps_per_block > 1 or tma is set */
+                              small FP32 plans (up to 300000 cells over all shots;
+                              variant U below 1000000 cells where they are estimated
+                              ahead, by the damped and free rows) step with
+                              one-thread-per-cell kernels, unless steps_per_block > 1
+                              or tma is set */
   int32_t steps_per_block; /* time steps per forward launch (FP32: 1, 2, 4, 8;
                               FP64: 1); 0 = automatic (1) */
   int32_t block_rows;      /* tile height of the time-blocked forward; 0 = automatic */
@@ -458,9 +460,10 @@ typedef struct ads_elastic_config {
                                 intermediate fields in device memory); 3 = three gather passes
                                 over intermediate fields, in place; 0 = automatic:
                                 one-thread-per-cell kernels (forward and adjoint) for
-                                FP64 plans and FP32 plans of up to 600000 cells over
-                                all shots, 1 for larger FP32 plans; with rows_per_warp
-                                set, 1 for FP32 and 3 for FP64 plans */
+                                FP64 plans and FP32 plans of up to 1500000 cells over
+                                all shots (from 200000 on with row-walking strips over
+                                the undamped interior), 1 for larger FP32 plans; with
+                                rows_per_warp set, 1 for FP32 and 3 for FP64 plans */
   int32_t reserved[3];
 } ads_elastic_config;
 
